@@ -27,6 +27,7 @@
 #include <cstdint>
 #include <vector>
 
+#include "dtw_block.cuh"
 #include "dtw_path.cuh"
 #include "dtw_pipe.cuh"
 #include "odba_internal.h"
@@ -46,28 +47,16 @@ constexpr int kMaxMoveNil = 255, kMoveOpenRight = 4, kMoveNilOpenRight = 5;
 
 template <typename T>
 struct PathTune;
-// RF: registers (columns) per lane of a full swath; the last, partial swath
-// of a member takes a multiple of RQ.  In the full-path round a last swath
-// within PAD registers of RF is swept at RF (the extra columns past the
-// series' end are swept and never walked), so that one loop body, not two of
-// nearly the same size, runs in most warps.
+// Stripe mode's one-warp swaths: RF registers (columns) per lane of a full
+// swath; the last, partial swath of a member takes a multiple of RQ.
 template <>
 struct PathTune<float> {
-  static constexpr int RF = 32, RQ = 4, PAD = 4;
+  static constexpr int RF = 32, RQ = 4;
 };
 template <>
 struct PathTune<double> {
-  static constexpr int RF = 16, RQ = 4, PAD = 0;
+  static constexpr int RF = 16, RQ = 4;
 };
-
-// Registers per lane of a full-path swath `width` columns wide (at most
-// 32 * RF).
-template <typename T>
-__host__ __device__ inline int path_regs(int width) {
-  constexpr int RF = PathTune<T>::RF, RQ = PathTune<T>::RQ;
-  const int rq = ((width + 31) / 32 + RQ - 1) / RQ * RQ;
-  return rq >= RF - PathTune<T>::PAD ? RF : rq;
-}
 
 // Geometry of one member's cost matrix, identical on host and device.
 struct MemberGeom {
@@ -83,9 +72,8 @@ __host__ __device__ inline MemberGeom member_geom(uint64_t len, uint64_t Lc, int
   g.m = int(g.flip ? Lc : len);
   g.n = int(g.flip ? len : Lc);
   g.r0 = os ? 1 : 0;
-  const int W = 32 * PathTune<T>::RF;
-  g.swaths = (g.n + W - 1) / W;
-  g.steps = (g.m - g.r0 + 1) / 2 + 31;
+  g.swaths = (g.n + kBlkCols - 1) / kBlkCols;
+  g.steps = block_steps(g.m - g.r0);
   g.words = (unsigned long long)g.swaths * g.steps * 64ull;
   return g;
 }
@@ -287,108 +275,22 @@ __global__ void fill_ranges_kernel(int2 *r, unsigned long long count) {
     r[i] = make_int2(1, 0);
 }
 
-template <typename T, int R>
-__device__ __forceinline__ void path_swath(const SwathJob<T> &job, const PathOut &po, T &emin,
-                                           T &etop) {
-  T col[R];
-  sweep_swath_path<T, R>(job, po, col, emin, etop);
-}
-
-template <typename T, int RF, int RQ, int WARPS>
-__global__ void __launch_bounds__(kRoundWarps * 32) path_dtw_kernel(RoundArgs<T> a) {
-  __shared__ __align__(16) T stage_mem[WARPS * kStageElems];
-  const int lane = threadIdx.x & 31;
-  const long long slot = (long long)blockIdx.x * WARPS + (threadIdx.x >> 5);
-  T *e0 = a.edges + slot * 2 * a.edge_stride;
-  T *e1 = e0 + a.edge_stride;
-  constexpr int W = 32 * RF;
-  for (;;) {
-    unsigned long long q = 0;
-    if (lane == 0) q = atomicAdd(a.counter, 1ull);
-    q = __shfl_sync(kFull, q, 0);
-    if (q >= (unsigned long long)a.nmem) break;
-    // longest members first when the caller's order (or member order) is by length
-    const int k = a.order ? a.order[q] : a.nmem - 1 - int(q);
-    int jb;
-    const MemberGeom g = geom_of<T>(a, k, jb);
-    const int flags = a.jflags[jb];
-    if (!(flags & 4)) continue;
-    const int os = flags & 1, oe = (flags >> 1) & 1;
-    const T *seq = a.series + a.offsets[a.mseries[k]];
-    const T *cen = a.centroids + a.coff[jb];
-    SwathJob<T> job;
-    job.x = g.flip ? cen : seq;
-    job.y = g.flip ? seq : cen;
-    job.m = g.m;
-    job.n = g.n;
-    job.r0 = g.r0;
-    job.open_end = oe != 0;
-    job.stage = stage_mem + (threadIdx.x >> 5) * kStageElems;
-    int shortcut = 0;
-    const bool check_short = oe && !os;
-    for (int s = 0; s < g.swaths; ++s) {
-      const int c0 = s * W;
-      const bool last = s == g.swaths - 1;
-      job.c0 = c0;
-      job.edge_in = c0 ? ((s & 1) ? e0 : e1) : nullptr;
-      job.edge_out = last ? nullptr : ((s & 1) ? e1 : e0);
-      job.free_diag0 = c0 > 0 && (c0 % kRefSwath) == 0;
-      job.corner_init = c0 == 0 ? (job.r0 ? Num<T>::big() : T(0)) : (job.r0 ? T(0) : Num<T>::big());
-      PathOut po;
-      po.words = a.words + a.path_off[k] + (unsigned long long)s * g.steps * 64ull;
-      po.track_min = true;
-      T emin, etop;
-      const int width = g.n - c0 < W ? g.n - c0 : W;
-      const int rq = path_regs<T>(width);
-      if (rq >= RF) {
-        path_swath<T, RF>(job, po, emin, etop);
-      } else {
-        switch (rq / RQ) {
-#define ODBA_CASE(K)                                                          \
-  case K:                                                                     \
-    if constexpr (K * RQ < RF) path_swath<T, K * RQ>(job, po, emin, etop);    \
-    break;
-          ODBA_CASE(1)
-          ODBA_CASE(2)
-          ODBA_CASE(3)
-          ODBA_CASE(4)
-          ODBA_CASE(5)
-          ODBA_CASE(6)
-          ODBA_CASE(7)
-#undef ODBA_CASE
-          default:
-            break;
-        }
-      }
-      // The reference checks, at every swath start past the first series'
-      // length, whether the top row already holds the column minimum; from
-      // the first hit on, the rest of the top row is OPEN_RIGHT.
-      const int cnext = c0 + W;
-      if (check_short && !shortcut && !last && cnext % kRefSwath == 0 && cnext > g.m &&
-          cnext < g.n && etop == emin)
-        shortcut = cnext;
-      __syncwarp();
-    }
-    if (lane == 0) a.shortcut[k] = shortcut;
-  }
-}
-
-// The open-end shortcut of swath-pipeline member k (the rule of
-// path_dtw_kernel, applied to the per-swath right-edge minima afterwards; a
-// swath's minimum is the least of its bands', its top-row value the top
-// band's, the other bands leaving theirs at big): the first qualifying
-// swath boundary, or 0.
+// The open-end shortcut of swath-pipeline member k, from the per-swath
+// right-edge minima (a swath's minimum is the least of its bands', its top-row
+// value the top band's, the other bands leaving theirs at big).  The reference
+// checks, at every swath start past the first series' length, whether the top
+// row already holds the column minimum; from the first hit on, the rest of the
+// top row is OPEN_RIGHT: the first qualifying swath boundary, or 0.
 template <typename T>
 __device__ __forceinline__ int member_shortcut(const RoundArgs<T> &a, int k, const MemberGeom &g,
                                                int flags) {
   const int os = flags & 1, oe = (flags >> 1) & 1;
-  constexpr int W = 32 * PathTune<T>::RF;
   if (!oe || os) return 0;
   const int nb = member_band(g, a.nbands, 0).count;
   const unsigned long long layer = (unsigned long long)a.nmem * a.max_swaths;
   for (int s = 0; s + 1 < g.swaths; ++s) {
-    const int cnext = (s + 1) * W;
-    if (cnext % kRefSwath != 0 || cnext <= g.m || cnext >= g.n) continue;
+    const int cnext = (s + 1) * kBlkCols;
+    if (cnext <= g.m || cnext >= g.n) continue;
     T emin = Num<T>::big(), etop = Num<T>::big();
     for (int b = 0; b < nb; ++b) {
       const T *et = a.emtop + ((unsigned long long)b * layer + (unsigned long long)k * a.max_swaths + s) * 2;
@@ -404,149 +306,171 @@ template <typename T>
 __device__ __forceinline__ bool walk_member_runs(const RoundArgs<T> &a, const MemberGeom &g, int k,
                                                  int os, int oe, int2 *runs);
 
-template <typename T, int R>
-__device__ __forceinline__ void path_pipe_swath(const SwathJob<T> &job, const PathOut &po,
-                                                BandGate gate, TileIn<T> tile, T &emin,
-                                                T &etop) {
-  T col[R];
-  sweep_swath_path<T, R, BandGate>(job, po, col, emin, etop, tile, gate);
-}
-
-// Path DTW as the swath pipeline: task q is band q / (nmem * max_swaths) of
-// swath (q / nmem) % max_swaths of the (q % nmem)-th member in alignment
-// order, so a member's swaths run on different warps at once (few or long
-// members keep the GPU busy).  The right edge of swath s goes to buffer s % 2
-// of the member with one progress word per (member, swath), as in the
-// all-pairs swath pipeline.  With more than one band (member_band), a band
-// starts from the last row and edge corner the band below left in the
-// (member, swath)'s row buffer, once that band has raised the (member,
-// swath)'s band word; bands only shorten the tasks, so the last wave of
-// warps is shorter, and leave every recorded move as it is.  Each band also
-// stores its right edge's minimum and top-row value for the open-end
-// shortcut, which shortcut_kernel resolves afterwards (it never changes a
-// recorded move).  Every wait is on a task taken earlier from the counter.
-template <typename T, int RF, int RQ>
-__global__ void __launch_bounds__(kRoundWarps * 32, sizeof(T) == 4 ? 3 : 2) path_pipe_kernel(RoundArgs<T> a) {
-  __shared__ __align__(16) T stage_mem[kRoundWarps * kStageElems];
-  constexpr int W = 32 * RF;
+// Path DTW, a block per swath (sweep_block).  PIPE: task q is band
+// q / (nmem * max_swaths) of swath (q / nmem) % max_swaths of the (q % nmem)-th
+// member in alignment order, so a member's swaths run in different blocks at
+// once (few or long members keep the GPU busy).  The right edge of swath s
+// goes to buffer s % 2 of the member with one progress word per (member,
+// swath), as in the all-pairs swath pipeline.  BAND (odba_round_set_bands,
+// member_band): a band starts from the last row and edge corner the band below
+// left in the (member, swath)'s row buffer, once that band has raised the
+// (member, swath)'s band word; the recorded moves are the same.  Each band
+// also stores its right edge's minimum and top-row value for the open-end
+// shortcut, which never changes a recorded move.  Every wait is on a task
+// taken earlier from the counter.  Without PIPE (edge columns of all members
+// too large) a task is a member, swath after swath, with two edge columns per
+// block.
+//
+// The block's cost per cell is the one-warp sweep's plus about 14 instructions
+// per 16 cells (loads of samples and edge, shuffles, stores); what it buys is
+// a step a quarter as long where a member's chain of swaths, and not the GPU's
+// throughput, sets a round's time.  One B200, one warp per swath against a
+// block per swath: 64 members of 512-1024 samples 0.73 -> 0.29 ms a round, 100
+// of 1000-4000 in double 2.51 -> 1.53, 400 of 3000-8000 (which fill the GPU)
+// 6.57 -> 5.86.
+//
+// Blocks per SM: four (two for double) fill the SM; more, which the registers
+// would allow, only spread its issue slots over more chains, and each chain's
+// last swath then ends later (400 members: 6.54 ms with six, 6.24 with five,
+// 5.86 with four, 5.83 with three; double 1.71 with four, 1.53 with two).
+constexpr int kRoundBlocksF32 = 4, kRoundBlocksF64 = 2;
+template <typename T, bool PIPE, bool BAND>
+__global__ void
+__launch_bounds__(kBlkThreads, sizeof(T) == 4 ? kRoundBlocksF32 : kRoundBlocksF64)
+    path_block_kernel(RoundArgs<T> a) {
+  __shared__ BlockSmem<T> sm;
   const int lane = threadIdx.x & 31;
+  const bool feeder = (threadIdx.x >> 5) == kBlkWarps;
   const unsigned long long layer = (unsigned long long)a.nmem * a.max_swaths;
-  const unsigned long long ntasks = layer * a.nbands;
+  const unsigned long long ntasks = PIPE ? layer * a.nbands : (unsigned long long)a.nmem;
+  auto member_of = [&](unsigned long long qi) {
+    return a.order ? a.order[qi] : a.nmem - 1 - int(qi);
+  };
   for (;;) {
-    unsigned long long q = 0;
-    if (lane == 0) q = atomicAdd(a.counter, 1ull);
-    q = __shfl_sync(kFull, q, 0);
+    if (feeder && lane == 0) {
+      // the next task that exists
+      unsigned long long q;
+      for (;;) {
+        q = atomicAdd(a.counter, 1ull);
+        if (q >= ntasks) break;
+        const unsigned long long ql = PIPE ? q % layer : q;
+        int jb;
+        const MemberGeom g = geom_of<T>(a, member_of(PIPE ? ql % a.nmem : q), jb);
+        if (!(a.jflags[jb] & 4)) continue;
+        if (PIPE && int(ql / a.nmem) >= g.swaths) continue;
+        if (PIPE && BAND && int(q / layer) >= member_band(g, a.nbands, 0).count) continue;
+        break;
+      }
+      sm.task = q;
+    }
+    __syncthreads();
+    const unsigned long long q = sm.task;
     if (q >= ntasks) break;
-    const int b = int(q / layer);
-    const unsigned long long ql = q - (unsigned long long)b * layer;
-    const int s = int(ql / a.nmem), qi = int(ql - (unsigned long long)s * a.nmem);
-    const int k = a.order ? a.order[qi] : a.nmem - 1 - qi;
+    const int b = PIPE && BAND ? int(q / layer) : 0;
+    const unsigned long long ql = PIPE ? q - (unsigned long long)b * layer : 0;
+    const int s_first = PIPE ? int(ql / a.nmem) : 0;
+    const int k = member_of(PIPE ? ql - (unsigned long long)s_first * a.nmem : q);
     int jb;
     const MemberGeom g = geom_of<T>(a, k, jb);
     const int flags = a.jflags[jb];
-    if (!(flags & 4) || s >= g.swaths) continue;
-    const Band bd = member_band(g, a.nbands, b);
-    if (b >= bd.count) continue;
-    const int oe = (flags >> 1) & 1;
+    const Band bd = member_band(g, PIPE && BAND ? a.nbands : 1, b);
+    const int os = flags & 1, oe = (flags >> 1) & 1;
     const T *seq = a.series + a.offsets[a.mseries[k]];
     const T *cen = a.centroids + a.coff[jb];
-    T *b0 = a.edges + (unsigned long long)k * 2 * a.edge_stride;
+    T *b0 = a.edges + (PIPE ? (unsigned long long)k : (unsigned long long)blockIdx.x) * 2 * a.edge_stride;
     T *b1 = b0 + a.edge_stride;
-    const int c0 = s * W;
-    const bool last = s == g.swaths - 1;
     const int base = bd.rb - g.r0;  // even: bands keep the step layout
-    const unsigned long long ks = (unsigned long long)k * a.max_swaths + s;
-    T *row = a.rowbuf ? a.rowbuf + ks * (W + 32) : nullptr;
-    TileIn<T> tile{nullptr, g.m - 1};
-    T corner = c0 == 0 ? (g.r0 ? Num<T>::big() : T(0)) : (g.r0 ? T(0) : Num<T>::big());
-    if (b > 0) {
-      // the band below, complete: its last row, and its left edge's value there
-      if (lane == 0) wait_word_at_least(a.bdone + ks, (unsigned long long)b, a.err, kWaitLimitNs);
-      __syncwarp();
-      (void)ld_acquire_gpu(a.bdone + ks);
-      tile.col_init = row;
-      corner = s ? row[W] : Num<T>::big();
-    }
-    if (b + 1 < bd.count) {
-      tile.row_out = row;
-      tile.corner_out = row + W;
-    }
-    SwathJob<T> job;
-    job.x = g.flip ? cen : seq;
-    job.y = g.flip ? seq : cen;
-    job.m = bd.re;
-    job.n = g.n;
-    job.c0 = c0;
-    job.r0 = bd.rb;
-    job.open_end = oe != 0;
-    job.edge_in = s ? (((s - 1) & 1) ? b1 : b0) + base : nullptr;
-    job.edge_out = last ? nullptr : ((s & 1) ? b1 : b0) + base;
-    job.free_diag0 = c0 > 0 && (c0 % kRefSwath) == 0;
-    job.corner_init = corner;
-    job.stage = stage_mem + (threadIdx.x >> 5) * kStageElems;
-    PathOut po;
-    po.words = a.words + a.path_off[k] + (unsigned long long)s * g.steps * 64ull +
-               (unsigned long long)(base / 2) * 64ull;
-    po.track_min = true;
-    unsigned long long *words = a.prog + (unsigned long long)k * a.max_swaths;
-    BandGate gate;
-    gate.g.prog_in = words + (s ? s - 1 : 0);
-    gate.g.prog_out = words + s;
-    gate.g.err = a.err;
-    gate.g.limit_ns = kWaitLimitNs;
-    gate.g.avail = 0;
-    gate.base = base;
-    T emin, etop;
-    const int width = g.n - c0 < W ? g.n - c0 : W;
-    const int rq = path_regs<T>(width);
-    if (rq >= RF) {
-      path_pipe_swath<T, RF>(job, po, gate, tile, emin, etop);
-    } else {
-      switch (rq / RQ) {
-#define ODBA_PPCASE(K)                                                                          \
-  case K:                                                                                       \
-    if constexpr (K * RQ < RF) path_pipe_swath<T, K * RQ>(job, po, gate, tile, emin, etop);     \
-    break;
-        ODBA_PPCASE(1)
-        ODBA_PPCASE(2)
-        ODBA_PPCASE(3)
-        ODBA_PPCASE(4)
-        ODBA_PPCASE(5)
-        ODBA_PPCASE(6)
-        ODBA_PPCASE(7)
-#undef ODBA_PPCASE
-        default:
-          break;
+    int shortcut = 0;               // !PIPE, feeder's lane 0
+    for (int s = s_first; s < (PIPE ? s_first + 1 : g.swaths); ++s) {
+      const int c0 = s * kBlkCols;
+      const bool last = s == g.swaths - 1;
+      const unsigned long long ks = (unsigned long long)k * a.max_swaths + s;
+      BlockJob<T> job;
+      job.x = g.flip ? cen : seq;
+      job.y = g.flip ? seq : cen;
+      job.m = bd.re;
+      job.n = g.n;
+      job.c0 = c0;
+      job.r0 = bd.rb;
+      job.edge_in = s ? (((s - 1) & 1) ? b1 : b0) + base : nullptr;
+      job.edge_out = last ? nullptr : ((s & 1) ? b1 : b0) + base;
+      job.open_end = oe != 0;
+      job.free_diag0 = c0 > 0;
+      job.corner_init = c0 == 0 ? (g.r0 ? Num<T>::big() : T(0)) : (g.r0 ? T(0) : Num<T>::big());
+      job.word_steps = g.steps;
+      job.words = reinterpret_cast<unsigned *>(a.words + a.path_off[k] +
+                                               (unsigned long long)s * g.steps * 64ull) +
+                  (size_t)(base / 2) * 32;
+      if (PIPE && BAND) {
+        T *row = a.rowbuf + ks * (kBlkCols + 32);
+        if (b > 0) {
+          // the band below, complete: its last row, and its left edge's value there
+          if (feeder && lane == 0)
+            wait_word_at_least(a.bdone + ks, (unsigned long long)b, a.err, kWaitLimitNs);
+          __syncthreads();
+          (void)ld_acquire_gpu(a.bdone + ks);
+          job.row_in = row;
+          job.corner_init = s ? row[kBlkCols] : Num<T>::big();
+        }
+        job.top_band = b == bd.count - 1;
+        if (b + 1 < bd.count) {
+          job.row_out = row;
+          job.corner_out = row + kBlkCols;
+        }
+      }
+      T unused = T(0);
+      EdgeStat<T> st;
+      if (PIPE) {
+        unsigned long long *words = a.prog + (unsigned long long)k * a.max_swaths;
+        BandGate gate;
+        gate.g.prog_in = words + (s ? s - 1 : 0);
+        gate.g.prog_out = words + s;
+        gate.g.err = a.err;
+        gate.g.limit_ns = kWaitLimitNs;
+        gate.g.avail = 0;
+        gate.base = base;
+        sweep_block<T, true, BAND, false, false>(job, sm, gate, CkptOut<T>{nullptr, 0, 1}, false,
+                                                 unused, st);
+        if (feeder && lane == 0) {
+          T *et = a.emtop + ((unsigned long long)b * layer + ks) * 2;
+          et[0] = st.emin;
+          et[1] = st.etop;
+        }
+        if (BAND && b + 1 < bd.count) {
+          // the row buffer and corner of every thread, then the band word
+          __threadfence();
+          __syncthreads();
+          if (feeder && lane == 0) st_release_gpu(a.bdone + ks, (unsigned long long)(b + 1));
+        }
+      } else {
+        sweep_block<T, true, false, false, false>(job, sm, NoGate(), CkptOut<T>{nullptr, 0, 1},
+                                                  false, unused, st);
+        const int cnext = c0 + kBlkCols;
+        if (oe && !os && !shortcut && !last && cnext > g.m && st.etop == st.emin) shortcut = cnext;
+        __syncthreads();
       }
     }
-    if (lane == 0) {
-      T *et = a.emtop + ((unsigned long long)b * layer + ks) * 2;
-      et[0] = emin;
-      et[1] = etop;
-    }
-    if (b + 1 < bd.count) {
-      // the row buffer and corner of every lane, then the band word
-      __threadfence();
-      __syncwarp();
-      if (lane == 0) st_release_gpu(a.bdone + ks, (unsigned long long)(b + 1));
-    }
-    if (a.walk_in_sweep) {
+    if (!PIPE && feeder && lane == 0) a.shortcut[k] = shortcut;
+    if (PIPE && a.walk_in_sweep) {
       // Member k's last task to finish resolves its shortcut and walks its
-      // path (pass 1 of the backtrack) while other warps sweep: every task
+      // path (pass 1 of the backtrack) while other blocks sweep: every task
       // makes its moves and edge values visible before it is counted.
       __threadfence();
-      __syncwarp();
-      unsigned long long n = 0;
-      if (lane == 0) n = atomicAdd(a.mdone + k, 1ull) + 1;
-      n = __shfl_sync(kFull, n, 0);
-      if (n == (unsigned long long)g.swaths * bd.count) {
-        __syncwarp();
-        (void)ld_acquire_gpu(a.mdone + k);  // every lane: after all the member's tasks
-        if (lane == 0) a.shortcut[k] = member_shortcut<T>(a, k, g, flags);
-        __syncwarp();
-        walk_member_runs<T>(a, g, k, flags & 1, oe, a.runs + a.runs_off[k]);
+      __syncthreads();
+      if (feeder) {
+        unsigned long long n = 0;
+        if (lane == 0) n = atomicAdd(a.mdone + k, 1ull) + 1;
+        n = __shfl_sync(kFull, n, 0);
+        if (n == (unsigned long long)g.swaths * bd.count) {
+          __syncwarp();
+          (void)ld_acquire_gpu(a.mdone + k);  // every lane: after all the member's tasks
+          if (lane == 0) a.shortcut[k] = member_shortcut<T>(a, k, g, flags);
+          __syncwarp();
+          walk_member_runs<T>(a, g, k, os, oe, a.runs + a.runs_off[k]);
+        }
       }
     }
+    __syncthreads();  // the task word and the rings are free again
   }
 }
 
@@ -563,15 +487,36 @@ __global__ void shortcut_kernel(RoundArgs<T> a) {
   a.shortcut[k] = member_shortcut<T>(a, k, g, flags);
 }
 
+// The moves of one row's 32 columns cb .. cb + 31 (cb a multiple of 32): bit
+// j of d (u) is column cb + j's D (U) bit.  Four lanes of the sweep own them,
+// each a step behind its left neighbour.  Row r >= 1.
+struct RowMoves {
+  unsigned d, u;
+};
+__device__ __forceinline__ const unsigned short *row_moves_at(const unsigned short *w,
+                                                              const MemberGeom &g, int r, int cb) {
+  const int k = r - g.r0, l = (cb / kBlkR) & 31;
+  const size_t idx = ((size_t)(cb / kBlkWarpCols) * g.steps + (k >> 1) + l) * 32 + l;
+  return w + idx * 2 + (k & 1);
+}
+__device__ __forceinline__ RowMoves load_row_moves(const unsigned short *p) {
+  const unsigned lo = unsigned(p[0]) | unsigned(p[66]) << 16;
+  const unsigned hi = unsigned(p[132]) | unsigned(p[198]) << 16;
+  return RowMoves{__byte_perm(lo, hi, 0x6420), __byte_perm(lo, hi, 0x7531)};
+}
+__device__ __forceinline__ RowMoves row_moves(const unsigned short *w, const MemberGeom &g, int r,
+                                              int cb) {
+  return load_row_moves(row_moves_at(w, g, r, cb));
+}
+
 // Walks member k's path from its end cell toward (0, 0) with one warp and
 // calls visit(move, r, c) for every cell; the last call has NIL or
 // NIL_OPEN_RIGHT.  Returns false if the walk failed.  Every lane holds the
-// move word of one of the 32 rows at and below the current cell (the word of
-// the lane that owned the current column in the path sweep), so the walk
-// advances by shuffles and reloads only when it leaves those 32 rows or that
-// owner's columns -- about once per 32 steps instead of one dependent global
-// load per step.  Every lane keeps the same walk state (visitors store from
-// lane 0 only).  Moves are decoded as the reference defines them: the
+// moves of one of the 32 rows at and below the current cell in a block of 32
+// columns, so the walk advances by shuffles and reloads only when it leaves
+// those rows or columns -- about once per 32 steps instead of one dependent
+// global load per step.  Every lane keeps the same walk state (visitors store
+// from lane 0 only).  Moves are decoded as the reference defines them: the
 // open-end shortcut overrides the top row first (with a single-row matrix that
 // row is row 0, dtw.hpp:105-108 runs before the row-0 loop), then row 0
 // (RIGHT or OPEN_RIGHT, NIL / NIL_OPEN_RIGHT at (0, 0)), then the recorded
@@ -580,8 +525,7 @@ template <typename T, typename Visit>
 __device__ __forceinline__ bool walk_member_path(const RoundArgs<T> &a, const MemberGeom &g, int k,
                                                  int os, int oe, Visit &&visit) {
   const int lane = threadIdx.x & 31;
-  constexpr int RF = PathTune<T>::RF, W = 32 * RF;
-  const unsigned long long *w = a.words + a.path_off[k];
+  const unsigned short *w = reinterpret_cast<const unsigned short *>(a.words + a.path_off[k]);
   const int shortcut = a.shortcut[k];
   // A path has at most m + n - 1 cells and never leaves the matrix; the checks
   // only keep a corrupt path buffer from turning into an endless or
@@ -590,26 +534,20 @@ __device__ __forceinline__ bool walk_member_path(const RoundArgs<T> &a, const Me
   long long steps = 0;
   int r = g.m - 1, c = g.n - 1;
   for (;;) {
-    const int s = c / W, c0 = s * W;
-    int R = RF;
-    if (s == g.swaths - 1) R = path_regs<T>(g.n - c0);
-    const int top = r, owner = (c - c0) / R, cbeg = c0 + owner * R;
-    unsigned long long word = 0;
-    const int my_row = top - lane;
-    if (my_row >= 1) {
-      const int rr = my_row - g.r0;
-      const unsigned long long t = (unsigned long long)owner + (rr >> 1);
-      word = w[(unsigned long long)s * g.steps * 64ull + (t * 32 + owner) * 2 + (rr & 1)];
-    }
+    const int top = r, cbeg = c & ~31;
+    RowMoves mine{0u, 0u};
+    if (top - lane >= 1) mine = row_moves(w, g, top - lane, cbeg);
     for (;;) {
-      const unsigned long long wv = __shfl_sync(kFull, word, (top - r) & 31);
+      const int src = (top - r) & 31;
+      const unsigned rd = __shfl_sync(kFull, mine.d, src), ru = __shfl_sync(kFull, mine.u, src);
       int mv;
       if (shortcut && r == g.m - 1 && c >= shortcut) {
         mv = kMoveOpenRight;
       } else if (r == 0) {
         mv = c == 0 ? (os ? kMoveNilOpenRight : kMaxMoveNil) : (os ? kMoveOpenRight : kMoveRight);
       } else {
-        mv = decode_move(wv, c - cbeg);
+        const int j = c - cbeg;
+        mv = ((rd >> j) & 1u) ? kMoveDiag : ((ru >> j) & 1u) ? kMoveUp : kMoveRight;
         if (mv == kMoveRight && oe && r == g.m - 1) mv = kMoveOpenRight;
       }
       if (mv == kMaxMoveNil || mv == kMoveNilOpenRight) {
@@ -636,24 +574,32 @@ __device__ __forceinline__ bool walk_member_path(const RoundArgs<T> &a, const Me
 // The backtrack's ranges alone (no path listing), in two passes.  Pass 1 (one
 // warp per member) walks the path a row at a time: in a row the backward walk
 // moves left through RIGHT cells until the first cell whose D or U bit is set,
-// one count-leading-zeros on the row's step word away, and the walk stores
-// the row's interval of contributing cells' columns at runs[r] ((1, 0) if
-// none).  The contributing cells are those of walk_member_path with the
-// backtrack's visitor: the top row's OPEN_RIGHT cells (from the open-end
-// shortcut's column on, and RIGHT on the open-end top row) contribute
-// nothing, so that row contributes only its last cell; row 0 is RIGHT
-// (OPEN_RIGHT with open start) down to (0, 0), which contributes unless it is
-// NIL_OPEN_RIGHT.  Pass 2 (runs_to_ranges_kernel) turns the intervals into
-// per-centroid-index ranges in parallel.  Returns false if the walk failed.
+// one count-leading-zeros on the row's bits away, and the walk keeps the row's
+// interval of contributing cells' columns for runs[r] ((1, 0) if none).  The
+// contributing cells are those of walk_member_path with the backtrack's
+// visitor: the top row's OPEN_RIGHT cells (from the open-end shortcut's column
+// on, and RIGHT on the open-end top row) contribute nothing, so that row
+// contributes only its last cell; row 0 is RIGHT (OPEN_RIGHT with open start)
+// down to (0, 0), which contributes unless it is NIL_OPEN_RIGHT.  Pass 2
+// (runs_to_ranges_kernel) turns the intervals into per-centroid-index ranges
+// in parallel.  Returns false if the walk failed.
+//
+// The walk is one serial chain per member, so what counts is the latency per
+// row: a row takes seven dependent instructions, unrolled eight rows at a time
+// without a branch (a walk that has left the window keeps a negative column),
+// and everything else -- the rows' bits, the intervals, the exit -- is off the
+// chain.  A window is 32 rows (one per lane) by 32 columns; the windows below
+// and to the left are loaded with it, and a lane keeps its row's interval in
+// registers until the warp stores them together.
 template <typename T>
 __device__ __forceinline__ bool walk_member_runs(const RoundArgs<T> &a, const MemberGeom &g, int k,
                                                  int os, int oe, int2 *runs) {
+  constexpr int G = 8;  // rows per group
   const int lane = threadIdx.x & 31;
-  constexpr int RF = PathTune<T>::RF, W = 32 * RF;
-  const unsigned long long *w = a.words + a.path_off[k];
+  const unsigned short *w = reinterpret_cast<const unsigned short *>(a.words + a.path_off[k]);
   const int shortcut = a.shortcut[k];
-  const bool lead = lane == 0;
-  // every window advances the walk by a row or an owner: a bound on windows
+  // every window advances the walk by a row or a block of columns: a bound on
+  // windows
   const long long max_windows = (long long)g.m + g.n + 64;
   long long windows = 0;
   int r = g.m - 1, c = g.n - 1;
@@ -661,98 +607,115 @@ __device__ __forceinline__ bool walk_member_runs(const RoundArgs<T> &a, const Me
   // the column the walk entered row r at; -1 on the open-end top row, whose
   // interval is its first cell alone
   int entry = oe ? -1 : c;
-  // A window: rows top .. top - 31 of one owner lane's columns cbeg .. cbeg +
-  // R - 1 (swath s, owner); lane l holds row top - l's planes, word idx of
-  // the member's path (step t = owner + (row - r0) / 2 of the swath: word
-  // (t * 32 + owner) * 2 + (row - r0) % 2).  The windows below (same owner,
-  // 32 rows = 16 steps down: idx - 1024) and to the left (owner - 1, idx -
-  // 66; or the previous swath's last owner) are loaded with it, so a window
-  // left through its last row or its first column is replaced without
-  // waiting on memory or dividing.
-  const long long swath_words = (long long)g.steps * 64;
-  int s = 0, owner = 0, cbeg = 0, R = RF, top = -1;
-  long long idx = 0, down_idx = 0, left_idx = 0;
-  int ls = 0, lowner = 0, lcbeg = 0, lR = RF;
-  unsigned long long word = 0, down_w = 0, left_w = 0;
-  int j = 0;
+  // A window: rows top .. top - 31 of columns cb .. cb + 31; lane l holds row
+  // top - l, its moves at `at`.
+  int top = -1, cb = 0;
+  RowMoves cur{0u, 0u}, down{0u, 0u}, left{0u, 0u};
+  const unsigned short *at = w, *at_left = w;
+  int2 iv = make_int2(1, 0);
+  bool have = false;
   for (;;) {
+    const bool below = top >= 0 && r == top - 32;
+    if ((below || r == 0) && have) {
+      runs[top - lane] = iv;
+      have = false;
+    }
     if (c < 0) return false;  // walked off column 0
     if (r == 0) {
-      if (lead) runs[0] = os ? make_int2(1, 0) : make_int2(0, c);
+      __syncwarp();
+      if (lane == 0) runs[0] = os ? make_int2(1, 0) : make_int2(0, c);
       return true;
     }
     if (++windows > max_windows) return false;
-    if (top >= 0 && j >= 0 && r == top - 32) {
-      top -= 32;  // the window below
-      word = down_w;
-      idx = down_idx;
-    } else if (top >= 0 && j < 0 && r > top - 32 && cbeg > 0) {
-      s = ls;  // the window to the left
-      owner = lowner;
-      cbeg = lcbeg;
-      R = lR;
-      word = left_w;
-      idx = left_idx;
+    if (below && c >= cb) {
+      top -= 32;
+      at -= 16 * 64;  // 16 steps of 32 words
+      cur = down;
+    } else if (top >= 0 && !below) {
+      cb -= 32;
+      at = at_left;
+      cur = left;
     } else {
-      s = c / W;
-      const int c0 = s * W;
-      R = RF;
-      if (s == g.swaths - 1) R = path_regs<T>(g.n - c0);
-      owner = (c - c0) / R;
-      cbeg = c0 + owner * R;
       top = r;
-      const int rr = top - lane - g.r0;
-      idx = s * swath_words + owner * 66 + (long long)(rr >> 1) * 64 + (rr & 1);
-      word = top - lane >= 1 ? w[idx] : 0ull;
+      cb = c & ~31;
+      at = row_moves_at(w, g, top - lane, cb);
+      if (top - lane >= 1) cur = load_row_moves(at);
     }
-    down_idx = idx - 1024;
-    down_w = top - 32 - lane >= 1 ? w[down_idx] : 0ull;
-    if (cbeg > 0) {
-      if (owner > 0) {
-        ls = s;
-        lowner = owner - 1;
-        lcbeg = cbeg - R;
-        lR = R;
-        left_idx = idx - 66;
-      } else {
-        ls = s - 1;
-        lowner = 31;
-        lcbeg = cbeg - RF;
-        lR = RF;
-        left_idx = idx - swath_words + 31 * 66;
+    if (top - 32 - lane >= 1) down = load_row_moves(at - 16 * 64);
+    if (cb > 0 && top - lane >= 1) {
+      at_left = (cb & (kBlkWarpCols - 1)) ? at - 4 * 66 : row_moves_at(w, g, top - lane, cb - 32);
+      left = load_row_moves(at_left);
+    }
+    // Rows that are not the walk's -- row 0 and below, and in the first group
+    // those above the walk's row -- get moves that leave the walk where it is.
+    const bool row_exists = top - lane >= 1;
+    const unsigned dul = row_exists ? cur.d | cur.u : ~0u, dl = row_exists ? cur.d : 0u;
+    const int rows = top < 32 ? top : 32;
+    int i = top - r, j = c - cb;  // the walk: row top - i, column cb + j
+    int i0 = i & ~(G - 1);        // the group: rows top - i0 - q, q < G
+    unsigned du[G], d[G];
+#pragma unroll
+    for (int q = 0; q < G; ++q) {
+      du[q] = __shfl_sync(kFull, dul, i0 + q);
+      d[q] = __shfl_sync(kFull, dl, i0 + q);
+      if (i0 + q < i) {
+        du[q] = ~0u;
+        d[q] = 0u;
       }
-      left_w = top - lane >= 1 ? w[left_idx] : 0ull;
     }
-    const unsigned dul = unsigned(word) | unsigned(word >> 32), dl = unsigned(word);
-    // j: the walk's column within the window; a row's planes are shuffled
-    // one row ahead, off the chain through j
-    const int lim = top - 32 > 0 ? top - 32 : 0;
-    j = c - cbeg;
-    int2 *rp = runs + r;
-    unsigned du_r = __shfl_sync(kFull, dul, (top - r) & 31);
-    unsigned d_r = __shfl_sync(kFull, dl, (top - r) & 31);
     for (;;) {
-      const int ln = (top - r + 1) & 31;
-      const unsigned du_n = __shfl_sync(kFull, dul, ln);
-      const unsigned d_n = __shfl_sync(kFull, dl, ln);
-      const unsigned x = du_r << (31 - j);  // the row's moves at or left of j, top-aligned
-      if (x == 0) {
-        // RIGHT through the owner's first column: on in the owner to the left
+      // The chain carries s = 31 - column: 32 or more once the walk has left
+      // the window (shifts by more than 31 give 0, and s only grows).
+      const int own = lane - i0;
+      unsigned s = 31u - unsigned(j), mine = 0u;
+#pragma unroll
+      for (int q = 0; q < G; ++q) {
+        if (own == q) mine = s;
+        unsigned x, t;  // the row's moves, and its D bits, from the walk's column on
+        asm("shl.b32 %0, %1, %2;" : "=r"(x) : "r"(du[q]), "r"(s));
+        const unsigned stop = s + unsigned(__clz(x));
+        asm("shl.b32 %0, %1, %2;" : "=r"(t) : "r"(d[q]), "r"(stop));
+        s = stop + (t >> 31);
+        du[q] = __shfl_sync(kFull, dul, (i0 + G + q) & 31);
+        d[q] = __shfl_sync(kFull, dl, (i0 + G + q) & 31);
+      }
+      // the rows before `end` were entered and left inside the window's
+      // columns; where the walk went out in row `end`, that row is complete if
+      // it left it by DIAG in the first column, and still the walk's row if
+      // its moves are all RIGHT
+      const bool out = s >= 32u;
+      int end = rows - i0 < G ? rows - i0 : G, after = 31 - int(s);
+      unsigned x = 0u;
+      if (mine < 32u) x = dul << mine;
+      bool whole = false;
+      if (out) {
+        end = __popc(__ballot_sync(kFull, own >= 1 && own < G && mine < 32u));
+        after = 31 - int(__shfl_sync(kFull, mine, i0 + end));
+        whole = __any_sync(kFull, own == end && x != 0);
+      }
+      if (lane >= i && own < end + (whole ? 1 : 0)) {
+        const int cp = cb + 31 - int(mine) - __clz(x);
+        const int from = lane == i ? entry : cb + 31 - int(mine);
+        iv = make_int2(cp, cp > from ? cp : from);
+        have = true;
+      }
+      if (out) {
+        if (whole)
+          entry = cb - 1;
+        else if (i0 + end > i)
+          entry = cb + after;
+        i = i0 + end + (whole ? 1 : 0);
         j = -1;
         break;
       }
-      const int jp = j - __clz(x);
-      const int cp = cbeg + jp;
-      if (lead) *rp = make_int2(cp, cp > entry ? cp : entry);
-      --rp;
-      --r;
-      j = jp - int((d_r >> jp) & 1u);  // one column left after DIAG
-      entry = cbeg + j;
-      du_r = du_n;
-      d_r = d_n;
-      if ((r <= lim) | (j < 0)) break;  // row 0, or a new window
+      i = i0 + end;
+      i0 = i;
+      j = after;
+      entry = cb + j;
+      if (i >= rows) break;
     }
-    c = cbeg + j;
+    r = top - i;
+    c = cb + j;
   }
 }
 
@@ -1022,9 +985,11 @@ __global__ void single_job_kernel(int *mseries, int *mjob, int n, int *clen, int
   }
 }
 
+// Resident blocks of the path kernel on the current device, cached per device
+// index (host threads may race; both compute the same value).
 template <typename T>
 int round_grid() {
-  static std::atomic<int> cached[64];  // per device; host threads may race (same value)
+  static std::atomic<int> cached[64];
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64) {
@@ -1033,8 +998,10 @@ int round_grid() {
   }
   int sms = 0, per_sm = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-      &per_sm, path_dtw_kernel<T, PathTune<T>::RF, PathTune<T>::RQ, kRoundWarps>, kRoundWarps * 32, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, path_block_kernel<T, true, false>,
+                                                kBlkThreads, 0);
+  constexpr int want = sizeof(T) == 4 ? kRoundBlocksF32 : kRoundBlocksF64;
+  if (per_sm > want) per_sm = want;
   if (per_sm < 1) per_sm = 1;
   const int g = sms * per_sm;
   if (dev >= 0 && dev < 64) cached[dev].store(g, std::memory_order_relaxed);
@@ -1056,19 +1023,10 @@ constexpr int kMaxBands = 8;
 constexpr size_t kMaxRowBufBytes = size_t(256) << 20;
 std::atomic<int> g_round_bands{0};  // odba_round_set_bands (0: chosen per launch)
 
-// Row bands of the swath pipeline for `tasks` (member, swath) tasks on
-// `slots` resident warps: two when the tasks make more than one wave and at
-// most four, one otherwise.  Tasks that fit one wave run at once, and bands
-// would only lengthen each (member, swath)'s chain.  Past one wave, halving
-// the tasks halves the last partial wave; more bands cost more than they
-// save, because a band taken from the counter before the band below it is
-// done holds its warp while it waits (400 members x 6 swaths on 1776 warps:
-// path DTW 7.02 ms with one band, 6.84 with two, 7.56 with three, 8.97 with
-// four; 800 members: 11.42, 10.97 and 11.71 ms).
-int pipe_bands(unsigned long long tasks, size_t slots) {
+// Row bands of the swath pipeline: those pinned, else none.
+int pipe_bands() {
   const int forced = g_round_bands.load(std::memory_order_relaxed);
-  if (forced > 0) return forced < kMaxBands ? forced : kMaxBands;
-  return (tasks > slots && tasks <= 4ull * slots) ? 2 : 1;
+  return forced > 0 ? (forced < kMaxBands ? forced : kMaxBands) : 1;
 }
 
 // Workspace layout for nmem members / njobs jobs with the given totals.
@@ -1079,7 +1037,7 @@ RoundLayout round_layout(int nmem, int njobs, unsigned long long words,
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
   RoundLayout L;
   L.edge_stride = (maxm + 32 + 31) / 32 * 32;
-  const size_t slots = size_t(round_grid<T>()) * kRoundWarps;
+  const size_t slots = size_t(round_grid<T>());
   L.max_swaths = max_swaths;
   L.pipe = max_swaths > 0 && size_t(nmem) * 2 * L.edge_stride * sizeof(T) <= kPipeEdgeBytes;
   const size_t edge_cols = L.pipe ? size_t(nmem) : slots;
@@ -1097,15 +1055,15 @@ RoundLayout round_layout(int nmem, int njobs, unsigned long long words,
   L.off_edges = o; o += up(edge_cols * 2 * L.edge_stride * sizeof(T));
   L.off_words = o; o += up(words * 8);
   const size_t ps = L.pipe ? size_t(nmem) * size_t(max_swaths) : 0;
-  L.nbands = L.pipe ? pipe_bands(tasks, slots) : 1;
+  L.nbands = L.pipe ? pipe_bands() : 1;
   // row buffers for at most kMaxRowBufBytes (many inactive members: no bands)
-  if (L.nbands > 1 && ps * (32 * PathTune<T>::RF + 32) * sizeof(T) > kMaxRowBufBytes) L.nbands = 1;
+  if (L.nbands > 1 && ps * (kBlkCols + 32) * sizeof(T) > kMaxRowBufBytes) L.nbands = 1;
   L.off_prog = o; o += up(ps * 8);
   L.off_bdone = o; o += up(ps * 8);  // cleared with the progress words
   L.off_mdone = o; o += L.pipe ? up(size_t(nmem) * 8) : 0;  // likewise
   L.off_order = o; o += L.pipe ? up(size_t(nmem) * 4) : 0;
   L.off_emtop = o; o += up(ps * L.nbands * 2 * sizeof(T));
-  L.off_rowbuf = o; o += L.nbands > 1 ? up(ps * (32 * PathTune<T>::RF + 32) * sizeof(T)) : 0;
+  L.off_rowbuf = o; o += L.nbands > 1 ? up(ps * (kBlkCols + 32) * sizeof(T)) : 0;
   L.total = o;
   (void)njobs;
   return L;
@@ -1164,9 +1122,10 @@ void launch_paths(RoundArgs<T> &a, const RoundLayout &L, char *base, cudaStream_
   cudaMemsetAsync(a.counter, 0, 16, stream);  // work counter and error word
   plan_kernel<T><<<1, kPlanThreads, 0, stream>>>(a);
   fill_ranges_kernel<<<int(nr / 256 + 1 < 4096 ? nr / 256 + 1 : 4096), 256, 0, stream>>>(a.ranges, nr);
-  // with fewer members than resident warps, one block per member spreads
-  // them over the SMs instead of leaving them to the first blocks placed
-  const bool spread = a.nmem < round_grid<T>() * kRoundWarps;
+  const unsigned long long tasks =
+      L.pipe ? (unsigned long long)a.nmem * L.max_swaths * L.nbands : (unsigned long long)a.nmem;
+  const int resident = round_grid<T>();
+  const int grid = tasks < (unsigned long long)resident ? int(tasks) : resident;
   if (L.pipe) {
     cudaMemsetAsync(a.prog, 0, L.off_order - L.off_prog, stream);  // progress, band, member words
     if (!a.order && a.nmem <= kRankMembers) {
@@ -1174,14 +1133,14 @@ void launch_paths(RoundArgs<T> &a, const RoundLayout &L, char *base, cudaStream_
       rank_members_kernel<T><<<(a.nmem + 255) / 256, 256, 0, stream>>>(a, ord);
       a.order = ord;
     }
-    path_pipe_kernel<T, PathTune<T>::RF, PathTune<T>::RQ>
-        <<<round_grid<T>(), kRoundWarps * 32, 0, stream>>>(a);
+    if (L.nbands > 1)
+      path_block_kernel<T, true, true><<<grid, kBlkThreads, 0, stream>>>(a);
+    else
+      path_block_kernel<T, true, false><<<grid, kBlkThreads, 0, stream>>>(a);
     if (!a.walk_in_sweep) shortcut_kernel<T><<<(a.nmem + 127) / 128, 128, 0, stream>>>(a);
-  } else if (spread)
-    path_dtw_kernel<T, PathTune<T>::RF, PathTune<T>::RQ, 1><<<a.nmem, 32, 0, stream>>>(a);
-  else
-    path_dtw_kernel<T, PathTune<T>::RF, PathTune<T>::RQ, kRoundWarps>
-        <<<round_grid<T>(), kRoundWarps * 32, 0, stream>>>(a);
+  } else {
+    path_block_kernel<T, false, false><<<grid, kBlkThreads, 0, stream>>>(a);
+  }
 }
 
 // The backtrack: with a path listing one kernel walking cell by cell; without,

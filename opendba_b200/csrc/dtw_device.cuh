@@ -308,6 +308,9 @@ struct NoGate {
   static constexpr bool kActive = false;
   __device__ __forceinline__ void wait_in(int) {}
   __device__ __forceinline__ void publish(int) {}
+  __device__ __forceinline__ bool ready(int) { return true; }
+  __device__ __forceinline__ void fail() {}
+  __device__ __forceinline__ unsigned *error() { return nullptr; }
 };
 constexpr int kPublishSteps = 64;  // lane 31 publishes every 64 steps (128 rows)
 

@@ -60,6 +60,23 @@ struct PipeGate {
     }
   }
   __device__ __forceinline__ void publish(int k) { st_release_gpu(prog_out, (unsigned long long)k); }
+  // wait_in without the wait: whether rows [0, k) may be read now (also when
+  // the launch's error word is up: nobody waits any more)
+  __device__ __forceinline__ bool ready(int k) {
+    if (k <= avail) return true;
+    const unsigned long long v = ld_acquire_gpu(prog_in);
+    if (v >= (unsigned long long)k) {
+      avail = int(v);
+      return true;
+    }
+    if (*reinterpret_cast<volatile unsigned *>(err)) {
+      avail = 0x7fffffff;
+      return true;
+    }
+    return false;
+  }
+  __device__ __forceinline__ void fail() { atomicExch(err, 1u); }
+  __device__ __forceinline__ unsigned *error() { return err; }
 };
 
 // The gate of a band of a swath's rows: the band's rows count from base (its
@@ -71,6 +88,9 @@ struct BandGate {
   int base;
   __device__ __forceinline__ void wait_in(int k) { g.wait_in(base + k); }
   __device__ __forceinline__ void publish(int k) { g.publish(base + k); }
+  __device__ __forceinline__ bool ready(int k) { return g.ready(base + k); }
+  __device__ __forceinline__ void fail() { g.fail(); }
+  __device__ __forceinline__ unsigned *error() { return g.err; }
 };
 
 // Bounded wait (one thread) until *p >= v, with the gate's error rules:
