@@ -45,17 +45,18 @@ constexpr int kRankMembers = 16384;  // longest-first task order computed up to 
 // kMoveRight and kMoveUp come with the path sweep (dtw_path.cuh)
 constexpr int kMaxMoveNil = 255, kMoveOpenRight = 4, kMoveNilOpenRight = 5;
 
+// Non-negative costs order like their bit patterns.
 template <typename T>
-struct PathTune;
-// Stripe mode's one-warp swaths: RF registers (columns) per lane of a full
-// swath; the last, partial swath of a member takes a multiple of RQ.
+struct CostBits;
 template <>
-struct PathTune<float> {
-  static constexpr int RF = 32, RQ = 4;
+struct CostBits<float> {
+  using U = unsigned;
+  static __device__ __forceinline__ U of(float v) { return __float_as_uint(v); }
 };
 template <>
-struct PathTune<double> {
-  static constexpr int RF = 16, RQ = 4;
+struct CostBits<double> {
+  using U = unsigned long long;
+  static __device__ __forceinline__ U of(double v) { return (U)__double_as_longlong(v); }
 };
 
 // Geometry of one member's cost matrix, identical on host and device.
@@ -591,22 +592,24 @@ __device__ __forceinline__ bool walk_member_path(const RoundArgs<T> &a, const Me
 // chain.  A window is 32 rows (one per lane) by 32 columns; the windows below
 // and to the left are loaded with it, and a lane keeps its row's interval in
 // registers until the warp stores them together.
-template <typename T>
-__device__ __forceinline__ bool walk_member_runs(const RoundArgs<T> &a, const MemberGeom &g, int k,
-                                                 int os, int oe, int2 *runs) {
+//
+// The walk starts (or goes on) at st.r, st.c; st.entry is the column it
+// entered row st.r at (-1 on the open-end top row, whose interval is its first
+// cell alone).  w holds the moves of the columns from cmin (a multiple of the
+// swath) on; the walk ends at the start cell (1), when it fails (2), or when
+// it leaves cmin to the left (0).
+struct RowWalk {
+  int r, c, entry;
+};
+__device__ __forceinline__ int walk_runs(const unsigned short *w, const MemberGeom &g, int cmin,
+                                         RowWalk &st, int os, int2 *runs) {
   constexpr int G = 8;  // rows per group
   const int lane = threadIdx.x & 31;
-  const unsigned short *w = reinterpret_cast<const unsigned short *>(a.words + a.path_off[k]);
-  const int shortcut = a.shortcut[k];
   // every window advances the walk by a row or a block of columns: a bound on
   // windows
   const long long max_windows = (long long)g.m + g.n + 64;
   long long windows = 0;
-  int r = g.m - 1, c = g.n - 1;
-  if (shortcut && c >= shortcut) c = shortcut - 1;  // OPEN_RIGHT from the shortcut's column on
-  // the column the walk entered row r at; -1 on the open-end top row, whose
-  // interval is its first cell alone
-  int entry = oe ? -1 : c;
+  int r = st.r, c = st.c, entry = st.entry;
   // A window: rows top .. top - 31 of columns cb .. cb + 31; lane l holds row
   // top - l, its moves at `at`.
   int top = -1, cb = 0;
@@ -616,17 +619,21 @@ __device__ __forceinline__ bool walk_member_runs(const RoundArgs<T> &a, const Me
   bool have = false;
   for (;;) {
     const bool below = top >= 0 && r == top - 32;
-    if ((below || r == 0) && have) {
+    if ((below || r == 0 || c < cmin) && have) {
       runs[top - lane] = iv;
       have = false;
     }
-    if (c < 0) return false;  // walked off column 0
+    if (c < 0) return 2;  // walked off column 0
     if (r == 0) {
       __syncwarp();
       if (lane == 0) runs[0] = os ? make_int2(1, 0) : make_int2(0, c);
-      return true;
+      return 1;
     }
-    if (++windows > max_windows) return false;
+    if (c < cmin) {
+      st = RowWalk{r, c, entry};
+      return 0;
+    }
+    if (++windows > max_windows) return 2;
     if (below && c >= cb) {
       top -= 32;
       at -= 16 * 64;  // 16 steps of 32 words
@@ -638,12 +645,12 @@ __device__ __forceinline__ bool walk_member_runs(const RoundArgs<T> &a, const Me
     } else {
       top = r;
       cb = c & ~31;
-      at = row_moves_at(w, g, top - lane, cb);
+      at = row_moves_at(w, g, top - lane, cb - cmin);
       if (top - lane >= 1) cur = load_row_moves(at);
     }
     if (top - 32 - lane >= 1) down = load_row_moves(at - 16 * 64);
-    if (cb > 0 && top - lane >= 1) {
-      at_left = (cb & (kBlkWarpCols - 1)) ? at - 4 * 66 : row_moves_at(w, g, top - lane, cb - 32);
+    if (cb > cmin && top - lane >= 1) {
+      at_left = (cb & (kBlkWarpCols - 1)) ? at - 4 * 66 : row_moves_at(w, g, top - lane, cb - 32 - cmin);
       left = load_row_moves(at_left);
     }
     // Rows that are not the walk's -- row 0 and below, and in the first group
@@ -719,30 +726,35 @@ __device__ __forceinline__ bool walk_member_runs(const RoundArgs<T> &a, const Me
   }
 }
 
-// Pass 2, one block per member: the contributing columns of row r are the
-// interval runs[r] = [x, y].  Member on the rows (centroid index t = column):
-// column t's range is [lowest, highest] row holding t.  Consecutive rows'
-// intervals share at most one column -- row r's first with row r - 1's last
-// (an UP move) and row r's last with row r + 1's first -- so row r stores a
-// column's high end unless row r + 1 also holds it and its low end unless row
-// r - 1 also holds it; every other column of the interval is row r's alone.
-// Centroid on the rows (t = row): the interval is the range.
 template <typename T>
-__global__ void runs_to_ranges_kernel(RoundArgs<T> a) {
-  const int k = blockIdx.x;
-  int jb;
-  const MemberGeom g = geom_of<T>(a, k, jb);
-  if (!(a.jflags[jb] & 4)) return;
-  const int2 *runs = a.runs + a.runs_off[k];
-  int2 *rg = a.ranges + a.rng_off[k];
-  for (int r = threadIdx.x; r < g.m; r += blockDim.x) {
+__device__ __forceinline__ bool walk_member_runs(const RoundArgs<T> &a, const MemberGeom &g, int k,
+                                                 int os, int oe, int2 *runs) {
+  const int shortcut = a.shortcut[k];
+  RowWalk st{g.m - 1, g.n - 1, 0};
+  if (shortcut && st.c >= shortcut) st.c = shortcut - 1;  // OPEN_RIGHT from the shortcut's column on
+  st.entry = oe ? -1 : st.c;
+  return walk_runs(reinterpret_cast<const unsigned short *>(a.words + a.path_off[k]), g, 0, st, os,
+                   runs) == 1;
+}
+
+// Pass 2: the contributing columns of row r are the interval runs[r] = [x, y].
+// Member on the rows (centroid index t = column): column t's range is [lowest,
+// highest] row holding t.  Consecutive rows' intervals share at most one
+// column -- row r's first with row r - 1's last (an UP move) and row r's last
+// with row r + 1's first -- so row r stores a column's high end unless row
+// r + 1 also holds it and its low end unless row r - 1 also holds it; every
+// other column of the interval is row r's alone.  Centroid on the rows (t =
+// row): the interval is the range.
+__device__ __forceinline__ void runs_to_ranges(const int2 *runs, int2 *rg, int m, bool flip,
+                                               int first, int stride) {
+  for (int r = first; r < m; r += stride) {
     const int2 iv = runs[r];
     if (iv.x > iv.y) continue;
-    if (g.flip) {
+    if (flip) {
       rg[r] = iv;
       continue;
     }
-    const int2 above = r + 1 < g.m ? runs[r + 1] : make_int2(1, 0);
+    const int2 above = r + 1 < m ? runs[r + 1] : make_int2(1, 0);
     const int2 below = r > 0 ? runs[r - 1] : make_int2(1, 0);
     const bool top_shared = above.x <= iv.y && iv.y <= above.y;
     const bool low_shared = below.x <= iv.x && iv.x <= below.y;
@@ -751,6 +763,15 @@ __global__ void runs_to_ranges_kernel(RoundArgs<T> a) {
       if (!(t == iv.x && low_shared)) rg[t].x = r;
     }
   }
+}
+template <typename T>
+__global__ void runs_to_ranges_kernel(RoundArgs<T> a) {
+  const int k = blockIdx.x;
+  int jb;
+  const MemberGeom g = geom_of<T>(a, k, jb);
+  if (!(a.jflags[jb] & 4)) return;
+  runs_to_ranges(a.runs + a.runs_off[k], a.ranges + a.rng_off[k], g.m, g.flip != 0, threadIdx.x,
+                 blockDim.x);
 }
 
 // The backtrack (updateCentroid's loop, dba.hpp:374-423): per member the
@@ -1360,15 +1381,14 @@ int dba_batch_launch(const T *centroids, const unsigned long long *coff, const i
 // memory (the reference's stripe mode, dba.hpp:515-763).  Per member, in the
 // orientation of the full-path round (centroid on the rows when an open end
 // flips the member, dba.hpp:497-501):
-//   1. forward: the swath pipeline (many warps, bounded hand-off waits) over
-//      the member's swaths; every swath's right edge is kept (E, one column of
+//   1. forward: the swath pipeline (a block per 1024-column swath, bounded
+//      hand-off waits); every swath's right edge is kept (E, one column of
 //      rows per swath) and every K-th cost row is kept across all columns (Q);
-//   2. backtrack, reference stripe by reference stripe (1024 columns) from the
-//      right: every K-row tile of the stripe's swaths below the current
-//      backtrack height H is recomputed with its moves in parallel (one warp
-//      per tile: its row below comes from Q, its left edge from E), then one
-//      warp continues the walk through the stripe and records the
-//      per-centroid-index sample ranges (and the path listing);
+//   2. backtrack, from the right: the K-row tiles of a group of reference
+//      stripes (1024 columns each) below the current backtrack height H are
+//      recomputed with their moves in parallel (one block per tile: its row
+//      below comes from Q, its left edge from E), then one warp continues the
+//      walk through the group;
 //   3. the ordered reducer of the full-path round.
 // The reference re-runs each stripe with the first sequence's length set to H
 // (dba.hpp:700-721), so with an open end its top-row rule acts on row H-1 and
@@ -1378,72 +1398,71 @@ int dba_batch_launch(const T *centroids, const unsigned long long *coff, const i
 // shortcut fired in the forward pass on take that branch too (the reference's
 // forward pass stopped there and left those edges unwritten).  The recompute
 // here does the same: rows below H-1 are the forward pass's, row H-1 follows
-// the open-end rules (for double, whose swaths are 512 wide, the second half
-// of a stripe continues the first half's recomputed top row).  Without an open
-// end the round equals the full-path round bit for bit.
+// the open-end rules.  A group is then one stripe.  Without an open end the
+// round equals the full-path round bit for bit.
+//
+// What the shapes are for: one member's forward pass is a chain of swaths and
+// its walk a chain of rows, so members run side by side (kStripeSlots, as many
+// as it takes to fill the GPU with swaths), and a group has as many stripes as
+// it takes to fill it with tiles.  3 members of 40k-80k samples against a 70k
+// centroid, 1024-row tiles: 203 ms a round with one member at a time, one warp
+// per swath and per tile and one stripe per launch (forward 60 ms, tiles 67,
+// walks 76).
 namespace {
+
+constexpr int kStripeSlots = 8;       // members side by side, at most
+constexpr int kStripeGroup = 8;       // stripes per group, at most
+constexpr size_t kStripeGroupBytes = size_t(1) << 30;  // move words of all slots' groups
+constexpr size_t kStripeSlotBytes = size_t(4) << 30;   // edges and checkpoint rows of all slots
+constexpr int kStripeFill = 512;      // swaths side by side that fill the GPU
 
 struct StripeWalk {
   int r, c, h, cur_t, lo, hi, state;  // state: 0 walking, 1 done, 2 failed
   int s_fwd;                          // first stripe whose forward shortcut fired, or INT_MAX
+  int entry;                          // row walk: the column row r was entered at
   long long nt;
+};
+
+// One member in a batch: its matrix in the round's orientation.
+struct StripeMember {
+  int member, flip, m, n, swaths;
+  unsigned long long trip;  // offset of its path listing, in triples
 };
 
 template <typename T>
 struct StripeArgs {
   const T *series;
   const uint64_t *offsets;
-  int member;                   // series + offsets[member]
   const T *centroid;
-  int flip;                     // centroid on the rows
-  int m, n, r0, oe, swaths, shift;  // tile height K = 1 << shift
+  int Lc, r0, oe, shift;        // tile height K = 1 << shift
+  int count;                    // members in the batch
+  StripeMember mem[kStripeSlots];
+  // per slot (member of the batch): strides between slots
   T *E;
-  unsigned long long e_stride;
+  unsigned long long e_stride, e_slot;
   T *Q;
-  unsigned long long q_stride;
+  unsigned long long q_stride, q_slot;
   unsigned long long *prog;     // one progress word per swath
+  unsigned long long prog_slot;
+  unsigned *words;              // move words of a group, the stripes in column order
+  unsigned long long words_slot;
+  int2 *runs;                   // row walk: the column interval of every row
+  unsigned long long runs_slot;
+  typename CostBits<T>::U *fmin, *cmin;  // per stripe: shortcut minima (forward, below H)
+  unsigned long long min_slot;
+  StripeWalk *walk;
   unsigned *err;
   unsigned long long *counter;
-  unsigned long long *words;    // move words of one swath, full-path layout (two buffers
-  unsigned long long words_stride;  // words_stride apart when a stripe has two swaths)
-  StripeWalk *walk;
-  int2 *ranges;                 // this member's ranges (one per centroid index)
-  int *extra;                   // this member's extra samples, or null
-  unsigned long long *fmin;     // per stripe: forward shortcut minimum (value bits)
-  unsigned long long *cmin;     // per stripe: shortcut minimum below H (value bits)
-  T *top_carry;                 // recomputed top row at the first half's right edge
-  int32_t *triples;             // this member's path listing, or null
-  int64_t *triple_count;        // or null
+  int2 *ranges;                 // all members' ranges, Lc per member
+  int *extra;                   // all members' extra samples, or null
+  int32_t *triples;             // path listings, or null
+  int64_t *triple_counts;       // or null
   unsigned long long limit_ns;
 };
 
 template <typename T>
-__device__ __forceinline__ const T *stripe_member_ptr(const StripeArgs<T> &a) {
-  return a.series + a.offsets[a.member];
-}
-template <typename T>
-__device__ __forceinline__ const T *stripe_rows_ptr(const StripeArgs<T> &a) {
-  return a.flip ? a.centroid : stripe_member_ptr(a);
-}
-template <typename T>
-__device__ __forceinline__ const T *stripe_cols_ptr(const StripeArgs<T> &a) {
-  return a.flip ? stripe_member_ptr(a) : a.centroid;
-}
-
-// Non-negative costs order like their bit patterns (float zero-extended).
-__device__ __forceinline__ unsigned long long cost_bits(float v) { return __float_as_uint(v); }
-__device__ __forceinline__ unsigned long long cost_bits(double v) {
-  return (unsigned long long)__double_as_longlong(v);
-}
-
-// Registers per lane of swath s (the last, partial swath is narrower).
-template <typename T>
-__host__ __device__ inline int stripe_regs(int n, int s) {
-  constexpr int RF = PathTune<T>::RF, RQ = PathTune<T>::RQ, W = 32 * RF;
-  const int c0 = s * W;
-  const int width = n - c0 < W ? n - c0 : W;
-  const int rq = ((width + 31) / 32 + RQ - 1) / RQ * RQ;
-  return rq < RF ? rq : RF;
+__device__ __forceinline__ const T *stripe_member_ptr(const StripeArgs<T> &a, int slot) {
+  return a.series + a.offsets[a.mem[slot].member];
 }
 
 template <typename T>
@@ -1451,116 +1470,106 @@ __device__ __forceinline__ T stripe_corner(int c0, int r0) {
   return c0 == 0 ? (r0 ? Num<T>::big() : T(0)) : (r0 ? T(0) : Num<T>::big());
 }
 
-// The stored right edge of the swath ending at column c - 1 (c a multiple of
-// the swath width, 0 < c < n).
+// The stored left edge of stripe t >= 1.
 template <typename T>
-__device__ __forceinline__ const T *stripe_edge_before(const StripeArgs<T> &a, int c) {
-  constexpr int W = 32 * PathTune<T>::RF;
-  return a.E + (unsigned long long)(c / W - 1) * a.e_stride;
+__device__ __forceinline__ const T *stripe_edge(const StripeArgs<T> &a, int slot, int t) {
+  return a.E + (unsigned long long)slot * a.e_slot + (unsigned long long)(t - 1) * a.e_stride;
+}
+
+// The lowest stripe of group gi, counted from the right, of `group` stripes;
+// [lo, hi) with hi <= lo: none.
+__host__ __device__ inline void stripe_group(int stripes, int group, int gi, int &lo, int &hi) {
+  hi = stripes - gi * group;
+  lo = hi - group > 0 ? hi - group : 0;
 }
 
 // Whether the reference's re-run of stripe t at height H takes its shortcut
 // branch (the whole of row H-1 OPEN_RIGHT).
 template <typename T>
-__device__ __forceinline__ bool stripe_fires(const StripeArgs<T> &a, int t, int H,
+__device__ __forceinline__ bool stripe_fires(const StripeArgs<T> &a, int slot, int t, int H,
                                              const StripeWalk &w) {
   if (!a.oe || a.r0) return false;
   const long long L = (long long)t * kRefSwath;
   if (L <= H) return false;
   if (t >= w.s_fwd) return true;
-  return cost_bits(stripe_edge_before(a, int(L))[H - 1]) == a.cmin[t];
+  return CostBits<T>::of(stripe_edge(a, slot, t)[H - 1]) == a.cmin[slot * a.min_slot + t];
 }
 
-template <typename T, int R>
-__device__ __forceinline__ void stripe_fwd_swath(const SwathJob<T> &job, const PipeGate &gate,
-                                                 const CkptOut<T> &ck) {
-  T col[R];
-  sweep_swath<T, R, PipeGate, true, false>(job, col, gate, ck);
-}
-
-// OE: open end; FLIP: centroid on the rows (compile-time switches, so that
-// one of the two series pointers stays a kernel parameter and the sweep keeps
-// its registers)
-template <typename T, int RF, int RQ, bool OE, bool FLIP>
-__global__ void __launch_bounds__(kRoundWarps * 32) stripe_forward_kernel(StripeArgs<T> a) {
-  __shared__ __align__(16) T stage_mem[kRoundWarps * kStageElems];
-  constexpr int W = 32 * RF;
-  const int lane = threadIdx.x & 31;
-  const T *x = FLIP ? a.centroid : stripe_member_ptr(a);
-  const T *y = FLIP ? stripe_member_ptr(a) : a.centroid;
+template <typename T>
+__global__ void
+__launch_bounds__(kBlkThreads, sizeof(T) == 4 ? kRoundBlocksF32 : kRoundBlocksF64)
+    stripe_forward_kernel(StripeArgs<T> a, int max_swaths) {
+  __shared__ BlockSmem<T> sm;
+  const unsigned long long ntasks = (unsigned long long)a.count * max_swaths;
   for (;;) {
-    unsigned long long q = 0;
-    if (lane == 0) q = atomicAdd(a.counter, 1ull);
-    q = __shfl_sync(kFull, q, 0);
-    if (q >= (unsigned long long)a.swaths) break;
-    const int sw = int(q), c0 = sw * W;
-    SwathJob<T> job;
-    job.x = x;
-    job.y = y;
-    job.m = a.m;
-    job.n = a.n;
+    if (threadIdx.x == 0) {
+      unsigned long long q;
+      do {
+        q = atomicAdd(a.counter, 1ull);
+      } while (q < ntasks && int(q / a.count) >= a.mem[q % a.count].swaths);
+      sm.task = q;
+    }
+    __syncthreads();
+    const unsigned long long q = sm.task;
+    if (q >= ntasks) break;
+    const int sw = int(q / a.count), slot = int(q - (unsigned long long)sw * a.count);
+    const StripeMember &mem = a.mem[slot];
+    const int c0 = sw * kBlkCols;
+    T *E = a.E + slot * a.e_slot;
+    BlockJob<T> job;
+    job.x = mem.flip ? a.centroid : stripe_member_ptr(a, slot);
+    job.y = mem.flip ? stripe_member_ptr(a, slot) : a.centroid;
+    job.m = mem.m;
+    job.n = mem.n;
     job.c0 = c0;
     job.r0 = a.r0;
-    job.edge_in = sw ? a.E + (unsigned long long)(sw - 1) * a.e_stride : nullptr;
-    job.edge_out = sw + 1 < a.swaths ? a.E + (unsigned long long)sw * a.e_stride : nullptr;
-    job.open_end = OE;
-    job.free_diag0 = c0 > 0 && (c0 % kRefSwath) == 0;
+    job.edge_in = sw ? E + (unsigned long long)(sw - 1) * a.e_stride : nullptr;
+    job.edge_out = sw + 1 < mem.swaths ? E + (unsigned long long)sw * a.e_stride : nullptr;
+    job.open_end = a.oe != 0;
+    job.free_diag0 = c0 > 0;
     job.corner_init = stripe_corner<T>(c0, a.r0);
-    job.stage = stage_mem + (threadIdx.x >> 5) * kStageElems;
+    job.words = nullptr;
+    job.word_steps = 0;
     PipeGate gate;
-    gate.prog_in = a.prog + (sw ? sw - 1 : 0);
-    gate.prog_out = a.prog + sw;
+    unsigned long long *prog = a.prog + slot * a.prog_slot;
+    gate.prog_in = prog + (sw ? sw - 1 : 0);
+    gate.prog_out = prog + sw;
     gate.err = a.err;
     gate.limit_ns = a.limit_ns;
     gate.avail = 0;
-    const CkptOut<T> ck{a.Q + c0, a.q_stride, a.shift};
-    const int R = stripe_regs<T>(a.n, sw);
-    if (R == RF) {
-      stripe_fwd_swath<T, RF>(job, gate, ck);
-    } else {
-      switch (R / RQ) {
-#define ODBA_SCASE(K)                                                         \
-  case K:                                                                     \
-    if constexpr (K * RQ < RF) stripe_fwd_swath<T, K * RQ>(job, gate, ck);    \
-    break;
-        ODBA_SCASE(1)
-        ODBA_SCASE(2)
-        ODBA_SCASE(3)
-        ODBA_SCASE(4)
-        ODBA_SCASE(5)
-        ODBA_SCASE(6)
-        ODBA_SCASE(7)
-#undef ODBA_SCASE
-        default:
-          break;
-      }
-    }
+    T unused = T(0);
+    EdgeStat<T> st;
+    sweep_block<T, false, false, true, false>(
+        job, sm, gate, CkptOut<T>{a.Q + slot * a.q_slot + c0, a.q_stride, a.shift}, false, unused,
+        st);
+    __syncthreads();
   }
 }
 
 // Shortcut minimum of the stored edge before stripe t over rows [0, H)
-// (ShortcutRows), reduced into slot[t].  Forward pass (fwd): every stripe t
-// in [tlo, thi] (stripes past the last row), H = m.  Backtrack: the one
-// stripe tlo, H the walk's height, skipped where the stripe's branch is
+// (ShortcutRows), reduced into the slot's minima.  Forward pass (fwd): every
+// stripe t in [tlo, thi] (stripes past the last row), H = m.  Backtrack: the
+// one stripe tlo, H the walk's height, skipped where the stripe's branch is
 // already decided.
 template <typename T>
-__global__ void stripe_min_kernel(StripeArgs<T> a, int tlo, int thi, int fwd) {
-  __shared__ unsigned long long smin[256];
-  const StripeWalk *wp = a.walk;
-  int H = a.m;
+__global__ void stripe_min_kernel(StripeArgs<T> a, int slot, int tlo, int thi, int fwd) {
+  using U = typename CostBits<T>::U;
+  __shared__ U smin[256];
+  const StripeWalk *wp = a.walk + slot;
+  int H = a.mem[slot].m;
   if (!fwd) {
     if (wp->state != 0) return;
     H = wp->h;
     if ((long long)tlo * kRefSwath <= H || tlo >= wp->s_fwd) return;
   }
-  unsigned long long *slot = fwd ? a.fmin : a.cmin;
+  U *out = (fwd ? a.fmin : a.cmin) + slot * a.min_slot;
   for (int t = tlo + int(blockIdx.y); t <= thi; t += int(gridDim.y)) {
-    const T *e = stripe_edge_before(a, t * kRefSwath);
-    unsigned long long best = ~0ull;
+    const T *e = stripe_edge(a, slot, t);
+    U best = ~U(0);
     for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < H;
          r += (long long)gridDim.x * blockDim.x) {
       if (!shortcut_row<T>(int(r))) continue;
-      const unsigned long long b = cost_bits(e[r]);
+      const U b = CostBits<T>::of(e[r]);
       best = b < best ? b : best;
     }
     smin[threadIdx.x] = best;
@@ -1570,139 +1579,155 @@ __global__ void stripe_min_kernel(StripeArgs<T> a, int tlo, int thi, int fwd) {
         smin[threadIdx.x] = smin[threadIdx.x + s];
       __syncthreads();
     }
-    if (threadIdx.x == 0 && smin[0] != ~0ull) atomicMin(slot + t, smin[0]);
+    if (threadIdx.x == 0 && smin[0] != ~U(0)) atomicMin(out + t, smin[0]);
     __syncthreads();
   }
 }
 
 // The first stripe in [tlo, thi] whose forward shortcut fires (one warp).
 template <typename T>
-__global__ void stripe_sfwd_kernel(StripeArgs<T> a, int tlo, int thi) {
+__global__ void stripe_sfwd_kernel(StripeArgs<T> a, int slot, int tlo, int thi) {
   const int lane = threadIdx.x & 31;
   for (int t0 = tlo; t0 <= thi; t0 += 32) {
     const int t = t0 + lane;
     bool f = false;
-    if (t <= thi) f = cost_bits(stripe_edge_before(a, t * kRefSwath)[a.m - 1]) == a.fmin[t];
+    if (t <= thi)
+      f = CostBits<T>::of(stripe_edge(a, slot, t)[a.mem[slot].m - 1]) == a.fmin[slot * a.min_slot + t];
     const unsigned ballot = __ballot_sync(kFull, f);
     if (ballot) {
-      if (lane == 0) a.walk->s_fwd = t0 + __ffs(ballot) - 1;
+      if (lane == 0) a.walk[slot].s_fwd = t0 + __ffs(ballot) - 1;
       return;
     }
   }
 }
 
-template <typename T, int R>
-__device__ __forceinline__ T stripe_tile_swath(const SwathJob<T> &job, const PathOut &po,
-                                               const TileIn<T> &tile) {
-  T col[R];
-  T emin, etop;
-  sweep_swath_path<T, R>(job, po, col, emin, etop, tile);
-  return etop;
-}
-
-// One warp per K-row tile of swath s below the backtrack height, into move
-// buffer buf.
-template <typename T, int RF, int RQ>
-__global__ void __launch_bounds__(kRoundWarps * 32) stripe_tile_kernel(StripeArgs<T> a, int s, int buf) {
-  __shared__ __align__(16) T stage_mem[kRoundWarps * kStageElems];
-  constexpr int W = 32 * RF;
-  const int kt = blockIdx.x * kRoundWarps + (threadIdx.x >> 5);
-  const StripeWalk w = *a.walk;
-  const int H = w.h;
-  const int K = 1 << a.shift;
+// Block (kt, b, slot): the K-row tile kt of the group's b-th stripe, where it
+// lies below the backtrack height.
+template <typename T>
+__global__ void
+__launch_bounds__(kBlkThreads, sizeof(T) == 4 ? kRoundBlocksF32 : kRoundBlocksF64)
+    stripe_tile_kernel(StripeArgs<T> a, int group, int gi) {
+  __shared__ BlockSmem<T> sm;
+  const int kt = blockIdx.x, slot = blockIdx.z;
+  const StripeMember &mem = a.mem[slot];
+  int lo, hi;
+  stripe_group(mem.swaths, group, gi, lo, hi);
+  const int t = lo + int(blockIdx.y);
+  if (t >= hi) return;
+  const StripeWalk w = a.walk[slot];
+  const int H = w.h, K = 1 << a.shift;
   const long long rb_l = (long long)a.r0 + (long long)kt * K;
-  const int c0 = s * W;
-  if (w.state != 0 || rb_l >= H || stripe_fires(a, c0 / kRefSwath, H, w)) return;
-  const int rb = int(rb_l);
-  const int re = rb + K < H ? rb + K : H;
-  SwathJob<T> job;
-  job.x = stripe_rows_ptr(a);
-  job.y = stripe_cols_ptr(a);
+  if (w.state != 0 || rb_l >= H || stripe_fires(a, slot, t, H, w)) return;
+  const int rb = int(rb_l), re = rb + K < H ? rb + K : H;
+  const int c0 = t * kBlkCols;
+  BlockJob<T> job;
+  job.x = mem.flip ? a.centroid : stripe_member_ptr(a, slot);
+  job.y = mem.flip ? stripe_member_ptr(a, slot) : a.centroid;
   job.m = re;
-  job.n = a.n;
+  job.n = mem.n;
   job.c0 = c0;
   job.r0 = rb;
-  const T *left = s ? a.E + (unsigned long long)(s - 1) * a.e_stride : nullptr;
+  const T *left = t ? stripe_edge(a, slot, t) : nullptr;
   job.edge_in = left ? left + (unsigned long long)kt * K : nullptr;
   job.edge_out = nullptr;
   job.open_end = a.oe != 0;
-  job.free_diag0 = c0 > 0 && (c0 % kRefSwath) == 0;
+  job.free_diag0 = c0 > 0;
   job.corner_init = kt == 0 ? stripe_corner<T>(c0, a.r0)
                             : (left ? left[(unsigned long long)kt * K - 1] : Num<T>::big());
-  job.stage = stage_mem + (threadIdx.x >> 5) * kStageElems;
-  TileIn<T> tile;
-  tile.col_init = kt ? a.Q + (unsigned long long)(kt - 1) * a.q_stride + c0 : nullptr;
-  // the re-run's top row is the backtrack height's (open end), the last row otherwise
-  tile.top_row = a.oe ? H - 1 : a.m - 1;
-  tile.top_left = (a.oe && (c0 % kRefSwath) != 0) ? a.top_carry : nullptr;
-  PathOut po;
-  po.words = a.words + (unsigned long long)buf * a.words_stride + (unsigned long long)kt * (K / 2) * 64ull;
-  po.track_min = false;
-  const int R = stripe_regs<T>(a.n, s);
-  T etop = T(0);
-  if (R == RF) {
-    etop = stripe_tile_swath<T, RF>(job, po, tile);
-  } else {
-    switch (R / RQ) {
-#define ODBA_TCASE(K)                                                         \
-  case K:                                                                     \
-    if constexpr (K * RQ < RF) etop = stripe_tile_swath<T, K * RQ>(job, po, tile); \
-    break;
-      ODBA_TCASE(1)
-      ODBA_TCASE(2)
-      ODBA_TCASE(3)
-      ODBA_TCASE(4)
-      ODBA_TCASE(5)
-      ODBA_TCASE(6)
-      ODBA_TCASE(7)
-#undef ODBA_TCASE
-      default:
-        break;
-    }
-  }
-  // the first half of a two-swath stripe hands its recomputed top row's last
-  // value to the second half
-  if (a.oe && re == H && (c0 % kRefSwath) == 0 && c0 + W < a.n && W < kRefSwath &&
-      (threadIdx.x & 31) == 0)
-    *a.top_carry = etop;
+  // the re-run's top row is the backtrack height's (open end)
+  job.top_band = re == H;
+  job.row_in = kt ? a.Q + slot * a.q_slot + (unsigned long long)(kt - 1) * a.q_stride + c0 : nullptr;
+  const int steps = block_steps(mem.m - a.r0);
+  job.word_steps = steps;
+  job.words = a.words + slot * a.words_slot + (size_t)(t - lo) * kBlkWarps * steps * 32 +
+              (size_t)kt * (K / 2) * 32;
+  T unused = T(0);
+  EdgeStat<T> st;
+  sweep_block<T, true, true, false, false>(job, sm, NoGate(), CkptOut<T>{nullptr, 0, 1}, false,
+                                           unused, st);
 }
 
-__global__ void stripe_walk_init_kernel(StripeWalk *w, int m, int n) {
-  if (threadIdx.x || blockIdx.x) return;
-  w->r = m - 1;
-  w->c = n - 1;
-  w->h = m;
+template <typename T>
+__global__ void stripe_walk_init_kernel(StripeArgs<T> a) {
+  const int slot = threadIdx.x;
+  if (slot >= a.count || blockIdx.x) return;
+  StripeWalk *w = a.walk + slot;
+  w->r = a.mem[slot].m - 1;
+  w->c = a.mem[slot].n - 1;
+  w->h = a.mem[slot].m;
   w->cur_t = -1;
   w->lo = 1;
   w->hi = 0;
   w->state = 0;
   w->s_fwd = INT_MAX;
+  w->entry = a.mem[slot].n - 1;
   w->nt = 0;
 }
 
-// Continues the backtrack through swath s (updateCentroid's loop,
-// dba.hpp:393-421, with the stripe branch's height, dba.hpp:384-386) until it
-// leaves the swath to the left or reaches the start cell.  One warp: every
-// lane holds the move word of one of the 32 rows at and below the current
-// cell (the word of the lane that owns the current column), so the walk
-// advances by shuffles and reloads the window only when it leaves those 32
-// rows or that owner's columns.  Every lane keeps the same walk state; lane 0
-// does the stores.  The height moves to the walk's row when it leaves a
-// reference stripe (with an open end only then; a shorter re-run is the same
-// without one).
+// The row walk (walk_runs) through a group, one warp per member: without an
+// open end and without a path listing.
 template <typename T>
-__global__ void stripe_walk_kernel(StripeArgs<T> a, int s, int buf) {
-  const int lane = threadIdx.x & 31;
-  if (blockIdx.x) return;
-  StripeWalk w = *a.walk;
-  if (w.state) return;
-  constexpr int W = 32 * PathTune<T>::RF;
-  const int c0 = s * W, R = stripe_regs<T>(a.n, s);
-  const int os = a.r0;
-  const long long max_cells = (long long)a.m + a.n - 1;
-  const unsigned long long *words = a.words + (unsigned long long)buf * a.words_stride;
-  int2 *rg = a.ranges;
-  int32_t *tri = a.triples;
+__global__ void __launch_bounds__(32) stripe_walk_runs_kernel(StripeArgs<T> a, int group, int gi) {
+  const int lane = threadIdx.x, slot = blockIdx.x;
+  const StripeMember &mem = a.mem[slot];
+  int lo, hi;
+  stripe_group(mem.swaths, group, gi, lo, hi);
+  StripeWalk w = a.walk[slot];
+  if (w.state || hi <= lo) return;
+  MemberGeom g;
+  g.m = mem.m;
+  g.n = mem.n;
+  g.r0 = a.r0;
+  g.steps = block_steps(mem.m - a.r0);
+  RowWalk rw{w.r, w.c, w.entry};
+  const int got = walk_runs(reinterpret_cast<const unsigned short *>(a.words + slot * a.words_slot),
+                            g, lo * kBlkCols, rw, a.r0, a.runs + slot * a.runs_slot);
+  if (lane == 0) {
+    w.r = rw.r;
+    w.c = rw.c;
+    w.entry = rw.entry;
+    w.h = rw.r + 1;
+    w.state = got;
+    a.walk[slot] = w;
+  }
+}
+
+// The rows' intervals as ranges (runs_to_ranges; the member on the rows).
+template <typename T>
+__global__ void stripe_ranges_kernel(StripeArgs<T> a) {
+  const int slot = blockIdx.y;
+  if (a.walk[slot].state != 1) return;
+  runs_to_ranges(a.runs + slot * a.runs_slot,
+                 a.ranges + (unsigned long long)a.mem[slot].member * a.Lc, a.mem[slot].m, false,
+                 blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+}
+
+// Continues the backtrack cell by cell through a group (updateCentroid's loop,
+// dba.hpp:393-421, with the stripe branch's height, dba.hpp:384-386) until it
+// leaves the group to the left or reaches the start cell.  One warp per
+// member: every lane holds the moves of one of the 32 rows at and below the
+// current cell in a block of 32 columns, so the walk advances by shuffles and
+// reloads the window only when it leaves those rows or columns.  Every lane
+// keeps the same walk state; lane 0 does the stores.  The height moves to the
+// walk's row when it leaves a reference stripe.
+template <typename T>
+__global__ void __launch_bounds__(32) stripe_walk_kernel(StripeArgs<T> a, int group, int gi) {
+  const int lane = threadIdx.x, slot = blockIdx.x;
+  const StripeMember &mem = a.mem[slot];
+  int t_lo, t_hi;
+  stripe_group(mem.swaths, group, gi, t_lo, t_hi);
+  StripeWalk w = a.walk[slot];
+  if (w.state || t_hi <= t_lo) return;
+  const int os = a.r0, flip = mem.flip;
+  const long long max_cells = (long long)mem.m + mem.n - 1;
+  MemberGeom g;
+  g.r0 = a.r0;
+  g.steps = block_steps(mem.m - a.r0);
+  const unsigned short *words = reinterpret_cast<const unsigned short *>(a.words + slot * a.words_slot);
+  int2 *rg = a.ranges + (unsigned long long)mem.member * a.Lc;
+  int *extra = a.extra ? a.extra + (unsigned long long)mem.member * a.Lc : nullptr;
+  int32_t *tri = a.triples ? a.triples + 3ull * mem.trip : nullptr;
+  int64_t *tri_count = a.triple_counts ? a.triple_counts + mem.member : nullptr;
   const bool lead = lane == 0;
   // rr: the member's sample index, cc: the centroid index
   auto contribute = [&](int rr, int cc) {
@@ -1713,13 +1738,13 @@ __global__ void stripe_walk_kernel(StripeArgs<T> a, int s, int buf) {
       w.hi = rr;
     } else if (rr == w.lo - 1) {
       w.lo = rr;
-    } else if (lead && a.extra) {
+    } else if (lead && extra) {
       // past an OPEN_RIGHT run on a re-run's top row (centroid on the rows)
-      a.extra[cc] = rr;
+      extra[cc] = rr;
     }
   };
   auto contribute_cell = [&](int r, int c) {
-    if (a.flip)
+    if (flip)
       contribute(c, r);
     else
       contribute(r, c);
@@ -1732,96 +1757,75 @@ __global__ void stripe_walk_kernel(StripeArgs<T> a, int s, int buf) {
     }
     ++w.nt;
   };
-  const int H = w.h;
-  if (stripe_fires(a, c0 / kRefSwath, H, w)) {
-    // the re-run's shortcut: row H-1 of the stripe is OPEN_RIGHT throughout
-    for (; w.c >= c0; --w.c) {
-      if (w.nt >= max_cells - 1) {
-        w.state = 2;
-        break;
+  for (int t = t_hi - 1; t >= t_lo && w.state == 0; --t) {
+    const int H = w.h, c0 = t * kBlkCols;
+    if (stripe_fires(a, slot, t, H, w)) {
+      // the re-run's shortcut: row H-1 of the stripe is OPEN_RIGHT throughout
+      for (; w.c >= c0; --w.c) {
+        if (w.nt >= max_cells - 1) {
+          w.state = 2;
+          break;
+        }
+        emit(kMoveOpenRight);
       }
-      emit(kMoveOpenRight);
     }
-  }
-  bool swath_done = w.c < c0 || w.state != 0;
-  while (!swath_done && w.state == 0) {
-    // window: rows w.r - lane, columns of the owner lane of w.c
-    const int top = w.r, owner = (w.c - c0) / R, cbeg = c0 + owner * R;
-    unsigned long long word = 0;
-    const int my_row = top - lane;
-    if (my_row >= 1) {
-      const int rr = my_row - a.r0;
-      const unsigned long long t = (unsigned long long)owner + (rr >> 1);
-      word = words[(t * 32 + owner) * 2 + (rr & 1)];
-    }
-    for (;;) {
-      int mv;
-      const unsigned long long wv = __shfl_sync(kFull, word, (top - w.r) & 31);
-      if (w.r == 0) {
-        mv = w.c == 0 ? (os ? kMoveNilOpenRight : kMaxMoveNil) : (os ? kMoveOpenRight : kMoveRight);
-      } else {
-        mv = decode_move(wv, w.c - cbeg);
-        if (mv == kMoveRight && a.oe && w.r == H - 1) mv = kMoveOpenRight;
-      }
-      if (mv == kMaxMoveNil || mv == kMoveNilOpenRight) {
-        // the start cell (dba.hpp:412-415)
-        if (mv != kMoveNilOpenRight) contribute(0, 0);
-        if (lead && w.cur_t >= 0 && w.hi >= w.lo) rg[w.cur_t] = make_int2(w.lo, w.hi);
+    bool stripe_done = w.c < c0 || w.state != 0;
+    while (!stripe_done && w.state == 0) {
+      // window: rows w.r - lane, columns cbeg .. cbeg + 31
+      const int top = w.r, cbeg = w.c & ~31;
+      RowMoves mine{0u, 0u};
+      if (top - lane >= 1) mine = row_moves(words, g, top - lane, cbeg - t_lo * kBlkCols);
+      for (;;) {
+        int mv;
+        const unsigned rd = __shfl_sync(kFull, mine.d, (top - w.r) & 31);
+        const unsigned ru = __shfl_sync(kFull, mine.u, (top - w.r) & 31);
+        if (w.r == 0) {
+          mv = w.c == 0 ? (os ? kMoveNilOpenRight : kMaxMoveNil) : (os ? kMoveOpenRight : kMoveRight);
+        } else {
+          const int j = w.c - cbeg;
+          mv = ((rd >> j) & 1u) ? kMoveDiag : ((ru >> j) & 1u) ? kMoveUp : kMoveRight;
+          if (mv == kMoveRight && a.oe && w.r == H - 1) mv = kMoveOpenRight;
+        }
+        if (mv == kMaxMoveNil || mv == kMoveNilOpenRight) {
+          // the start cell (dba.hpp:412-415)
+          if (mv != kMoveNilOpenRight) contribute(0, 0);
+          if (lead && w.cur_t >= 0 && w.hi >= w.lo) rg[w.cur_t] = make_int2(w.lo, w.hi);
+          emit(mv);
+          if (lead && tri_count) *tri_count = w.nt;
+          w.state = 1;
+          break;
+        }
+        if (w.nt >= max_cells - 1) {
+          w.state = 2;
+          break;
+        }
         emit(mv);
-        if (lead && a.triple_count) *a.triple_count = w.nt;
-        w.state = 1;
-        break;
+        if (mv != kMoveOpenRight) contribute_cell(w.r, w.c);
+        if (mv == kMoveDiag) {
+          --w.r;
+          --w.c;
+        } else if (mv == kMoveUp) {
+          --w.r;
+        } else {
+          --w.c;
+        }
+        if (w.r < 0 || w.c < 0) {
+          w.state = 2;
+          break;
+        }
+        if (w.c < c0) {
+          stripe_done = true;
+          break;
+        }
+        if (top - w.r >= 32 || w.c < cbeg) break;  // reload the window
       }
-      if (w.nt >= max_cells - 1) {
-        w.state = 2;
-        break;
-      }
-      emit(mv);
-      if (mv != kMoveOpenRight) contribute_cell(w.r, w.c);
-      if (mv == kMoveDiag) {
-        --w.r;
-        --w.c;
-      } else if (mv == kMoveUp) {
-        --w.r;
-      } else {
-        --w.c;
-      }
-      if (w.r < 0 || w.c < 0) {
-        w.state = 2;
-        break;
-      }
-      if (w.c < c0) {
-        swath_done = true;
-        break;
-      }
-      if (top - w.r >= 32 || w.c < cbeg) break;  // reload the window
     }
+    if (w.state == 0 && w.c < c0) w.h = w.r + 1;
   }
-  if (w.state == 0 && w.c < c0 && (!a.oe || (c0 % kRefSwath) == 0)) w.h = w.r + 1;
   if (lead) {
-    if (w.state == 2 && a.triple_count) *a.triple_count = -1;
-    *a.walk = w;
+    if (w.state == 2 && tri_count) *tri_count = -1;
+    a.walk[slot] = w;
   }
-}
-
-template <typename T>
-int stripe_grid() {
-  static std::atomic<int> cached[64];  // per device; host threads may race (same value)
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev >= 0 && dev < 64) {
-    const int c = cached[dev].load(std::memory_order_relaxed);
-    if (c) return c;
-  }
-  int sms = 0, per_sm = 0;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-      &per_sm, stripe_forward_kernel<T, PathTune<T>::RF, PathTune<T>::RQ, false, false>,
-      kRoundWarps * 32, 0);
-  if (per_sm < 1) per_sm = 1;
-  const int g = sms * per_sm;
-  if (dev >= 0 && dev < 64) cached[dev].store(g, std::memory_order_relaxed);
-  return g;
 }
 
 // One member's matrix: rows x columns in the round's orientation.
@@ -1839,15 +1843,15 @@ inline StripeDims stripe_dims(uint64_t len, uint64_t Lc, int oe) {
 
 struct StripeLayout {
   RoundLayout round;
-  size_t off_head, off_prog, off_E, off_Q, off_W, off_min, off_extra, total;
-  unsigned long long e_stride, q_stride, words_stride;
-  int swaths_max, stripes_max;
+  size_t off_head, off_prog, off_E, off_Q, off_W, off_runs, off_min, off_extra, total;
+  unsigned long long e_stride, q_stride, words_slot, e_slot, q_slot, runs_slot, min_slot;
+  int swaths_max;
+  int slots, group;
 };
 
 template <typename T>
 StripeLayout stripe_layout(const uint64_t *h_lens, int n, uint64_t Lc, int os, int oe, int shift) {
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
-  constexpr int W = 32 * PathTune<T>::RF;
   uint64_t max_rows = 1, max_cols = 1;
   for (int k = 0; k < n; ++k) {
     const StripeDims d = stripe_dims(h_lens[k], Lc, oe);
@@ -1856,23 +1860,36 @@ StripeLayout stripe_layout(const uint64_t *h_lens, int n, uint64_t Lc, int os, i
   }
   StripeLayout S;
   S.round = round_layout<T>(n, 1, 0, (unsigned long long)n * Lc, 1);
-  S.swaths_max = int((max_cols + W - 1) / W);
-  S.stripes_max = int((max_cols + kRefSwath - 1) / kRefSwath);
+  S.swaths_max = int((max_cols + kBlkCols - 1) / kBlkCols);
   S.e_stride = (max_rows + 64 + 31) / 32 * 32;
-  S.q_stride = (unsigned long long)S.swaths_max * W;
+  S.q_stride = (unsigned long long)S.swaths_max * kBlkCols;
   const unsigned long long K = 1ull << shift;
   const unsigned long long nq = (max_rows - (os ? 1 : 0)) / K + 1;
-  const unsigned long long steps = (max_rows + 1) / 2 + 32;
-  S.words_stride = steps * 64;
-  const int bufs = (oe && W < kRefSwath) ? 2 : 1;
+  S.e_slot = (unsigned long long)(S.swaths_max > 1 ? S.swaths_max - 1 : 1) * S.e_stride;
+  S.q_slot = nq * S.q_stride;
+  const size_t slot_bytes = size_t(S.e_slot + S.q_slot) * sizeof(T);
+  int slots = (kStripeFill + S.swaths_max - 1) / S.swaths_max;
+  if (slots > kStripeSlots) slots = kStripeSlots;
+  if (slots > n) slots = n;
+  while (slots > 1 && slot_bytes * slots > kStripeSlotBytes) --slots;
+  S.slots = slots;
+  const size_t stripe_bytes = size_t(kBlkWarps) * block_steps(int(max_rows)) * 32 * 4;
+  int group = S.swaths_max < kStripeGroup ? S.swaths_max : kStripeGroup;
+  while (group > 1 && stripe_bytes * group * slots > kStripeGroupBytes) --group;
+  S.group = group;
+  S.words_slot = stripe_bytes / 4 * group;
+  S.runs_slot = max_rows;
+  S.min_slot = (unsigned long long)S.swaths_max + 1;
   size_t o = S.round.total;
-  S.off_head = o; o += 256;
-  S.off_prog = o; o += up(size_t(S.swaths_max) * 8);
-  S.off_E = o; o += up(size_t(S.swaths_max > 1 ? S.swaths_max - 1 : 1) * S.e_stride * sizeof(T));
-  S.off_Q = o; o += up(size_t(nq) * S.q_stride * sizeof(T));
-  S.off_W = o; o += up(size_t(bufs) * S.words_stride * 8);
-  S.off_min = o; o += up(size_t(2) * (S.stripes_max + 1) * 8);
+  S.off_head = o; o += 1024;
+  S.off_prog = o; o += up(size_t(slots) * S.swaths_max * 8);
+  S.off_E = o; o += up(size_t(slots) * S.e_slot * sizeof(T));
+  S.off_Q = o; o += up(size_t(slots) * S.q_slot * sizeof(T));
+  S.off_W = o; o += up(size_t(slots) * S.words_slot * 4);
+  S.off_runs = o; o += up(size_t(slots) * S.runs_slot * sizeof(int2));
+  // with an open end: the extra samples, and the shortcut minima of every stripe
   S.off_extra = o; o += oe ? up(size_t(n) * Lc * 4) : 0;
+  S.off_min = o; o += oe ? (size_t(2) * slots * S.min_slot * sizeof(T) + 63) / 64 * 64 : 0;
   S.total = o;
   return S;
 }
@@ -1907,30 +1924,9 @@ int dba_round_stripe_launch(const T *centroid, uint64_t Lc, const T *series,
   if (ws_bytes < S.total) return fail(ODBA_ERR_WORKSPACE_TOO_SMALL, "stripe DBA round workspace too small");
   const RoundLayout &L = S.round;
   char *base = static_cast<char *>(ws);
-  int *single = reinterpret_cast<int *>(base + L.off_single);
-  int *mseries = single, *mjob = single + n, *d_clen = single + 2 * n, *d_flags = single + 2 * n + 1,
-      *d_mbeg = single + 2 * n + 2, *d_mend = single + 2 * n + 3;
-  unsigned long long *d_coff =
-      reinterpret_cast<unsigned long long *>(base + L.off_single + ((size_t(2 * n + 4) * 4 + 7) / 8) * 8);
   const int flags = (os ? 1 : 0) | (oe ? 2 : 0) | 4;
-  single_job_kernel<<<(n + 255) / 256, 256, 0, stream>>>(mseries, mjob, n, d_clen, int(Lc), d_flags,
-                                                        flags, d_mbeg, d_mend, d_coff);
   int *extra = oe ? reinterpret_cast<int *>(base + S.off_extra) : nullptr;
-  RoundArgs<T> a;
-  a.centroids = centroid;
-  a.coff = d_coff;
-  a.clen = d_clen;
-  a.jflags = d_flags;
-  a.mbeg = d_mbeg;
-  a.mend = d_mend;
-  a.njobs = 1;
-  a.series = series;
-  a.offsets = offsets;
-  a.lens = lens;
-  a.mseries = mseries;
-  a.mjob = mjob;
-  a.order = nullptr;
-  a.nmem = n;
+  RoundArgs<T> a = single_job_round<T>(centroid, Lc, series, offsets, lens, n, flags, L, base, stream);
   a.means = mean;
   a.counts = counts;
   a.deltas = delta;
@@ -1952,92 +1948,100 @@ int dba_round_stripe_launch(const T *centroid, uint64_t Lc, const T *series,
   if (extra) cudaMemsetAsync(extra, 0xff, size_t(nr) * 4, stream);
   if (int rc = check_launch("stripe DBA round set-up")) return rc;
 
-  constexpr int RF = PathTune<T>::RF, RQ = PathTune<T>::RQ;
-  constexpr int W = 32 * RF;
-  constexpr int kPerStripe = kRefSwath / W;  // swaths per reference stripe
   char *head = base + S.off_head;
   StripeArgs<T> sa;
   sa.series = series;
   sa.offsets = offsets;
   sa.centroid = centroid;
+  sa.Lc = int(Lc);
   sa.r0 = os ? 1 : 0;
   sa.oe = oe ? 1 : 0;
   sa.shift = sh;
   sa.E = reinterpret_cast<T *>(base + S.off_E);
   sa.e_stride = S.e_stride;
+  sa.e_slot = S.e_slot;
   sa.Q = reinterpret_cast<T *>(base + S.off_Q);
   sa.q_stride = S.q_stride;
+  sa.q_slot = S.q_slot;
   sa.prog = reinterpret_cast<unsigned long long *>(base + S.off_prog);
+  sa.prog_slot = (unsigned long long)S.swaths_max;
+  sa.words = reinterpret_cast<unsigned *>(base + S.off_W);
+  sa.words_slot = S.words_slot;
+  sa.runs = reinterpret_cast<int2 *>(base + S.off_runs);
+  sa.runs_slot = S.runs_slot;
+  sa.fmin = oe ? reinterpret_cast<typename CostBits<T>::U *>(base + S.off_min) : nullptr;
+  sa.min_slot = S.min_slot;
+  sa.cmin = oe ? sa.fmin + S.slots * S.min_slot : nullptr;
   sa.counter = reinterpret_cast<unsigned long long *>(head);
+  sa.walk = reinterpret_cast<StripeWalk *>(head + 64);
   // the wait error word is byte 8 of the workspace, as in the full-path round
   sa.err = reinterpret_cast<unsigned *>(base + L.off_counter + 8);
   cudaMemsetAsync(base + L.off_counter, 0, 16, stream);
-  sa.walk = reinterpret_cast<StripeWalk *>(head + 64);
-  sa.top_carry = reinterpret_cast<T *>(head + 192);
-  sa.words = reinterpret_cast<unsigned long long *>(base + S.off_W);
-  sa.words_stride = S.words_stride;
-  sa.fmin = reinterpret_cast<unsigned long long *>(base + S.off_min);
-  sa.cmin = sa.fmin + (S.stripes_max + 1);
+  sa.ranges = a.ranges;
+  sa.extra = extra;
+  sa.triples = triples;
+  sa.triple_counts = triple_counts;
   sa.limit_ns = kWaitLimitNs;
+  static_assert(64 + kStripeSlots * sizeof(StripeWalk) <= 1024, "walk states fit the header");
   const bool check_short = oe && !os;
+  const bool by_rows = !oe && !triples;
   const int K = 1 << sh;
+  const int group = oe ? 1 : S.group;
   unsigned long long trip = 0;
-  for (int k = 0; k < n; ++k) {
-    const StripeDims d = stripe_dims(h_lens[k], Lc, oe);
-    const int m = int(d.rows), ncols = int(d.cols);
-    const int swaths = (ncols + W - 1) / W;
-    const int stripes = (ncols + kRefSwath - 1) / kRefSwath;
-    sa.member = k;
-    sa.flip = d.flip;
-    sa.m = m;
-    sa.n = ncols;
-    sa.swaths = swaths;
-    sa.ranges = a.ranges + (unsigned long long)k * Lc;
-    sa.extra = extra ? extra + (unsigned long long)k * Lc : nullptr;
-    sa.triples = triples ? triples + 3ull * trip : nullptr;
-    sa.triple_count = triple_counts ? triple_counts + k : nullptr;
-    trip += h_lens[k] + Lc + 1;
-    cudaMemsetAsync(head, 0, 64, stream);
-    cudaMemsetAsync(sa.prog, 0, size_t(swaths) * 8, stream);
-    if (check_short) cudaMemsetAsync(sa.fmin, 0xff, size_t(2) * (S.stripes_max + 1) * 8, stream);
-    stripe_walk_init_kernel<<<1, 32, 0, stream>>>(sa.walk, m, ncols);
-    const int fgrid = swaths < stripe_grid<T>() * kRoundWarps ? (swaths + kRoundWarps - 1) / kRoundWarps
-                                                              : stripe_grid<T>();
-    if (!oe)
-      stripe_forward_kernel<T, RF, RQ, false, false><<<fgrid, kRoundWarps * 32, 0, stream>>>(sa);
-    else if (!d.flip)
-      stripe_forward_kernel<T, RF, RQ, true, false><<<fgrid, kRoundWarps * 32, 0, stream>>>(sa);
-    else
-      stripe_forward_kernel<T, RF, RQ, true, true><<<fgrid, kRoundWarps * 32, 0, stream>>>(sa);
-    // stripes past the last row: where the forward pass's shortcut fired first
-    const int tlo = m / kRefSwath + 1, thi = stripes - 1;
-    const int gx = (m + 2047) / 2048 < 64 ? (m + 2047) / 2048 : 64;
-    if (check_short && tlo <= thi) {
-      const int gy = thi - tlo + 1 < 1024 ? thi - tlo + 1 : 1024;
-      stripe_min_kernel<T><<<dim3(gx, gy), 256, 0, stream>>>(sa, tlo, thi, 1);
-      stripe_sfwd_kernel<T><<<1, 32, 0, stream>>>(sa, tlo, thi);
+  for (int k0 = 0; k0 < n; k0 += S.slots) {
+    sa.count = n - k0 < S.slots ? n - k0 : S.slots;
+    int max_swaths = 0, max_m = 0;
+    unsigned long long all_swaths = 0;
+    for (int i = 0; i < sa.count; ++i) {
+      const StripeDims d = stripe_dims(h_lens[k0 + i], Lc, oe);
+      StripeMember &mem = sa.mem[i];
+      mem.member = k0 + i;
+      mem.flip = d.flip;
+      mem.m = int(d.rows);
+      mem.n = int(d.cols);
+      mem.swaths = (mem.n + kBlkCols - 1) / kBlkCols;
+      mem.trip = trip;
+      trip += h_lens[k0 + i] + Lc + 1;
+      max_swaths = mem.swaths > max_swaths ? mem.swaths : max_swaths;
+      max_m = mem.m > max_m ? mem.m : max_m;
+      all_swaths += mem.swaths;
     }
-    const int tiles = (m - sa.r0 + K - 1) / K;
-    const int tgrid = ((tiles > 1 ? tiles : 1) + kRoundWarps - 1) / kRoundWarps;
-    auto tile = [&](int s, int buf) {
-      stripe_tile_kernel<T, RF, RQ><<<tgrid, kRoundWarps * 32, 0, stream>>>(sa, s, buf);
-    };
-    auto walk = [&](int s, int buf) { stripe_walk_kernel<T><<<1, 32, 0, stream>>>(sa, s, buf); };
-    for (int t = stripes - 1; t >= 0; --t) {
-      if (check_short && t >= 1) stripe_min_kernel<T><<<dim3(gx, 1), 256, 0, stream>>>(sa, t, t, 0);
-      const int s_lo = t * kPerStripe;
-      const int s_hi = s_lo + kPerStripe - 1 < swaths - 1 ? s_lo + kPerStripe - 1 : swaths - 1;
-      if (oe && s_hi > s_lo) {
-        // the second half continues the first half's recomputed top row
-        for (int s = s_lo; s <= s_hi; ++s) tile(s, s - s_lo);
-        for (int s = s_hi; s >= s_lo; --s) walk(s, s - s_lo);
-      } else {
-        for (int s = s_hi; s >= s_lo; --s) {
-          tile(s, 0);
-          walk(s, 0);
-        }
+    cudaMemsetAsync(head, 0, 64, stream);
+    cudaMemsetAsync(sa.prog, 0, size_t(S.slots) * S.swaths_max * 8, stream);
+    if (check_short)
+      cudaMemsetAsync(sa.fmin, 0xff, size_t(2) * S.slots * S.min_slot * sizeof(T), stream);
+    stripe_walk_init_kernel<T><<<1, 32, 0, stream>>>(sa);
+    const int resident = round_grid<T>();
+    const int fgrid = all_swaths < (unsigned long long)resident ? int(all_swaths) : resident;
+    stripe_forward_kernel<T><<<fgrid, kBlkThreads, 0, stream>>>(sa, max_swaths);
+    auto min_blocks = [](int m) { return (m + 2047) / 2048 < 64 ? (m + 2047) / 2048 : 64; };
+    if (check_short) {
+      // stripes past the last row: where the forward pass's shortcut fired first
+      for (int i = 0; i < sa.count; ++i) {
+        const int tlo = sa.mem[i].m / kRefSwath + 1, thi = sa.mem[i].swaths - 1;
+        if (tlo > thi) continue;
+        const int gy = thi - tlo + 1 < 1024 ? thi - tlo + 1 : 1024;
+        stripe_min_kernel<T><<<dim3(min_blocks(sa.mem[i].m), gy), 256, 0, stream>>>(sa, i, tlo, thi, 1);
+        stripe_sfwd_kernel<T><<<1, 32, 0, stream>>>(sa, i, tlo, thi);
       }
     }
+    const int tiles = (max_m - sa.r0 + K - 1) / K > 0 ? (max_m - sa.r0 + K - 1) / K : 1;
+    for (int gi = 0; gi * group < max_swaths; ++gi) {
+      if (check_short)
+        for (int i = 0; i < sa.count; ++i) {
+          const int t = sa.mem[i].swaths - 1 - gi;
+          // (rows below H reach a stripe's shortcut only past column H)
+          if (t >= 1) stripe_min_kernel<T><<<dim3(min_blocks(sa.mem[i].m), 1), 256, 0, stream>>>(sa, i, t, t, 0);
+        }
+      stripe_tile_kernel<T><<<dim3(tiles, group, sa.count), kBlkThreads, 0, stream>>>(sa, group, gi);
+      if (by_rows)
+        stripe_walk_runs_kernel<T><<<sa.count, 32, 0, stream>>>(sa, group, gi);
+      else
+        stripe_walk_kernel<T><<<sa.count, 32, 0, stream>>>(sa, group, gi);
+    }
+    if (by_rows)
+      stripe_ranges_kernel<T><<<dim3((max_m + 255) / 256 < 256 ? (max_m + 255) / 256 : 256, sa.count), 256,
+                                0, stream>>>(sa);
     if (int rc = check_launch("stripe DBA round member kernels")) return rc;
   }
   dim3 rg((unsigned(Lc) + kReduceWarps - 1) / kReduceWarps, 1);

@@ -127,6 +127,18 @@ __device__ __forceinline__ void wait_count(const int *p, int v, int more, unsign
   __syncwarp();
 }
 
+// Row checkpoints (the stripe-mode forward pass): the full cost row
+// r = r0 + k*K - 1 (k >= 1, K = 2^shift >= 2) of this swath's columns is
+// stored at q + (k - 1) * stride + (c - c0) -- q points at this swath's first
+// column.  K is even, so these rows are always the second row of a lane's
+// step pair.
+template <typename T>
+struct CkptOut {
+  T *q;
+  unsigned long long stride;
+  int shift;
+};
+
 // One swath for one block (see SwathJob for the matrix convention).
 template <typename T>
 struct BlockJob {

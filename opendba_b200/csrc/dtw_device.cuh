@@ -314,26 +314,13 @@ struct NoGate {
 };
 constexpr int kPublishSteps = 64;  // lane 31 publishes every 64 steps (128 rows)
 
-// Row checkpoints (the stripe-mode forward pass): the full cost row
-// r = r0 + k*K - 1 (k >= 1, K = 2^shift >= 2) of this swath's columns is
-// stored at q + (k - 1) * stride + (c - c0) -- q points at this swath's first
-// column.  K is even, so these rows are always the second row of a lane's
-// step pair.
-template <typename T>
-struct CkptOut {
-  T *q;
-  unsigned long long stride;
-  int shift;
-};
-
 // Sweeps one swath.  On return col[] holds, per lane, the costs of the last
 // row m-1 at the lane's columns.  Swath-edge buffers are indexed by r - r0,
 // two rows per 8/16-byte access.  Returns the right edge's EdgeStat (lane 31;
 // the big value unless TRACK and job.track).
-template <typename T, int R, typename Gate = NoGate, bool CKPT = false, bool TRACK = true>
+template <typename T, int R, typename Gate = NoGate, bool TRACK = true>
 __device__ __forceinline__ EdgeStat<T> sweep_swath(const SwathJob<T> &job, T (&col)[R],
-                                                   Gate gate = Gate(),
-                                                   CkptOut<T> ckpt = CkptOut<T>{nullptr, 0, 1}) {
+                                                   Gate gate = Gate()) {
   using V2 = typename Pair2<T>::V;
   const int lane = threadIdx.x & 31;
   const int m = job.m;
@@ -381,15 +368,6 @@ __device__ __forceinline__ EdgeStat<T> sweep_swath(const SwathJob<T> &job, T (&c
     }
   };
 
-  auto store_ckpt = [&](int ra) {
-    const int kk = ra - r0 + 2;
-    if ((kk & ((1 << ckpt.shift) - 1)) == 0) {
-      T *dst = ckpt.q + (unsigned long long)((kk >> ckpt.shift) - 1) * ckpt.stride + lane * R;
-#pragma unroll
-      for (int j = 0; j < R; ++j) dst[j] = col[j];
-    }
-  };
-
   auto masked_step = [&](int t) {
     const int ra = r0 + 2 * (t - lane);
     T xa = __shfl_up_sync(kFull, xa_cur, 1);
@@ -416,7 +394,6 @@ __device__ __forceinline__ EdgeStat<T> sweep_swath(const SwathJob<T> &job, T (&c
       if (act_a) note(ra, a_last);
       if (act_b) note(ra + 1, col[R - 1]);
     }
-    if (CKPT && act_b) store_ckpt(ra);
   };
 
   // chunk c of lane 0's rows (k = ra - r0 in [64c, 64c + 64)) into slot c % 2;
@@ -509,7 +486,6 @@ __device__ __forceinline__ EdgeStat<T> sweep_swath(const SwathJob<T> &job, T (&c
       a_last = step_rows2_steady<T, R>(col, yv, xa, xb, la, lb, diag);
       xa_cur = xa;
       xb_cur = xb;
-      if (CKPT) store_ckpt(r0 + 2 * (t - lane));
       if (has_out) {
         if (lane31) {
           V2 v;

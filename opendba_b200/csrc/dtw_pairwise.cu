@@ -185,7 +185,7 @@ template <typename T, int R, bool TRACK>
 __device__ __forceinline__ EdgeStat<T> pipe_swath(const SwathJob<T> &job, const PipeGate &gate,
                                                   bool last, T &corner) {
   T col[R];
-  const EdgeStat<T> st = sweep_swath<T, R, PipeGate, false, TRACK>(job, col, gate);
+  const EdgeStat<T> st = sweep_swath<T, R, PipeGate, TRACK>(job, col, gate);
   if (last) corner = pick_column<T, R>(col, job.c0, job.n - 1);
   return st;
 }

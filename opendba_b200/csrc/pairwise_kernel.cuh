@@ -70,7 +70,7 @@ __device__ __forceinline__ T pair_distance(T corner, int m, int n, int os, int o
 template <typename T, int R, bool TRACK>
 __device__ __forceinline__ EdgeStat<T> run_swath(const SwathJob<T> &job, bool last, T &corner) {
   T col[R];
-  const EdgeStat<T> st = sweep_swath<T, R, NoGate, false, TRACK>(job, col);
+  const EdgeStat<T> st = sweep_swath<T, R, NoGate, TRACK>(job, col);
   if (last) corner = pick_column<T, R>(col, job.c0, job.n - 1);
   return st;
 }
