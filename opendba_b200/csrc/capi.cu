@@ -4,6 +4,7 @@
 
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 #include "odba_internal.h"
@@ -17,6 +18,53 @@ thread_local char g_err[512] = "";
 int fail(int status, const char *msg) {
   std::snprintf(g_err, sizeof(g_err), "%s", msg);
   return status;
+}
+
+namespace {
+constexpr uint64_t kScratchKeepBytes = uint64_t(256) << 20;
+constexpr int kScratchDevices = 64;
+
+// The current device's scratch pool, or null (no stream-ordered pools).
+cudaMemPool_t scratch_pool() {
+  static std::mutex mu;
+  static cudaMemPool_t pools[kScratchDevices] = {};
+  static bool tried[kScratchDevices] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kScratchDevices) return nullptr;
+  std::lock_guard<std::mutex> g(mu);
+  if (!tried[dev]) {
+    tried[dev] = true;
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    if (cudaMemPoolCreate(&pools[dev], &props) == cudaSuccess) {
+      uint64_t keep = kScratchKeepBytes;
+      cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep);
+    } else {
+      cudaGetLastError();
+      pools[dev] = nullptr;
+    }
+  }
+  return pools[dev];
+}
+}  // namespace
+
+cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t stream) {
+  const cudaMemPool_t pool = scratch_pool();
+  if (!pool) return cudaMallocAsync(p, bytes, stream);
+  cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, stream);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    cudaStreamSynchronize(stream);
+    cudaMemPoolTrimTo(pool, 0);
+    e = cudaMallocFromPoolAsync(p, bytes, pool, stream);
+  }
+  return e;
+}
+
+void scratch_free(void *p, cudaStream_t stream) {
+  if (p) cudaFreeAsync(p, stream);
 }
 
 int check_launch(const char *what) {
@@ -96,32 +144,33 @@ int medoid_pass_host(const T *h_series, const uint64_t *h_lens, int n, int os, i
   }
   const size_t npairs = size_t(n) * (n - 1) / 2;
   const size_t ws_bytes = pairwise_workspace_bytes_n<T>(npairs, max_len);
-  // one device allocation: series | offsets | lens | dists | sos | means | sigmas | medoid | workspace
+  // one device allocation: series | offsets, lens | dists | sos | means, sigmas | medoid |
+  // workspace; the figures from the means to the workspace's error word come
+  // back in one copy
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
-  const size_t b_series = up((total + 16) * sizeof(T)), b_meta = up(n * sizeof(uint64_t)),
+  const size_t b_series = up((total + 16) * sizeof(T)), b_meta = up(2 * n * sizeof(uint64_t)),
                b_d = up((npairs + 1) * sizeof(T)), b_sos = up(n * sizeof(T)),
-               b_mv = up(n * sizeof(double)), b_med = 256;
-  const size_t bytes = b_series + 2 * b_meta + b_d + b_sos + 2 * b_mv + b_med + ws_bytes;
+               b_mv = up(2 * n * sizeof(double)), b_med = 256;
+  const size_t o_meta = b_series, o_d = o_meta + b_meta, o_sos = o_d + b_d, o_mv = o_sos + b_sos,
+               o_med = o_mv + b_mv, o_ws = o_med + b_med;
   char *base = nullptr;
-  ODBA_CUDA(cudaMallocAsync(reinterpret_cast<void **>(&base), bytes, stream), "device allocation");
+  ODBA_CUDA(scratch_alloc(reinterpret_cast<void **>(&base), o_ws + ws_bytes, stream), "device allocation");
   T *d_series = reinterpret_cast<T *>(base);
-  uint64_t *d_offs = reinterpret_cast<uint64_t *>(base + b_series);
-  uint64_t *d_lens = reinterpret_cast<uint64_t *>(base + b_series + b_meta);
-  T *d_dists = reinterpret_cast<T *>(base + b_series + 2 * b_meta);
-  T *d_sos = reinterpret_cast<T *>(base + b_series + 2 * b_meta + b_d);
-  double *d_means = reinterpret_cast<double *>(base + b_series + 2 * b_meta + b_d + b_sos);
-  double *d_sigmas = d_means + b_mv / sizeof(double);
-  int *d_medoid = reinterpret_cast<int *>(base + b_series + 2 * b_meta + b_d + b_sos + 2 * b_mv);
-  void *d_ws = base + b_series + 2 * b_meta + b_d + b_sos + 2 * b_mv + b_med;
-  int rc = ODBA_OK;
-  unsigned wait_err = 0;
+  uint64_t *d_offs = reinterpret_cast<uint64_t *>(base + o_meta);
+  uint64_t *d_lens = d_offs + n;
+  T *d_dists = reinterpret_cast<T *>(base + o_d);
+  T *d_sos = reinterpret_cast<T *>(base + o_sos);
+  double *d_means = reinterpret_cast<double *>(base + o_mv);
+  double *d_sigmas = d_means + n;
+  int *d_medoid = reinterpret_cast<int *>(base + o_med);
+  void *d_ws = base + o_ws;
+  offs.insert(offs.end(), h_lens, h_lens + n);
+  std::vector<char> figures(o_ws + 16 - o_mv);
   auto run = [&]() -> int {
     ODBA_CUDA(cudaMemcpyAsync(d_series, h_series, total * sizeof(T), cudaMemcpyHostToDevice, stream),
               "series upload");
-    ODBA_CUDA(cudaMemcpyAsync(d_offs, offs.data(), n * sizeof(uint64_t), cudaMemcpyHostToDevice, stream),
-              "offsets upload");
-    ODBA_CUDA(cudaMemcpyAsync(d_lens, h_lens, n * sizeof(uint64_t), cudaMemcpyHostToDevice, stream),
-              "lengths upload");
+    ODBA_CUDA(cudaMemcpyAsync(d_offs, offs.data(), 2 * n * sizeof(uint64_t), cudaMemcpyHostToDevice, stream),
+              "offsets and lengths upload");
     if (norm) {
       if (int r = znorm_launch<T>(d_series, d_offs, d_lens, n, d_means, d_sigmas, stream)) return r;
     }
@@ -134,25 +183,20 @@ int medoid_pass_host(const T *h_series, const uint64_t *h_lens, int n, int os, i
     if (n >= 2)
       ODBA_CUDA(cudaMemcpyAsync(h_dists, d_dists, npairs * sizeof(T), cudaMemcpyDeviceToHost, stream),
                 "distance download");
-    ODBA_CUDA(cudaMemcpyAsync(h_medoid, d_medoid, sizeof(int), cudaMemcpyDeviceToHost, stream),
-              "medoid download");
-    if (norm && h_means)
-      ODBA_CUDA(cudaMemcpyAsync(h_means, d_means, n * sizeof(double), cudaMemcpyDeviceToHost, stream),
-                "means download");
-    if (norm && h_sigmas)
-      ODBA_CUDA(cudaMemcpyAsync(h_sigmas, d_sigmas, n * sizeof(double), cudaMemcpyDeviceToHost, stream),
-                "sigmas download");
-    if (n >= 2)
-      ODBA_CUDA(cudaMemcpyAsync(&wait_err, static_cast<char *>(d_ws) + 8, sizeof(unsigned),
-                                cudaMemcpyDeviceToHost, stream),
-                "error word download");
+    ODBA_CUDA(cudaMemcpyAsync(figures.data(), base + o_mv, n >= 2 ? figures.size() : o_ws - o_mv,
+                              cudaMemcpyDeviceToHost, stream),
+              "medoid, means and sigmas download");
     ODBA_CUDA(cudaStreamSynchronize(stream), "medoid pass");
+    std::memcpy(h_medoid, figures.data() + (o_med - o_mv), sizeof(int));
+    if (norm && h_means) std::memcpy(h_means, figures.data(), n * sizeof(double));
+    if (norm && h_sigmas) std::memcpy(h_sigmas, figures.data() + n * sizeof(double), n * sizeof(double));
+    unsigned wait_err = 0;
+    if (n >= 2) std::memcpy(&wait_err, figures.data() + (o_ws - o_mv) + 8, sizeof wait_err);
     if (wait_err) return fail(ODBA_ERR_TIMEOUT, "a swath hand-off wait ran out in the pair kernel");
     return ODBA_OK;
   };
-  rc = run();
-  cudaFreeAsync(base, stream);
-  if (rc == ODBA_OK) ODBA_CUDA(cudaStreamSynchronize(stream), "medoid pass teardown");
+  const int rc = run();
+  scratch_free(base, stream);
   return rc;
 }
 

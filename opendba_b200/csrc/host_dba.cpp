@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "opendba.hpp"
+#include "odba_internal.h"
 #include "opendba_b200.h"
 #include "text_parse.h"
 
@@ -168,21 +169,32 @@ struct DevBuf {
   void *p = nullptr;
   size_t bytes = 0;
   explicit DevBuf(size_t b = 0) { resize(b); }
+  // Scratch in the order of one stream, which all its uses must be on.
+  DevBuf(size_t b, cudaStream_t stream) : st(stream), scratch(true) { resize(b); }
   void resize(size_t b) {
     if (b <= bytes && p) return;
-    if (p) cudaFree(p);
-    p = nullptr;
-    bytes = 0;
+    release();
     if (b) {
-      check_cuda(cudaMalloc(&p, b), "device allocation in the host façade");
+      check_cuda(scratch ? odba::scratch_alloc(&p, b, st) : cudaMalloc(&p, b),
+                 "device allocation in the host façade");
       bytes = b;
     }
   }
-  ~DevBuf() {
-    if (p) cudaFree(p);
-  }
+  ~DevBuf() { release(); }
   DevBuf(const DevBuf &) = delete;
   DevBuf &operator=(const DevBuf &) = delete;
+
+ private:
+  cudaStream_t st = nullptr;
+  bool scratch = false;
+  void release() {
+    if (p && scratch)
+      odba::scratch_free(p, st);
+    else if (p)
+      cudaFree(p);
+    p = nullptr;
+    bytes = 0;
+  }
 };
 
 template <typename U>
@@ -198,8 +210,41 @@ struct DeviceSet {
   int n = 0;
   uint64_t max_len = 0, total = 0;
 
+  DeviceSet() = default;
+  explicit DeviceSet(cudaStream_t scratch) : data(0, scratch), offs(0, scratch), lens(0, scratch) {}
+
   // Copies sequences[i][0..lens[i]) from any memory space.
   void upload(T *const *sequences, const size_t *lengths, int count, cudaStream_t st) {
+    layout(lengths, count);
+    for (int i = 0; i < n; ++i)
+      check_cuda(cudaMemcpyAsync(ptr<T>(data) + h_offs[i], sequences[i], lengths[i] * sizeof(T),
+                                 cudaMemcpyDefault, st),
+                 "series upload");
+    upload_meta(st);
+  }
+
+  // The same for series in host memory: short ones are packed first, since a
+  // copy of a few kilobytes costs about as much as its call.
+  void upload_host(T *const *sequences, const size_t *lengths, int count, cudaStream_t st) {
+    constexpr size_t kPackBytes = size_t(64) << 20;
+    size_t bytes = 0;
+    for (int i = 0; i < count; ++i) bytes += lengths[i] * sizeof(T);
+    if (count < 2 || bytes > kPackBytes) {
+      upload(sequences, lengths, count, st);
+      return;
+    }
+    layout(lengths, count);
+    std::vector<T> packed(total);
+    for (int i = 0; i < n; ++i)
+      std::memcpy(packed.data() + h_offs[i], sequences[i], lengths[i] * sizeof(T));
+    // (pageable: the copy has left the host buffer when the call returns)
+    check_cuda(cudaMemcpyAsync(data.p, packed.data(), total * sizeof(T), cudaMemcpyHostToDevice, st),
+               "series upload");
+    upload_meta(st);
+  }
+
+ private:
+  void layout(const size_t *lengths, int count) {
     n = count;
     h_offs.assign(n, 0);
     h_lens.assign(n, 0);
@@ -214,10 +259,8 @@ struct DeviceSet {
     data.resize((total + 16) * sizeof(T));
     offs.resize(std::max(1, n) * sizeof(uint64_t));
     lens.resize(std::max(1, n) * sizeof(uint64_t));
-    for (int i = 0; i < n; ++i)
-      check_cuda(cudaMemcpyAsync(ptr<T>(data) + h_offs[i], sequences[i], lengths[i] * sizeof(T),
-                                 cudaMemcpyDefault, st),
-                 "series upload");
+  }
+  void upload_meta(cudaStream_t st) {
     check_cuda(cudaMemcpyAsync(offs.p, h_offs.data(), n * sizeof(uint64_t), cudaMemcpyHostToDevice, st),
                "offsets upload");
     check_cuda(cudaMemcpyAsync(lens.p, h_lens.data(), n * sizeof(uint64_t), cudaMemcpyHostToDevice, st),
@@ -812,16 +855,21 @@ void performDBA(T **sequences, int num_sequences, size_t *sequence_lengths, char
 // Block-edge merge and sentinel removal after the segmentation kernel
 // (segmentation.hpp:486-578).  segmented_sequences / segmented_seq_lengths are
 // allocated with cudaMallocManaged, as the reference does, for the caller to free.
-template <typename T>
-void adaptive_segmentation(T **sequences, size_t *seq_lengths, int num_seqs, int min_segment_length,
-                           T ***segmented_sequences, size_t **segmented_seq_lengths,
-                           int prefix_length_to_skip, cudaStream_t stream) {
-  const int n = num_seqs;
-  DeviceSet<T> ds;
-  ds.upload(sequences, seq_lengths, n, stream);
+namespace {
+
+// The segment medians of every series: done(i, medians, count) per series, in
+// order.  host: the sequences are in host memory.
+template <typename T, typename Done>
+void segment_series(T *const *sequences, const size_t *seq_lengths, int n, int min_segment_length,
+                    int prefix_length_to_skip, cudaStream_t stream, bool host, Done &&done) {
+  DeviceSet<T> ds(stream);
+  if (host)
+    ds.upload_host(sequences, seq_lengths, n, stream);
+  else
+    ds.upload(sequences, seq_lengths, n, stream);
   const size_t cap = odba_segment_capacity(ds.h_lens.data(), n, min_segment_length);
-  DevBuf d_med(std::max<size_t>(cap, 1) * sizeof(T));
-  DevBuf ws(odba_segment_workspace_bytes(n));
+  DevBuf d_med(std::max<size_t>(cap, 1) * sizeof(T), stream);
+  DevBuf ws(odba_segment_workspace_bytes(n), stream);
   check(Ops<T>::segment(ptr<T>(ds.data), ptr<uint64_t>(ds.offs), ptr<uint64_t>(ds.lens),
                         ds.h_lens.data(), n, min_segment_length, ptr<T>(d_med), ws.p, ws.bytes,
                         stream),
@@ -829,8 +877,6 @@ void adaptive_segmentation(T **sequences, size_t *seq_lengths, int num_seqs, int
   std::vector<T> med(cap);
   check_cuda(cudaMemcpyAsync(med.data(), d_med.p, cap * sizeof(T), cudaMemcpyDeviceToHost, stream), "segment download");
   check_cuda(cudaStreamSynchronize(stream), "segmentation");
-  check_cuda(cudaMallocManaged(segmented_sequences, sizeof(T *) * std::max(1, n)), "segmented sequence pointers");
-  check_cuda(cudaMallocManaged(segmented_seq_lengths, sizeof(size_t) * std::max(1, n)), "segmented lengths");
   int dw = (min_segment_length + 2) / 3;
   const int spb = 256 * dw;
   const float per = float(min_segment_length) / float(dw);
@@ -885,11 +931,26 @@ void adaptive_segmentation(T **sequences, size_t *seq_lengths, int num_seqs, int
         cursor -= prefix_length_to_skip;
       }
     }
-    (*segmented_seq_lengths)[i] = size_t(cursor);
-    check_cuda(cudaMallocManaged(&(*segmented_sequences)[i], sizeof(T) * std::max<long>(cursor, 1)),
-               "a segmented sequence");
-    std::memcpy((*segmented_sequences)[i], seg + skipped, sizeof(T) * size_t(cursor));
+    done(i, seg + skipped, size_t(cursor));
   }
+}
+
+}  // namespace
+
+template <typename T>
+void adaptive_segmentation(T **sequences, size_t *seq_lengths, int num_seqs, int min_segment_length,
+                           T ***segmented_sequences, size_t **segmented_seq_lengths,
+                           int prefix_length_to_skip, cudaStream_t stream) {
+  const int n = num_seqs;
+  check_cuda(cudaMallocManaged(segmented_sequences, sizeof(T *) * std::max(1, n)), "segmented sequence pointers");
+  check_cuda(cudaMallocManaged(segmented_seq_lengths, sizeof(size_t) * std::max(1, n)), "segmented lengths");
+  segment_series<T>(sequences, seq_lengths, n, min_segment_length, prefix_length_to_skip, stream,
+                    false, [&](int i, const T *medians, size_t count) {
+    (*segmented_seq_lengths)[i] = count;
+    check_cuda(cudaMallocManaged(&(*segmented_sequences)[i], sizeof(T) * std::max<size_t>(count, 1)),
+               "a segmented sequence");
+    std::memcpy((*segmented_sequences)[i], medians, sizeof(T) * count);
+  });
 }
 
 // ---------------------------------------------------------------------------
@@ -1346,18 +1407,18 @@ int segment_host(const T *h_series, const uint64_t *h_lens, int n, int minseg, i
     lens[i] = h_lens[i];
     off += h_lens[i];
   }
-  T **segs = nullptr;
-  size_t *seglens = nullptr;
-  adaptive_segmentation<T>(ptrs.data(), lens.data(), n, minseg, &segs, &seglens, prefix_skip);
+  // (device memory is copied as it is)
+  cudaPointerAttributes attr = {};
+  const bool device = cudaPointerGetAttributes(&attr, h_series) == cudaSuccess &&
+                      attr.type == cudaMemoryTypeDevice;
+  cudaGetLastError();
   size_t pos = 0;
-  for (int i = 0; i < n; ++i) {
-    std::memcpy(h_out + pos, segs[i], seglens[i] * sizeof(T));
-    pos += seglens[i];
-    h_out_lens[i] = seglens[i];
-    cudaFree(segs[i]);
-  }
-  cudaFree(segs);
-  cudaFree(seglens);
+  segment_series<T>(ptrs.data(), lens.data(), n, minseg, prefix_skip, nullptr, !device,
+                    [&](int i, const T *medians, size_t count) {
+    std::memcpy(h_out + pos, medians, count * sizeof(T));
+    pos += count;
+    h_out_lens[i] = count;
+  });
   return ODBA_OK;
 }
 }  // namespace
@@ -1394,6 +1455,7 @@ struct JobSet {
   std::vector<int> jbeg, jend, flags;         // series range per job in the sorted table
   std::vector<std::vector<int>> order;        // per job: sorted position -> input position
   DeviceSet<T> ds;                            // all jobs' series, sorted within each job
+  explicit JobSet(cudaStream_t st) : ds(st) {}
 };
 
 // Truncation and stable sort per job (dba.hpp:868-885), then upload.
@@ -1439,7 +1501,7 @@ void build_jobs(const T *h_series, const uint64_t *h_lens, const int *job_begin,
     js.jend[j] = int(ptrs.size());
     js.order[j] = idx;
   }
-  js.ds.upload(ptrs.data(), lens.data(), int(ptrs.size()), st);
+  js.ds.upload_host(ptrs.data(), lens.data(), int(ptrs.size()), st);
 }
 
 template <typename T>
@@ -1459,10 +1521,10 @@ int run_jobs(const T *h_series, const uint64_t *h_lens, const int *job_begin, co
              const int *job_flags, int njobs, int norm, int max_rounds, bool batched,
              int *h_medoids, uint64_t *h_centroid_offsets, T *h_centroids, int *h_rounds,
              double *h_deltas, cudaStream_t st) {
-  JobSet<T> js;
+  JobSet<T> js(st);
   build_jobs<T>(h_series, h_lens, job_begin, job_end, job_flags, njobs, js, st);
   const int n = js.ds.n;
-  DevBuf d_means(std::max(1, n) * sizeof(double)), d_sig(std::max(1, n) * sizeof(double));
+  DevBuf d_means(std::max(1, n) * sizeof(double), st), d_sig(std::max(1, n) * sizeof(double), st);
   std::vector<double> means(n, 0.0), sigmas(n, 1.0);
   if (norm) {
     check(Ops<T>::znorm(ptr<T>(js.ds.data), ptr<uint64_t>(js.ds.offs), ptr<uint64_t>(js.ds.lens), n,
@@ -1477,9 +1539,9 @@ int run_jobs(const T *h_series, const uint64_t *h_lens, const int *job_begin, co
     const unsigned long long m = (unsigned long long)(js.jend[j] - js.jbeg[j]);
     tri_off[j + 1] = tri_off[j] + m * (m - 1) / 2;
   }
-  DevBuf d_dists(std::max<unsigned long long>(tri_off[njobs], 1) * sizeof(T));
-  DevBuf d_sos(std::max(1, n) * sizeof(T)), d_med(std::max(1, njobs) * sizeof(int));
-  DevBuf ws(odba_dtw_pairwise_workspace_bytes(sizeof(T), std::max<uint64_t>(js.ds.max_len, 1)));
+  DevBuf d_dists(std::max<unsigned long long>(tri_off[njobs], 1) * sizeof(T), st);
+  DevBuf d_sos(std::max(1, n) * sizeof(T), st), d_med(std::max(1, njobs) * sizeof(int), st);
+  DevBuf ws(odba_dtw_pairwise_workspace_bytes(sizeof(T), std::max<uint64_t>(js.ds.max_len, 1)), st);
   if (batched) {
     // one launch for every pair of every job, largest m*n first
     std::vector<odba_pair_task> tasks;
@@ -1502,7 +1564,7 @@ int run_jobs(const T *h_series, const uint64_t *h_lens, const int *job_begin, co
     std::stable_sort(perm.begin(), perm.end(), [&](size_t a, size_t b) { return cost[a] > cost[b]; });
     std::vector<odba_pair_task> sorted(tasks.size());
     for (size_t i = 0; i < perm.size(); ++i) sorted[i] = tasks[perm[i]];
-    DevBuf d_tasks(std::max<size_t>(sorted.size(), 1) * sizeof(odba_pair_task));
+    DevBuf d_tasks(std::max<size_t>(sorted.size(), 1) * sizeof(odba_pair_task), st);
     check_cuda(cudaMemcpyAsync(d_tasks.p, sorted.data(), sorted.size() * sizeof(odba_pair_task),
                                cudaMemcpyHostToDevice, st), "task upload");
     if (!sorted.empty())
@@ -1555,8 +1617,9 @@ int run_jobs(const T *h_series, const uint64_t *h_lens, const int *job_begin, co
     h_medoids[j] = js.order[j][med[j]];
     h_centroid_offsets[j] = coff[j];
   }
-  DevBuf cbuf[2] = {DevBuf(std::max<uint64_t>(ctot, 1) * sizeof(T)), DevBuf(std::max<uint64_t>(ctot, 1) * sizeof(T))};
-  DevBuf d_counts(std::max<uint64_t>(ctot, 1) * sizeof(uint32_t)), d_deltas(njobs * sizeof(double));
+  DevBuf cbuf[2] = {DevBuf(std::max<uint64_t>(ctot, 1) * sizeof(T), st),
+                    DevBuf(std::max<uint64_t>(ctot, 1) * sizeof(T), st)};
+  DevBuf d_counts(std::max<uint64_t>(ctot, 1) * sizeof(uint32_t), st), d_deltas(njobs * sizeof(double), st);
   for (int j = 0; j < njobs; ++j)
     check_cuda(cudaMemcpyAsync(ptr<T>(cbuf[0]) + coff[j], ptr<T>(js.ds.data) + js.ds.h_offs[js.jbeg[j] + med[j]],
                                clen[j] * sizeof(T), cudaMemcpyDeviceToDevice, st), "seed centroids");
@@ -1597,9 +1660,9 @@ int run_jobs(const T *h_series, const uint64_t *h_lens, const int *job_begin, co
     for (int j = 0; j < njobs; ++j) h_flags[j] = (js.flags[j] & 3) | (active[j] ? 4 : 0);
   };
   flags_now();
-  DevBuf d_mseries(n * sizeof(int)), d_mjob(n * sizeof(int)), d_mbeg(njobs * sizeof(int)),
-      d_mend(njobs * sizeof(int)), d_flags(njobs * sizeof(int)), d_clen(njobs * sizeof(int)),
-      d_coff(njobs * sizeof(uint64_t)), d_order(n * sizeof(int));
+  DevBuf d_mseries(n * sizeof(int), st), d_mjob(n * sizeof(int), st), d_mbeg(njobs * sizeof(int), st),
+      d_mend(njobs * sizeof(int), st), d_flags(njobs * sizeof(int), st), d_clen(njobs * sizeof(int), st),
+      d_coff(njobs * sizeof(uint64_t), st), d_order(n * sizeof(int), st);
   check_cuda(cudaMemcpyAsync(d_mseries.p, mseries.data(), n * sizeof(int), cudaMemcpyHostToDevice, st), "members");
   check_cuda(cudaMemcpyAsync(d_mjob.p, mjob.data(), n * sizeof(int), cudaMemcpyHostToDevice, st), "members");
   check_cuda(cudaMemcpyAsync(d_mbeg.p, mbeg.data(), njobs * sizeof(int), cudaMemcpyHostToDevice, st), "jobs");
@@ -1652,7 +1715,7 @@ int run_jobs(const T *h_series, const uint64_t *h_lens, const int *job_begin, co
       for (int j : w) fl[j] |= 4;
       ws_max = std::max(ws_max, ws_for(fl));
     }
-    DevBuf rws(ws_max);
+    DevBuf rws(ws_max, st);
     const std::vector<int> was_active = active;
     for (auto &wave : waves) {
       std::vector<int> size_flags = none;
@@ -1696,8 +1759,11 @@ int run_jobs(const T *h_series, const uint64_t *h_lens, const int *job_begin, co
         check_cuda(cudaGraphLaunch(exec[cur], st), "graph launch");
         check_cuda(cudaMemcpyAsync(nb.data(), cbuf[1 - cur].p, ctot * sizeof(T), cudaMemcpyDeviceToHost, st), "means");
         check_cuda(cudaMemcpyAsync(deltas.data(), d_deltas.p, njobs * sizeof(double), cudaMemcpyDeviceToHost, st), "deltas");
+        unsigned wait_err = 0;  // the round's hand-off wait error word (byte 8 of its workspace)
+        check_cuda(cudaMemcpyAsync(&wait_err, static_cast<char *>(rws.p) + 8, sizeof wait_err,
+                                   cudaMemcpyDeviceToHost, st), "wait error word");
         check_cuda(cudaStreamSynchronize(st), "batched round");
-        if (wait_ran_out(rws.p)) {
+        if (wait_err) {
           for (int g = 0; g < 2; ++g) cudaGraphExecDestroy(exec[g]);
           return ODBA_ERR_TIMEOUT;
         }
@@ -1725,7 +1791,7 @@ int run_jobs(const T *h_series, const uint64_t *h_lens, const int *job_begin, co
       if (!active[j]) continue;
       const int b = js.jbeg[j], m = js.jend[j] - js.jbeg[j];
       const int os = js.flags[j] & 1, oe = (js.flags[j] >> 1) & 1;
-      DevBuf rws(odba_dba_round_workspace_bytes(sizeof(T), js.ds.h_lens.data() + b, m, clen[j], os, oe));
+      DevBuf rws(odba_dba_round_workspace_bytes(sizeof(T), js.ds.h_lens.data() + b, m, clen[j], os, oe), st);
       T *cin = ptr<T>(cbuf[0]) + coff[j];
       T *cout = ptr<T>(cbuf[1]) + coff[j];
       std::vector<T> v(clen[j]);

@@ -18,6 +18,13 @@ int fail(int status, const char *msg);
 int check_launch(const char *what);
 // Returns ODBA_OK if the current device is a compute capability 10.x part.
 int require_sm100();
+// Stream-ordered scratch of the host-buffer entry points, from a pool of the
+// library's own per device that keeps up to 256 MB mapped between calls (the
+// default pool unmaps what is freed at every synchronisation: mapping the
+// scratch again cost 0.4-0.7 ms a call).  Memory beyond that goes back at the
+// next synchronisation, all of it when an allocation fails.
+cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t stream);
+void scratch_free(void *p, cudaStream_t stream);
 
 template <typename T>
 size_t pairwise_workspace_bytes(uint64_t max_len);
