@@ -21,6 +21,7 @@
 #include <mutex>
 #include <vector>
 
+#include "dtw_block.cuh"
 #include "dtw_device.cuh"
 #include "dtw_pipe.cuh"
 #include "odba_internal.h"
@@ -132,32 +133,36 @@ int whole_pairlist_launch(const T *series, const uint64_t *offsets, const uint64
 }  // namespace odba
 
 // ---------------------------------------------------------------------------
-// Few long pairs: swath-pipelined sweeps.
+// Few pairs: swath-pipelined sweeps.
 //
 // With fewer pairs than warps (16 series of 1M-4M samples give 120 pairs for
 // ~1776 resident warps), one warp per pair would leave most of the GPU idle.
-// Here the unit of work is one swath of one pair: task k is swath k / P of
-// pair k % P (P pairs), so swath s of a pair is always handed out after swath
-// s - 1 of the same pair.  Each pair owns two edge buffers (swath s writes
-// buffer s % 2 and reads buffer (s - 1) % 2), and every swath of every pair
-// has its own progress word (rows stored so far), which the producing warp's
-// lane 31 publishes with a gpu-scope release every 128 rows and at the end of
-// its swath.  The consuming warp's lane 0 acquires the word before reading
-// rows it has not seen published.  Why this cannot deadlock: a warp waits only
-// on the previous swath of its pair, which was handed out earlier to a warp
-// that is already running and waits only on earlier tasks, so the earliest
-// unfinished task never waits.  Why two buffers suffice: swath s + 1
-// overwrites row r of buffer (s - 1) % 2 only after swath s has published row
-// r, and swath s reads its input rows before it computes (and publishes)
-// them; swaths s and s + 2 do write one buffer at the same time, at different
-// rows, which is why the progress words are per swath and not per buffer.
+// Here the unit of work is one 1024-column swath of one pair, swept by a block
+// (sweep_block): task k is swath k / P of pair k % P (P pairs), so swath s of a
+// pair is always handed out after swath s - 1 of the same pair.  Each pair owns
+// two edge buffers (swath s writes buffer s % 2 and reads buffer (s - 1) % 2),
+// and every swath of every pair has its own progress word (rows stored so far),
+// which the producing block's feeder publishes with a gpu-scope release every
+// 8 or 16 row pairs and at the end of its swath.  The consuming block's feeder
+// acquires the word before reading rows it has not seen published.  Why this
+// cannot deadlock: a block waits only on the previous swath of its pair, which
+// was handed out earlier to a block that is already running and waits only on
+// earlier tasks, so the earliest unfinished task never waits.  Why two buffers
+// suffice: swath s + 1 overwrites row r of buffer (s - 1) % 2 only after swath
+// s has published row r, and swath s reads its input rows before it computes
+// (and publishes) them; swaths s and s + 2 do write one buffer at the same
+// time, at different rows, which is why the progress words are per swath and
+// not per buffer.
 //
-// Every wait is bounded: after kWaitLimitNs of polling (%globaltimer) the warp
-// raises the launch's error word and continues; every other waiting warp sees
+// Every wait is bounded: after its limit of polling (%globaltimer) a block
+// raises the launch's error word and continues; every other waiting block sees
 // the word and stops waiting, so a fault in the hand-off ends the launch
 // quickly with the pairs it touched written as NaN.
 namespace odba {
 namespace {
+
+// Blocks per SM of the swath pipeline.
+constexpr int kPipeBlocksF32 = 4, kPipeBlocksF64 = 3;
 
 template <typename T>
 struct PipeArgs {
@@ -181,108 +186,158 @@ struct PipeArgs {
   unsigned long long limit_ns;
 };
 
-template <typename T, int R, bool TRACK>
-__device__ __forceinline__ EdgeStat<T> pipe_swath(const SwathJob<T> &job, const PipeGate &gate,
-                                                  bool last, T &corner) {
-  T col[R];
-  const EdgeStat<T> st = sweep_swath<T, R, PipeGate, TRACK>(job, col, gate);
-  if (last) corner = pick_column<T, R>(col, job.c0, job.n - 1);
-  return st;
+// One pair of a launch: its series (rows, columns), modes and output.  Without
+// an open end the matrix of (b, a) is the transpose of (a, b)'s with the same
+// costs bit for bit (the differences change sign, the cell rule is symmetric),
+// so the shorter series takes the rows: a pair's time is the steps down its
+// rows plus about 200 steps for each swath after the first, and 1024 columns
+// cost less than 1024 rows.
+struct PipePair {
+  int s, j, os, oe;
+  unsigned long long out;
+  uint64_t m, n;
+};
+template <typename T>
+__device__ __forceinline__ PipePair pipe_pair(const PipeArgs<T> &a, unsigned long long qi) {
+  PipePair p;
+  if (a.list) {
+    const odba_pair_task task = a.list[qi];
+    p.s = int(task.first);
+    p.j = int(task.second);
+    p.os = int((task.out >> 62) & 1ull);
+    p.oe = int((task.out >> 63) & 1ull);
+    p.out = task.out & ((1ull << 62) - 1);
+  } else {
+    const long long i = (long long)(a.pbeg + a.npairs - 1 - qi);
+    pair_of(i, a.n, p.s, p.j);
+    p.os = a.open_start;
+    p.oe = a.open_end;
+    p.out = (unsigned long long)i;
+  }
+  p.m = a.lens[p.s];
+  p.n = a.lens[p.j];
+  if (!p.os && !p.oe && p.m > p.n) {
+    const int t = p.s;
+    p.s = p.j;
+    p.j = t;
+    const uint64_t l = p.m;
+    p.m = p.n;
+    p.n = l;
+  }
+  return p;
 }
 
-// TRACK: some pair may take the open-end shortcut (see sweep_pair)
-template <typename T, int RF, int RQ, bool TRACK>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32, kMinBlocksPerSM)
+// A block per swath (sweep_block).  TRACK: some pair may take the open-end
+// shortcut (see sweep_pair).  A pair with more swaths than the launch counts
+// (a list's second series may be longer than its longest first one) has the
+// rest of them swept by the block of its last counted one, in turn.
+template <typename T, bool TRACK>
+__global__ void __launch_bounds__(kBlkThreads, sizeof(T) == 4 ? kPipeBlocksF32 : kPipeBlocksF64)
     swathpipe_kernel(PipeArgs<T> a) {
-  constexpr int W = 32 * RF;
-  __shared__ __align__(16) T stage_mem[kWarpsPerBlock * kStageElems];
+  __shared__ BlockSmem<T> sm;
   const int lane = threadIdx.x & 31;
+  const bool feeder = (threadIdx.x >> 5) == kBlkWarps;
   const unsigned long long ntasks = a.npairs * a.max_swaths;
   for (;;) {
-    unsigned long long q = 0;
-    if (lane == 0) q = atomicAdd(a.counter, 1ull);
-    q = __shfl_sync(kFull, q, 0);
-    if (q >= ntasks) break;
-    const unsigned long long sw = q / a.npairs, qi = q - sw * a.npairs;
-    int s, j, os, oe;
-    unsigned long long out;
-    if (a.list) {
-      const odba_pair_task task = a.list[qi];
-      s = int(task.first);
-      j = int(task.second);
-      os = int((task.out >> 62) & 1ull);
-      oe = int((task.out >> 63) & 1ull);
-      out = task.out & ((1ull << 62) - 1);
-    } else {
-      const long long p = (long long)(a.pbeg + a.npairs - 1 - qi);
-      pair_of(p, a.n, s, j);
-      os = a.open_start;
-      oe = a.open_end;
-      out = (unsigned long long)p;
+    if (feeder && lane == 0) {
+      // the next task that exists
+      unsigned long long q;
+      for (;;) {
+        q = atomicAdd(a.counter, 1ull);
+        if (q >= ntasks) break;
+        const unsigned long long sw = q / a.npairs;
+        if (sw * kBlkCols < pipe_pair(a, q - sw * a.npairs).n) break;
+      }
+      sm.task = q;
     }
-    SwathJob<T> job;
-    job.stage = stage_mem + (threadIdx.x >> 5) * kStageElems;
-    job.x = a.series + a.offsets[s];
-    job.m = int(a.lens[s]);
-    job.y = a.series + a.offsets[j];
-    job.n = int(a.lens[j]);
-    const unsigned long long nsw = (unsigned long long)(job.n + W - 1) / W;
-    if (sw >= nsw) continue;
-    const int c0 = int(sw) * W;
-    const bool last = sw + 1 == nsw;
+    __syncthreads();
+    const unsigned long long q = sm.task;
+    if (q >= ntasks) break;
+    const unsigned long long first = q / a.npairs, qi = q - first * a.npairs;
+    const PipePair p = pipe_pair(a, qi);
+    const int m = int(p.m), n = int(p.n);
     T *b0 = a.edges + qi * 2 * a.edge_stride;
     T *b1 = b0 + a.edge_stride;
-    job.c0 = c0;
-    job.r0 = os;
-    job.open_end = oe != 0;
-    job.edge_in = sw ? (((sw - 1) & 1) ? b1 : b0) : nullptr;
-    job.edge_out = last ? nullptr : ((sw & 1) ? b1 : b0);
-    job.free_diag0 = c0 > 0 && (c0 % kRefSwath) == 0;
-    job.corner_init = c0 == 0 ? (job.r0 ? Num<T>::big() : T(0)) : (job.r0 ? T(0) : Num<T>::big());
-    job.track = TRACK && swath_checks_shortcut<T>(c0, W, job.m, job.n, job.open_end, job.r0);
-    PipeGate gate;
     unsigned long long *words = a.progress + qi * a.max_swaths;
-    gate.prog_in = words + (sw ? sw - 1 : 0);
-    gate.prog_out = words + sw;
-    gate.err = a.err;
-    gate.limit_ns = a.limit_ns;
-    gate.avail = 0;
-    T corner = T(0);
-    const int width = job.n - c0 < W ? job.n - c0 : W;
-    const int rneed = (width + 31) / 32;
-    const int rq = (rneed + RQ - 1) / RQ * RQ;
-    EdgeStat<T> st{Num<T>::big(), Num<T>::big()};
-    if (rq >= RF) {
-      st = pipe_swath<T, RF, TRACK>(job, gate, last, corner);
-    } else {
-      switch (rq / RQ) {
-#define ODBA_PCASE(K)                                                       \
-  case K:                                                                   \
-    if constexpr (K * RQ < RF) st = pipe_swath<T, K * RQ, TRACK>(job, gate, last, corner); \
-    break;
-        ODBA_PCASE(1)
-        ODBA_PCASE(2)
-        ODBA_PCASE(3)
-        ODBA_PCASE(4)
-        ODBA_PCASE(5)
-        ODBA_PCASE(6)
-        ODBA_PCASE(7)
-#undef ODBA_PCASE
-        default:
-          break;
+    const bool to_end = first + 1 == a.max_swaths;
+    bool stop = false;  // the shortcut fired past the counted boundaries
+    for (unsigned long long sw = first;; ++sw) {
+      const int c0 = int(sw) * kBlkCols;
+      const bool last = c0 + kBlkCols >= n;
+      BlockJob<T> job;
+      job.x = a.series + a.offsets[p.s];
+      job.y = a.series + a.offsets[p.j];
+      job.m = m;
+      job.n = n;
+      job.c0 = c0;
+      job.r0 = p.os;
+      job.edge_in = sw ? (((sw - 1) & 1) ? b1 : b0) : nullptr;
+      job.edge_out = last ? nullptr : ((sw & 1) ? b1 : b0);
+      job.open_end = p.oe != 0;
+      job.free_diag0 = c0 > 0;
+      job.corner_init = c0 == 0 ? (p.os ? Num<T>::big() : T(0)) : (p.os ? T(0) : Num<T>::big());
+      job.words = nullptr;
+      job.word_steps = 0;
+      PipeGate gate;
+      gate.prog_in = words + (first ? first - 1 : 0);
+      gate.prog_out = words + first;
+      gate.err = a.err;
+      gate.limit_ns = a.limit_ns;
+      gate.avail = sw == first ? 0 : 0x7fffffff;
+      T corner = T(0);
+      EdgeStat<T> st;
+      bool mine = sweep_block<T, false, false, false, true>(
+          job, sm, gate, CkptOut<T>{nullptr, 0, 1}, last, corner, st);
+      if (TRACK && swath_checks_shortcut<T>(c0, kBlkCols, m, n, p.oe != 0, p.os)) {
+        // this swath's right edge is the left edge of reference swath k + 1
+        const unsigned long long k = sw;
+        T v = T(-1);
+        if (feeder && lane == 0) {
+          if (!shortcut_fires<T>(st, m, v)) v = T(-1);
+          if (k < a.max_bounds) a.bstat[qi * a.max_bounds + k] = v;
+        }
+        if (k >= a.max_bounds) {
+          if (feeder && lane == 0) sm.task = v >= T(0) ? 1ull : 0ull;
+          __syncthreads();
+          if (sm.task) {
+            stop = true;
+            mine = feeder && lane == 0;
+            corner = v;
+          }
+        }
       }
-    }
-    if (TRACK && job.track && lane == 31) {
-      // this swath's right edge is the left edge of reference swath k + 1
-      const unsigned long long k = (unsigned long long)(c0 + W) / kRefSwath - 1;
-      T v;
-      a.bstat[qi * a.max_bounds + k] = shortcut_fires<T>(st, job.m, v) ? v : T(-1);
-    }
-    if (last && lane == 0) {
-      const bool bad = *reinterpret_cast<volatile unsigned *>(a.err) != 0;
-      a.dists[out] = bad ? T(NAN) : pair_distance<T>(corner, job.m, job.n, os, oe);
+      if (m <= p.os && last) mine = threadIdx.x == 0;  // open start over a single row: all zeros
+      if (mine) {
+        const bool bad = *reinterpret_cast<volatile unsigned *>(a.err) != 0;
+        a.dists[p.out] = bad ? T(NAN) : pair_distance<T>(corner, m, n, p.os, p.oe);
+      }
+      __syncthreads();  // the task word and the rings are free again
+      if (last || stop || !to_end) break;
     }
   }
+}
+
+// Resident blocks of swathpipe_kernel on the current device (cached like
+// grid_size).
+template <typename T>
+int pipe_grid() {
+  static std::atomic<int> cached[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64) {
+    const int c = cached[dev].load(std::memory_order_relaxed);
+    if (c) return c;
+  }
+  int sms = 0, per_sm = 0;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, swathpipe_kernel<T, false>, kBlkThreads, 0);
+  constexpr int want = sizeof(T) == 4 ? kPipeBlocksF32 : kPipeBlocksF64;
+  if (per_sm > want) per_sm = want;
+  if (per_sm < 1) per_sm = 1;
+  if (sms < 1) sms = 1;
+  const int g = sms * per_sm;
+  if (dev >= 0 && dev < 64) cached[dev].store(g, std::memory_order_relaxed);
+  return g;
 }
 
 // After the pipeline: a pair whose open-end shortcut fired on some checked
@@ -313,6 +368,7 @@ __global__ void pipe_shortcut_kernel(PipeArgs<T> a) {
   const int m = int(a.lens[s]), n = int(a.lens[j]);
   for (int cnext = kRefSwath; cnext < n; cnext += kRefSwath) {
     if (cnext <= m) continue;
+    if ((unsigned long long)(cnext / kRefSwath - 1) >= a.max_bounds) return;
     const T v = a.bstat[qi * a.max_bounds + (unsigned long long)(cnext / kRefSwath - 1)];
     if (v >= T(0)) {
       a.dists[out] = pair_distance<T>(v, m, n, os, oe);
@@ -326,8 +382,7 @@ __global__ void pipe_shortcut_kernel(PipeArgs<T> a) {
 // counter and error word | progress words | shortcut values | edge buffers
 template <typename T>
 size_t swathpipe_progress_bytes(unsigned long long npairs, uint64_t max_len) {
-  constexpr int W = 32 * Tune<T>::RF;
-  const unsigned long long max_swaths = (max_len + W - 1) / W;
+  const unsigned long long max_swaths = (max_len + kBlkCols - 1) / kBlkCols;
   return (size_t(npairs) * max_swaths * 8 + 255) / 256 * 256;
 }
 
@@ -353,7 +408,6 @@ int swathpipe_launch(const T *series, const uint64_t *offsets, const uint64_t *l
   if (npairs == 0) return ODBA_OK;
   if (ws_bytes < swathpipe_workspace_bytes<T>(npairs, max_len))
     return fail(ODBA_ERR_WORKSPACE_TOO_SMALL, "workspace too small for the swath pipeline");
-  constexpr int W = 32 * Tune<T>::RF;
   PipeArgs<T> a;
   a.series = series;
   a.offsets = offsets;
@@ -362,7 +416,7 @@ int swathpipe_launch(const T *series, const uint64_t *offsets, const uint64_t *l
   a.list = list;
   a.pbeg = pbeg;
   a.npairs = npairs;
-  a.max_swaths = (max_len + W - 1) / W;
+  a.max_swaths = (max_len + kBlkCols - 1) / kBlkCols;
   a.dists = dists;
   char *base = static_cast<char *>(workspace);
   a.counter = reinterpret_cast<unsigned long long *>(base);
@@ -380,11 +434,14 @@ int swathpipe_launch(const T *series, const uint64_t *offsets, const uint64_t *l
   if (cudaMemsetAsync(base, 0, 256 + swathpipe_progress_bytes<T>(npairs, max_len), stream) != cudaSuccess)
     return fail(ODBA_ERR_CUDA, "clearing the pipeline state failed");
   const bool track = list || (oe && !os);
+  const unsigned long long tasks = npairs * a.max_swaths;
+  const int resident = pipe_grid<T>();
+  const int grid = tasks < (unsigned long long)resident ? int(tasks) : resident;
   if (track) {
-    swathpipe_kernel<T, Tune<T>::RF, Tune<T>::RQ, true><<<grid_size<T>(), kWarpsPerBlock * 32, 0, stream>>>(a);
+    swathpipe_kernel<T, true><<<grid, kBlkThreads, 0, stream>>>(a);
     pipe_shortcut_kernel<T><<<unsigned((npairs + 127) / 128), 128, 0, stream>>>(a);
   } else {
-    swathpipe_kernel<T, Tune<T>::RF, Tune<T>::RQ, false><<<grid_size<T>(), kWarpsPerBlock * 32, 0, stream>>>(a);
+    swathpipe_kernel<T, false><<<grid, kBlkThreads, 0, stream>>>(a);
   }
   return check_launch("swath-pipelined DTW kernel");
 }
@@ -410,9 +467,8 @@ template int swathpipe_launch<double>(const double *, const uint64_t *, const ui
 // and the swath pipeline above (many warps per pair).  The plan is chosen per
 // key (element size, floor(log2 max_len), floor(log2 pairs)): a plan pinned by
 // odba_tune_set; else, in tuning mode, every eligible plan not yet measured for
-// the key, in turn; else the fastest measured plan; else a rule of thumb (the
-// pipeline when there are fewer pairs than resident warps and the longest
-// series spans four or more swaths).  Measured throughput is pair-cells per
+// the key, in turn; else the fastest measured plan; else a rule of thumb
+// (rule_of_thumb).  Measured throughput is pair-cells per
 // second with max_len^2 per pair standing in for the cells (the lengths live
 // on the device); CUDA events around each tuning launch are read back on the
 // next call or by odba_tune_flush.
@@ -462,26 +518,38 @@ void harvest_locked(bool block) {
 
 template <typename T>
 bool plan_fits(int plan, unsigned long long npairs, uint64_t max_len, size_t ws_bytes) {
-  constexpr int W = 32 * Tune<T>::RF;
   const unsigned long long slots = (unsigned long long)grid_size<T>() * kWarpsPerBlock;
   switch (plan) {
     case ODBA_PLAN_WHOLE_PAIR:
     case ODBA_PLAN_WHOLE_PAIR_HALF_SWATH:
       return ws_bytes >= whole_workspace_bytes<T>(max_len);
     case ODBA_PLAN_SWATH_PIPELINE:
-      return npairs <= 2 * slots && (max_len + W - 1) / W >= 2 &&
-             ws_bytes >= swathpipe_workspace_bytes<T>(npairs, max_len);
+      return npairs <= 2 * slots && ws_bytes >= swathpipe_workspace_bytes<T>(npairs, max_len);
     default:
       return false;
   }
 }
 
+// The pipeline pays while its blocks are few enough to run a pair's swaths side
+// by side: it takes a pair's steps a quarter to a half of the one-warp sweep's
+// time, but fills the GPU with a third as many pairs.  Measured on one B200
+// (one-warp time / pipeline time, all pairs of n series): float, 2000-4000
+// samples, 1128 / 1770 / 2016 pairs 1.72 / 1.23 / 1.09, 1000-2000 samples 1.45 /
+// 1.07 / 0.92, 900-1100 samples 630 / 1128 / 1540 pairs 1.70 / 1.07 / 0.79,
+// 512-1024 samples 1.66 / 1.11 / 0.86, 20-40 samples 276 / 630 pairs 1.08 / 0.71;
+// double, 2000-4000 samples 1128 / 1770 pairs 1.68 / 1.08, 900-1100 samples 630 /
+// 1128 pairs 1.59 / 0.94, 150-400 samples 276 / 630 pairs 1.76 / 0.92, 20-40
+// samples 276 pairs 0.81.
 template <typename T>
 int rule_of_thumb(unsigned long long npairs, uint64_t max_len) {
-  constexpr int W = 32 * Tune<T>::RF;
   const unsigned long long slots = (unsigned long long)grid_size<T>() * kWarpsPerBlock;
-  return (npairs < slots && (max_len + W - 1) / W >= 4) ? ODBA_PLAN_SWATH_PIPELINE
-                                                         : ODBA_PLAN_WHOLE_PAIR;
+  const uint64_t swaths = (max_len + kBlkCols - 1) / kBlkCols;
+  unsigned long long most;
+  if (sizeof(T) == 4)
+    most = swaths >= 3 ? slots : swaths == 2 ? slots * 2 / 3 : max_len >= 64 ? slots / 2 : slots / 6;
+  else
+    most = swaths >= 3 ? slots * 2 / 3 : swaths == 2 ? slots * 2 / 5 : max_len >= 64 ? slots / 4 : 0;
+  return npairs < most ? ODBA_PLAN_SWATH_PIPELINE : ODBA_PLAN_WHOLE_PAIR;
 }
 
 // Chooses the plan; *measure tells the caller to time the launch for the table.
