@@ -1,7 +1,7 @@
 // A thread block sweeps one 1024-column swath of a cost matrix: four compute
 // warps in a row and a fifth warp feeding them.
 //
-// Why a block per swath: a one-warp swath (dtw_device.cuh) is the cheapest
+// Why a block per swath: a one-warp swath (dtw_warp.cuh) is the cheapest
 // way to fill the GPU with many matrices, but a matrix is then a chain of
 // long steps -- 64 cells per lane, about 800 cycles for a warp that records
 // moves and has the scheduler to itself -- and few matrices leave most
@@ -66,29 +66,6 @@ __host__ __device__ inline int block_steps(int rows) {
   return ((rows + 1) / 2 + 31 + kBlkChunk - 1) / kBlkChunk * kBlkChunk;
 }
 
-// The staged samples of a row pair: float twice each, so that a step reads the
-// two operand pairs of its packed differences as they are.
-template <typename T>
-struct XPair;
-template <>
-struct XPair<float> {
-  float4 v;
-  __device__ __forceinline__ float a() const { return v.x; }
-  __device__ __forceinline__ float b() const { return v.z; }
-  static __device__ __forceinline__ void put(XPair *p, int row, float x) {
-    reinterpret_cast<float2 *>(p)[row & 1] = make_float2(x, x);
-  }
-};
-template <>
-struct XPair<double> {
-  double2 v;
-  __device__ __forceinline__ double a() const { return v.x; }
-  __device__ __forceinline__ double b() const { return v.y; }
-  static __device__ __forceinline__ void put(XPair *p, int row, double x) {
-    reinterpret_cast<double *>(p)[row & 1] = x;
-  }
-};
-
 template <typename T>
 struct BlockSmem {
   // the first kBlkChunk pairs again past the end: a chunk's reads never wrap
@@ -139,7 +116,7 @@ struct CkptOut {
   int shift;
 };
 
-// One swath for one block (see SwathJob for the matrix convention).
+// One swath for one block.
 template <typename T>
 struct BlockJob {
   const T *x, *y;
@@ -158,97 +135,6 @@ struct BlockJob {
   const T *row_in = nullptr;
   T *row_out = nullptr, *corner_out = nullptr;
 };
-
-// One cell; PATH adds its move bits B (D) and B + 8 (U) to w.
-template <typename T, bool PATH, bool TOP, int B>
-__device__ __forceinline__ T block_cell(T d, T up, T diag, T left, bool top, bool fd, unsigned &w) {
-  if constexpr (PATH) {
-    const T uv = Num<T>::cell(d, up);
-    T dv = Num<T>::cell(d, diag);
-    T rv = Num<T>::cell(d, left);
-    if (TOP) {
-      rv = top ? left : rv;
-      dv = (top && fd) ? diag : dv;
-    }
-    const T v = Num<T>::min3(uv, dv, rv);
-    or_bit_if_eq<B>(w, dv, v);
-    or_bit_if_eq<B + 8>(w, uv, v);
-    return v;
-  } else if constexpr (TOP) {
-    return cell_rule<T>(d, up, diag, left, top, fd);
-  } else {
-    return Num<T>::cell(d, Num<T>::min3(up, diag, left));
-  }
-}
-
-// The differences of a step's two rows from staged samples.
-template <typename T>
-struct BlockDiffs : RowDiffs<T, kBlkR> {
-  __device__ __forceinline__ explicit BlockDiffs(const XPair<T> &x)
-      : RowDiffs<T, kBlkR>(x.a(), x.b()) {}
-};
-template <>
-struct BlockDiffs<float> {
-  unsigned long long xa2, xb2, pa = 0, pb = 0;
-  __device__ __forceinline__ explicit BlockDiffs(const XPair<float> &x)
-      : xa2(pack_f32x2(x.v.x, x.v.y)), xb2(pack_f32x2(x.v.z, x.v.w)) {}
-  __device__ __forceinline__ float a(const YCols<float, kBlkR> &y, int j) {
-    if ((j & 1) == 0) pa = sub_f32x2(xa2, y.p[j / 2]);
-    return (j & 1) ? half_f32x2<1>(pa) : half_f32x2<0>(pa);
-  }
-  __device__ __forceinline__ float b(const YCols<float, kBlkR> &y, int j) {
-    if ((j & 1) == 0) pb = sub_f32x2(xb2, y.p[j / 2]);
-    return (j & 1) ? half_f32x2<1>(pb) : half_f32x2<0>(pb);
-  }
-};
-
-// Two rows of a lane's 8 columns, row b one column behind row a
-// (step_rows2_steady).  CAP: cap receives the value of column capj in row a
-// (capb: in row b).
-template <typename T>
-struct BlockRowState {
-  T a_left, a_diag, b_left, b_diag, va_prev;
-  unsigned wa, wb;
-};
-template <typename T, bool PATH, bool TOP, bool CAP, int J>
-struct BlockCols {
-  static __device__ __forceinline__ void run(T (&col)[kBlkR], const YCols<T, kBlkR> &yv,
-                                             BlockDiffs<T> &df, BlockRowState<T> &z, bool top_a,
-                                             bool top_b, bool fd0, int capj, bool capb, T &cap) {
-    if constexpr (J < kBlkR) {
-      const T up = col[J];
-      const T va = block_cell<T, PATH, TOP, J>(df.a(yv, J), up, z.a_diag, z.a_left, top_a,
-                                               J == 0 && fd0, z.wa);
-      z.a_diag = up;
-      z.a_left = va;
-      if (CAP) cap = (capj == J && !capb) ? va : cap;
-      if constexpr (J > 0) {
-        const T vb = block_cell<T, PATH, TOP, 16 + J - 1>(df.b(yv, J - 1), z.va_prev, z.b_diag,
-                                                          z.b_left, top_b, J == 1 && fd0, z.wb);
-        z.b_diag = z.va_prev;
-        z.b_left = vb;
-        col[J - 1] = vb;
-        if (CAP) cap = (capj == J - 1 && capb) ? vb : cap;
-      }
-      z.va_prev = va;
-      BlockCols<T, PATH, TOP, CAP, J + 1>::run(col, yv, df, z, top_a, top_b, fd0, capj, capb, cap);
-    }
-  }
-};
-template <typename T, bool PATH, bool TOP, bool CAP>
-__device__ __forceinline__ T block_rows2(T (&col)[kBlkR], const YCols<T, kBlkR> &yv,
-                                         const XPair<T> &x, T la, T lb, T dg, bool top_a,
-                                         bool top_b, bool fd0, unsigned &word, int capj, bool capb,
-                                         T &cap) {
-  BlockRowState<T> z{la, dg, lb, la, T(0), 0u, 0u};
-  BlockDiffs<T> df(x);
-  BlockCols<T, PATH, TOP, CAP, 0>::run(col, yv, df, z, top_a, top_b, fd0, capj, capb, cap);
-  col[kBlkR - 1] = block_cell<T, PATH, TOP, 16 + kBlkR - 1>(
-      df.b(yv, kBlkR - 1), z.va_prev, z.b_diag, z.b_left, top_b, kBlkR == 1 && fd0, z.wb);
-  if (CAP) cap = (capj == kBlkR - 1 && capb) ? col[kBlkR - 1] : cap;
-  if (PATH) word = z.wa | z.wb;
-  return z.a_left;
-}
 
 // The sweep.  All kBlkThreads threads call it with the same job.  PATH
 // records moves; BAND: the job may be a band of a swath's rows (rows counted
@@ -433,9 +319,9 @@ __device__ __forceinline__ bool sweep_block(const BlockJob<T> &job, BlockSmem<T>
       unsigned word = 0u;
       const bool top = SLOW && oe_top && k == last_pair;
       T c2 = cap;
-      a_last = block_rows2<T, PATH, SLOW, SLOW && CAP>(col, yv, xv, la, lb, diag,
-                                                       top && !last_is_b, top && last_is_b, fd0,
-                                                       word, capj, last_is_b, c2);
+      a_last = step_row_pair<T, kBlkR, PATH, SLOW, SLOW && CAP>(
+          col, yv, xv, la, lb, diag, top && !last_is_b, top && last_is_b, fd0, word, capj, last_is_b,
+          c2);
       if (SLOW && CAP) cap = k == last_pair ? c2 : cap;
       V2 v;
       v.x = a_last;

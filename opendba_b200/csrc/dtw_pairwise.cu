@@ -59,11 +59,9 @@ int whole_pairwise_launch(const T *series, const uint64_t *offsets, const uint64
   a.edge_stride = (max_len + 32 + 31) / 32 * 32;
   a.open_start = os;
   a.open_end = oe;
+  a.classes = size_classes(a.npairs, grid_size<T>() * kWarpsPerBlock);
   cudaMemsetAsync(a.counter, 0, 16, stream);  // work counter and error word
-  if (oe && !os)
-    pairwise_kernel<T, RF, Tune<T>::RQ, true><<<grid_size<T>(), kWarpsPerBlock * 32, 0, stream>>>(a);
-  else
-    pairwise_kernel<T, RF, Tune<T>::RQ, false><<<grid_size<T>(), kWarpsPerBlock * 32, 0, stream>>>(a);
+  pairwise_kernel<T, RF, Tune<T>::RQ><<<grid_size<T>(), kWarpsPerBlock * 32, 0, stream>>>(a);
   return check_launch("pairwise DTW kernel");
 }
 
@@ -82,7 +80,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, kMinBlocksPerSM)
     pairlist_kernel(const T *series, const uint64_t *offsets, const uint64_t *lens,
                     const odba_pair_task *tasks, unsigned long long ntasks, T *dists,
                     unsigned long long *counter, T *edges, unsigned long long edge_stride) {
-  __shared__ __align__(16) T stage_mem[kWarpsPerBlock * kStageElems];
+  __shared__ WarpSmem<T> sm[kWarpsPerBlock];
   const int lane = threadIdx.x & 31;
   const long long slot = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   T *e0 = edges + slot * 2 * edge_stride;
@@ -96,7 +94,6 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, kMinBlocksPerSM)
     const int os = int((task.out >> 62) & 1ull), oe = int((task.out >> 63) & 1ull);
     const unsigned long long out = task.out & ((1ull << 62) - 1);
     SwathJob<T> job;
-    job.stage = stage_mem + (threadIdx.x >> 5) * kStageElems;
     job.x = series + offsets[task.first];
     job.m = int(lens[task.first]);
     job.y = series + offsets[task.second];
@@ -104,7 +101,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, kMinBlocksPerSM)
     job.r0 = os;
     job.open_end = oe != 0;
     T corner = T(0);
-    sweep_pair<T, RF, RQ, true>(job, e0, e1, corner);
+    sweep_pair<T, RF, RQ>(job, sm[threadIdx.x >> 5], e0, e1, corner);
     if (lane == 0) dists[out] = pair_distance<T>(corner, job.m, job.n, os, oe);
   }
 }

@@ -136,13 +136,11 @@ int pairwise_noalloc(const T *series, const uint64_t *offsets, const uint64_t *l
   a.edge_stride = stride;
   a.open_start = os ? 1 : 0;
   a.open_end = oe ? 1 : 0;
+  a.classes = size_classes(a.npairs, grid * kWarpsPerBlock);
   // the counter is the only state that must start at zero
   cudaError_t e = cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), stream);
   if (e != cudaSuccess) return fail(ODBA_ERR_CUDA, "clearing the work counter failed");
-  if (a.open_end && !a.open_start)
-    pairwise_kernel<T, Tune<T>::RF, Tune<T>::RQ, true><<<grid, kWarpsPerBlock * 32, 0, stream>>>(a);
-  else
-    pairwise_kernel<T, Tune<T>::RF, Tune<T>::RQ, false><<<grid, kWarpsPerBlock * 32, 0, stream>>>(a);
+  pairwise_kernel<T, Tune<T>::RF, Tune<T>::RQ><<<grid, kWarpsPerBlock * 32, 0, stream>>>(a);
   return check_launch("pairwise DTW kernel (no-allocation variant)");
 }
 

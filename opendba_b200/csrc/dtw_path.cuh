@@ -1,4 +1,4 @@
-// Moves recorded by the path sweep of the DBA round (DBAUpdate's DTWDistance
+// The row-pair step of the sweeps, and the moves recorded by the path sweep of the DBA round (DBAUpdate's DTWDistance
 // launches with a path matrix, dba.hpp:589-617).
 //
 // Each cell also records the reference's move choice (dtw.hpp:202-227):
@@ -9,8 +9,7 @@
 // DIAGONAL > UP > RIGHT, i.e. move = DIAGONAL if diag == min, else UP if
 // up == min, else RIGHT.  Two bits per cell are kept as two bit planes: D
 // (the diagonal candidate equals the minimum) and U (the up candidate does),
-// each set by one compare and one predicated OR of an immediate; decode_move
-// applies the priority.  The codes the reference derives from position alone
+// each set by one compare and one predicated OR of an immediate.  The codes the reference derives from position alone
 // (row 0, (0, 0), the open-end OPEN_RIGHT) are rebuilt by the backtrack.
 #pragma once
 
@@ -35,5 +34,76 @@ __device__ __forceinline__ void or_bit_if_eq(unsigned &w, double a, double b) {
 
 // Move codes the sweep records (dtw.hpp:10-16).
 constexpr int kMoveDiag = 1, kMoveRight = 2, kMoveUp = 3;
+
+// One cell; PATH adds its move bits B (D) and B + 8 (U) to w.
+template <typename T, bool PATH, bool TOP, int B>
+__device__ __forceinline__ T row_pair_cell(T d, T up, T diag, T left, bool top, bool fd, unsigned &w) {
+  if constexpr (PATH) {
+    const T uv = Num<T>::cell(d, up);
+    T dv = Num<T>::cell(d, diag);
+    T rv = Num<T>::cell(d, left);
+    if (TOP) {
+      rv = top ? left : rv;
+      dv = (top && fd) ? diag : dv;
+    }
+    const T v = Num<T>::min3(uv, dv, rv);
+    or_bit_if_eq<B>(w, dv, v);
+    or_bit_if_eq<B + 8>(w, uv, v);
+    return v;
+  } else if constexpr (TOP) {
+    return cell_rule<T>(d, up, diag, left, top, fd);
+  } else {
+    return Num<T>::cell(d, Num<T>::min3(up, diag, left));
+  }
+}
+
+// Two rows of a lane's R columns, row b one column behind row a: the two
+// chains interleave, and since row a at column j reads the old col[j - 1] as its
+// diagonal before row b writes the new one, no column changes registers (in
+// column order all of them would rotate).  CAP: cap receives the value of column capj in row a
+// (capb: in row b).
+template <typename T>
+struct RowPairState {
+  T a_left, a_diag, b_left, b_diag, va_prev;
+  unsigned wa, wb;
+};
+template <typename T, int R, bool PATH, bool TOP, bool CAP, int J>
+struct RowPairCols {
+  static __device__ __forceinline__ void run(T (&col)[R], const YCols<T, R> &yv,
+                                             RowDiffs<T, R> &df, RowPairState<T> &z, bool top_a,
+                                             bool top_b, bool fd0, int capj, bool capb, T &cap) {
+    if constexpr (J < R) {
+      const T up = col[J];
+      const T va = row_pair_cell<T, PATH, TOP, J>(df.a(yv, J), up, z.a_diag, z.a_left, top_a,
+                                               J == 0 && fd0, z.wa);
+      z.a_diag = up;
+      z.a_left = va;
+      if (CAP) cap = (capj == J && !capb) ? va : cap;
+      if constexpr (J > 0) {
+        const T vb = row_pair_cell<T, PATH, TOP, 16 + J - 1>(df.b(yv, J - 1), z.va_prev, z.b_diag,
+                                                          z.b_left, top_b, J == 1 && fd0, z.wb);
+        z.b_diag = z.va_prev;
+        z.b_left = vb;
+        col[J - 1] = vb;
+        if (CAP) cap = (capj == J - 1 && capb) ? vb : cap;
+      }
+      z.va_prev = va;
+      RowPairCols<T, R, PATH, TOP, CAP, J + 1>::run(col, yv, df, z, top_a, top_b, fd0, capj, capb, cap);
+    }
+  }
+};
+template <typename T, int R, bool PATH, bool TOP, bool CAP>
+__device__ __forceinline__ T step_row_pair(T (&col)[R], const YCols<T, R> &yv, const XPair<T> &x,
+                                           T la, T lb, T dg, bool top_a, bool top_b, bool fd0,
+                                           unsigned &word, int capj, bool capb, T &cap) {
+  RowPairState<T> z{la, dg, lb, la, T(0), 0u, 0u};
+  RowDiffs<T, R> df(x);
+  RowPairCols<T, R, PATH, TOP, CAP, 0>::run(col, yv, df, z, top_a, top_b, fd0, capj, capb, cap);
+  col[R - 1] = row_pair_cell<T, PATH, TOP, 16 + R - 1>(
+      df.b(yv, R - 1), z.va_prev, z.b_diag, z.b_left, top_b, R == 1 && fd0, z.wb);
+  if (CAP) cap = (capj == R - 1 && capb) ? col[R - 1] : cap;
+  if (PATH) word = z.wa | z.wb;
+  return z.a_left;
+}
 
 }  // namespace odba

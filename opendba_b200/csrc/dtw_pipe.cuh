@@ -86,7 +86,6 @@ struct BandGate {
   static constexpr bool kActive = true;
   PipeGate g;
   int base;
-  __device__ __forceinline__ void wait_in(int k) { g.wait_in(base + k); }
   __device__ __forceinline__ void publish(int k) { g.publish(base + k); }
   __device__ __forceinline__ bool ready(int k) { return g.ready(base + k); }
   __device__ __forceinline__ void fail() { g.fail(); }

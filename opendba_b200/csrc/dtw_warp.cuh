@@ -1,0 +1,195 @@
+// One warp sweeps one swath of a cost matrix (distances only): the form that
+// fills the GPU with many matrices at the least cost per cell.
+//
+// Rows come in chunks of 32 pairs.  The warp stages a chunk's samples and
+// left-edge values in shared memory while it sweeps the chunk before, collects
+// the right edge there and stores it 32 pairs at a time, so that a step is the
+// cells, two shuffles, two shared loads and one shared store and no lane
+// branches.  Lanes outside the matrix compute values nobody reads: above the
+// first row a lane is re-set when it reaches it (the first 31 steps), below the
+// last row nothing is stored; only the steps that need the open-end top row or
+// the last cell run a slower form.
+//
+// What bounds it: the issue port.  A float cell is half a packed subtraction, a
+// three-input minimum and a multiply-add, 3.9 cycles per warp cell and scheduler
+// in a loop of nothing else; a double one two compare-and-selects, 13.6.  300
+// float series of 2000-8000 samples (all pairs): 4.5 cycles per cell, padding
+// and fill included, 141 ms (a form that shuffled and packed the samples and
+// stored the edge from one lane by branch: 147).
+#pragma once
+
+#include <type_traits>
+
+#include "dtw_path.cuh"
+
+namespace odba {
+
+constexpr int kWarpChunk = 32;  // row pairs (steps) per chunk
+
+template <typename T>
+struct WarpSmem {
+  // the pairs of two chunks, twice: a chunk's reads (pair t - lane) never wrap
+  alignas(16) XPair<T> x[4 * kWarpChunk];
+  alignas(16) T ein[2 * kWarpChunk];   // left edge of the chunk
+  alignas(16) T eout[2 * kWarpChunk];  // right edge, pair t - 31 at step t
+  alignas(16) T sink[2 * kWarpChunk];  // where the lanes without a right edge store
+};
+
+// One swath for one warp.
+template <typename T>
+struct SwathJob {
+  const T *x;         // first series (rows), length m
+  const T *y;         // second series (columns), length n
+  int m, n;
+  int c0;             // first column of this swath
+  int r0;             // first computed row: 0, or 1 with open start (row 0 is all zeros)
+  const T *edge_in;   // C[r][c0-1] by r - r0, or nullptr for the first swath
+  T *edge_out;        // receives C[r][c_last] by r - r0, or nullptr
+  bool open_end;
+  bool free_diag0;    // column c0 is a reference swath-left column (c0 % 1024 == 0, c0 > 0)
+  bool track = false; // keep the right edge's EdgeStat (needs edge_out)
+  T corner_init;      // diagonal input of lane 0 at its first row
+};
+
+// Sweeps one swath.  last: the swath holds column n - 1; corner then receives
+// cell (m - 1, n - 1) in every lane.  Returns the right edge's EdgeStat in
+// every lane (the big value unless job.track).
+template <typename T, int R>
+__device__ __forceinline__ EdgeStat<T> sweep_warp(const SwathJob<T> &job, WarpSmem<T> &sm, bool last,
+                                                  T &corner) {
+  using V2 = typename Pair2<T>::V;
+  const int lane = threadIdx.x & 31;
+  const int r0 = job.r0, rows = job.m - r0;
+  const T init = r0 ? T(0) : Num<T>::big();
+  EdgeStat<T> st{Num<T>::big(), Num<T>::big()};
+  if (rows <= 0) {  // open start over a single row: all zeros
+    if (last) corner = init;
+    return st;
+  }
+  const int pairs = (rows + 1) / 2, steps = pairs + 31;
+  YCols<T, R> yv;
+  yv.load(job.y, job.c0 + lane * R, job.n);
+  T col[R];
+#pragma unroll
+  for (int j = 0; j < R; ++j) col[j] = init;
+  T a_last = init, dg = init, cap = T(0);
+  const bool lane0 = lane == 0, lane31 = lane == 31;
+  const T dinit = lane0 ? job.corner_init : init;
+  const bool fd0 = job.free_diag0 && lane0;
+  const bool has_in = job.edge_in != nullptr, has_out = job.edge_out != nullptr;
+  const int last_pair = (rows - 1) >> 1;
+  const bool last_is_b = ((rows - 1) & 1) != 0;
+  const bool oe_top = job.open_end && job.m >= 2;  // a single-row matrix has no open-end rule
+  // the lane and register of column n - 1
+  const int cap_lane = last ? (job.n - 1 - job.c0) / R : 0;
+  const int capj = last && lane == cap_lane ? job.n - 1 - job.c0 - cap_lane * R : -1;
+  // steps [slow0, slow1) run the slow form
+  const int slow0 = oe_top ? last_pair : last ? last_pair + cap_lane : steps;
+  const int slow1 = oe_top ? last_pair + 32 : last ? slow0 + 1 : steps;
+
+  // this lane's row pair of the next chunk
+  T nx0 = T(0), nx1 = T(0), ne0 = T(0), ne1 = T(0);
+  auto load = [&](int k) {
+    if (k >= pairs) return;
+    const int row = 2 * k;
+    nx0 = job.x[r0 + row];
+    nx1 = job.x[r0 + (row + 1 < rows ? row + 1 : row)];
+    if (has_in) {
+      const V2 e = __ldcg(reinterpret_cast<const V2 *>(job.edge_in + row));
+      ne0 = e.x;
+      ne1 = e.y;
+    }
+  };
+  auto put = [&](int k) {
+    if (k >= pairs) return;
+    XPair<T> *p = &sm.x[k & (2 * kWarpChunk - 1)];
+    XPair<T>::put(p, 0, nx0);
+    XPair<T>::put(p, 1, nx1);
+    p[2 * kWarpChunk] = p[0];
+    if (has_in) {
+      sm.ein[2 * lane] = ne0;
+      sm.ein[2 * lane + 1] = ne1;
+    }
+  };
+  if (!has_in) sm.ein[2 * lane] = sm.ein[2 * lane + 1] = Num<T>::big();
+  load(lane);
+  put(lane);
+  __syncwarp();
+
+  V2 *os = reinterpret_cast<V2 *>(lane31 ? sm.eout : sm.sink);
+  const V2 *es = reinterpret_cast<const V2 *>(sm.ein);
+  for (int t0 = 0; t0 < steps; t0 += kWarpChunk) {
+    const int lim = steps - t0 < kWarpChunk ? steps - t0 : kWarpChunk;
+    load(t0 + kWarpChunk + lane);
+    const XPair<T> *xs = sm.x + ((t0 - lane) & (2 * kWarpChunk - 1));
+    auto step = [&](auto slow_c, int s) {
+      constexpr bool SLOW = decltype(slow_c)::value;
+      const XPair<T> xv = xs[s];
+      const V2 ev = es[s];
+      T la = __shfl_up_sync(kFull, a_last, 1);
+      T lb = __shfl_up_sync(kFull, col[R - 1], 1);
+      la = lane0 ? ev.x : la;
+      lb = lane0 ? ev.y : lb;
+      const T diag = dg;
+      dg = lb;
+      unsigned word = 0u;
+      const int k = t0 + s - lane;
+      const bool top = SLOW && oe_top && k == last_pair;
+      T c2 = cap;
+      a_last = step_row_pair<T, R, false, SLOW, SLOW>(col, yv, xv, la, lb, diag, top && !last_is_b,
+                                                      top && last_is_b, fd0, word, capj, last_is_b,
+                                                      c2);
+      if (SLOW) cap = k == last_pair ? c2 : cap;
+      V2 v;
+      v.x = a_last;
+      v.y = col[R - 1];
+      os[s] = v;
+    };
+    // one copy of each form of the step: what runs next to other swath widths
+    // has to share the instruction cache with them
+    for (int s = 0; s < lim;) {
+      if (t0 == 0 && s == lane) {  // the lane's first row pair
+        dg = dinit;
+#pragma unroll
+        for (int j = 0; j < R; ++j) col[j] = init;
+      }
+      int s1 = t0 == 0 ? s + 1 : lim;
+      if (t0 + s < slow0 || t0 + s >= slow1) {
+        if (t0 + s < slow0 && s1 > slow0 - t0) s1 = slow0 - t0;
+#pragma unroll 1
+        for (; s < s1; ++s) step(std::false_type{}, s);
+      } else {
+        step(std::true_type{}, s++);
+      }
+    }
+    __syncwarp();
+    if (has_out) {
+      const int k = t0 - 31 + lane, row = 2 * k;
+      if (lane < lim && k >= 0 && row < rows) {
+        const V2 v = reinterpret_cast<const V2 *>(sm.eout)[lane];
+        __stcg(reinterpret_cast<V2 *>(job.edge_out + row), v);
+        if (job.track) {
+          if (shortcut_row<T>(r0 + row)) st.emin = Num<T>::min2(st.emin, v.x);
+          if (row == rows - 1) st.etop = v.x;
+          if (row + 1 < rows) {
+            if (shortcut_row<T>(r0 + row + 1)) st.emin = Num<T>::min2(st.emin, v.y);
+            if (row + 1 == rows - 1) st.etop = v.y;
+          }
+        }
+      }
+    }
+    put(t0 + kWarpChunk + lane);
+    __syncwarp();
+  }
+  if (job.track) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      st.emin = Num<T>::min2(st.emin, __shfl_xor_sync(kFull, st.emin, off));
+      st.etop = Num<T>::min2(st.etop, __shfl_xor_sync(kFull, st.etop, off));
+    }
+  }
+  if (last) corner = __shfl_sync(kFull, cap, cap_lane);
+  return st;
+}
+
+}  // namespace odba

@@ -17,13 +17,15 @@
 #include <cmath>
 #include <cstdint>
 
-#include "dtw_device.cuh"
+#include "dtw_warp.cuh"
 
 namespace odba {
 namespace {
 
 constexpr int kWarpsPerBlock = 4;
-constexpr int kMinBlocksPerSM = 3;  // 12 warps per SM measured fastest (16 is slower, 20 spills)
+// 12 warps per SM: 300 float series of 2000-8000 samples take 140 ms, with 8
+// warps 155, with 16 (128 registers: the widest swaths spill) 152.
+constexpr int kMinBlocksPerSM = 3;
 
 template <typename T>
 struct PairwiseArgs {
@@ -38,7 +40,25 @@ struct PairwiseArgs {
   T *edges;
   unsigned long long edge_stride;  // elements per edge buffer
   int open_start, open_end;
+  int classes;                     // passes over the pairs, largest first (size_classes)
 };
+
+// Largest pairs first, without a sort: the warps go over the range
+// kSizeClasses times and take, each time, the pairs of one class of matrix
+// size (sixteenths of max_len^2, the largest class first), so that the pairs
+// left for the end are the small ones.  A skipped pair costs an atomic and two
+// loads.  100 double series of 1000-4000 samples (2.8 pairs per warp): 14.30 ms
+// in index order, 14.48 / 13.99 / 13.45 with 4 / 8 / 16 classes; 300 float
+// series of 2000-8000 (25 per warp): 142.0 and 141.3.  Below two pairs per warp
+// nearly all start at once and the skips cost more than the order gives (64
+// series, 1.1 per warp: 288 and 296 us); above kClassWaves the tail is less
+// than the skips.
+constexpr int kSizeClasses = 16;
+constexpr unsigned long long kClassWaves = 64;
+
+inline int size_classes(unsigned long long npairs, int warps) {
+  return npairs >= 2ull * warps && npairs <= kClassWaves * warps ? kSizeClasses : 1;
+}
 
 __device__ __forceinline__ long long row_start(long long s, long long n) {
   return s * n - s * (s + 1) / 2;
@@ -67,14 +87,6 @@ __device__ __forceinline__ T pair_distance(T corner, int m, int n, int os, int o
   return T(v);
 }
 
-template <typename T, int R, bool TRACK>
-__device__ __forceinline__ EdgeStat<T> run_swath(const SwathJob<T> &job, bool last, T &corner) {
-  T col[R];
-  const EdgeStat<T> st = sweep_swath<T, R, NoGate, TRACK>(job, col);
-  if (last) corner = pick_column<T, R>(col, job.c0, job.n - 1);
-  return st;
-}
-
 // The reference's open-end shortcut (dtw.hpp:74-129, open end without open
 // start) is checked on the left edge of every 1024-column reference swath that
 // starts past the last row: if that edge's value on the last row equals its
@@ -96,18 +108,21 @@ __device__ __forceinline__ bool shortcut_fires(const EdgeStat<T> &st, int m, T &
 }
 
 // Full swaths use RF registers per lane (swath width 32*RF); the last, partial
-// swath uses the smallest multiple of RQ registers that covers it.  TRACK:
-// the pair may take the open-end shortcut (off at compile time for launches
-// without an open end, so that their sweep carries no extra work).
-template <typename T, int RF, int RQ, bool TRACK>
-__device__ void sweep_pair(SwathJob<T> job, T *e0, T *e1, T &corner) {
+// swath uses the smallest multiple of RQ registers that covers it.  RQ = 8:
+// every width is code of its own, and the warps of an SM run different widths
+// next to each other.  With RQ = 4 (8 float widths) and five copies of the step
+// per width they spend half of their time waiting for instructions: pairs of
+// 8-48 series of 200-2000 samples took 4.46 ms, with two copies and RQ = 8
+// 1.57, RQ = 16 1.54; full-width work pays 0.4% for RQ = 8 and 2% for 16.
+template <typename T, int RF, int RQ>
+__device__ void sweep_pair(SwathJob<T> job, WarpSmem<T> &sm, T *e0, T *e1, T &corner) {
   constexpr int W = 32 * RF;
   int k = 0;
   for (int c0 = 0; c0 < job.n; c0 += W, ++k) {
     const int width = job.n - c0 < W ? job.n - c0 : W;
     const bool last = c0 + W >= job.n;
     job.c0 = c0;
-    job.track = TRACK && swath_checks_shortcut<T>(c0, W, job.m, job.n, job.open_end, job.r0);
+    job.track = swath_checks_shortcut<T>(c0, W, job.m, job.n, job.open_end, job.r0);
     // ping-pong: swath k writes buffer k%2 and reads buffer (k+1)%2
     job.edge_in = c0 ? ((k & 1) ? e0 : e1) : nullptr;
     job.edge_out = last ? nullptr : ((k & 1) ? e1 : e0);
@@ -117,12 +132,12 @@ __device__ void sweep_pair(SwathJob<T> job, T *e0, T *e1, T &corner) {
     const int rq = (rneed + RQ - 1) / RQ * RQ;
     EdgeStat<T> st{Num<T>::big(), Num<T>::big()};
     if (rq >= RF) {
-      st = run_swath<T, RF, TRACK>(job, last, corner);
+      st = sweep_warp<T, RF>(job, sm, last, corner);
     } else {
       switch (rq / RQ) {
-#define ODBA_CASE(K)                                          \
-  case K:                                                     \
-    if constexpr (K * RQ < RF) st = run_swath<T, K * RQ, TRACK>(job, last, corner); \
+#define ODBA_CASE(K)                                                       \
+  case K:                                                                  \
+    if constexpr (K * RQ < RF) st = sweep_warp<T, K * RQ>(job, sm, last, corner); \
     break;
         ODBA_CASE(1)
         ODBA_CASE(2)
@@ -136,20 +151,16 @@ __device__ void sweep_pair(SwathJob<T> job, T *e0, T *e1, T &corner) {
           break;
       }
     }
-    // the next swath's lane 0 reads what this swath's lane 31 wrote
+    // the next swath reads what this swath's lanes stored
     __syncwarp();
-    if (TRACK && job.track) {
-      st.emin = __shfl_sync(kFull, st.emin, 31);
-      st.etop = __shfl_sync(kFull, st.etop, 31);
-      if (shortcut_fires<T>(st, job.m, corner)) return;
-    }
+    if (job.track && shortcut_fires<T>(st, job.m, corner)) return;
   }
 }
 
-template <typename T, int RF, int RQ, bool TRACK>
+template <typename T, int RF, int RQ>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, kMinBlocksPerSM)
     pairwise_kernel(PairwiseArgs<T> a) {
-  __shared__ __align__(16) T stage_mem[kWarpsPerBlock * kStageElems];
+  __shared__ WarpSmem<T> sm[kWarpsPerBlock];
   const int lane = threadIdx.x & 31;
   const long long slot = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   T *e0 = a.edges + slot * 2 * a.edge_stride;
@@ -158,12 +169,22 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, kMinBlocksPerSM)
     unsigned long long q = 0;
     if (lane == 0) q = atomicAdd(a.counter, 1ull);
     q = __shfl_sync(kFull, q, 0);
-    if (q >= a.npairs) break;
+    int cls = 0;
+    while (q >= a.npairs && cls < a.classes) {
+      q -= a.npairs;
+      ++cls;
+    }
+    if (cls == a.classes) break;
     const long long p = (long long)(a.pbeg + a.npairs - 1 - q);
     int s, j;
     pair_of(p, a.n, s, j);
+    if (a.classes > 1) {
+      const float top = float(a.edge_stride - 32);
+      const float part = float(a.lens[s]) * float(a.lens[j]) / (top * top);  // of the largest matrix
+      const int c = a.classes - 1 - int(part * float(a.classes));
+      if ((c < 0 ? 0 : c) != cls) continue;
+    }
     SwathJob<T> job;
-    job.stage = stage_mem + (threadIdx.x >> 5) * kStageElems;
     job.x = a.series + a.offsets[s];
     job.m = int(a.lens[s]);
     job.y = a.series + a.offsets[j];
@@ -177,7 +198,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, kMinBlocksPerSM)
       continue;
     }
     T corner = T(0);
-    sweep_pair<T, RF, RQ, TRACK>(job, e0, e1, corner);
+    sweep_pair<T, RF, RQ>(job, sm[threadIdx.x >> 5], e0, e1, corner);
     if (lane == 0) a.dists[p] = pair_distance<T>(corner, job.m, job.n, a.open_start, a.open_end);
   }
 }
@@ -186,11 +207,11 @@ template <typename T>
 struct Tune;
 template <>
 struct Tune<float> {
-  static constexpr int RF = 32, RQ = 4;
+  static constexpr int RF = 32, RQ = 8;
 };
 template <>
 struct Tune<double> {
-  static constexpr int RF = 16, RQ = 4;
+  static constexpr int RF = 16, RQ = 8;
 };
 
 // Resident blocks of pairwise_kernel on the current device, cached per device
@@ -208,7 +229,7 @@ int grid_size() {
   int sms = 0, per_sm = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-      &per_sm, pairwise_kernel<T, Tune<T>::RF, Tune<T>::RQ, false>, kWarpsPerBlock * 32, 0);
+      &per_sm, pairwise_kernel<T, Tune<T>::RF, Tune<T>::RQ>, kWarpsPerBlock * 32, 0);
   if (per_sm < 1) per_sm = 1;
   if (sms < 1) sms = 1;
   const int g = sms * per_sm;
