@@ -39,6 +39,7 @@ namespace {
 constexpr int kRoundWarps = 4;
 constexpr int kReduceWarps = 4;  // centroid indices per block of the ordered reducer
 constexpr int kReduceThreads = kReduceWarps * 32;
+constexpr int kReduceBlocksF32 = 6, kReduceBlocksF64 = 4;
 constexpr int kPlanThreads = 1024;  // members per step of the plan's prefix sums
 constexpr int kRankMembers = 16384;  // longest-first task order computed up to this many members
 // move codes of the reference's path matrix (dtw.hpp:10-16); kMoveDiag,
@@ -894,16 +895,26 @@ __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(
 
 // grid: (ceil(max centroid length / 256), jobs)
 template <typename T>
-__global__ void __launch_bounds__(kReduceThreads) reduce_kernel(RoundArgs<T> a) {
+__global__ void
+__launch_bounds__(kReduceThreads, sizeof(T) == 4 ? kReduceBlocksF32 : kReduceBlocksF64)
+    reduce_kernel(RoundArgs<T> a) {
   // One warp per centroid index: the index's sum is a chain of additions in
   // the reference's order (members in order, each member's samples from the
   // highest down, the stripe-mode extra sample last), so the warp's lanes
   // load the samples of consecutive members at once (lane l the l-th group
-  // of kMpl members of a chunk) and lay them out in that order in the warp's
-  // shared-memory buffer; lane 0 then adds the buffer.  Many warps per SM
-  // keep the loads and the chains of different indices in flight together.
+  // of mpl <= kMpl members of a chunk) and lay them out in that order in the
+  // warp's shared-memory buffer; lane 0 then adds the buffer.  Many warps per
+  // SM keep the loads and the chains of different indices in flight together.
+  //
+  // What bounds it is the chain of four dependent loads per member (offset,
+  // range, series, sample).  The members of a chunk spread evenly over the
+  // lanes, and each lane has its members' first samples in flight together.
+  // 8 members per lane always, one load after the other, against this: 64
+  // members of 512-1024 samples 33 -> 13 us, 690 in 24 jobs 79 -> 28, 400 of
+  // 3000-8000 203 -> 112 (184 with kMpl = 8, four blocks per SM), 100 double of
+  // 1000-4000 67 -> 57.
   constexpr int kCap = 8192 / int(sizeof(T));  // samples per warp's buffer
-  constexpr int kMpl = 8;                      // members per lane per chunk
+  constexpr int kMpl = 4;                      // members per lane per chunk
   __shared__ T s_buf[kReduceWarps][kCap];
   __shared__ double s_max[kReduceWarps];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -918,23 +929,31 @@ __global__ void __launch_bounds__(kReduceThreads) reduce_kernel(RoundArgs<T> a) 
     T *buf = s_buf[wid];
     const int kb = a.mbeg[jb], ke = a.mend[jb];
     for (int k0 = kb; k0 < ke; k0 += 32 * kMpl) {
+      const int mpl = ke - k0 >= 32 * kMpl ? kMpl : (ke - k0 + 31) / 32;
       int2 r[kMpl];
       int e[kMpl];
       const T *sq[kMpl];
+      T first[kMpl];
       int n_l = 0;
 #pragma unroll
       for (int u = 0; u < kMpl; ++u) {
-        const int m = k0 + lane * kMpl + u;
+        const int m = k0 + lane * mpl + u;
         r[u] = make_int2(1, 0);
         e[u] = -1;
         sq[u] = a.series;
-        if (m < ke) {
+        if (u < mpl && m < ke) {
           const unsigned long long ro = a.rng_off[m];
           r[u] = a.ranges[ro + t];
           sq[u] = a.series + a.offsets[a.mseries[m]];
           if (a.extra) e[u] = a.extra[ro + t];
         }
-        if (r[u].y >= r[u].x) n_l += r[u].y - r[u].x + 1 + (e[u] >= 0 ? 1 : 0);
+      }
+#pragma unroll
+      for (int u = 0; u < kMpl; ++u) {
+        first[u] = T(0);
+        if (r[u].y < r[u].x) continue;
+        n_l += r[u].y - r[u].x + 1 + (e[u] >= 0 ? 1 : 0);
+        first[u] = __ldg(sq[u] + r[u].y);
       }
       int incl = n_l;
 #pragma unroll
@@ -949,7 +968,8 @@ __global__ void __launch_bounds__(kReduceThreads) reduce_kernel(RoundArgs<T> a) 
 #pragma unroll
         for (int u = 0; u < kMpl; ++u) {
           if (r[u].y < r[u].x) continue;
-          for (int i = r[u].y; i >= r[u].x; --i) buf[p++] = __ldg(sq[u] + i);
+          buf[p++] = first[u];
+          for (int i = r[u].y - 1; i >= r[u].x; --i) buf[p++] = __ldg(sq[u] + i);
           if (e[u] >= 0) buf[p++] = __ldg(sq[u] + e[u]);
         }
         __syncwarp();
