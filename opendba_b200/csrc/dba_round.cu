@@ -309,9 +309,13 @@ __device__ __forceinline__ bool walk_member_runs(const RoundArgs<T> &a, const Me
                                                  int os, int oe, int2 *runs);
 
 // Path DTW, a block per swath (sweep_block).  PIPE: task q is band
-// q / (nmem * max_swaths) of swath (q / nmem) % max_swaths of the (q % nmem)-th
-// member in alignment order, so a member's swaths run in different blocks at
-// once (few or long members keep the GPU busy).  The right edge of swath s
+// q / (nmem * max_swaths) of a swath of the (q % nmem)-th member in alignment
+// order, in turn (q / nmem) % max_swaths, so a member's swaths run in different
+// blocks at once (few or long members keep the GPU busy).  The last swaths of
+// all members share the last turn: a member of one swath does not go before the
+// second swath of a longer one, whose chain ends later (690 members of 200-2000
+// samples in 24 jobs: 480 us with the first swaths in one turn, 441 so; where
+// all members have the same swaths nothing changes).  The right edge of swath s
 // goes to buffer s % 2 of the member with one progress word per (member,
 // swath), as in the all-pairs swath pipeline.  BAND (odba_round_set_bands,
 // member_band): a band starts from the last row and edge corner the band below
@@ -331,11 +335,12 @@ __device__ __forceinline__ bool walk_member_runs(const RoundArgs<T> &a, const Me
 // of 1000-4000 in double 2.51 -> 1.53, 400 of 3000-8000 (which fill the GPU)
 // 6.57 -> 5.86.
 //
-// Blocks per SM: four (two for double) fill the SM; more, which the registers
+// Blocks per SM: three (two for double) fill the SM; more, which the registers
 // would allow, only spread its issue slots over more chains, and each chain's
 // last swath then ends later (400 members: 6.54 ms with six, 6.24 with five,
-// 5.86 with four, 5.83 with three; double 1.71 with four, 1.53 with two).
-constexpr int kRoundBlocksF32 = 4, kRoundBlocksF64 = 2;
+// 5.86 with four, 5.79 with three, 6.8 with two; 690 of 200-2000 492 us with
+// four, 480 with three, 557 with two; double 1.71 with four, 1.53 with two).
+constexpr int kRoundBlocksF32 = 3, kRoundBlocksF64 = 2;
 template <typename T, bool PIPE, bool BAND>
 __global__ void
 __launch_bounds__(kBlkThreads, sizeof(T) == 4 ? kRoundBlocksF32 : kRoundBlocksF64)
@@ -348,6 +353,8 @@ __launch_bounds__(kBlkThreads, sizeof(T) == 4 ? kRoundBlocksF32 : kRoundBlocksF6
   auto member_of = [&](unsigned long long qi) {
     return a.order ? a.order[qi] : a.nmem - 1 - int(qi);
   };
+  // the turn of a member's first swath
+  auto late = [&](const MemberGeom &g) { return g.swaths < a.max_swaths ? a.max_swaths - g.swaths : 0; };
   for (;;) {
     if (feeder && lane == 0) {
       // the next task that exists
@@ -359,7 +366,7 @@ __launch_bounds__(kBlkThreads, sizeof(T) == 4 ? kRoundBlocksF32 : kRoundBlocksF6
         int jb;
         const MemberGeom g = geom_of<T>(a, member_of(PIPE ? ql % a.nmem : q), jb);
         if (!(a.jflags[jb] & 4)) continue;
-        if (PIPE && int(ql / a.nmem) >= g.swaths) continue;
+        if (PIPE && (unsigned)(int(ql / a.nmem) - late(g)) >= (unsigned)g.swaths) continue;
         if (PIPE && BAND && int(q / layer) >= member_band(g, a.nbands, 0).count) continue;
         break;
       }
@@ -370,10 +377,11 @@ __launch_bounds__(kBlkThreads, sizeof(T) == 4 ? kRoundBlocksF32 : kRoundBlocksF6
     if (q >= ntasks) break;
     const int b = PIPE && BAND ? int(q / layer) : 0;
     const unsigned long long ql = PIPE ? q - (unsigned long long)b * layer : 0;
-    const int s_first = PIPE ? int(ql / a.nmem) : 0;
-    const int k = member_of(PIPE ? ql - (unsigned long long)s_first * a.nmem : q);
+    const int turn = PIPE ? int(ql / a.nmem) : 0;
+    const int k = member_of(PIPE ? ql - (unsigned long long)turn * a.nmem : q);
     int jb;
     const MemberGeom g = geom_of<T>(a, k, jb);
+    const int s_first = PIPE ? turn - late(g) : 0;
     const int flags = a.jflags[jb];
     const Band bd = member_band(g, PIPE && BAND ? a.nbands : 1, b);
     const int os = flags & 1, oe = (flags >> 1) & 1;

@@ -68,3 +68,17 @@ def test_more_swaths_than_blocks(env, mode, dtype):
         got = _ranges(env, centroid, members, *mode)
         for k in range(len(members)):
             assert np.array_equal(got[k], want[k % len(kinds)]), f"member {k}"
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_mixed_swath_counts(env, dtype):
+    # open end, centroid shorter: the members take the columns, one to four
+    # swaths each, and only the last swaths share a turn
+    rng = np.random.default_rng(5)
+    centroid = _signal(rng, 300, dtype)
+    kinds = [_signal(rng, L, dtype) for L in (100, 299, 301, 1000, 1024, 1025, 2048, 2049, 3073, 4000)]
+    members = kinds * 60
+    want = O.member_ranges(centroid, kinds, 0, 1, fma_mode=1)
+    got = _ranges(env, centroid, members, 0, 1)
+    for k in range(len(members)):
+        assert np.array_equal(got[k], want[k % len(kinds)]), f"member {k}"
