@@ -539,23 +539,41 @@ bool plan_fits(int plan, unsigned long long npairs, uint64_t max_len, size_t ws_
 
 // The pipeline pays while its blocks are few enough to run a pair's swaths side
 // by side: it takes a pair's steps a quarter to a half of the one-warp sweep's
-// time, but fills the GPU with a third as many pairs.  Measured on one B200
-// (one-warp time / pipeline time, all pairs of n series): float, 2000-4000
-// samples, 1128 / 1770 / 2016 pairs 1.72 / 1.23 / 1.09, 1000-2000 samples 1.45 /
-// 1.07 / 0.92, 900-1100 samples 630 / 1128 / 1540 pairs 1.70 / 1.07 / 0.79,
-// 512-1024 samples 1.66 / 1.11 / 0.86, 20-40 samples 276 / 630 pairs 1.08 / 0.71;
-// double, 2000-4000 samples 1128 / 1770 pairs 1.68 / 1.08, 900-1100 samples 630 /
-// 1128 pairs 1.59 / 0.94, 150-400 samples 276 / 630 pairs 1.76 / 0.92, 20-40
-// samples 276 pairs 0.81.
+// time, but fills the GPU with a third as many pairs, and a second swath that is
+// nearly empty costs it a block all the same.  Measured on one B200 (one-warp
+// time / pipeline time, all pairs of n series), float:
+//   2000-4000 samples  1431 / 1770 / 2016 / 2278 pairs  1.37 / 1.18 / 1.02 / 0.95
+//   1000-2000          1128 / 1431 / 1770               1.46 / 1.18 / 0.95
+//   1200-1500          780 / 1128 / 1770                1.42 / 1.01 / 0.68
+//   900-1100           861 / 1128                       1.17 / 0.92
+//   512-1024           861 / 1128 / 1431                1.23 / 1.08 / 0.90
+//   150-400            630 / 861                        1.22 / 0.92
+//   64-128             378 / 780                        1.14 / 0.71
+//   20-40              435 / 630                        1.02 / 0.72
+// double:
+//   2000-4000          1770 / 2278                      1.34 / 1.13
+//   1000-2000          1770 / 2016                      1.15 / 1.04
+//   900-1100           861 / 1128 / 1431                1.39 / 1.13 / 0.89
+//   512-1024           1128 / 1431                      1.17 / 0.98
+//   150-400            630 / 861 / 1128                 1.15 / 1.08 / 0.81
+//   64-128             378 / 780                        1.14 / 0.70
+//   20-40              276 / 630                        0.93 / 0.57
+// Above one pair per resident warp (1776) the workspace that does not know the
+// number of pairs would not hold the pipeline's edges, so the rule ends there.
 template <typename T>
 int rule_of_thumb(unsigned long long npairs, uint64_t max_len) {
   const unsigned long long slots = (unsigned long long)grid_size<T>() * kWarpsPerBlock;
   const uint64_t swaths = (max_len + kBlkCols - 1) / kBlkCols;
+  const bool f32 = sizeof(T) == 4;
   unsigned long long most;
-  if (sizeof(T) == 4)
-    most = swaths >= 3 ? slots : swaths == 2 ? slots * 2 / 3 : max_len >= 64 ? slots / 2 : slots / 6;
+  if (swaths >= 3)
+    most = slots;
+  else if (swaths == 2)
+    most = max_len >= 1536 ? (f32 ? slots * 15 / 16 : slots) : (f32 ? slots * 5 / 8 : slots * 2 / 3);
+  else if (max_len >= 256)
+    most = max_len >= 512 ? (f32 ? slots * 2 / 3 : slots * 3 / 4) : (f32 ? slots * 3 / 7 : slots / 2);
   else
-    most = swaths >= 3 ? slots * 2 / 3 : swaths == 2 ? slots * 2 / 5 : max_len >= 64 ? slots / 4 : 0;
+    most = f32 || max_len >= 64 ? slots / 4 : 0;
   return npairs < most ? ODBA_PLAN_SWATH_PIPELINE : ODBA_PLAN_WHOLE_PAIR;
 }
 
