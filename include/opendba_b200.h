@@ -95,9 +95,10 @@ int odba_dtw_pairwise_range_f64(const double *series, const uint64_t *offsets, c
  *   ODBA_PLAN_WHOLE_PAIR             one warp per pair, 1024-column swaths
  *                                    (512 for double), persistent work queue;
  *   ODBA_PLAN_WHOLE_PAIR_HALF_SWATH  the same with half-width swaths;
- *   ODBA_PLAN_SWATH_PIPELINE         many warps per pair: swaths of one pair
- *                                    run on different warps, each waiting
- *                                    (bounded) on the previous swath's edge.
+ *   ODBA_PLAN_SWATH_PIPELINE         a block of warps per 1024-column swath:
+ *                                    swaths of one pair run in different
+ *                                    blocks, each waiting (bounded) on the
+ *                                    previous swath's edge.
  * The plan is chosen per key (element size, len_bucket = floor(log2 max_len),
  * count_bucket = floor(log2 pairs)): a plan pinned with odba_tune_set; else,
  * in tuning mode (odba_tune_mode(1)), each eligible plan not yet measured for
@@ -123,11 +124,9 @@ int odba_tune_load(const char *path);
 
 /* ---- row bands of the DBA round's path DTW ----------------------------------------
  * No reference counterpart (a tuning knob; results do not depend on it).
- * When a round's (member, swath) tasks are fewer than about three waves of
- * the GPU's resident warps, the path DTW cuts each member's rows into bands
- * so that the last wave of tasks is short.  n in 1..8 pins the number of
- * bands for the following launches (1: none), 0 restores the automatic
- * choice.  A workspace size queried under one setting fits launches under the
+ * The path DTW can cut each member's rows into bands, tasks of their own.
+ * n in 1..8 pins the number of bands for the following launches (1: none),
+ * 0 restores the automatic choice (none).  A workspace size queried under one setting fits launches under the
  * same setting. */
 int odba_round_set_bands(int n);
 
@@ -305,9 +304,10 @@ int odba_dba_reduce_ranges_f64(const double *centroid, uint64_t centroid_len, co
  * recomputes, 1024-column stripe by stripe from the right, the tiles of
  * ckpt_rows rows below the path in parallel.  Workspace for the longest
  * member m and centroid length Lc (rows x columns after the open-end flip):
- * about (Lc/1024 * m + m/ckpt_rows * Lc) values plus m * 256 bytes (float;
- * double swaths are 512 wide) -- 80 GB for 4 M x 4 M in float with the
- * default, where a full path needs 4 TB.  In global and open-start alignment
+ * about (Lc/1024 * m + m/ckpt_rows * Lc) values plus m * 256 bytes, times the
+ * members and stripes worked on side by side (up to eight each, fewer where
+ * that would exceed 4 GB and 1 GB) -- 80 GB for 4 M x 4 M in float with
+ * 1024 rows, where a full path needs 4 TB.  In global and open-start alignment
  * the results equal odba_dba_round_* bit for bit.  With an open end they
  * follow the reference's stripe re-run, which sees the backtrack height H as
  * the first sequence's length (dba.hpp:700-721): the open-end top-row rule

@@ -4,16 +4,16 @@
 //  1. plan:      per member the orientation (the centroid goes on the Y axis
 //                when open_end and it is the shorter one, dba.hpp:497-501),
 //                the size and offset of its 2-bit path, and its path-file slot.
-//  2. path DTW:  persistent launch, one warp per member, swath by swath with the
-//                register wavefront of dtw_path.cuh; records every move and the
-//                right-edge minima the open-end shortcut needs.
-//  3. backtrack: one thread per member walks its path from the end cell back to
+//  2. path DTW:  persistent launch, a block per swath (dtw_block.cuh); records
+//                every move and the right-edge minima the open-end shortcut
+//                needs.
+//  3. backtrack: one warp per member walks its path from the end cell back to
 //                (0, 0) (updateCentroid's loop) and stores, per centroid index,
 //                the contiguous range of member samples that index receives --
 //                a path crosses every centroid index in one contiguous run.
 //                Optionally it also emits the path as (i, j, move) triples in
 //                the order of the reference's path file (io_utils.hpp:287-323).
-//  4. reduce:    one thread per centroid index adds the member samples in the
+//  4. reduce:    one warp per centroid index adds the member samples in the
 //                reference's exact order -- members in order, each member's
 //                samples from its last path row down to its first -- then
 //                divides by the pile-up count in T (dba.hpp:820-822) and takes
