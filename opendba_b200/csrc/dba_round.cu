@@ -1439,7 +1439,7 @@ int dba_batch_launch(const T *centroids, const unsigned long long *coff, const i
 namespace {
 
 constexpr int kStripeSlots = 8;       // members side by side, at most
-constexpr int kStripeGroup = 8;       // stripes per group, at most
+constexpr int kStripeGroup = 4;       // stripes per group, at most
 constexpr size_t kStripeGroupBytes = size_t(1) << 30;  // move words of all slots' groups
 constexpr size_t kStripeSlotBytes = size_t(4) << 30;   // edges and checkpoint rows of all slots
 constexpr int kStripeFill = 512;      // swaths side by side that fill the GPU
@@ -1474,6 +1474,8 @@ struct StripeArgs {
   unsigned long long prog_slot;
   unsigned *words;              // move words of a group, the stripes in column order
   unsigned long long words_slot;
+  unsigned long long words_all; // of all slots: the second buffer's offset
+  int odd_words;                // 1: groups take two buffers in turn, 0: one buffer
   int2 *runs;                   // row walk: the column interval of every row
   unsigned long long runs_slot;
   typename CostBits<T>::U *fmin, *cmin;  // per stripe: shortcut minima (forward, below H)
@@ -1509,6 +1511,12 @@ __device__ __forceinline__ const T *stripe_edge(const StripeArgs<T> &a, int slot
 __host__ __device__ inline void stripe_group(int stripes, int group, int gi, int &lo, int &hi) {
   hi = stripes - gi * group;
   lo = hi - group > 0 ? hi - group : 0;
+}
+
+// Group gi's move words: with two buffers, groups take them in turn.
+template <typename T>
+__device__ __forceinline__ unsigned *stripe_words(const StripeArgs<T> &a, int slot, int gi) {
+  return a.words + (unsigned long long)(gi & a.odd_words) * a.words_all + slot * a.words_slot;
 }
 
 // Whether the reference's re-run of stripe t at height H takes its shortcut
@@ -1629,20 +1637,16 @@ __global__ void stripe_sfwd_kernel(StripeArgs<T> a, int slot, int tlo, int thi) 
   }
 }
 
-// Block (kt, b, slot): the K-row tile kt of the group's b-th stripe, where it
-// lies below the backtrack height.
+// The K-row tile kt of group gi's b-th stripe, where it lies below the
+// backtrack height in w, for one block.
 template <typename T>
-__global__ void
-__launch_bounds__(kBlkThreads, sizeof(T) == 4 ? kRoundBlocksF32 : kRoundBlocksF64)
-    stripe_tile_kernel(StripeArgs<T> a, int group, int gi) {
-  __shared__ BlockSmem<T> sm;
-  const int kt = blockIdx.x, slot = blockIdx.z;
+__device__ __forceinline__ void stripe_tile(const StripeArgs<T> &a, BlockSmem<T> &sm, int group,
+                                            int gi, int kt, int b, int slot, const StripeWalk &w) {
   const StripeMember &mem = a.mem[slot];
   int lo, hi;
   stripe_group(mem.swaths, group, gi, lo, hi);
-  const int t = lo + int(blockIdx.y);
+  const int t = lo + b;
   if (t >= hi) return;
-  const StripeWalk w = a.walk[slot];
   const int H = w.h, K = 1 << a.shift;
   const long long rb_l = (long long)a.r0 + (long long)kt * K;
   if (w.state != 0 || rb_l >= H || stripe_fires(a, slot, t, H, w)) return;
@@ -1667,12 +1671,22 @@ __launch_bounds__(kBlkThreads, sizeof(T) == 4 ? kRoundBlocksF32 : kRoundBlocksF6
   job.row_in = kt ? a.Q + slot * a.q_slot + (unsigned long long)(kt - 1) * a.q_stride + c0 : nullptr;
   const int steps = block_steps(mem.m - a.r0);
   job.word_steps = steps;
-  job.words = a.words + slot * a.words_slot + (size_t)(t - lo) * kBlkWarps * steps * 32 +
+  job.words = stripe_words(a, slot, gi) + (size_t)(t - lo) * kBlkWarps * steps * 32 +
               (size_t)kt * (K / 2) * 32;
   T unused = T(0);
   EdgeStat<T> st;
   sweep_block<T, true, true, false, false>(job, sm, NoGate(), CkptOut<T>{nullptr, 0, 1}, false,
                                            unused, st);
+}
+
+// Block (kt, b, slot): one tile of the group.
+template <typename T>
+__global__ void
+__launch_bounds__(kBlkThreads, sizeof(T) == 4 ? kRoundBlocksF32 : kRoundBlocksF64)
+    stripe_tile_kernel(StripeArgs<T> a, int group, int gi) {
+  __shared__ BlockSmem<T> sm;
+  const StripeWalk w = a.walk[blockIdx.z];
+  stripe_tile(a, sm, group, gi, int(blockIdx.x), int(blockIdx.y), int(blockIdx.z), w);
 }
 
 template <typename T>
@@ -1695,8 +1709,8 @@ __global__ void stripe_walk_init_kernel(StripeArgs<T> a) {
 // The row walk (walk_runs) through a group, one warp per member: without an
 // open end and without a path listing.
 template <typename T>
-__global__ void __launch_bounds__(32) stripe_walk_runs_kernel(StripeArgs<T> a, int group, int gi) {
-  const int lane = threadIdx.x, slot = blockIdx.x;
+__device__ __forceinline__ void stripe_walk_runs(const StripeArgs<T> &a, int group, int gi, int slot) {
+  const int lane = threadIdx.x & 31;
   const StripeMember &mem = a.mem[slot];
   int lo, hi;
   stripe_group(mem.swaths, group, gi, lo, hi);
@@ -1708,8 +1722,8 @@ __global__ void __launch_bounds__(32) stripe_walk_runs_kernel(StripeArgs<T> a, i
   g.r0 = a.r0;
   g.steps = block_steps(mem.m - a.r0);
   RowWalk rw{w.r, w.c, w.entry};
-  const int got = walk_runs(reinterpret_cast<const unsigned short *>(a.words + slot * a.words_slot),
-                            g, lo * kBlkCols, rw, a.r0, a.runs + slot * a.runs_slot);
+  const int got = walk_runs(reinterpret_cast<const unsigned short *>(stripe_words(a, slot, gi)), g,
+                            lo * kBlkCols, rw, a.r0, a.runs + slot * a.runs_slot);
   if (lane == 0) {
     w.r = rw.r;
     w.c = rw.c;
@@ -1718,6 +1732,44 @@ __global__ void __launch_bounds__(32) stripe_walk_runs_kernel(StripeArgs<T> a, i
     w.state = got;
     a.walk[slot] = w;
   }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(32) stripe_walk_runs_kernel(StripeArgs<T> a, int group, int gi) {
+  stripe_walk_runs(a, group, gi, int(blockIdx.x));
+}
+
+// The row walk through group gi by the first blocks, one per member, and the
+// tiles of group gi + 1 by the others (two word buffers, no open end).  A tile
+// of group gi + 1 takes part or not by the height before or after the walk
+// through group gi, whichever its block finds: the rows above the later height
+// are computed for nothing, those below are the same.
+//
+// 3 members of 40k-80k samples against a 70k centroid: a group of 4 stripes takes
+// 0.33 ms on three warps and its tiles 0.25 on the whole GPU; one after the
+// other a round took 20.7 ms, beside each other 17.7 (groups of 8 stripes 18.2,
+// of 2 18.3).
+template <typename T>
+__global__ void
+__launch_bounds__(kBlkThreads, sizeof(T) == 4 ? kRoundBlocksF32 : kRoundBlocksF64)
+    stripe_walk_tile_kernel(StripeArgs<T> a, int group, int gi, int tiles) {
+  __shared__ BlockSmem<T> sm;
+  __shared__ StripeWalk s_walk;
+  if (int(blockIdx.x) < a.count) {
+    if (threadIdx.x < 32) stripe_walk_runs(a, group, gi, int(blockIdx.x));
+    return;
+  }
+  const unsigned q = blockIdx.x - a.count, per_slot = unsigned(tiles) * group;
+  const int slot = int(q / per_slot), u = int(q - slot * per_slot), b = u / tiles;
+  if (threadIdx.x == 0) {
+    const volatile StripeWalk *w = a.walk + slot;
+    s_walk.h = w->h;
+    s_walk.state = w->state;
+    s_walk.s_fwd = INT_MAX;
+  }
+  __syncthreads();
+  const StripeWalk w = s_walk;
+  stripe_tile(a, sm, group, gi + 1, u - b * tiles, b, slot, w);
 }
 
 // The rows' intervals as ranges (runs_to_ranges; the member on the rows).
@@ -1751,7 +1803,7 @@ __global__ void __launch_bounds__(32) stripe_walk_kernel(StripeArgs<T> a, int gr
   MemberGeom g;
   g.r0 = a.r0;
   g.steps = block_steps(mem.m - a.r0);
-  const unsigned short *words = reinterpret_cast<const unsigned short *>(a.words + slot * a.words_slot);
+  const unsigned short *words = reinterpret_cast<const unsigned short *>(stripe_words(a, slot, gi));
   int2 *rg = a.ranges + (unsigned long long)mem.member * a.Lc;
   int *extra = a.extra ? a.extra + (unsigned long long)mem.member * a.Lc : nullptr;
   int32_t *tri = a.triples ? a.triples + 3ull * mem.trip : nullptr;
@@ -1875,6 +1927,7 @@ struct StripeLayout {
   unsigned long long e_stride, q_stride, words_slot, e_slot, q_slot, runs_slot, min_slot;
   int swaths_max;
   int slots, group;
+  bool two;  // two word buffers (row walks beside the next group's tiles)
 };
 
 template <typename T>
@@ -1905,6 +1958,7 @@ StripeLayout stripe_layout(const uint64_t *h_lens, int n, uint64_t Lc, int os, i
   int group = S.swaths_max < kStripeGroup ? S.swaths_max : kStripeGroup;
   while (group > 1 && stripe_bytes * group * slots > kStripeGroupBytes) --group;
   S.group = group;
+  S.two = !oe && S.swaths_max > group && 2 * stripe_bytes * group * slots <= kStripeGroupBytes;
   S.words_slot = stripe_bytes / 4 * group;
   S.runs_slot = max_rows;
   S.min_slot = (unsigned long long)S.swaths_max + 1;
@@ -1913,7 +1967,7 @@ StripeLayout stripe_layout(const uint64_t *h_lens, int n, uint64_t Lc, int os, i
   S.off_prog = o; o += up(size_t(slots) * S.swaths_max * 8);
   S.off_E = o; o += up(size_t(slots) * S.e_slot * sizeof(T));
   S.off_Q = o; o += up(size_t(slots) * S.q_slot * sizeof(T));
-  S.off_W = o; o += up(size_t(slots) * S.words_slot * 4);
+  S.off_W = o; o += up(size_t(slots) * S.words_slot * 4 * (S.two ? 2 : 1));
   S.off_runs = o; o += up(size_t(slots) * S.runs_slot * sizeof(int2));
   // with an open end: the extra samples, and the shortcut minima of every stripe
   S.off_extra = o; o += oe ? up(size_t(n) * Lc * 4) : 0;
@@ -1995,6 +2049,7 @@ int dba_round_stripe_launch(const T *centroid, uint64_t Lc, const T *series,
   sa.prog_slot = (unsigned long long)S.swaths_max;
   sa.words = reinterpret_cast<unsigned *>(base + S.off_W);
   sa.words_slot = S.words_slot;
+  sa.words_all = (unsigned long long)S.slots * S.words_slot;
   sa.runs = reinterpret_cast<int2 *>(base + S.off_runs);
   sa.runs_slot = S.runs_slot;
   sa.fmin = oe ? reinterpret_cast<typename CostBits<T>::U *>(base + S.off_min) : nullptr;
@@ -2015,6 +2070,8 @@ int dba_round_stripe_launch(const T *centroid, uint64_t Lc, const T *series,
   const bool by_rows = !oe && !triples;
   const int K = 1 << sh;
   const int group = oe ? 1 : S.group;
+  const bool beside = by_rows && S.two;
+  sa.odd_words = beside ? 1 : 0;
   unsigned long long trip = 0;
   for (int k0 = 0; k0 < n; k0 += S.slots) {
     sa.count = n - k0 < S.slots ? n - k0 : S.slots;
@@ -2061,8 +2118,12 @@ int dba_round_stripe_launch(const T *centroid, uint64_t Lc, const T *series,
           // (rows below H reach a stripe's shortcut only past column H)
           if (t >= 1) stripe_min_kernel<T><<<dim3(min_blocks(sa.mem[i].m), 1), 256, 0, stream>>>(sa, i, t, t, 0);
         }
-      stripe_tile_kernel<T><<<dim3(tiles, group, sa.count), kBlkThreads, 0, stream>>>(sa, group, gi);
-      if (by_rows)
+      if (!beside || gi == 0)
+        stripe_tile_kernel<T><<<dim3(tiles, group, sa.count), kBlkThreads, 0, stream>>>(sa, group, gi);
+      if (beside && (gi + 1) * group < max_swaths)
+        stripe_walk_tile_kernel<T><<<sa.count + tiles * group * sa.count, kBlkThreads, 0, stream>>>(
+            sa, group, gi, tiles);
+      else if (by_rows)
         stripe_walk_runs_kernel<T><<<sa.count, 32, 0, stream>>>(sa, group, gi);
       else
         stripe_walk_kernel<T><<<sa.count, 32, 0, stream>>>(sa, group, gi);
