@@ -314,8 +314,8 @@ __device__ __forceinline__ bool walk_member_runs(const RoundArgs<T> &a, const Me
 // blocks at once (few or long members keep the GPU busy).  The last swaths of
 // all members share the last turn: a member of one swath does not go before the
 // second swath of a longer one, whose chain ends later (690 members of 200-2000
-// samples in 24 jobs: 480 us with the first swaths in one turn, 441 so; where
-// all members have the same swaths nothing changes).  The right edge of swath s
+// samples in 24 jobs, three blocks per SM: 480 us with the first swaths in one
+// turn, 441 so; where all members have the same swaths nothing changes).  The right edge of swath s
 // goes to buffer s % 2 of the member with one progress word per (member,
 // swath), as in the all-pairs swath pipeline.  BAND (odba_round_set_bands,
 // member_band): a band starts from the last row and edge corner the band below
@@ -335,12 +335,17 @@ __device__ __forceinline__ bool walk_member_runs(const RoundArgs<T> &a, const Me
 // of 1000-4000 in double 2.51 -> 1.53, 400 of 3000-8000 (which fill the GPU)
 // 6.57 -> 5.86.
 //
-// Blocks per SM: three (two for double) fill the SM; more, which the registers
-// would allow, only spread its issue slots over more chains, and each chain's
-// last swath then ends later (400 members: 6.54 ms with six, 6.24 with five,
-// 5.86 with four, 5.79 with three, 6.8 with two; 690 of 200-2000 492 us with
-// four, 480 with three, 557 with two; double 1.71 with four, 1.53 with two).
-constexpr int kRoundBlocksF32 = 3, kRoundBlocksF64 = 2;
+// Blocks per SM: four (two for double).  More, which the registers would allow,
+// only spread the issue slots over more chains, and each chain's last swath then
+// ends later; three are a little better where one wave of chains is all there
+// is, but lose on larger rounds.  Float, with three / four / five / six: 400
+// members of 3000-8000 samples 5.79 / 5.86 / 6.24 / 6.54 ms, 600 8.61 / 8.11 /
+// 8.39 / 8.67, 1000 13.75 / 12.95 / 13.06 / 13.09, 512 of 1000-2000 (open end)
+// 1.10 / 1.00 / 1.07 / 1.14; double 1.71 with four, 1.53 with two.
+//
+// Above about a thousand members the one-warp sweep's lower cost per cell would
+// win (2000 of 3000-8000: 22.6 ms against 25.5).
+constexpr int kRoundBlocksF32 = 4, kRoundBlocksF64 = 2;
 template <typename T, bool PIPE, bool BAND>
 __global__ void
 __launch_bounds__(kBlkThreads, sizeof(T) == 4 ? kRoundBlocksF32 : kRoundBlocksF64)
