@@ -304,10 +304,13 @@ int odba_dba_reduce_ranges_f64(const double *centroid, uint64_t centroid_len, co
  * recomputes, 1024-column stripe by stripe from the right, the tiles of
  * ckpt_rows rows below the path in parallel.  Workspace for the longest
  * member m and centroid length Lc (rows x columns after the open-end flip):
- * about (Lc/1024 * m + m/ckpt_rows * Lc) values plus m * 256 bytes, times the
- * members and stripes worked on side by side (up to eight each, fewer where
- * that would exceed 4 GB and 1 GB) -- 80 GB for 4 M x 4 M in float with
- * 1024 rows, where a full path needs 4 TB.  In global and open-start alignment
+ * (Lc/1024 * m + m/ckpt_rows * Lc) values plus m * 256 bytes for one member
+ * and one stripe at a time -- 80 GB for 4 M x 4 M in float with the default
+ * of 4096 rows, 126 GB with 1024, where a full path needs 4 TB.  Up to eight
+ * members and four stripes are worked on side by side while that takes at
+ * most 4 GB (members) and 1 GB (stripes): the size function gives the most
+ * that fits 95 % of the free device memory, and a round takes what fits the
+ * workspace it is given, down to one member and one stripe.  In global and open-start alignment
  * the results equal odba_dba_round_* bit for bit.  With an open end they
  * follow the reference's stripe re-run, which sees the backtrack height H as
  * the first sequence's length (dba.hpp:700-721): the open-end top-row rule

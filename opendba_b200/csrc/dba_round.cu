@@ -1445,8 +1445,10 @@ namespace {
 
 constexpr int kStripeSlots = 8;       // members side by side, at most
 constexpr int kStripeGroup = 4;       // stripes per group, at most
-constexpr size_t kStripeGroupBytes = size_t(1) << 30;  // move words of all slots' groups
-constexpr size_t kStripeSlotBytes = size_t(4) << 30;   // edges and checkpoint rows of all slots
+// at most, of a workspace of any size: move words of all slots' groups, and edges
+// and checkpoint rows of all slots (one stripe and one slot whatever they take)
+constexpr size_t kStripeGroupBytes = size_t(1) << 30;
+constexpr size_t kStripeSlotBytes = size_t(4) << 30;
 constexpr int kStripeFill = 512;      // swaths side by side that fill the GPU
 
 struct StripeWalk {
@@ -1935,8 +1937,11 @@ struct StripeLayout {
   bool two;  // two word buffers (row walks beside the next group's tiles)
 };
 
+// The layout with the most members and stripes side by side whose total is at
+// most `limit` bytes; the smallest layout if none is.
 template <typename T>
-StripeLayout stripe_layout(const uint64_t *h_lens, int n, uint64_t Lc, int os, int oe, int shift) {
+StripeLayout stripe_layout(const uint64_t *h_lens, int n, uint64_t Lc, int os, int oe, int shift,
+                           size_t limit) {
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
   uint64_t max_rows = 1, max_cols = 1;
   for (int k = 0; k < n; ++k) {
@@ -1953,32 +1958,57 @@ StripeLayout stripe_layout(const uint64_t *h_lens, int n, uint64_t Lc, int os, i
   const unsigned long long nq = (max_rows - (os ? 1 : 0)) / K + 1;
   S.e_slot = (unsigned long long)(S.swaths_max > 1 ? S.swaths_max - 1 : 1) * S.e_stride;
   S.q_slot = nq * S.q_stride;
+  S.min_slot = (unsigned long long)S.swaths_max + 1;
+  const size_t stripe_bytes = size_t(kBlkWarps) * block_steps(int(max_rows)) * 32 * 4;
+  // the offsets of one choice of slots, stripes per group, word buffers and
+  // row intervals
+  auto place = [&](int slots, int group, bool two, bool by_runs) {
+    S.slots = slots;
+    S.group = group;
+    S.two = two;
+    S.words_slot = stripe_bytes / 4 * group;
+    S.runs_slot = by_runs ? max_rows : 0;
+    size_t o = S.round.total;
+    S.off_head = o; o += 1024;
+    S.off_prog = o; o += up(size_t(slots) * S.swaths_max * 8);
+    S.off_E = o; o += up(size_t(slots) * S.e_slot * sizeof(T));
+    S.off_Q = o; o += up(size_t(slots) * S.q_slot * sizeof(T));
+    S.off_W = o; o += up(size_t(slots) * S.words_slot * 4 * (two ? 2 : 1));
+    S.off_runs = o; o += up(size_t(slots) * S.runs_slot * sizeof(int2));
+    // with an open end: the extra samples, and the shortcut minima of every stripe
+    S.off_extra = o; o += oe ? up(size_t(n) * Lc * 4) : 0;
+    S.off_min = o; o += oe ? (size_t(2) * slots * S.min_slot * sizeof(T) + 63) / 64 * 64 : 0;
+    S.total = o;
+    return S.total <= limit;
+  };
   const size_t slot_bytes = size_t(S.e_slot + S.q_slot) * sizeof(T);
   int slots = (kStripeFill + S.swaths_max - 1) / S.swaths_max;
   if (slots > kStripeSlots) slots = kStripeSlots;
   if (slots > n) slots = n;
   while (slots > 1 && slot_bytes * slots > kStripeSlotBytes) --slots;
-  S.slots = slots;
-  const size_t stripe_bytes = size_t(kBlkWarps) * block_steps(int(max_rows)) * 32 * 4;
-  int group = S.swaths_max < kStripeGroup ? S.swaths_max : kStripeGroup;
-  while (group > 1 && stripe_bytes * group * slots > kStripeGroupBytes) --group;
-  S.group = group;
-  S.two = !oe && S.swaths_max > group && 2 * stripe_bytes * group * slots <= kStripeGroupBytes;
-  S.words_slot = stripe_bytes / 4 * group;
-  S.runs_slot = max_rows;
-  S.min_slot = (unsigned long long)S.swaths_max + 1;
-  size_t o = S.round.total;
-  S.off_head = o; o += 1024;
-  S.off_prog = o; o += up(size_t(slots) * S.swaths_max * 8);
-  S.off_E = o; o += up(size_t(slots) * S.e_slot * sizeof(T));
-  S.off_Q = o; o += up(size_t(slots) * S.q_slot * sizeof(T));
-  S.off_W = o; o += up(size_t(slots) * S.words_slot * 4 * (S.two ? 2 : 1));
-  S.off_runs = o; o += up(size_t(slots) * S.runs_slot * sizeof(int2));
-  // with an open end: the extra samples, and the shortcut minima of every stripe
-  S.off_extra = o; o += oe ? up(size_t(n) * Lc * 4) : 0;
-  S.off_min = o; o += oe ? (size_t(2) * slots * S.min_slot * sizeof(T) + 63) / 64 * 64 : 0;
-  S.total = o;
+  // the most side by side that fits: first without the second word buffer,
+  // then with fewer stripes per group, then fewer members; last one member,
+  // one stripe and no row intervals (the walk goes cell by cell)
+  for (; slots >= 1; --slots) {
+    int group = S.swaths_max < kStripeGroup ? S.swaths_max : kStripeGroup;
+    while (group > 1 && stripe_bytes * group * slots > kStripeGroupBytes) --group;
+    if (S.swaths_max > group && 2 * stripe_bytes * group * slots <= kStripeGroupBytes &&
+        place(slots, group, true, true))
+      return S;
+    for (; group >= 1; --group)
+      if (place(slots, group, false, true)) return S;
+  }
+  place(1, 1, false, false);
   return S;
+}
+
+// What a workspace may take: 95 % of the device memory that is free, or no
+// limit where there is no device to ask.
+size_t stripe_memory_limit() {
+  size_t fr = 0, tot = 0;
+  if (cudaMemGetInfo(&fr, &tot) == cudaSuccess) return fr / 20 * 19;
+  cudaGetLastError();
+  return SIZE_MAX;
 }
 
 int stripe_shift(int ckpt_rows) {
@@ -1996,7 +2026,7 @@ size_t dba_round_stripe_workspace_bytes(const uint64_t *h_lens, int n, uint64_t 
                                         int ckpt_rows) {
   const int sh = stripe_shift(ckpt_rows);
   if (sh < 0 || n < 1 || Lc == 0) return 0;
-  return stripe_layout<T>(h_lens, n, Lc, os, oe, sh).total;
+  return stripe_layout<T>(h_lens, n, Lc, os, oe, sh, stripe_memory_limit()).total;
 }
 
 template <typename T>
@@ -2007,7 +2037,7 @@ int dba_round_stripe_launch(const T *centroid, uint64_t Lc, const T *series,
                             size_t ws_bytes, cudaStream_t stream) {
   const int sh = stripe_shift(ckpt_rows);
   if (sh < 0) return fail(ODBA_ERR_INVALID_ARGUMENT, "checkpoint rows must be a power of two >= 2 (0: default)");
-  const StripeLayout S = stripe_layout<T>(h_lens, n, Lc, os, oe, sh);
+  const StripeLayout S = stripe_layout<T>(h_lens, n, Lc, os, oe, sh, ws_bytes);
   if (ws_bytes < S.total) return fail(ODBA_ERR_WORKSPACE_TOO_SMALL, "stripe DBA round workspace too small");
   const RoundLayout &L = S.round;
   char *base = static_cast<char *>(ws);
@@ -2072,7 +2102,7 @@ int dba_round_stripe_launch(const T *centroid, uint64_t Lc, const T *series,
   sa.limit_ns = kWaitLimitNs;
   static_assert(64 + kStripeSlots * sizeof(StripeWalk) <= 1024, "walk states fit the header");
   const bool check_short = oe && !os;
-  const bool by_rows = !oe && !triples;
+  const bool by_rows = !oe && !triples && S.runs_slot;
   const int K = 1 << sh;
   const int group = oe ? 1 : S.group;
   const bool beside = by_rows && S.two;
