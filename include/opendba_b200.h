@@ -55,6 +55,8 @@ int odba_device_check(void);
  * odba_dtw_pairwise_workspace_bytes_n is the tighter size of the plan chosen
  * by default for n series (few long series: per-pair edge buffers instead of
  * per-warp ones).  A smaller workspace restricts the plans to those that fit.
+ * max_len is the longest series: under every plan a pair whose first series is
+ * longer than the launch was sized for gets NaN.
  * use_open_start / use_open_end have the reference's meaning
  * (openDBA.cu:72-104), including its open-end shortcut (dtw.hpp:74-129):
  * where it fires the distance is the last-row value of that swath's left

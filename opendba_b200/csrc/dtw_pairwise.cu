@@ -100,6 +100,10 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, kMinBlocksPerSM)
     job.n = int(lens[task.second]);
     job.r0 = os;
     job.open_end = oe != 0;
+    if ((unsigned long long)job.m + 32 > edge_stride) {  // longer than max_len (pairwise_kernel)
+      if (lane == 0) dists[out] = Num<T>::quiet_nan();
+      continue;
+    }
     T corner = T(0);
     sweep_pair<T, RF, RQ>(job, sm[threadIdx.x >> 5], e0, e1, corner);
     if (lane == 0) dists[out] = pair_distance<T>(corner, job.m, job.n, os, oe);
@@ -189,10 +193,15 @@ struct PipeArgs {
 // so the shorter series takes the rows: a pair's time is the steps down its
 // rows plus about 200 steps for each swath after the first, and 1024 columns
 // cost less than 1024 rows.
+//
+// fits: the first series (before the exchange) is within the max_len the
+// launch sized its edge buffers for; a longer one's edges would run into the
+// next pair's buffers, so its pair is given NaN, as in the one-warp plans.
 struct PipePair {
   int s, j, os, oe;
   unsigned long long out;
   uint64_t m, n;
+  bool fits;
 };
 template <typename T>
 __device__ __forceinline__ PipePair pipe_pair(const PipeArgs<T> &a, unsigned long long qi) {
@@ -213,6 +222,7 @@ __device__ __forceinline__ PipePair pipe_pair(const PipeArgs<T> &a, unsigned lon
   }
   p.m = a.lens[p.s];
   p.n = a.lens[p.j];
+  p.fits = p.m + 32 <= a.edge_stride;
   if (!p.os && !p.oe && p.m > p.n) {
     const int t = p.s;
     p.s = p.j;
@@ -262,6 +272,11 @@ __global__ void __launch_bounds__(kBlkThreads, sizeof(T) == 4 ? kPipeBlocksF32 :
     const unsigned long long turn = q / a.npairs, qi = q - turn * a.npairs;
     const PipePair p = pipe_pair(a, qi);
     const unsigned long long first = turn - late(p);
+    if (!p.fits) {
+      if (first == 0 && threadIdx.x == 0) a.dists[p.out] = Num<T>::quiet_nan();
+      __syncthreads();  // the task word is free again
+      continue;
+    }
     const int m = int(p.m), n = int(p.n);
     T *b0 = a.edges + qi * 2 * a.edge_stride;
     T *b1 = b0 + a.edge_stride;
@@ -355,30 +370,15 @@ __global__ void pipe_shortcut_kernel(PipeArgs<T> a) {
   const unsigned long long qi = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (qi >= a.npairs) return;
   if (*reinterpret_cast<volatile unsigned *>(a.err) != 0) return;
-  int s, j, os, oe;
-  unsigned long long out;
-  if (a.list) {
-    const odba_pair_task task = a.list[qi];
-    s = int(task.first);
-    j = int(task.second);
-    os = int((task.out >> 62) & 1ull);
-    oe = int((task.out >> 63) & 1ull);
-    out = task.out & ((1ull << 62) - 1);
-  } else {
-    const long long p = (long long)(a.pbeg + a.npairs - 1 - qi);
-    pair_of(p, a.n, s, j);
-    os = a.open_start;
-    oe = a.open_end;
-    out = (unsigned long long)p;
-  }
-  if (!oe || os) return;
-  const int m = int(a.lens[s]), n = int(a.lens[j]);
+  const PipePair p = pipe_pair(a, qi);  // (never exchanged with an open end)
+  if (!p.oe || p.os || !p.fits) return;
+  const int m = int(p.m), n = int(p.n);
   for (int cnext = kRefSwath; cnext < n; cnext += kRefSwath) {
     if (cnext <= m) continue;
     if ((unsigned long long)(cnext / kRefSwath - 1) >= a.max_bounds) return;
     const T v = a.bstat[qi * a.max_bounds + (unsigned long long)(cnext / kRefSwath - 1)];
     if (v >= T(0)) {
-      a.dists[out] = pair_distance<T>(v, m, n, os, oe);
+      a.dists[p.out] = pair_distance<T>(v, m, n, p.os, p.oe);
       return;
     }
   }
