@@ -81,6 +81,19 @@ __device__ __forceinline__ int smem_count(const int *p) {
   return *reinterpret_cast<const volatile int *>(p);
 }
 
+// What lane 0 reads, in every lane of the calling warp, with what was written
+// before it: a warp whose lanes decide by a word that changes under them must
+// decide by one read of it (lanes need not run in step).
+__device__ __forceinline__ int warp_count(const int *p) {
+  const int v = __shfl_sync(kFull, smem_count(p), 0);
+  __threadfence_block();
+  __syncwarp();
+  return v;
+}
+__device__ __forceinline__ unsigned long long warp_timer_ns() {
+  return __shfl_sync(kFull, global_timer_ns(), 0);
+}
+
 // Waits until the counter is at least v (every lane of the calling warp);
 // one that has to wait waits for `more` instead, so that a neighbour of nearly
 // the same pace is not waited for again at every chunk.
@@ -173,8 +186,7 @@ __device__ __forceinline__ bool sweep_block(const BlockJob<T> &job, BlockSmem<T>
     const int *last_done = &sm.done[wact - 1];
     unsigned long long t0 = 0;
     for (unsigned idle = 0; staged < pairs || drained < pairs;) {
-      const int ld = smem_count(last_done);
-      __threadfence_block();
+      const int ld = warp_count(last_done);
       bool moved = false;
       if (drained < pairs) {
         // whole chunks of the right edge, up to kBlkStage pairs
@@ -202,7 +214,7 @@ __device__ __forceinline__ bool sweep_block(const BlockJob<T> &job, BlockSmem<T>
         // room in the sample ring (the last warp's lane 31 reads the oldest
         // pair) and in the left-edge ring, and the left edge published
         const int k1 = staged + kBlkStage < pairs ? staged + kBlkStage : pairs;
-        bool ok = k1 + 31 - ld <= kBlkXPairs && k1 - smem_count(&sm.done[0]) <= kBlkRing;
+        bool ok = k1 + 31 - ld <= kBlkXPairs && k1 - warp_count(&sm.done[0]) <= kBlkRing;
         if (ok && has_in && Gate::kActive) {
           int have = 0;
           if (lane == 0) have = gate.ready(2 * k1 < rows ? 2 * k1 : rows) ? 1 : 0;
@@ -239,7 +251,7 @@ __device__ __forceinline__ bool sweep_block(const BlockJob<T> &job, BlockSmem<T>
         __nanosleep(idle < 4 ? 128u << idle : 2000u);
         if ((++idle & 255u) == 0) {
           // bounded like the compute warps' waits
-          const unsigned long long now = global_timer_ns();
+          const unsigned long long now = warp_timer_ns();
           if (t0 == 0) {
             t0 = now;
           } else if (now - t0 > 2 * kWaitLimitNs) {

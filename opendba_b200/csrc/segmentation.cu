@@ -129,6 +129,7 @@ __device__ __forceinline__ void seg_rows_fast(const unsigned (&cost)[kSegRegs], 
   static_assert(REGS <= kSegRegs, "costs held per thread");
   const int t = threadIdx.x, n = t / kSegGroups + 1, g = t % kSegGroups;
   const int nmax = (t | 31) / kSegGroups + 1;  // the warp's longest prefix
+  const unsigned live = __ballot_sync(kFull, n <= N_ds);  // whole groups of kSegGroups lanes
   for (int p = from + 1; p <= to; ++p) {
     const unsigned *prev = rows + ((p - 1) & 1) * kSegRowWords + kSegLens;
     unsigned *cur = rows + (p & 1) * kSegRowWords + kSegLens;
@@ -145,7 +146,6 @@ __device__ __forceinline__ void seg_rows_fast(const unsigned (&cost)[kSegRegs], 
             best = __viaddmin_u32(q[-i * kSegGroups], cost[i], best);
         }
       }
-      const unsigned live = __activemask();
 #pragma unroll
       for (int off = 1; off < kSegGroups; off <<= 1) {
         const unsigned o = __shfl_xor_sync(live, best, off);

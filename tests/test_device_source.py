@@ -1,0 +1,28 @@
+"""Rules the device sources keep that no run can show to be broken reliably."""
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(__file__), "..", "opendba_b200", "csrc")
+
+
+def _source(name):
+    with open(os.path.join(CSRC, name)) as f:
+        text = f.read()
+    return re.sub(r"//[^\n]*", "", text)
+
+
+def test_no_collective_over_the_lanes_that_happen_to_be_together():
+    # __activemask() names the lanes that run together at the moment, not those
+    # that will reach a shuffle
+    for name in os.listdir(CSRC):
+        if name.endswith((".cu", ".cuh")):
+            assert "__activemask" not in _source(name), name
+
+
+def test_feeder_decides_by_one_read():
+    # the feeding warp's lanes take part in shuffles by what shared counters and
+    # the timer say: one lane reads them for all
+    text = _source("dtw_block.cuh")
+    feeder = text[text.index("if (w == kBlkWarps) {"):text.index("if (w >= wact) return false;")]
+    assert "warp_count(" in feeder and "warp_timer_ns(" in feeder
+    assert "smem_count(" not in feeder and "global_timer_ns(" not in feeder
