@@ -128,15 +128,15 @@ int odba_tune_load(const char *path);
  * No reference counterpart (a tuning knob; results do not depend on it).
  * The path DTW can cut each member's rows into bands, tasks of their own.
  * n in 1..8 pins the number of bands for the following launches (1: none),
- * 0 restores the automatic choice (none).  A workspace size queried under one setting fits launches under the
- * same setting. */
+ * 0 restores the automatic choice (none).  A workspace size queried under one
+ * setting fits launches under the same setting. */
 int odba_round_set_bands(int n);
 
 /* ---- self-test of the bounded device wait --------------------------------------
- * No reference counterpart.  One warp runs the swath pipeline's wait on a
- * progress word that nothing publishes, with the given limit (at most 10 s);
- * returns ODBA_ERR_TIMEOUT when the wait ran out and raised the error word,
- * as it must. */
+ * No reference counterpart.  A block sweeps a swath whose left neighbour's
+ * progress word nothing publishes, with the swath pipeline's own sweep and
+ * wait and the given limit (at most 10 s); returns ODBA_ERR_TIMEOUT when the
+ * wait ran out and raised the error word, as it must. */
 int odba_selftest_wait_timeout(uint64_t limit_ns, void *stream);
 
 /* ---- DTW distances of an arbitrary pair list (batched jobs, queries) ----------

@@ -37,7 +37,7 @@
 // without waiting on the waiter (a warp waits for its left neighbour's steps,
 // or for room its right neighbour frees; the feeder never blocks on one of
 // its duties while another could go on); they are bounded like the waits
-// between blocks.
+// between blocks (dtw_pipe.cuh).
 #pragma once
 
 #include <type_traits>
@@ -81,14 +81,11 @@ __device__ __forceinline__ int smem_count(const int *p) {
   return *reinterpret_cast<const volatile int *>(p);
 }
 
-// What lane 0 reads, in every lane of the calling warp, with what was written
-// before it: a warp whose lanes decide by a word that changes under them must
-// decide by one read of it (lanes need not run in step).
+// What lane 0 reads, in every lane of the calling warp: a warp whose lanes decide
+// by a word that changes under them must decide by one read of it (lanes need
+// not run in step).
 __device__ __forceinline__ int warp_count(const int *p) {
-  const int v = __shfl_sync(kFull, smem_count(p), 0);
-  __threadfence_block();
-  __syncwarp();
-  return v;
+  return __shfl_sync(kFull, smem_count(p), 0);
 }
 __device__ __forceinline__ unsigned long long warp_timer_ns() {
   return __shfl_sync(kFull, global_timer_ns(), 0);
@@ -96,17 +93,20 @@ __device__ __forceinline__ unsigned long long warp_timer_ns() {
 
 // Waits until the counter is at least v (every lane of the calling warp);
 // one that has to wait waits for `more` instead, so that a neighbour of nearly
-// the same pace is not waited for again at every chunk.
-__device__ __forceinline__ void wait_count(const int *p, int v, int more, unsigned *err) {
+// the same pace is not waited for again at every chunk.  Bounded: past limit_ns
+// the launch's error word is raised; a word already up ends the wait.
+__device__ __forceinline__ void wait_count(const int *p, int v, int more, unsigned *err,
+                                           unsigned long long limit_ns) {
   if (smem_count(p) < v) {
     unsigned long long t0 = 0;
     for (unsigned it = 0; smem_count(p) < more; ++it) {
       __nanosleep(it < 4 ? 64u << it : 1000u);
-      if ((it & 1023u) == 1023u) {
+      if ((it & 63u) == 63u) {
+        if (err && *reinterpret_cast<volatile unsigned *>(err)) break;
         const unsigned long long now = global_timer_ns();
-        if (t0 == 0)
+        if (t0 == 0) {
           t0 = now;
-        else if (now - t0 > 4 * kWaitLimitNs) {  // past every wait between blocks
+        } else if (now - t0 > limit_ns) {
           if (err) atomicExch(err, 1u);
           break;
         }
@@ -186,7 +186,9 @@ __device__ __forceinline__ bool sweep_block(const BlockJob<T> &job, BlockSmem<T>
     const int *last_done = &sm.done[wact - 1];
     unsigned long long t0 = 0;
     for (unsigned idle = 0; staged < pairs || drained < pairs;) {
-      const int ld = warp_count(last_done);
+      const int ld = warp_count(last_done), d0 = warp_count(&sm.done[0]);
+      __threadfence_block();
+      __syncwarp();
       bool moved = false;
       if (drained < pairs) {
         // whole chunks of the right edge, up to kBlkStage pairs
@@ -214,7 +216,7 @@ __device__ __forceinline__ bool sweep_block(const BlockJob<T> &job, BlockSmem<T>
         // room in the sample ring (the last warp's lane 31 reads the oldest
         // pair) and in the left-edge ring, and the left edge published
         const int k1 = staged + kBlkStage < pairs ? staged + kBlkStage : pairs;
-        bool ok = k1 + 31 - ld <= kBlkXPairs && k1 - warp_count(&sm.done[0]) <= kBlkRing;
+        bool ok = k1 + 31 - ld <= kBlkXPairs && k1 - d0 <= kBlkRing;
         if (ok && has_in && Gate::kActive) {
           int have = 0;
           if (lane == 0) have = gate.ready(2 * k1 < rows ? 2 * k1 : rows) ? 1 : 0;
@@ -249,12 +251,12 @@ __device__ __forceinline__ bool sweep_block(const BlockJob<T> &job, BlockSmem<T>
         t0 = 0;
       } else {
         __nanosleep(idle < 4 ? 128u << idle : 2000u);
-        if ((++idle & 255u) == 0) {
-          // bounded like the compute warps' waits
+        if ((++idle & 15u) == 0) {
+          // bounded, before the compute warps' waits are
           const unsigned long long now = warp_timer_ns();
           if (t0 == 0) {
             t0 = now;
-          } else if (now - t0 > 2 * kWaitLimitNs) {
+          } else if (now - t0 > gate.limit()) {
             if (Gate::kActive && lane == 0) gate.fail();
             staged = drained = pairs;
             if (lane == 0) {
@@ -359,6 +361,7 @@ __device__ __forceinline__ bool sweep_block(const BlockJob<T> &job, BlockSmem<T>
   // the steps at which some lane is on row m - 1 are slow where that row has
   // rules of its own (open end) or its value is wanted
   const bool slow_end = oe_top || (CAP && cap_last);
+  const unsigned long long wait_limit = 4 * gate.limit();  // past every wait of a feeder
 #pragma unroll 1
   for (int t0 = 0; t0 < steps; t0 += kBlkChunk) {
     // this chunk's left-edge pairs, and room in the right-edge ring
@@ -366,13 +369,14 @@ __device__ __forceinline__ bool sweep_block(const BlockJob<T> &job, BlockSmem<T>
     need = need < pairs ? need : pairs;
     if (w) need = need + 31 < steps ? need + 31 : steps;
     const int most = w ? steps : pairs;
-    wait_count(from, need, need + kBlkSlack < most ? need + kBlkSlack : most, gate.error());
+    wait_count(from, need, need + kBlkSlack < most ? need + kBlkSlack : most, gate.error(),
+               wait_limit);
     if (has_next) {
       const int room = t0 + kBlkChunk - 31 - kBlkRing;
       if (room > 0) {
         // (the right neighbour can go on to step t0 - 39 whatever this warp does)
         const int v = room < pairs ? room : pairs, more = room + 4 * kBlkChunk;
-        wait_count(to, v, more < pairs ? more : pairs, gate.error());
+        wait_count(to, v, more < pairs ? more : pairs, gate.error(), wait_limit);
       }
     }
     if (slow_end && t0 + kBlkChunk > last_pair)

@@ -200,12 +200,14 @@ struct Pair2<double> {
 
 // Hand-off of swath-edge rows.  NoGate: the edge buffer is complete or the
 // sweep's own, nothing to wait for (PipeGate in dtw_pipe.cuh is the other).
+constexpr unsigned long long kWaitLimitNs = 2000000000ull;  // 2 s
 struct NoGate {
   static constexpr bool kActive = false;
   __device__ __forceinline__ void publish(int) {}
   __device__ __forceinline__ bool ready(int) { return true; }
   __device__ __forceinline__ void fail() {}
   __device__ __forceinline__ unsigned *error() { return nullptr; }
+  __device__ __forceinline__ unsigned long long limit() { return kWaitLimitNs; }
 };
 
 }  // namespace odba

@@ -155,10 +155,10 @@ int whole_pairlist_launch(const T *series, const uint64_t *offsets, const uint64
 // time, at different rows, which is why the progress words are per swath and
 // not per buffer.
 //
-// Every wait is bounded: after its limit of polling (%globaltimer) a block
-// raises the launch's error word and continues; every other waiting block sees
-// the word and stops waiting, so a fault in the hand-off ends the launch
-// quickly with the pairs it touched written as NaN.
+// Every wait is bounded: a block whose feeder could not go on for limit_ns
+// (%globaltimer) raises the launch's error word and continues; every other
+// waiting block sees the word and stops waiting, so a fault in the hand-off
+// ends the launch quickly with the pairs it touched written as NaN.
 namespace odba {
 namespace {
 
@@ -713,19 +713,43 @@ int pairlist_launch(const T *series, const uint64_t *offsets, const uint64_t *le
 }
 
 namespace {
-// One warp waits on a progress word that nothing publishes, with the swath
-// pipeline's own bounded wait.
-__global__ void gate_selftest_kernel(unsigned long long *word, unsigned *err,
-                                     unsigned long long limit_ns, int *seen) {
-  if (threadIdx.x != 0) return;
+// The self-test's buffer: the error word, the progress words, samples, an edge.
+constexpr int kSelfRows = 64, kSelfCols = 1024 + 300;
+struct SelfTest {
+  unsigned err[4];
+  unsigned long long prog[2];
+  float x[kSelfRows], y[kSelfCols], edge[kSelfRows + 32];
+};
+
+// A block sweeps the second swath of a pair whose first swath nobody sweeps:
+// the pipeline's own wait on a progress word that nothing publishes.
+__global__ void __launch_bounds__(kBlkThreads) gate_selftest_kernel(SelfTest *t,
+                                                                    unsigned long long limit_ns) {
+  __shared__ BlockSmem<float> sm;
+  BlockJob<float> job;
+  job.x = t->x;
+  job.y = t->y;
+  job.m = kSelfRows;
+  job.n = kSelfCols;
+  job.c0 = kBlkCols;
+  job.r0 = 0;
+  job.edge_in = t->edge;
+  job.edge_out = nullptr;
+  job.open_end = false;
+  job.free_diag0 = true;
+  job.corner_init = Num<float>::big();
+  job.words = nullptr;
+  job.word_steps = 0;
   PipeGate gate;
-  gate.prog_in = word;
-  gate.prog_out = word + 1;
-  gate.err = err;
+  gate.prog_in = t->prog;
+  gate.prog_out = t->prog + 1;
+  gate.err = t->err;
   gate.limit_ns = limit_ns;
   gate.avail = 0;
-  gate.wait_in(1);
-  *seen = ld_acquire_gpu(word) != 0;
+  float corner = 0.f;
+  EdgeStat<float> st;
+  sweep_block<float, false, false, false, true>(job, sm, gate, CkptOut<float>{nullptr, 0, 1}, true,
+                                                corner, st);
 }
 }  // namespace
 
@@ -733,23 +757,19 @@ int gate_selftest(unsigned long long limit_ns, cudaStream_t stream) {
   if (limit_ns == 0 || limit_ns > 10000000000ull)
     return fail(ODBA_ERR_INVALID_ARGUMENT, "limit must be in (0, 10 s]");
   if (int rc = require_sm100()) return rc;
-  char *buf = nullptr;
-  if (cudaMallocAsync(reinterpret_cast<void **>(&buf), 256, stream) != cudaSuccess)
+  SelfTest *t = nullptr;
+  if (cudaMallocAsync(reinterpret_cast<void **>(&t), sizeof *t, stream) != cudaSuccess)
     return fail(ODBA_ERR_OUT_OF_MEMORY, "self-test buffer");
-  unsigned err = 0;
-  int seen = 0;
-  cudaMemsetAsync(buf, 0, 256, stream);
-  gate_selftest_kernel<<<1, 32, 0, stream>>>(reinterpret_cast<unsigned long long *>(buf),
-                                            reinterpret_cast<unsigned *>(buf + 64), limit_ns,
-                                            reinterpret_cast<int *>(buf + 128));
+  unsigned err[4] = {0u, 0u, 0u, 0u};
+  cudaMemsetAsync(t, 0, sizeof *t, stream);
+  gate_selftest_kernel<<<1, kBlkThreads, 0, stream>>>(t, limit_ns);
   int rc = check_launch("wait self-test kernel");
-  cudaMemcpyAsync(&err, buf + 64, sizeof err, cudaMemcpyDeviceToHost, stream);
-  cudaMemcpyAsync(&seen, buf + 128, sizeof seen, cudaMemcpyDeviceToHost, stream);
-  cudaFreeAsync(buf, stream);
+  cudaMemcpyAsync(err, t->err, sizeof err, cudaMemcpyDeviceToHost, stream);
+  cudaFreeAsync(t, stream);
   if (cudaStreamSynchronize(stream) != cudaSuccess) return fail(ODBA_ERR_CUDA, "wait self-test");
   if (rc) return rc;
-  if (err) return fail(ODBA_ERR_TIMEOUT, "the wait ran out and raised the error word");
-  return seen ? ODBA_OK : fail(ODBA_ERR_CUDA, "the wait returned without the word or a timeout");
+  if (err[0]) return fail(ODBA_ERR_TIMEOUT, "the wait ran out and raised the error word");
+  return fail(ODBA_ERR_CUDA, "the wait returned without the word or a timeout");
 }
 
 int tune_set(int elem_size, int len_bucket, int count_bucket, int plan) {

@@ -1,17 +1,19 @@
-// Bounded hand-off of swath-edge rows between warps (the swath pipeline).
+// Bounded hand-off of swath-edge rows between blocks (the swath pipeline).
 //
-// The producing warp's lane 31 publishes "rows stored so far" with a
-// gpu-scope release; the consuming warp's lane 0 acquires the word before it
-// reads rows it has not seen published.  Every wait is bounded: after the
-// limit (%globaltimer) the waiter raises the launch's error word and goes on,
+// The producing block's feeding warp publishes "rows stored so far" with a
+// gpu-scope release; the consuming block's feeder acquires the word before it
+// reads rows it has not seen published (PipeGate::ready, polled between its
+// other duties: dtw_block.cuh).  Every wait is bounded: a feeder none of whose
+// duties could go on for the gate's limit (%globaltimer) raises the launch's
+// error word and goes on, a compute warp does so after four times the limit,
 // and every other waiter that sees the word stops waiting too.
 #pragma once
 
 #include <cstdint>
 
-namespace odba {
+#include "dtw_device.cuh"
 
-constexpr unsigned long long kWaitLimitNs = 2000000000ull;  // 2 s
+namespace odba {
 
 __device__ __forceinline__ unsigned long long ld_acquire_gpu(const unsigned long long *p) {
   unsigned long long v;
@@ -35,33 +37,9 @@ struct PipeGate {
   unsigned long long limit_ns;
   int avail;                          // input rows known to be published
 
-  __device__ __forceinline__ void wait_in(int k) {
-    if (k <= avail) return;
-    unsigned long long t0 = 0;
-    for (unsigned it = 0;; ++it) {
-      const unsigned long long v = ld_acquire_gpu(prog_in);
-      if (v >= (unsigned long long)k) {
-        avail = int(v);
-        return;
-      }
-      if (*reinterpret_cast<volatile unsigned *>(err)) {
-        avail = 0x7fffffff;
-        return;
-      }
-      const unsigned long long now = global_timer_ns();
-      if (it == 0) {
-        t0 = now;
-      } else if (now - t0 > limit_ns) {
-        atomicExch(err, 1u);
-        avail = 0x7fffffff;
-        return;
-      }
-      __nanosleep(128);
-    }
-  }
   __device__ __forceinline__ void publish(int k) { st_release_gpu(prog_out, (unsigned long long)k); }
-  // wait_in without the wait: whether rows [0, k) may be read now (also when
-  // the launch's error word is up: nobody waits any more)
+  // whether rows [0, k) may be read now (also when the launch's error word is
+  // up: nobody waits any more)
   __device__ __forceinline__ bool ready(int k) {
     if (k <= avail) return true;
     const unsigned long long v = ld_acquire_gpu(prog_in);
@@ -77,6 +55,7 @@ struct PipeGate {
   }
   __device__ __forceinline__ void fail() { atomicExch(err, 1u); }
   __device__ __forceinline__ unsigned *error() { return err; }
+  __device__ __forceinline__ unsigned long long limit() { return limit_ns; }
 };
 
 // The gate of a band of a swath's rows: the band's rows count from base (its
@@ -90,6 +69,7 @@ struct BandGate {
   __device__ __forceinline__ bool ready(int k) { return g.ready(base + k); }
   __device__ __forceinline__ void fail() { g.fail(); }
   __device__ __forceinline__ unsigned *error() { return g.err; }
+  __device__ __forceinline__ unsigned long long limit() { return g.limit_ns; }
 };
 
 // Bounded wait (one thread) until *p >= v, with the gate's error rules:

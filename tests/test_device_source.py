@@ -26,3 +26,14 @@ def test_feeder_decides_by_one_read():
     feeder = text[text.index("if (w == kBlkWarps) {"):text.index("if (w >= wact) return false;")]
     assert "warp_count(" in feeder and "warp_timer_ns(" in feeder
     assert "smem_count(" not in feeder and "global_timer_ns(" not in feeder
+
+
+def test_waits_of_the_sweep_take_the_launch_limit():
+    # the limit a launch (or the self-test) gives is the one its sweep's waits
+    # run out by, and there is no second wait beside them to test instead
+    text = _source("dtw_block.cuh")
+    assert "gate.limit()" in text and "kWaitLimitNs" not in text
+    assert "wait_in" not in _source("dtw_pipe.cuh")
+    pairs = _source("dtw_pairwise.cu")
+    kernel = pairs[pairs.index("gate_selftest_kernel(SelfTest"):]
+    assert "sweep_block<" in kernel[:kernel.index("int gate_selftest(")]
