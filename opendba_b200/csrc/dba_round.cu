@@ -458,7 +458,7 @@ __launch_bounds__(kBlkThreads, sizeof(T) == 4 ? kRoundBlocksF32 : kRoundBlocksF6
           if (feeder && lane == 0) st_release_gpu(a.bdone + ks, (unsigned long long)(b + 1));
         }
       } else {
-        sweep_block<T, true, false, false, false>(job, sm, NoGate(), CkptOut<T>{nullptr, 0, 1},
+        sweep_block<T, true, false, false, false>(job, sm, NoGate(a.err), CkptOut<T>{nullptr, 0, 1},
                                                   false, unused, st);
         const int cnext = c0 + kBlkCols;
         if (oe && !os && !shortcut && !last && cnext > g.m && st.etop == st.emin) shortcut = cnext;
@@ -1682,8 +1682,8 @@ __device__ __forceinline__ void stripe_tile(const StripeArgs<T> &a, BlockSmem<T>
               (size_t)kt * (K / 2) * 32;
   T unused = T(0);
   EdgeStat<T> st;
-  sweep_block<T, true, true, false, false>(job, sm, NoGate(), CkptOut<T>{nullptr, 0, 1}, false,
-                                           unused, st);
+  sweep_block<T, true, true, false, false>(job, sm, NoGate(a.err, a.limit_ns),
+                                           CkptOut<T>{nullptr, 0, 1}, false, unused, st);
 }
 
 // Block (kt, b, slot): one tile of the group.

@@ -102,12 +102,12 @@ __device__ __forceinline__ void wait_count(const int *p, int v, int more, unsign
     for (unsigned it = 0; smem_count(p) < more; ++it) {
       __nanosleep(it < 4 ? 64u << it : 1000u);
       if ((it & 63u) == 63u) {
-        if (err && *reinterpret_cast<volatile unsigned *>(err)) break;
+        if (*reinterpret_cast<volatile unsigned *>(err)) break;
         const unsigned long long now = global_timer_ns();
         if (t0 == 0) {
           t0 = now;
         } else if (now - t0 > limit_ns) {
-          if (err) atomicExch(err, 1u);
+          atomicExch(err, 1u);
           break;
         }
       }
@@ -257,7 +257,7 @@ __device__ __forceinline__ bool sweep_block(const BlockJob<T> &job, BlockSmem<T>
           if (t0 == 0) {
             t0 = now;
           } else if (now - t0 > gate.limit()) {
-            if (Gate::kActive && lane == 0) gate.fail();
+            if (lane == 0) gate.fail();
             staged = drained = pairs;
             if (lane == 0) {
               *reinterpret_cast<volatile int *>(&sm.staged) = staged;

@@ -199,15 +199,21 @@ struct Pair2<double> {
 };
 
 // Hand-off of swath-edge rows.  NoGate: the edge buffer is complete or the
-// sweep's own, nothing to wait for (PipeGate in dtw_pipe.cuh is the other).
+// sweep's own, no other block to wait for (PipeGate in dtw_pipe.cuh is the
+// other).  The block's warps still wait for one another, and such a wait that
+// runs out raises the launch's error word as any other.
 constexpr unsigned long long kWaitLimitNs = 2000000000ull;  // 2 s
 struct NoGate {
   static constexpr bool kActive = false;
+  unsigned *err;
+  unsigned long long limit_ns;
+  __device__ __forceinline__ explicit NoGate(unsigned *e, unsigned long long limit = kWaitLimitNs)
+      : err(e), limit_ns(limit) {}
   __device__ __forceinline__ void publish(int) {}
   __device__ __forceinline__ bool ready(int) { return true; }
-  __device__ __forceinline__ void fail() {}
-  __device__ __forceinline__ unsigned *error() { return nullptr; }
-  __device__ __forceinline__ unsigned long long limit() { return kWaitLimitNs; }
+  __device__ __forceinline__ void fail() { atomicExch(err, 1u); }
+  __device__ __forceinline__ unsigned *error() { return err; }
+  __device__ __forceinline__ unsigned long long limit() { return limit_ns; }
 };
 
 }  // namespace odba

@@ -723,9 +723,7 @@ struct SelfTest {
 
 // A block sweeps the second swath of a pair whose first swath nobody sweeps:
 // the pipeline's own wait on a progress word that nothing publishes.
-__global__ void __launch_bounds__(kBlkThreads) gate_selftest_kernel(SelfTest *t,
-                                                                    unsigned long long limit_ns) {
-  __shared__ BlockSmem<float> sm;
+__device__ __forceinline__ BlockJob<float> selftest_job(SelfTest *t) {
   BlockJob<float> job;
   job.x = t->x;
   job.y = t->y;
@@ -740,6 +738,11 @@ __global__ void __launch_bounds__(kBlkThreads) gate_selftest_kernel(SelfTest *t,
   job.corner_init = Num<float>::big();
   job.words = nullptr;
   job.word_steps = 0;
+  return job;
+}
+__global__ void __launch_bounds__(kBlkThreads) gate_selftest_kernel(SelfTest *t,
+                                                                    unsigned long long limit_ns) {
+  __shared__ BlockSmem<float> sm;
   PipeGate gate;
   gate.prog_in = t->prog;
   gate.prog_out = t->prog + 1;
@@ -748,8 +751,20 @@ __global__ void __launch_bounds__(kBlkThreads) gate_selftest_kernel(SelfTest *t,
   gate.avail = 0;
   float corner = 0.f;
   EdgeStat<float> st;
-  sweep_block<float, false, false, false, true>(job, sm, gate, CkptOut<float>{nullptr, 0, 1}, true,
-                                                corner, st);
+  sweep_block<float, false, false, false, true>(selftest_job(t), sm, gate,
+                                                CkptOut<float>{nullptr, 0, 1}, true, corner, st);
+}
+
+// The same swath with nothing to wait for outside the block, by the compute
+// warps alone (kBlkThreads - 32 threads): their wait for a feeder that is not
+// there.
+__global__ void __launch_bounds__(kBlkThreads) block_selftest_kernel(SelfTest *t,
+                                                                     unsigned long long limit_ns) {
+  __shared__ BlockSmem<float> sm;
+  float corner = 0.f;
+  EdgeStat<float> st;
+  sweep_block<float, false, false, false, true>(selftest_job(t), sm, NoGate(t->err + 1, limit_ns),
+                                                CkptOut<float>{nullptr, 0, 1}, true, corner, st);
 }
 }  // namespace
 
@@ -763,13 +778,15 @@ int gate_selftest(unsigned long long limit_ns, cudaStream_t stream) {
   unsigned err[4] = {0u, 0u, 0u, 0u};
   cudaMemsetAsync(t, 0, sizeof *t, stream);
   gate_selftest_kernel<<<1, kBlkThreads, 0, stream>>>(t, limit_ns);
+  block_selftest_kernel<<<1, kBlkThreads - 32, 0, stream>>>(t, limit_ns);
   int rc = check_launch("wait self-test kernel");
   cudaMemcpyAsync(err, t->err, sizeof err, cudaMemcpyDeviceToHost, stream);
   cudaFreeAsync(t, stream);
   if (cudaStreamSynchronize(stream) != cudaSuccess) return fail(ODBA_ERR_CUDA, "wait self-test");
   if (rc) return rc;
-  if (err[0]) return fail(ODBA_ERR_TIMEOUT, "the wait ran out and raised the error word");
-  return fail(ODBA_ERR_CUDA, "the wait returned without the word or a timeout");
+  if (err[0] && err[1]) return fail(ODBA_ERR_TIMEOUT, "the waits ran out and raised the error words");
+  return fail(ODBA_ERR_CUDA, err[0] ? "a wait inside a block returned without a timeout"
+                                    : "the wait returned without the word or a timeout");
 }
 
 int tune_set(int elem_size, int len_bucket, int count_bucket, int plan) {

@@ -37,3 +37,10 @@ def test_waits_of_the_sweep_take_the_launch_limit():
     pairs = _source("dtw_pairwise.cu")
     kernel = pairs[pairs.index("gate_selftest_kernel(SelfTest"):]
     assert "sweep_block<" in kernel[:kernel.index("int gate_selftest(")]
+
+
+def test_every_sweep_has_an_error_word():
+    # a wait that runs out without one would leave a wrong result unsaid
+    for name in ("dba_round.cu", "dtw_pairwise.cu"):
+        assert "NoGate()" not in _source(name), name
+    assert "return nullptr" not in _source("dtw_device.cuh")
