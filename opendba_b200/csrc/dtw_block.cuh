@@ -182,7 +182,7 @@ __device__ __forceinline__ bool sweep_block(const BlockJob<T> &job, BlockSmem<T>
       for (int i = lane; i < 2 * kBlkRing; i += 32) sm.ring[0][i] = Num<T>::big();
     T emin = Num<T>::big(), etop = Num<T>::big();
     int staged = 0, drained = has_out ? 0 : pairs;
-    int published = 0;
+    int published = 0, top_lane = 0;  // top_lane: the lane that stores the top row
     const int *last_done = &sm.done[wact - 1];
     unsigned long long t0 = 0;
     for (unsigned idle = 0; staged < pairs || drained < pairs;) {
@@ -202,6 +202,7 @@ __device__ __forceinline__ bool sweep_block(const BlockJob<T> &job, BlockSmem<T>
             if (shortcut_row<T>(r0 + row)) emin = Num<T>::min2(emin, v);
             if (row == rows - 1 && job.top_band) etop = v;
           }
+          top_lane = (rows - 1 - 2 * drained) & 31;  // (the last time through)
           __syncwarp();
           drained = avail;
           if (lane == 0) *reinterpret_cast<volatile int *>(&sm.drained) = drained;
@@ -269,10 +270,9 @@ __device__ __forceinline__ bool sweep_block(const BlockJob<T> &job, BlockSmem<T>
     }
     if (Gate::kActive && has_out && published < rows && lane == 0) gate.publish(rows);
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
+    for (int off = 16; off > 0; off >>= 1)
       emin = Num<T>::min2(emin, __shfl_xor_sync(kFull, emin, off));
-      etop = Num<T>::min2(etop, __shfl_xor_sync(kFull, etop, off));
-    }
+    etop = __shfl_sync(kFull, etop, top_lane);  // (no minimum: it may be NaN or infinite)
     st.emin = emin;
     st.etop = etop;
     return false;

@@ -183,10 +183,13 @@ __device__ __forceinline__ EdgeStat<T> sweep_warp(const SwathJob<T> &job, WarpSm
   }
   if (job.track) {
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
+    for (int off = 16; off > 0; off >>= 1)
       st.emin = Num<T>::min2(st.emin, __shfl_xor_sync(kFull, st.emin, off));
-      st.etop = Num<T>::min2(st.etop, __shfl_xor_sync(kFull, st.etop, off));
-    }
+    // every lane the same figures, whatever the values: the warp goes on or
+    // stops by them.  The last row's value is the one of the lane that stored
+    // it (a minimum with the other lanes' big would lose a NaN or an infinity).
+    st.emin = __shfl_sync(kFull, st.emin, 0);
+    st.etop = __shfl_sync(kFull, st.etop, (last_pair + 31) & 31);
   }
   if (last) corner = __shfl_sync(kFull, cap, cap_lane);
   return st;
