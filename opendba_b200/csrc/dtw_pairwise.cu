@@ -188,11 +188,15 @@ struct PipeArgs {
 };
 
 // One pair of a launch: its series (rows, columns), modes and output.  Without
-// an open end the matrix of (b, a) is the transpose of (a, b)'s with the same
-// costs bit for bit (the differences change sign, the cell rule is symmetric),
-// so the shorter series takes the rows: a pair's time is the steps down its
-// rows plus about 200 steps for each swath after the first, and 1024 columns
-// cost less than 1024 rows.
+// an open end the matrix of (b, a) is the transpose of (a, b)'s, in float with
+// the same costs bit for bit (the differences change sign, the cell rule is
+// symmetric), so the shorter series takes the rows: a pair's time is the steps
+// down its rows plus about 200 steps for each swath after the first, and 1024
+// columns cost less than 1024 rows.  Not in double: its compare-and-select
+// minimum is not symmetric in NaN, so a pair with a NaN (or two infinities)
+// would depend on the plan.  The same order of the minimum in a second copy of
+// the sweep costs more than the exchange gives (15 series of 10000-30000: 24.4
+// ms exchanged, 25.2 not, 27.9 with the copy).
 //
 // fits: the first series (before the exchange) is within the max_len the
 // launch sized its edge buffers for; a longer one's edges would run into the
@@ -223,7 +227,7 @@ __device__ __forceinline__ PipePair pipe_pair(const PipeArgs<T> &a, unsigned lon
   p.m = a.lens[p.s];
   p.n = a.lens[p.j];
   p.fits = p.m + 32 <= a.edge_stride;
-  if (!p.os && !p.oe && p.m > p.n) {
+  if (sizeof(T) == 4 && !p.os && !p.oe && p.m > p.n) {
     const int t = p.s;
     p.s = p.j;
     p.j = t;

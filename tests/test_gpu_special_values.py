@@ -116,3 +116,11 @@ def _check(env, plan, dtype, mode, value, lens, seed):
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])
 def test_open_end(env, dtype, value, plan):
     _check(env, plan, dtype, (0, 1), value, [1, 3, 40, 1025, 1100, 2100], 7)
+
+
+@pytest.mark.parametrize("plan", list(PLANS))
+@pytest.mark.parametrize("value", [np.nan, np.inf, 1e30])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_global_either_series_the_longer_one(env, dtype, value, plan):
+    # the pipeline puts the shorter series on the rows
+    _check(env, plan, dtype, (0, 0), value, [2100, 1100, 600, 40, 3, 1, 700, 1030], 9)
