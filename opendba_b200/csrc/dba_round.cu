@@ -610,8 +610,9 @@ __device__ __forceinline__ bool walk_member_path(const RoundArgs<T> &a, const Me
 // The walk starts (or goes on) at st.r, st.c; st.entry is the column it
 // entered row st.r at (-1 on the open-end top row, whose interval is its first
 // cell alone).  w holds the moves of the columns from cmin (a multiple of the
-// swath) on; the walk ends at the start cell (1), when it fails (2), or when
-// it leaves cmin to the left (0).
+// swath) on; the walk ends at the start cell (1), when it fails (2: NaN or
+// infinite costs can lead it off column 0, in row st.r, whose interval is then
+// not stored), or when it leaves cmin to the left (0).
 struct RowWalk {
   int r, c, entry;
 };
@@ -637,7 +638,10 @@ __device__ __forceinline__ int walk_runs(const unsigned short *w, const MemberGe
       runs[top - lane] = iv;
       have = false;
     }
-    if (c < 0) return 2;  // walked off column 0
+    if (c < 0) {  // walked off column 0
+      st = RowWalk{r, c, entry};
+      return 2;
+    }
     if (r == 0) {
       __syncwarp();
       if (lane == 0) runs[0] = os ? make_int2(1, 0) : make_int2(0, c);
@@ -759,9 +763,10 @@ __device__ __forceinline__ bool walk_member_runs(const RoundArgs<T> &a, const Me
 // r + 1 also holds it and its low end unless row r - 1 also holds it; every
 // other column of the interval is row r's alone.  Centroid on the rows (t =
 // row): the interval is the range.
+// lo, t_min: the lowest row walked and the first column taken (a failed walk).
 __device__ __forceinline__ void runs_to_ranges(const int2 *runs, int2 *rg, int m, bool flip,
-                                               int first, int stride) {
-  for (int r = first; r < m; r += stride) {
+                                               int first, int stride, int lo = 0, int t_min = 0) {
+  for (int r = lo + first; r < m; r += stride) {
     const int2 iv = runs[r];
     if (iv.x > iv.y) continue;
     if (flip) {
@@ -769,10 +774,10 @@ __device__ __forceinline__ void runs_to_ranges(const int2 *runs, int2 *rg, int m
       continue;
     }
     const int2 above = r + 1 < m ? runs[r + 1] : make_int2(1, 0);
-    const int2 below = r > 0 ? runs[r - 1] : make_int2(1, 0);
+    const int2 below = r > lo ? runs[r - 1] : make_int2(1, 0);
     const bool top_shared = above.x <= iv.y && iv.y <= above.y;
     const bool low_shared = below.x <= iv.x && iv.x <= below.y;
-    for (int t = iv.x; t <= iv.y; ++t) {
+    for (int t = iv.x > t_min ? iv.x : t_min; t <= iv.y; ++t) {
       if (!(t == iv.y && top_shared)) rg[t].y = r;
       if (!(t == iv.x && low_shared)) rg[t].x = r;
     }
@@ -1732,6 +1737,7 @@ __device__ __forceinline__ void stripe_walk_runs(const StripeArgs<T> &a, int gro
   const int got = walk_runs(reinterpret_cast<const unsigned short *>(stripe_words(a, slot, gi)), g,
                             lo * kBlkCols, rw, a.r0, a.runs + slot * a.runs_slot);
   if (lane == 0) {
+    if (got == 2 && rw.entry >= 0) a.runs[slot * a.runs_slot + rw.r] = make_int2(0, rw.entry);
     w.r = rw.r;
     w.c = rw.c;
     w.entry = rw.entry;
@@ -1779,14 +1785,19 @@ __launch_bounds__(kBlkThreads, sizeof(T) == 4 ? kRoundBlocksF32 : kRoundBlocksF6
   stripe_tile(a, sm, group, gi + 1, u - b * tiles, b, slot, w);
 }
 
-// The rows' intervals as ranges (runs_to_ranges; the member on the rows).
+// The rows' intervals as ranges (runs_to_ranges; the member on the rows).  A
+// walk that failed has what it passed, as the walk by cells leaves it: all but
+// the column it was in, the first.
 template <typename T>
 __global__ void stripe_ranges_kernel(StripeArgs<T> a) {
   const int slot = blockIdx.y;
-  if (a.walk[slot].state != 1) return;
+  const StripeWalk &w = a.walk[slot];
+  const bool failed = w.state == 2;
+  if (w.state != 1 && !failed) return;
   runs_to_ranges(a.runs + slot * a.runs_slot,
                  a.ranges + (unsigned long long)a.mem[slot].member * a.Lc, a.mem[slot].m, false,
-                 blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+                 blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x,
+                 failed ? (w.entry >= 0 ? w.r : w.r + 1) : 0, failed ? 1 : 0);
 }
 
 // Continues the backtrack cell by cell through a group (updateCentroid's loop,

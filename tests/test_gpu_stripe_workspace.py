@@ -78,3 +78,41 @@ def test_any_workspace_gives_the_same_round(env, mode, dtype):
     assert taken >= 5
     with pytest.raises(native.OdbaError):
         run(small // 4)
+
+
+def _least(run, high, native):
+    """The smallest workspace a round takes (nothing smaller is launched)."""
+    low = 0
+    while high - low > 4096:
+        mid = (low + high) // 2
+        try:
+            run(mid)
+            high = mid
+        except native.OdbaError:
+            low = mid
+    return high
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("value", [np.nan, np.inf, 1e30])
+def test_walks_that_fail_leave_the_same_samples(env, value, dtype):
+    # with the least workspace a member's path is walked cell by cell, with more
+    # row by row; NaN and infinite costs lead some walks off the first column
+    torch, api, native = env
+    rng = np.random.default_rng(23)
+    lens = [2200, 700, 1500, 3, 40, 1100, 2500, 65]
+    series = [np.cumsum(rng.standard_normal(L)).astype(dtype) for L in lens]
+    for s in series:
+        if rng.random() < 0.6:
+            s[rng.integers(0, len(s), size=2)] = value
+    ds = api.DeviceSeries.from_host(series)
+    for c in (2, 5, 6):
+        for open_both in (0, 1):
+            cen = torch.from_numpy(series[c].copy()).cuda()
+
+            def run(nbytes):
+                ws = None if nbytes is None else torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+                got = api.dba_round(cen, ds, open_both, 0, workspace=ws, stripe_rows=ROWS)
+                return got[0].cpu().numpy().tobytes(), got[1].cpu().numpy().tobytes(), got[2]
+
+            assert run(None) == run(_least(run, 64 << 20, native)), (c, open_both)
