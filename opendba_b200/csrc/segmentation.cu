@@ -19,7 +19,7 @@
 // Kept as the reference computes them: the down-averaging loop bound (which
 // averages zero samples -- NaN -- for the upper part of a block), the
 // FLT_MIN/partial-warp rules of the min/max reduction, the block minimum that
-// only thread 0 sees, the saturating 8-bit conversion, the wrapping int product
+// only thread 0 sees, the 8-bit conversion (seg_byte), the wrapping int product
 // in DIST, and the even-span median pick (segmentation.hpp:327-332).  Where the
 // reference races (a 2-sample segment's median reads the first sample of the
 // next segment while that one is being sorted) the sorted value is used.
@@ -67,6 +67,15 @@ __device__ __forceinline__ T warp_max(T v) {
     if (o > v) v = o;
   }
   return v;
+}
+
+// The conversion to 8 bits as the device compiles the reference's cast
+// (segmentation.hpp:168): truncated to an unsigned 32-bit value, which saturates
+// (negative and NaN give a low byte of 0), and of that the low byte.  Points past
+// the last whole group of 32 are not part of the block's range and can lie
+// outside it: 256 gives 0, 300 gives 44.
+__device__ __forceinline__ unsigned char seg_byte(double v) {
+  return (unsigned char)(__double2uint_rz(v) & 255u);
 }
 
 struct SegParams {
@@ -287,7 +296,7 @@ __global__ void __launch_bounds__(kSegThreads) segment_kernel(const T *series,
   unsigned pv = 0, pq = 0;
   if (t < 256) {
     if (t < N_ds) {
-      q[t] = (unsigned char)(256.0 * ((dsv - mn) / (gmax - mn + 1)));
+      q[t] = seg_byte(256.0 * ((dsv - mn) / (gmax - mn + 1)));
       pv = q[t];
       pq = pv * pv;
     }

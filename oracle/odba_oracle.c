@@ -588,11 +588,11 @@ int oracle_pairwise_fp64ref(const double *series, const uint64_t *offsets, const
  * sorted), the sorted value is used.  smem is the device's opt-in shared
  * memory per block; it sets the DP extent e. */
 static unsigned char seg_quant(double v) {
-  /* float -> unsigned char conversion on the GPU clamps to [0, 255], NaN -> 0 */
-  if (!(v == v)) return 0;
-  if (v <= 0.0) return 0;
-  if (v >= 255.0) return 255;
-  return (unsigned char)v;
+  /* the GPU's double -> unsigned char cast: to unsigned 32 bits with saturation
+   * (NaN -> 2^31), then the low byte */
+  if (!(v == v) || v <= 0.0) return 0;
+  if (v >= 4294967295.0) return 255;
+  return (unsigned char)((unsigned)v & 255u);
 }
 
 #define DEFINE_SEG(T, SFX, TMAX, TMIN)                                                         \
