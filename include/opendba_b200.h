@@ -44,6 +44,11 @@ const char *odba_status_string(int status);
 const char *odba_last_error(void);
 /* ODBA_OK when the current CUDA device is a compute capability 10.x (B200) part. */
 int odba_device_check(void);
+/* The entry points that take host buffers (odba_medoid_pass_host_*,
+ * odba_dba_jobs_*, odba_segment_host_*) keep up to 256 MB of device scratch per
+ * device between calls; this gives the current device's back (what calls in
+ * flight in other threads use stays theirs). */
+int odba_scratch_release(void);
 
 /* ---- all-vs-all DTW distances (the medoid pass) ----------------------------
  * Replaces the DTWDistance launch loop of approximateMedoidIndices

@@ -30,6 +30,7 @@ SIGNATURES = {
     "odba_status_string": (ctypes.c_char_p, [I32]),
     "odba_last_error": (ctypes.c_char_p, []),
     "odba_device_check": (I32, []),
+    "odba_scratch_release": (I32, []),
     "odba_dtw_pairwise_workspace_bytes": (ctypes.c_size_t, [I32, U64]),
     "odba_dtw_pairwise_workspace_bytes_n": (ctypes.c_size_t, [I32, I32, U64]),
     "odba_dtw_pairwise_range_f32": (I32, [P, P, P, I32, U64, I32, I32, U64, U64, P, P, ctypes.c_size_t, P]),

@@ -63,8 +63,16 @@ cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t stream) {
   return e;
 }
 
-void scratch_free(void *p, cudaStream_t stream) {
-  if (p) cudaFreeAsync(p, stream);
+void scratch_free(void *p, size_t bytes, cudaStream_t stream) {
+  if (!p) return;
+  cudaFreeAsync(p, stream);
+  if (bytes >= kScratchSyncBytes) cudaStreamSynchronize(stream);
+}
+
+int scratch_trim() {
+  const cudaMemPool_t pool = scratch_pool();
+  if (pool && cudaMemPoolTrimTo(pool, 0) != cudaSuccess) return check_launch("scratch pool");
+  return ODBA_OK;
 }
 
 int check_launch(const char *what) {
@@ -196,7 +204,7 @@ int medoid_pass_host(const T *h_series, const uint64_t *h_lens, int n, int os, i
     return ODBA_OK;
   };
   const int rc = run();
-  scratch_free(base, stream);
+  scratch_free(base, o_ws + ws_bytes, stream);
   return rc;
 }
 
@@ -298,6 +306,11 @@ const char *odba_status_string(int status) {
 const char *odba_last_error(void) { return odba::g_err; }
 
 int odba_device_check(void) { return require_sm100(); }
+
+int odba_scratch_release(void) {
+  if (int rc = require_sm100()) return rc;
+  return scratch_trim();
+}
 
 size_t odba_dtw_pairwise_workspace_bytes(int elem_size, uint64_t max_len) {
   if (elem_size == 8) return pairwise_workspace_bytes<double>(max_len);

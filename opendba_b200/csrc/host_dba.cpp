@@ -189,7 +189,7 @@ struct DevBuf {
   bool scratch = false;
   void release() {
     if (p && scratch)
-      odba::scratch_free(p, st);
+      odba::scratch_free(p, bytes, st);
     else if (p)
       cudaFree(p);
     p = nullptr;

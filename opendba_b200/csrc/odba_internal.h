@@ -21,10 +21,14 @@ int require_sm100();
 // Stream-ordered scratch of the host-buffer entry points, from a pool of the
 // library's own per device that keeps up to 256 MB mapped between calls (the
 // default pool unmaps what is freed at every synchronisation: mapping the
-// scratch again cost 0.4-0.7 ms a call).  Memory beyond that goes back at the
-// next synchronisation, all of it when an allocation fails.
+// scratch again cost 0.4-0.7 ms a call).  Memory beyond that goes back when a
+// block of kScratchSyncBytes or more is freed (which waits for the stream: the
+// pool looks at its size when it is synchronised with), all of it when an
+// allocation fails or when the program asks (scratch_trim).
+constexpr size_t kScratchSyncBytes = size_t(16) << 20;
 cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t stream);
-void scratch_free(void *p, cudaStream_t stream);
+void scratch_free(void *p, size_t bytes, cudaStream_t stream);
+int scratch_trim();
 
 template <typename T>
 size_t pairwise_workspace_bytes(uint64_t max_len);
