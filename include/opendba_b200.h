@@ -138,12 +138,12 @@ int odba_tune_load(const char *path);
 int odba_round_set_bands(int n);
 
 /* ---- self-test of the bounded device wait --------------------------------------
- * No reference counterpart.  A block sweeps a swath whose left neighbour's
- * progress word nothing publishes, with the swath pipeline's own sweep and
- * wait and the given limit (at most 10 s); then the warps of a block wait for
- * a feeding warp that is not there (four times the limit).  Returns
- * ODBA_ERR_TIMEOUT when both waits ran out and raised their error words, as
- * they must. */
+ * No reference counterpart.  A block, then a warp, sweeps a swath whose left
+ * neighbour's progress word nothing publishes, with the swath pipelines' own
+ * sweeps and waits and the given limit (at most 10 s); between them the warps
+ * of a block wait for a feeding warp that is not there (four times the limit).
+ * Returns ODBA_ERR_TIMEOUT when all three waits ran out and raised their error
+ * words, as they must. */
 int odba_selftest_wait_timeout(uint64_t limit_ns, void *stream);
 
 /* ---- DTW distances of an arbitrary pair list (batched jobs, queries) ----------

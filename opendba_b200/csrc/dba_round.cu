@@ -4,9 +4,9 @@
 //  1. plan:      per member the orientation (the centroid goes on the Y axis
 //                when open_end and it is the shorter one, dba.hpp:497-501),
 //                the size and offset of its 2-bit path, and its path-file slot.
-//  2. path DTW:  persistent launch, a block per swath (dtw_block.cuh); records
-//                every move and the right-edge minima the open-end shortcut
-//                needs.
+//  2. path DTW:  persistent launch, a block per swath (dtw_block.cuh) or, in
+//                large rounds, a warp (dtw_warp.cuh); records every move and
+//                the right-edge minima the open-end shortcut needs.
 //  3. backtrack: one warp per member walks its path from the end cell back to
 //                (0, 0) (updateCentroid's loop) and stores, per centroid index,
 //                the contiguous range of member samples that index receives --
@@ -30,6 +30,7 @@
 #include "dtw_block.cuh"
 #include "dtw_path.cuh"
 #include "dtw_pipe.cuh"
+#include "dtw_warp.cuh"
 #include "odba_internal.h"
 
 namespace odba {
@@ -141,6 +142,7 @@ struct RoundArgs {
   T *emtop;  // per (band, member, swath)
   unsigned *err;
   int max_swaths;
+  int one_warp = 0;  // a warp per swath, whose moves are laid out as WarpMap has them
   // row bands of the swath pipeline (member_band): per (member, swath) the
   // last row and edge corner of the band done so far, and that band's count
   int nbands = 1;
@@ -285,14 +287,14 @@ __global__ void fill_ranges_kernel(int2 *r, unsigned long long count) {
 // top row is OPEN_RIGHT: the first qualifying swath boundary, or 0.
 template <typename T>
 __device__ __forceinline__ int member_shortcut(const RoundArgs<T> &a, int k, const MemberGeom &g,
-                                               int flags) {
+                                               int flags, int cols) {
   const int os = flags & 1, oe = (flags >> 1) & 1;
   if (!oe || os) return 0;
   const int nb = member_band(g, a.nbands, 0).count;
   const unsigned long long layer = (unsigned long long)a.nmem * a.max_swaths;
-  for (int s = 0; s + 1 < g.swaths; ++s) {
-    const int cnext = (s + 1) * kBlkCols;
-    if (cnext <= g.m || cnext >= g.n) continue;
+  for (int s = 0; (s + 1) * cols < g.n; ++s) {
+    const int cnext = (s + 1) * cols;  // (a swath of `cols` columns)
+    if (cnext % kRefSwath || cnext <= g.m) continue;
     T emin = Num<T>::big(), etop = Num<T>::big();
     for (int b = 0; b < nb; ++b) {
       const T *et = a.emtop + ((unsigned long long)b * layer + (unsigned long long)k * a.max_swaths + s) * 2;
@@ -304,11 +306,96 @@ __device__ __forceinline__ int member_shortcut(const RoundArgs<T> &a, int k, con
   return 0;
 }
 
-template <typename T>
-__device__ __forceinline__ bool walk_member_runs(const RoundArgs<T> &a, const MemberGeom &g, int k,
-                                                 int os, int oe, int2 *runs);
+// The moves of one row's 32 columns cb .. cb + 31 (cb a multiple of 32): bit
+// j of d (u) is column cb + j's D (U) bit.
+struct RowMoves {
+  unsigned d, u;
+};
 
-// Path DTW, a block per swath (sweep_block).  PIPE: task q is band
+// Where a matrix's moves are, as the block sweep lays them out (from column cmin,
+// a multiple of the swath, on): four lanes of 8 columns hold a row's 32 columns,
+// each a step behind its left neighbour.  Rows r >= 1.
+struct BlockMap {
+  const unsigned short *w;
+  int r0, steps, cmin;
+  struct At {
+    const unsigned short *p;
+  };
+  __device__ __forceinline__ At at(int r, int cb) const {
+    const int k = r - r0, l = ((cb - cmin) / kBlkR) & 31;
+    return At{w + (((size_t)((cb - cmin) / kBlkWarpCols) * steps + (k >> 1) + l) * 32 + l) * 2 + (k & 1)};
+  }
+  // the 32 columns cb .. to the left of a's, and the rows 32 below a's
+  __device__ __forceinline__ At left(At a, int r, int cb) const {
+    return ((cb - cmin + 32) & (kBlkWarpCols - 1)) ? At{a.p - 4 * 66} : at(r, cb);
+  }
+  static __device__ __forceinline__ At below(At a) { return At{a.p - 16 * 64}; }
+  static __device__ __forceinline__ RowMoves load(At a) {
+    const unsigned lo = unsigned(a.p[0]) | unsigned(a.p[66]) << 16;
+    const unsigned hi = unsigned(a.p[132]) | unsigned(a.p[198]) << 16;
+    return RowMoves{__byte_perm(lo, hi, 0x6420), __byte_perm(lo, hi, 0x7531)};
+  }
+};
+
+// The one-warp sweep: columns per lane of a full swath, and of a last one of
+// `width` columns (the least of 8, 16 and 32 that covers it: a row's 32 columns
+// are then 1, 2 or 4 lanes').
+template <typename T>
+constexpr int kWarpR = sizeof(T) == 4 ? 32 : 16;
+template <typename T>
+__host__ __device__ inline int warp_cols() {
+  return 32 * kWarpR<T>;
+}
+template <typename T>
+__host__ __device__ inline int warp_regs(int width) {
+  return width <= 256 ? 8 : width <= 512 ? 16 : kWarpR<T>;
+}
+template <typename T>
+struct WarpMap {
+  static constexpr int KW = WarpMoves<T>::kWords;
+  const unsigned *w;
+  int r0, steps, n;
+  struct At {
+    const unsigned *p;
+    int lanes;
+  };
+  __device__ __forceinline__ At at(int r, int cb) const {
+    const int k = r - r0, s = cb / warp_cols<T>(), c = cb - s * warp_cols<T>();
+    const int R = warp_regs<T>(n - cb + c), l = c / R;
+    return At{w + (((size_t)s * steps + (k >> 1) + l) * 64 + l * 2 + (k & 1)) * KW, 32 / R};
+  }
+  __device__ __forceinline__ At left(At a, int r, int cb) const {
+    return (cb + 32) % warp_cols<T>() ? At{a.p - a.lanes * 66 * KW, a.lanes} : at(r, cb);
+  }
+  static __device__ __forceinline__ At below(At a) { return At{a.p - 16 * 64 * KW, a.lanes}; }
+  static __device__ __forceinline__ RowMoves load(At a) {
+    RowMoves m{0u, 0u};
+    const int R = 32 / a.lanes;
+    for (int i = 0; i < a.lanes; ++i) {
+      const unsigned *p = a.p + i * 66 * KW;
+      const unsigned d = KW == 2 ? p[0] : p[0] & 0xffffu, u = KW == 2 ? p[1] : p[0] >> 16;
+      m.d |= d << (i * R);
+      m.u |= u << (i * R);
+    }
+    return m;
+  }
+};
+
+template <typename T>
+__device__ __forceinline__ BlockMap block_map(const RoundArgs<T> &a, const MemberGeom &g, int k) {
+  return BlockMap{reinterpret_cast<const unsigned short *>(a.words + a.path_off[k]), g.r0, g.steps, 0};
+}
+template <typename T>
+__device__ __forceinline__ WarpMap<T> warp_map(const RoundArgs<T> &a, const MemberGeom &g, int k) {
+  return WarpMap<T>{reinterpret_cast<const unsigned *>(a.words + a.path_off[k]), g.r0, g.steps, g.n};
+}
+
+template <typename T, typename Map>
+__device__ __forceinline__ bool walk_member_runs(const RoundArgs<T> &a, const Map &map,
+                                                 const MemberGeom &g, int k, int os, int oe,
+                                                 int2 *runs);
+
+// Path DTW, a block per swath (sweep_block): task q is band
 // q / (nmem * max_swaths) of a swath of the (q % nmem)-th member in alignment
 // order, in turn (q / nmem) % max_swaths, so a member's swaths run in different
 // blocks at once (few or long members keep the GPU busy).  The last swaths of
@@ -323,9 +410,7 @@ __device__ __forceinline__ bool walk_member_runs(const RoundArgs<T> &a, const Me
 // (member, swath)'s band word; the recorded moves are the same.  Each band
 // also stores its right edge's minimum and top-row value for the open-end
 // shortcut, which never changes a recorded move.  Every wait is on a task
-// taken earlier from the counter.  Without PIPE (edge columns of all members
-// too large) a task is a member, swath after swath, with two edge columns per
-// block.
+// taken earlier from the counter.
 //
 // The block's cost per cell is the one-warp sweep's plus about 14 instructions
 // per 16 cells (loads of samples and edge, shuffles, stores); what it buys is
@@ -342,11 +427,8 @@ __device__ __forceinline__ bool walk_member_runs(const RoundArgs<T> &a, const Me
 // members of 3000-8000 samples 5.79 / 5.86 / 6.24 / 6.54 ms, 600 8.61 / 8.11 /
 // 8.39 / 8.67, 1000 13.75 / 12.95 / 13.06 / 13.09, 512 of 1000-2000 (open end)
 // 1.10 / 1.00 / 1.07 / 1.14; double 1.71 with four, 1.53 with two.
-//
-// Above about a thousand members the one-warp sweep's lower cost per cell would
-// win (2000 of 3000-8000: 22.6 ms against 25.5).
 constexpr int kRoundBlocksF32 = 4, kRoundBlocksF64 = 2;
-template <typename T, bool PIPE, bool BAND>
+template <typename T, bool BAND>
 __global__ void
 __launch_bounds__(kBlkThreads, sizeof(T) == 4 ? kRoundBlocksF32 : kRoundBlocksF64)
     path_block_kernel(RoundArgs<T> a) {
@@ -354,7 +436,7 @@ __launch_bounds__(kBlkThreads, sizeof(T) == 4 ? kRoundBlocksF32 : kRoundBlocksF6
   const int lane = threadIdx.x & 31;
   const bool feeder = (threadIdx.x >> 5) == kBlkWarps;
   const unsigned long long layer = (unsigned long long)a.nmem * a.max_swaths;
-  const unsigned long long ntasks = PIPE ? layer * a.nbands : (unsigned long long)a.nmem;
+  const unsigned long long ntasks = layer * a.nbands;
   auto member_of = [&](unsigned long long qi) {
     return a.order ? a.order[qi] : a.nmem - 1 - int(qi);
   };
@@ -367,12 +449,12 @@ __launch_bounds__(kBlkThreads, sizeof(T) == 4 ? kRoundBlocksF32 : kRoundBlocksF6
       for (;;) {
         q = atomicAdd(a.counter, 1ull);
         if (q >= ntasks) break;
-        const unsigned long long ql = PIPE ? q % layer : q;
+        const unsigned long long ql = q % layer;
         int jb;
-        const MemberGeom g = geom_of<T>(a, member_of(PIPE ? ql % a.nmem : q), jb);
+        const MemberGeom g = geom_of<T>(a, member_of(ql % a.nmem), jb);
         if (!(a.jflags[jb] & 4)) continue;
-        if (PIPE && (unsigned)(int(ql / a.nmem) - late(g)) >= (unsigned)g.swaths) continue;
-        if (PIPE && BAND && int(q / layer) >= member_band(g, a.nbands, 0).count) continue;
+        if ((unsigned)(int(ql / a.nmem) - late(g)) >= (unsigned)g.swaths) continue;
+        if (BAND && int(q / layer) >= member_band(g, a.nbands, 0).count) continue;
         break;
       }
       sm.task = q;
@@ -380,93 +462,81 @@ __launch_bounds__(kBlkThreads, sizeof(T) == 4 ? kRoundBlocksF32 : kRoundBlocksF6
     __syncthreads();
     const unsigned long long q = sm.task;
     if (q >= ntasks) break;
-    const int b = PIPE && BAND ? int(q / layer) : 0;
-    const unsigned long long ql = PIPE ? q - (unsigned long long)b * layer : 0;
-    const int turn = PIPE ? int(ql / a.nmem) : 0;
-    const int k = member_of(PIPE ? ql - (unsigned long long)turn * a.nmem : q);
+    const int b = BAND ? int(q / layer) : 0;
+    const unsigned long long ql = q - (unsigned long long)b * layer;
+    const int turn = int(ql / a.nmem);
+    const int k = member_of(ql - (unsigned long long)turn * a.nmem);
     int jb;
     const MemberGeom g = geom_of<T>(a, k, jb);
-    const int s_first = PIPE ? turn - late(g) : 0;
+    const int s = turn - late(g);
     const int flags = a.jflags[jb];
-    const Band bd = member_band(g, PIPE && BAND ? a.nbands : 1, b);
+    const Band bd = member_band(g, BAND ? a.nbands : 1, b);
     const int os = flags & 1, oe = (flags >> 1) & 1;
     const T *seq = a.series + a.offsets[a.mseries[k]];
     const T *cen = a.centroids + a.coff[jb];
-    T *b0 = a.edges + (PIPE ? (unsigned long long)k : (unsigned long long)blockIdx.x) * 2 * a.edge_stride;
+    T *b0 = a.edges + (unsigned long long)k * 2 * a.edge_stride;
     T *b1 = b0 + a.edge_stride;
     const int base = bd.rb - g.r0;  // even: bands keep the step layout
-    int shortcut = 0;               // !PIPE, feeder's lane 0
-    for (int s = s_first; s < (PIPE ? s_first + 1 : g.swaths); ++s) {
-      const int c0 = s * kBlkCols;
-      const bool last = s == g.swaths - 1;
-      const unsigned long long ks = (unsigned long long)k * a.max_swaths + s;
-      BlockJob<T> job;
-      job.x = g.flip ? cen : seq;
-      job.y = g.flip ? seq : cen;
-      job.m = bd.re;
-      job.n = g.n;
-      job.c0 = c0;
-      job.r0 = bd.rb;
-      job.edge_in = s ? (((s - 1) & 1) ? b1 : b0) + base : nullptr;
-      job.edge_out = last ? nullptr : ((s & 1) ? b1 : b0) + base;
-      job.open_end = oe != 0;
-      job.free_diag0 = c0 > 0;
-      job.corner_init = c0 == 0 ? (g.r0 ? Num<T>::big() : T(0)) : (g.r0 ? T(0) : Num<T>::big());
-      job.word_steps = g.steps;
-      job.words = reinterpret_cast<unsigned *>(a.words + a.path_off[k] +
-                                               (unsigned long long)s * g.steps * 64ull) +
-                  (size_t)(base / 2) * 32;
-      if (PIPE && BAND) {
-        T *row = a.rowbuf + ks * (kBlkCols + 32);
-        if (b > 0) {
-          // the band below, complete: its last row, and its left edge's value there
-          if (feeder && lane == 0)
-            wait_word_at_least(a.bdone + ks, (unsigned long long)b, a.err, kWaitLimitNs);
-          __syncthreads();
-          (void)ld_acquire_gpu(a.bdone + ks);
-          job.row_in = row;
-          job.corner_init = s ? row[kBlkCols] : Num<T>::big();
-        }
-        job.top_band = b == bd.count - 1;
-        if (b + 1 < bd.count) {
-          job.row_out = row;
-          job.corner_out = row + kBlkCols;
-        }
-      }
-      T unused = T(0);
-      EdgeStat<T> st;
-      if (PIPE) {
-        unsigned long long *words = a.prog + (unsigned long long)k * a.max_swaths;
-        BandGate gate;
-        gate.g.prog_in = words + (s ? s - 1 : 0);
-        gate.g.prog_out = words + s;
-        gate.g.err = a.err;
-        gate.g.limit_ns = kWaitLimitNs;
-        gate.g.avail = 0;
-        gate.base = base;
-        sweep_block<T, true, BAND, false, false>(job, sm, gate, CkptOut<T>{nullptr, 0, 1}, false,
-                                                 unused, st);
-        if (feeder && lane == 0) {
-          T *et = a.emtop + ((unsigned long long)b * layer + ks) * 2;
-          et[0] = st.emin;
-          et[1] = st.etop;
-        }
-        if (BAND && b + 1 < bd.count) {
-          // the row buffer and corner of every thread, then the band word
-          __threadfence();
-          __syncthreads();
-          if (feeder && lane == 0) st_release_gpu(a.bdone + ks, (unsigned long long)(b + 1));
-        }
-      } else {
-        sweep_block<T, true, false, false, false>(job, sm, NoGate(a.err), CkptOut<T>{nullptr, 0, 1},
-                                                  false, unused, st);
-        const int cnext = c0 + kBlkCols;
-        if (oe && !os && !shortcut && !last && cnext > g.m && st.etop == st.emin) shortcut = cnext;
+    const int c0 = s * kBlkCols;
+    const bool last = s == g.swaths - 1;
+    const unsigned long long ks = (unsigned long long)k * a.max_swaths + s;
+    BlockJob<T> job;
+    job.x = g.flip ? cen : seq;
+    job.y = g.flip ? seq : cen;
+    job.m = bd.re;
+    job.n = g.n;
+    job.c0 = c0;
+    job.r0 = bd.rb;
+    job.edge_in = s ? (((s - 1) & 1) ? b1 : b0) + base : nullptr;
+    job.edge_out = last ? nullptr : ((s & 1) ? b1 : b0) + base;
+    job.open_end = oe != 0;
+    job.free_diag0 = c0 > 0;
+    job.corner_init = c0 == 0 ? (g.r0 ? Num<T>::big() : T(0)) : (g.r0 ? T(0) : Num<T>::big());
+    job.word_steps = g.steps;
+    job.words = reinterpret_cast<unsigned *>(a.words + a.path_off[k] +
+                                             (unsigned long long)s * g.steps * 64ull) +
+                (size_t)(base / 2) * 32;
+    if (BAND) {
+      T *row = a.rowbuf + ks * (kBlkCols + 32);
+      if (b > 0) {
+        // the band below, complete: its last row, and its left edge's value there
+        if (feeder && lane == 0)
+          wait_word_at_least(a.bdone + ks, (unsigned long long)b, a.err, kWaitLimitNs);
         __syncthreads();
+        (void)ld_acquire_gpu(a.bdone + ks);
+        job.row_in = row;
+        job.corner_init = s ? row[kBlkCols] : Num<T>::big();
+      }
+      job.top_band = b == bd.count - 1;
+      if (b + 1 < bd.count) {
+        job.row_out = row;
+        job.corner_out = row + kBlkCols;
       }
     }
-    if (!PIPE && feeder && lane == 0) a.shortcut[k] = shortcut;
-    if (PIPE && a.walk_in_sweep) {
+    T unused = T(0);
+    EdgeStat<T> st;
+    unsigned long long *words = a.prog + (unsigned long long)k * a.max_swaths;
+    BandGate gate;
+    gate.g.prog_in = words + (s ? s - 1 : 0);
+    gate.g.prog_out = words + s;
+    gate.g.err = a.err;
+    gate.g.limit_ns = kWaitLimitNs;
+    gate.g.avail = 0;
+    gate.base = base;
+    sweep_block<T, true, BAND, false, false>(job, sm, gate, CkptOut<T>{nullptr, 0, 1}, false, unused,
+                                             st);
+    if (feeder && lane == 0) {
+      T *et = a.emtop + ((unsigned long long)b * layer + ks) * 2;
+      et[0] = st.emin;
+      et[1] = st.etop;
+    }
+    if (BAND && b + 1 < bd.count) {
+      // the row buffer and corner of every thread, then the band word
+      __threadfence();
+      __syncthreads();
+      if (feeder && lane == 0) st_release_gpu(a.bdone + ks, (unsigned long long)(b + 1));
+    }
+    if (a.walk_in_sweep) {
       // Member k's last task to finish resolves its shortcut and walks its
       // path (pass 1 of the backtrack) while other blocks sweep: every task
       // makes its moves and edge values visible before it is counted.
@@ -479,13 +549,143 @@ __launch_bounds__(kBlkThreads, sizeof(T) == 4 ? kRoundBlocksF32 : kRoundBlocksF6
         if (n == (unsigned long long)g.swaths * bd.count) {
           __syncwarp();
           (void)ld_acquire_gpu(a.mdone + k);  // every lane: after all the member's tasks
-          if (lane == 0) a.shortcut[k] = member_shortcut<T>(a, k, g, flags);
+          if (lane == 0) a.shortcut[k] = member_shortcut<T>(a, k, g, flags, kBlkCols);
           __syncwarp();
-          walk_member_runs<T>(a, g, k, os, oe, a.runs + a.runs_off[k]);
+          walk_member_runs<T>(a, block_map<T>(a, g, k), g, k, os, oe, a.runs + a.runs_off[k]);
         }
       }
     }
     __syncthreads();  // the task word and the rings are free again
+  }
+}
+
+// Path DTW, a warp per swath (sweep_warp; fills_with_warps): the same pipeline,
+// tasks and turns, swaths of 512 columns in double.  Without PIPE (edge columns of
+// all members too large) a task is a member, swath after swath, with two edge
+// columns per warp.
+//
+// What bounds it is the issue port: 12 warps per SM (8 in double), 2000 float
+// members of 3000-8000 samples 11.1 cycles per cell and scheduler.
+constexpr int kRoundWarpBlocksF32 = 3, kRoundWarpBlocksF64 = 2;
+template <typename T, int R, typename Gate>
+__device__ __forceinline__ EdgeStat<T> path_warp_swath(const SwathJob<T> &job, WarpSmem<T> &sm,
+                                                       Gate gate) {
+  T unused = T(0);
+  return sweep_warp<T, R, true, Gate>(job, sm, false, unused, gate);
+}
+template <typename T, typename Gate>
+__device__ __forceinline__ EdgeStat<T> path_warp_any(const SwathJob<T> &job, WarpSmem<T> &sm,
+                                                     Gate gate) {
+  const int R = warp_regs<T>(job.n - job.c0);
+  if (R == kWarpR<T>) return path_warp_swath<T, kWarpR<T>>(job, sm, gate);
+  if (sizeof(T) == 4 && R == 16) return path_warp_swath<T, 16>(job, sm, gate);
+  return path_warp_swath<T, 8>(job, sm, gate);
+}
+template <typename T, bool PIPE>
+__global__ void
+__launch_bounds__(kRoundWarps * 32, sizeof(T) == 4 ? kRoundWarpBlocksF32 : kRoundWarpBlocksF64)
+    path_warp_kernel(RoundArgs<T> a) {
+  __shared__ WarpSmem<T> s_warp[kRoundWarps];
+  WarpSmem<T> &sm = s_warp[threadIdx.x >> 5];
+  constexpr int W = 32 * kWarpR<T>;
+  const int lane = threadIdx.x & 31;
+  const unsigned long long ntasks =
+      PIPE ? (unsigned long long)a.nmem * a.max_swaths : (unsigned long long)a.nmem;
+  auto member_of = [&](unsigned long long qi) {
+    return a.order ? a.order[qi] : a.nmem - 1 - int(qi);
+  };
+  auto swaths_of = [&](const MemberGeom &g) { return (g.n + W - 1) / W; };
+  // the swath of a turn (negative or past the last one: none)
+  auto swath_of = [&](const MemberGeom &g, int turn) {
+    const int n = swaths_of(g);
+    return turn - (n < a.max_swaths ? a.max_swaths - n : 0);
+  };
+  for (;;) {
+    unsigned long long q = 0;
+    if (lane == 0) {
+      // the next task that exists
+      for (;;) {
+        q = atomicAdd(a.counter, 1ull);
+        if (q >= ntasks) break;
+        int jb;
+        const MemberGeom g = geom_of<T>(a, member_of(PIPE ? q % a.nmem : q), jb);
+        if (!(a.jflags[jb] & 4)) continue;
+        if (PIPE && (unsigned)swath_of(g, int(q / a.nmem)) >= (unsigned)swaths_of(g)) continue;
+        break;
+      }
+    }
+    q = __shfl_sync(kFull, q, 0);
+    if (q >= ntasks) break;
+    const int k = member_of(PIPE ? q % a.nmem : q);
+    int jb;
+    const MemberGeom g = geom_of<T>(a, k, jb);
+    const int flags = a.jflags[jb], os = flags & 1, oe = (flags >> 1) & 1;
+    const int nsw = swaths_of(g), s0 = PIPE ? swath_of(g, int(q / a.nmem)) : 0;
+    const T *seq = a.series + a.offsets[a.mseries[k]];
+    const T *cen = a.centroids + a.coff[jb];
+    const unsigned long long col =
+        PIPE ? (unsigned long long)k
+             : (unsigned long long)blockIdx.x * kRoundWarps + (threadIdx.x >> 5);
+    T *b0 = a.edges + col * 2 * a.edge_stride;
+    T *b1 = b0 + a.edge_stride;
+    int shortcut = 0;
+    for (int s = s0; s < (PIPE ? s0 + 1 : nsw); ++s) {
+      const int c0 = s * W;
+      const bool last = s == nsw - 1;
+      SwathJob<T> job;
+      job.x = g.flip ? cen : seq;
+      job.y = g.flip ? seq : cen;
+      job.m = g.m;
+      job.n = g.n;
+      job.c0 = c0;
+      job.r0 = g.r0;
+      job.edge_in = s ? (((s - 1) & 1) ? b1 : b0) : nullptr;
+      job.edge_out = last ? nullptr : ((s & 1) ? b1 : b0);
+      job.open_end = oe != 0;
+      job.free_diag0 = c0 > 0 && c0 % kRefSwath == 0;
+      job.track = oe && !os && !last;
+      job.corner_init = c0 == 0 ? (g.r0 ? Num<T>::big() : T(0)) : (g.r0 ? T(0) : Num<T>::big());
+      job.words = reinterpret_cast<unsigned *>(a.words + a.path_off[k]) +
+                  (size_t)s * g.steps * 64 * WarpMoves<T>::kWords;
+      if (PIPE) {
+        unsigned long long *words = a.prog + (unsigned long long)k * a.max_swaths;
+        PipeGate gate;
+        gate.prog_in = words + (s ? s - 1 : 0);
+        gate.prog_out = words + s;
+        gate.err = a.err;
+        gate.limit_ns = kWaitLimitNs;
+        gate.avail = 0;
+        const EdgeStat<T> st = path_warp_any<T>(job, sm, gate);
+        if (lane == 0) {
+          T *et = a.emtop + ((unsigned long long)k * a.max_swaths + s) * 2;
+          et[0] = st.emin;
+          et[1] = st.etop;
+        }
+      } else {
+        const EdgeStat<T> st = path_warp_any<T>(job, sm, SoloGate());
+        const int cnext = c0 + W;
+        if (job.track && !shortcut && cnext % kRefSwath == 0 && cnext > g.m && st.etop == st.emin)
+          shortcut = cnext;
+        __syncwarp();  // the next swath reads what this one's lanes stored
+      }
+    }
+    if (!PIPE && lane == 0) a.shortcut[k] = shortcut;
+    if (PIPE && a.walk_in_sweep) {
+      // as in path_block_kernel: the member's last task to finish walks its path
+      __threadfence();
+      __syncwarp();
+      unsigned long long n = 0;
+      if (lane == 0) n = atomicAdd(a.mdone + k, 1ull) + 1;
+      n = __shfl_sync(kFull, n, 0);
+      if (n == (unsigned long long)nsw) {
+        __syncwarp();
+        (void)ld_acquire_gpu(a.mdone + k);  // every lane: after all the member's tasks
+        if (lane == 0) a.shortcut[k] = member_shortcut<T>(a, k, g, flags, W);
+        __syncwarp();
+        walk_member_runs<T>(a, warp_map<T>(a, g, k), g, k, os, oe, a.runs + a.runs_off[k]);
+      }
+    }
+    __syncwarp();
   }
 }
 
@@ -499,29 +699,7 @@ __global__ void shortcut_kernel(RoundArgs<T> a) {
   const MemberGeom g = geom_of<T>(a, k, jb);
   const int flags = a.jflags[jb];
   if (!(flags & 4)) return;
-  a.shortcut[k] = member_shortcut<T>(a, k, g, flags);
-}
-
-// The moves of one row's 32 columns cb .. cb + 31 (cb a multiple of 32): bit
-// j of d (u) is column cb + j's D (U) bit.  Four lanes of the sweep own them,
-// each a step behind its left neighbour.  Row r >= 1.
-struct RowMoves {
-  unsigned d, u;
-};
-__device__ __forceinline__ const unsigned short *row_moves_at(const unsigned short *w,
-                                                              const MemberGeom &g, int r, int cb) {
-  const int k = r - g.r0, l = (cb / kBlkR) & 31;
-  const size_t idx = ((size_t)(cb / kBlkWarpCols) * g.steps + (k >> 1) + l) * 32 + l;
-  return w + idx * 2 + (k & 1);
-}
-__device__ __forceinline__ RowMoves load_row_moves(const unsigned short *p) {
-  const unsigned lo = unsigned(p[0]) | unsigned(p[66]) << 16;
-  const unsigned hi = unsigned(p[132]) | unsigned(p[198]) << 16;
-  return RowMoves{__byte_perm(lo, hi, 0x6420), __byte_perm(lo, hi, 0x7531)};
-}
-__device__ __forceinline__ RowMoves row_moves(const unsigned short *w, const MemberGeom &g, int r,
-                                              int cb) {
-  return load_row_moves(row_moves_at(w, g, r, cb));
+  a.shortcut[k] = member_shortcut<T>(a, k, g, flags, a.one_warp ? warp_cols<T>() : kBlkCols);
 }
 
 // Walks member k's path from its end cell toward (0, 0) with one warp and
@@ -536,11 +714,11 @@ __device__ __forceinline__ RowMoves row_moves(const unsigned short *w, const Mem
 // row is row 0, dtw.hpp:105-108 runs before the row-0 loop), then row 0
 // (RIGHT or OPEN_RIGHT, NIL / NIL_OPEN_RIGHT at (0, 0)), then the recorded
 // code with RIGHT on the open-end top row meaning OPEN_RIGHT.
-template <typename T, typename Visit>
-__device__ __forceinline__ bool walk_member_path(const RoundArgs<T> &a, const MemberGeom &g, int k,
-                                                 int os, int oe, Visit &&visit) {
+template <typename T, typename Map, typename Visit>
+__device__ __forceinline__ bool walk_member_path(const RoundArgs<T> &a, const Map &map,
+                                                 const MemberGeom &g, int k, int os, int oe,
+                                                 Visit &&visit) {
   const int lane = threadIdx.x & 31;
-  const unsigned short *w = reinterpret_cast<const unsigned short *>(a.words + a.path_off[k]);
   const int shortcut = a.shortcut[k];
   // A path has at most m + n - 1 cells and never leaves the matrix; the checks
   // only keep a corrupt path buffer from turning into an endless or
@@ -551,7 +729,7 @@ __device__ __forceinline__ bool walk_member_path(const RoundArgs<T> &a, const Me
   for (;;) {
     const int top = r, cbeg = c & ~31;
     RowMoves mine{0u, 0u};
-    if (top - lane >= 1) mine = row_moves(w, g, top - lane, cbeg);
+    if (top - lane >= 1) mine = map.load(map.at(top - lane, cbeg));
     for (;;) {
       const int src = (top - r) & 31;
       const unsigned rd = __shfl_sync(kFull, mine.d, src), ru = __shfl_sync(kFull, mine.u, src);
@@ -609,15 +787,16 @@ __device__ __forceinline__ bool walk_member_path(const RoundArgs<T> &a, const Me
 //
 // The walk starts (or goes on) at st.r, st.c; st.entry is the column it
 // entered row st.r at (-1 on the open-end top row, whose interval is its first
-// cell alone).  w holds the moves of the columns from cmin (a multiple of the
+// cell alone).  map holds the moves of the columns from cmin (a multiple of the
 // swath) on; the walk ends at the start cell (1), when it fails (2: NaN or
 // infinite costs can lead it off column 0, in row st.r, whose interval is then
 // not stored), or when it leaves cmin to the left (0).
 struct RowWalk {
   int r, c, entry;
 };
-__device__ __forceinline__ int walk_runs(const unsigned short *w, const MemberGeom &g, int cmin,
-                                         RowWalk &st, int os, int2 *runs) {
+template <typename Map>
+__device__ __forceinline__ int walk_runs(const Map &map, const MemberGeom &g, int cmin, RowWalk &st,
+                                         int os, int2 *runs) {
   constexpr int G = 8;  // rows per group
   const int lane = threadIdx.x & 31;
   // every window advances the walk by a row or a block of columns: a bound on
@@ -629,7 +808,7 @@ __device__ __forceinline__ int walk_runs(const unsigned short *w, const MemberGe
   // top - l, its moves at `at`.
   int top = -1, cb = 0;
   RowMoves cur{0u, 0u}, down{0u, 0u}, left{0u, 0u};
-  const unsigned short *at = w, *at_left = w;
+  typename Map::At at{}, at_left{};
   int2 iv = make_int2(1, 0);
   bool have = false;
   for (;;) {
@@ -654,7 +833,7 @@ __device__ __forceinline__ int walk_runs(const unsigned short *w, const MemberGe
     if (++windows > max_windows) return 2;
     if (below && c >= cb) {
       top -= 32;
-      at -= 16 * 64;  // 16 steps of 32 words
+      at = Map::below(at);
       cur = down;
     } else if (top >= 0 && !below) {
       cb -= 32;
@@ -663,13 +842,13 @@ __device__ __forceinline__ int walk_runs(const unsigned short *w, const MemberGe
     } else {
       top = r;
       cb = c & ~31;
-      at = row_moves_at(w, g, top - lane, cb - cmin);
-      if (top - lane >= 1) cur = load_row_moves(at);
+      at = map.at(top - lane, cb);
+      if (top - lane >= 1) cur = map.load(at);
     }
-    if (top - 32 - lane >= 1) down = load_row_moves(at - 16 * 64);
+    if (top - 32 - lane >= 1) down = map.load(Map::below(at));
     if (cb > cmin && top - lane >= 1) {
-      at_left = (cb & (kBlkWarpCols - 1)) ? at - 4 * 66 : row_moves_at(w, g, top - lane, cb - 32 - cmin);
-      left = load_row_moves(at_left);
+      at_left = map.left(at, top - lane, cb - 32);
+      left = map.load(at_left);
     }
     // Rows that are not the walk's -- row 0 and below, and in the first group
     // those above the walk's row -- get moves that leave the walk where it is.
@@ -744,15 +923,15 @@ __device__ __forceinline__ int walk_runs(const unsigned short *w, const MemberGe
   }
 }
 
-template <typename T>
-__device__ __forceinline__ bool walk_member_runs(const RoundArgs<T> &a, const MemberGeom &g, int k,
-                                                 int os, int oe, int2 *runs) {
+template <typename T, typename Map>
+__device__ __forceinline__ bool walk_member_runs(const RoundArgs<T> &a, const Map &map,
+                                                 const MemberGeom &g, int k, int os, int oe,
+                                                 int2 *runs) {
   const int shortcut = a.shortcut[k];
   RowWalk st{g.m - 1, g.n - 1, 0};
   if (shortcut && st.c >= shortcut) st.c = shortcut - 1;  // OPEN_RIGHT from the shortcut's column on
   st.entry = oe ? -1 : st.c;
-  return walk_runs(reinterpret_cast<const unsigned short *>(a.words + a.path_off[k]), g, 0, st, os,
-                   runs) == 1;
+  return walk_runs(map, g, 0, st, os, runs) == 1;
 }
 
 // Pass 2: the contributing columns of row r are the interval runs[r] = [x, y].
@@ -809,7 +988,10 @@ __global__ void __launch_bounds__(kRoundWarps * 32) backtrack_kernel(RoundArgs<T
   const int os = flags & 1, oe = (flags >> 1) & 1;
   int2 *rg = a.ranges + a.rng_off[k];
   if (!a.triples) {
-    walk_member_runs<T>(a, g, k, os, oe, a.runs + a.runs_off[k]);
+    if (a.one_warp)
+      walk_member_runs<T>(a, warp_map<T>(a, g, k), g, k, os, oe, a.runs + a.runs_off[k]);
+    else
+      walk_member_runs<T>(a, block_map<T>(a, g, k), g, k, os, oe, a.runs + a.runs_off[k]);
     return;
   }
   int32_t *tri = a.triples + 3ull * a.trip_off[k];
@@ -828,7 +1010,7 @@ __global__ void __launch_bounds__(kRoundWarps * 32) backtrack_kernel(RoundArgs<T
       lo = mi;  // the walk only moves toward smaller indices
     }
   };
-  const bool ok = walk_member_path<T>(a, g, k, os, oe, [&](int mv, int r, int c) {
+  auto visit = [&](int mv, int r, int c) {
     if (mv == kMaxMoveNil || mv == kMoveNilOpenRight) {
       // the start cell (dba.hpp:412-415)
       if (mv != kMoveNilOpenRight) contribute(0, 0);
@@ -842,7 +1024,9 @@ __global__ void __launch_bounds__(kRoundWarps * 32) backtrack_kernel(RoundArgs<T
       tri[3 * nt + 2] = mv;
     }
     ++nt;
-  });
+  };
+  const bool ok = a.one_warp ? walk_member_path<T>(a, warp_map<T>(a, g, k), g, k, os, oe, visit)
+                             : walk_member_path<T>(a, block_map<T>(a, g, k), g, k, os, oe, visit);
   if (lead && a.triple_counts) a.triple_counts[k] = ok ? nt : -1;
 }
 
@@ -867,7 +1051,7 @@ __global__ void __launch_bounds__(kRoundWarps * 32) chop_walk_kernel(RoundArgs<T
   bool skipping = true;
   long long pos = -1;
   int row = -1, count = 0;
-  const bool ok = walk_member_path<T>(a, g, k, flags & 1, (flags >> 1) & 1, [&](int mv, int r, int c) {
+  auto visit = [&](int mv, int r, int c) {
     if (skipping) {
       if (mv == kMoveOpenRight) return;
       skipping = false;
@@ -883,7 +1067,10 @@ __global__ void __launch_bounds__(kRoundWarps * 32) chop_walk_kernel(RoundArgs<T
       row = r;
       count = 1;
     }
-  });
+  };
+  const int os = flags & 1, oe = (flags >> 1) & 1;
+  const bool ok = a.one_warp ? walk_member_path<T>(a, warp_map<T>(a, g, k), g, k, os, oe, visit)
+                             : walk_member_path<T>(a, block_map<T>(a, g, k), g, k, os, oe, visit);
   if (lead) {
     if (ok && row >= 0) h[row] = count;
     chop[k] = ok ? pos : -1;
@@ -1057,9 +1244,29 @@ int round_grid() {
   }
   int sms = 0, per_sm = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, path_block_kernel<T, true, false>,
-                                                kBlkThreads, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, path_block_kernel<T, false>, kBlkThreads, 0);
   constexpr int want = sizeof(T) == 4 ? kRoundBlocksF32 : kRoundBlocksF64;
+  if (per_sm > want) per_sm = want;
+  if (per_sm < 1) per_sm = 1;
+  const int g = sms * per_sm;
+  if (dev >= 0 && dev < 64) cached[dev].store(g, std::memory_order_relaxed);
+  return g;
+}
+
+// Resident blocks of the one-warp path kernel (cached like round_grid).
+template <typename T>
+int round_warp_grid() {
+  static std::atomic<int> cached[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64) {
+    const int c = cached[dev].load(std::memory_order_relaxed);
+    if (c) return c;
+  }
+  int sms = 0, per_sm = 0;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, path_warp_kernel<T, true>, kRoundWarps * 32, 0);
+  constexpr int want = sizeof(T) == 4 ? kRoundWarpBlocksF32 : kRoundWarpBlocksF64;
   if (per_sm > want) per_sm = want;
   if (per_sm < 1) per_sm = 1;
   const int g = sms * per_sm;
@@ -1075,6 +1282,7 @@ struct RoundLayout {
   int max_swaths;
   int nbands;  // row bands of the swath pipeline
   bool pipe;   // path DTW as the swath pipeline (two edge columns per member)
+  bool one_warp;  // a warp per swath, not a block
 };
 
 constexpr size_t kPipeEdgeBytes = size_t(8) << 30;  // per-member edge columns up to 8 GB
@@ -1088,7 +1296,39 @@ int pipe_bands() {
   return forced > 0 ? (forced < kMaxBands ? forced : kMaxBands) : 1;
 }
 
-// Workspace layout for nmem members / njobs jobs with the given totals.
+// Whether a round of `tasks` (member, 1024-column swath) pairs, the most swaths
+// of a member being max_swaths, fills the GPU with one warp per swath.  At full
+// load the one-warp sweep takes three quarters of the block sweep's issue slots
+// per cell; the block sweep ends a chain of swaths in a quarter of the steps, and
+// the longer the chains the more of them it takes to hide their ends.  One
+// B200, block time / one-warp time of a round (centroid of a middling member):
+//   float, 1 swath   100-400 samples    1000 / 1500 / 2000 / 2500 tasks  0.99 / 1.03 / 1.10 / 1.10
+//                    400-800            1000 / 2000 / 2500               0.93 / 0.94 / 1.07
+//          2         1000-2000          1200 / 1600 / 2000 / 2400        0.97 / 1.01 / 1.11 / 1.28
+//          3         2000-4000          1200 / 1800 / 2100 / 2700        0.81 / 0.99 / 1.03 / 1.04
+//          5-6       3000-8000          1800 / 2700 / 3000 / 3600        0.92 / 1.02 / 0.98 / 1.07
+//          12-13     8000-16000         2400 / 3000 / 3900               0.92 / 0.96 / 1.04
+//   double, 1        100-400            500 / 700 / 900                  0.99 / 1.11 / 1.24
+//                    400-800            300 / 500 / 700                  0.79 / 1.01 / 1.23
+//          2         1000-2000          400 / 600 / 800                  0.82 / 1.03 / 1.15
+//          3-4       2000-4000          600 / 1200                       0.86 / 1.13
+//          5-6       3000-8000          1200 / 1500 / 1800               0.96 / 1.02 / 1.03
+//          11-12     8000-16000         1200 / 1650                      0.96 / 0.99
+// Larger ones: 2000 float members of 3000-8000 25.2 ms (block) and 20.0, 1000
+// double ones 28.2 and 22.3.
+template <typename T>
+bool fills_with_warps(unsigned long long tasks, int max_swaths) {
+  const unsigned long long slots = (unsigned long long)round_warp_grid<T>() * kRoundWarps;
+  if (sizeof(T) == 4)
+    return max_swaths <= 4 ? tasks * 5 >= slots * 6 : max_swaths <= 8 ? tasks * 5 >= slots * 8 : tasks >= slots * 2;
+  return max_swaths <= 2   ? tasks * 2 >= slots
+         : max_swaths <= 4 ? tasks * 6 >= slots * 5
+         : max_swaths <= 8 ? tasks * 2 >= slots * 3
+                           : tasks * 4 >= slots * 7;
+}
+
+// Workspace layout for nmem members / njobs jobs with the given totals; tasks:
+// (member, 1024-column swath) pairs of active members.
 template <typename T>
 RoundLayout round_layout(int nmem, int njobs, unsigned long long words,
                          unsigned long long ranges, unsigned long long maxm, int max_swaths = 0,
@@ -1096,10 +1336,12 @@ RoundLayout round_layout(int nmem, int njobs, unsigned long long words,
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
   RoundLayout L;
   L.edge_stride = (maxm + 32 + 31) / 32 * 32;
-  const size_t slots = size_t(round_grid<T>());
-  L.max_swaths = max_swaths;
   L.pipe = max_swaths > 0 && size_t(nmem) * 2 * L.edge_stride * sizeof(T) <= kPipeEdgeBytes;
-  const size_t edge_cols = L.pipe ? size_t(nmem) : slots;
+  L.nbands = L.pipe ? pipe_bands() : 1;
+  L.one_warp = max_swaths > 0 && (!L.pipe || (L.nbands == 1 && fills_with_warps<T>(tasks, max_swaths)));
+  L.max_swaths = L.one_warp ? max_swaths * (kBlkCols / warp_cols<T>()) : max_swaths;
+  const size_t edge_cols = L.pipe ? size_t(nmem)
+                           : L.one_warp ? size_t(round_warp_grid<T>()) * kRoundWarps : 0;
   size_t o = 0;
   L.off_counter = o; o += 256;
   L.off_path = o; o += up(size_t(nmem) * 8);
@@ -1113,8 +1355,7 @@ RoundLayout round_layout(int nmem, int njobs, unsigned long long words,
   L.off_runs = o; o += up(size_t(rows) * sizeof(int2));  // cleared with the ranges
   L.off_edges = o; o += up(edge_cols * 2 * L.edge_stride * sizeof(T));
   L.off_words = o; o += up(words * 8);
-  const size_t ps = L.pipe ? size_t(nmem) * size_t(max_swaths) : 0;
-  L.nbands = L.pipe ? pipe_bands() : 1;
+  const size_t ps = L.pipe ? size_t(nmem) * size_t(L.max_swaths) : 0;
   // row buffers for at most kMaxRowBufBytes (many inactive members: no bands)
   if (L.nbands > 1 && ps * (kBlkCols + 32) * sizeof(T) > kMaxRowBufBytes) L.nbands = 1;
   L.off_prog = o; o += up(ps * 8);
@@ -1181,25 +1422,29 @@ void launch_paths(RoundArgs<T> &a, const RoundLayout &L, char *base, cudaStream_
   cudaMemsetAsync(a.counter, 0, 16, stream);  // work counter and error word
   plan_kernel<T><<<1, kPlanThreads, 0, stream>>>(a);
   fill_ranges_kernel<<<int(nr / 256 + 1 < 4096 ? nr / 256 + 1 : 4096), 256, 0, stream>>>(a.ranges, nr);
+  a.one_warp = L.one_warp ? 1 : 0;
   const unsigned long long tasks =
       L.pipe ? (unsigned long long)a.nmem * L.max_swaths * L.nbands : (unsigned long long)a.nmem;
-  const int resident = round_grid<T>();
-  const int grid = tasks < (unsigned long long)resident ? int(tasks) : resident;
-  if (L.pipe) {
-    cudaMemsetAsync(a.prog, 0, L.off_order - L.off_prog, stream);  // progress, band, member words
-    if (!a.order && a.nmem <= kRankMembers) {
-      int *ord = reinterpret_cast<int *>(base + L.off_order);
-      rank_members_kernel<T><<<(a.nmem + 255) / 256, 256, 0, stream>>>(a, ord);
-      a.order = ord;
-    }
-    if (L.nbands > 1)
-      path_block_kernel<T, true, true><<<grid, kBlkThreads, 0, stream>>>(a);
-    else
-      path_block_kernel<T, true, false><<<grid, kBlkThreads, 0, stream>>>(a);
-    if (!a.walk_in_sweep) shortcut_kernel<T><<<(a.nmem + 127) / 128, 128, 0, stream>>>(a);
-  } else {
-    path_block_kernel<T, false, false><<<grid, kBlkThreads, 0, stream>>>(a);
+  const unsigned long long wgrid = L.one_warp ? round_warp_grid<T>() : round_grid<T>(),
+                           wblocks = L.one_warp ? (tasks + kRoundWarps - 1) / kRoundWarps : tasks;
+  const int grid = int(wblocks < wgrid ? wblocks : wgrid);
+  if (!L.pipe) {
+    path_warp_kernel<T, false><<<grid, kRoundWarps * 32, 0, stream>>>(a);
+    return;
   }
+  cudaMemsetAsync(a.prog, 0, L.off_order - L.off_prog, stream);  // progress, band, member words
+  if (!a.order && a.nmem <= kRankMembers) {
+    int *ord = reinterpret_cast<int *>(base + L.off_order);
+    rank_members_kernel<T><<<(a.nmem + 255) / 256, 256, 0, stream>>>(a, ord);
+    a.order = ord;
+  }
+  if (L.one_warp)
+    path_warp_kernel<T, true><<<grid, kRoundWarps * 32, 0, stream>>>(a);
+  else if (L.nbands > 1)
+    path_block_kernel<T, true><<<grid, kBlkThreads, 0, stream>>>(a);
+  else
+    path_block_kernel<T, false><<<grid, kBlkThreads, 0, stream>>>(a);
+  if (!a.walk_in_sweep) shortcut_kernel<T><<<(a.nmem + 127) / 128, 128, 0, stream>>>(a);
 }
 
 // The backtrack: with a path listing one kernel walking cell by cell; without,
@@ -1373,6 +1618,22 @@ size_t dba_batch_workspace_bytes(const uint64_t *h_mlens, const int *h_mjob, int
     if (h_clen[j] > maxm) maxm = h_clen[j];
   return round_layout<T>(nmem, njobs, words, ranges, maxm, ms, rows, tasks).total;
 }
+
+template <typename T>
+bool dba_batch_by_warp(const uint64_t *h_mlens, const int *h_mjob, int nmem, const uint64_t *h_clen,
+                       const int *h_flags, int njobs) {
+  unsigned long long words, ranges, maxm;
+  int ms = 1;
+  unsigned long long rows = 0, tasks = 0;
+  host_totals<T>(h_mlens, h_mjob, nmem, h_clen, h_flags, words, ranges, maxm, &ms, &rows, &tasks);
+  for (int j = 0; j < njobs; ++j)
+    if (h_clen[j] > maxm) maxm = h_clen[j];
+  return round_layout<T>(nmem, njobs, words, ranges, maxm, ms, rows, tasks).one_warp;
+}
+template bool dba_batch_by_warp<float>(const uint64_t *, const int *, int, const uint64_t *,
+                                       const int *, int);
+template bool dba_batch_by_warp<double>(const uint64_t *, const int *, int, const uint64_t *,
+                                        const int *, int);
 
 template <typename T>
 int dba_batch_launch(const T *centroids, const unsigned long long *coff, const int *clen,
@@ -1734,8 +1995,9 @@ __device__ __forceinline__ void stripe_walk_runs(const StripeArgs<T> &a, int gro
   g.r0 = a.r0;
   g.steps = block_steps(mem.m - a.r0);
   RowWalk rw{w.r, w.c, w.entry};
-  const int got = walk_runs(reinterpret_cast<const unsigned short *>(stripe_words(a, slot, gi)), g,
-                            lo * kBlkCols, rw, a.r0, a.runs + slot * a.runs_slot);
+  const BlockMap map{reinterpret_cast<const unsigned short *>(stripe_words(a, slot, gi)), g.r0, g.steps,
+                     lo * kBlkCols};
+  const int got = walk_runs(map, g, lo * kBlkCols, rw, a.r0, a.runs + slot * a.runs_slot);
   if (lane == 0) {
     if (got == 2 && rw.entry >= 0) a.runs[slot * a.runs_slot + rw.r] = make_int2(0, rw.entry);
     w.r = rw.r;
@@ -1818,10 +2080,8 @@ __global__ void __launch_bounds__(32) stripe_walk_kernel(StripeArgs<T> a, int gr
   if (w.state || t_hi <= t_lo) return;
   const int os = a.r0, flip = mem.flip;
   const long long max_cells = (long long)mem.m + mem.n - 1;
-  MemberGeom g;
-  g.r0 = a.r0;
-  g.steps = block_steps(mem.m - a.r0);
-  const unsigned short *words = reinterpret_cast<const unsigned short *>(stripe_words(a, slot, gi));
+  const BlockMap map{reinterpret_cast<const unsigned short *>(stripe_words(a, slot, gi)), a.r0,
+                     block_steps(mem.m - a.r0), t_lo * kBlkCols};
   int2 *rg = a.ranges + (unsigned long long)mem.member * a.Lc;
   int *extra = a.extra ? a.extra + (unsigned long long)mem.member * a.Lc : nullptr;
   int32_t *tri = a.triples ? a.triples + 3ull * mem.trip : nullptr;
@@ -1872,7 +2132,7 @@ __global__ void __launch_bounds__(32) stripe_walk_kernel(StripeArgs<T> a, int gr
       // window: rows w.r - lane, columns cbeg .. cbeg + 31
       const int top = w.r, cbeg = w.c & ~31;
       RowMoves mine{0u, 0u};
-      if (top - lane >= 1) mine = row_moves(words, g, top - lane, cbeg - t_lo * kBlkCols);
+      if (top - lane >= 1) mine = map.load(map.at(top - lane, cbeg));
       for (;;) {
         int mv;
         const unsigned rd = __shfl_sync(kFull, mine.d, (top - w.r) & 31);
@@ -2210,9 +2470,10 @@ size_t prefix_chop_workspace_bytes(const uint64_t *h_lens, int n, uint64_t P) {
   const uint64_t clen = P;
   const int flags = kChopFlags;
   int ms = 1;
-  host_totals<T>(h_lens, nullptr, n, &clen, &flags, words, ranges, maxm, &ms);
+  unsigned long long tasks = 0;
+  host_totals<T>(h_lens, nullptr, n, &clen, &flags, words, ranges, maxm, &ms, nullptr, &tasks);
   if (P > maxm) maxm = P;
-  return round_layout<T>(n, 1, words, ranges, maxm, ms).total;
+  return round_layout<T>(n, 1, words, ranges, maxm, ms, 0, tasks).total;
 }
 
 template <typename T>
@@ -2223,9 +2484,10 @@ int prefix_chop_launch(const T *prefix, uint64_t P, const T *series, const uint6
   const uint64_t clen = P;
   const int flags = kChopFlags;
   int ms = 1;
-  host_totals<T>(h_lens, nullptr, n, &clen, &flags, words, ranges, maxm, &ms);
+  unsigned long long tasks = 0;
+  host_totals<T>(h_lens, nullptr, n, &clen, &flags, words, ranges, maxm, &ms, nullptr, &tasks);
   if (P > maxm) maxm = P;
-  const RoundLayout L = round_layout<T>(n, 1, words, ranges, maxm, ms);
+  const RoundLayout L = round_layout<T>(n, 1, words, ranges, maxm, ms, 0, tasks);
   if (ws_bytes < L.total) return fail(ODBA_ERR_WORKSPACE_TOO_SMALL, "prefix chop workspace too small");
   char *base = static_cast<char *>(ws);
   int *single = reinterpret_cast<int *>(base + L.off_single);

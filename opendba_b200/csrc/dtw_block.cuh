@@ -330,7 +330,7 @@ __device__ __forceinline__ bool sweep_block(const BlockJob<T> &job, BlockSmem<T>
           for (int j = 0; j < kBlkR; ++j) col[j] = job.row_in[c_lane - job.c0 + j];
         }
       }
-      unsigned word = 0u;
+      unsigned word[4] = {0u, 0u, 0u, 0u};
       const bool top = SLOW && oe_top && k == last_pair;
       T c2 = cap;
       a_last = step_row_pair<T, kBlkR, PATH, SLOW, SLOW && CAP>(
@@ -342,7 +342,7 @@ __device__ __forceinline__ bool sweep_block(const BlockJob<T> &job, BlockSmem<T>
       v.y = col[kBlkR - 1];
       os[(t0 + s - 31) & (kBlkRing - 1)] = v;
       // (a band's idle lanes would hit its neighbours' slots)
-      if (PATH && (!BAND || (k >= 0 && k <= last_pair))) wp[(size_t)(t0 + s) * 32] = word;
+      if (PATH && (!BAND || (k >= 0 && k <= last_pair))) wp[(size_t)(t0 + s) * 32] = word[0];
       if (BAND && k == last_pair && job.row_out) {
 #pragma unroll
         for (int j = 0; j < kBlkR; ++j) job.row_out[c_lane - job.c0 + j] = col[j];

@@ -770,6 +770,32 @@ __global__ void __launch_bounds__(kBlkThreads) block_selftest_kernel(SelfTest *t
   sweep_block<float, false, false, false, true>(selftest_job(t), sm, NoGate(t->err + 1, limit_ns),
                                                 CkptOut<float>{nullptr, 0, 1}, true, corner, st);
 }
+
+// The same swath by one warp (the one-warp pipeline of the rounds).
+__global__ void __launch_bounds__(32) warp_selftest_kernel(SelfTest *t, unsigned long long limit_ns) {
+  __shared__ WarpSmem<float> sm;
+  const BlockJob<float> b = selftest_job(t);
+  SwathJob<float> job;
+  job.x = b.x;
+  job.y = b.y;
+  job.m = b.m;
+  job.n = b.n;
+  job.c0 = b.c0;
+  job.r0 = b.r0;
+  job.edge_in = b.edge_in;
+  job.edge_out = nullptr;
+  job.open_end = false;
+  job.free_diag0 = true;
+  job.corner_init = b.corner_init;
+  PipeGate gate;
+  gate.prog_in = t->prog;
+  gate.prog_out = t->prog + 1;
+  gate.err = t->err + 2;
+  gate.limit_ns = limit_ns;
+  gate.avail = 0;
+  float corner = 0.f;
+  sweep_warp<float, 16, false, PipeGate>(job, sm, true, corner, gate);
+}
 }  // namespace
 
 int gate_selftest(unsigned long long limit_ns, cudaStream_t stream) {
@@ -783,14 +809,16 @@ int gate_selftest(unsigned long long limit_ns, cudaStream_t stream) {
   cudaMemsetAsync(t, 0, sizeof *t, stream);
   gate_selftest_kernel<<<1, kBlkThreads, 0, stream>>>(t, limit_ns);
   block_selftest_kernel<<<1, kBlkThreads - 32, 0, stream>>>(t, limit_ns);
+  warp_selftest_kernel<<<1, 32, 0, stream>>>(t, limit_ns);
   int rc = check_launch("wait self-test kernel");
   cudaMemcpyAsync(err, t->err, sizeof err, cudaMemcpyDeviceToHost, stream);
   cudaFreeAsync(t, stream);
   if (cudaStreamSynchronize(stream) != cudaSuccess) return fail(ODBA_ERR_CUDA, "wait self-test");
   if (rc) return rc;
-  if (err[0] && err[1]) return fail(ODBA_ERR_TIMEOUT, "the waits ran out and raised the error words");
-  return fail(ODBA_ERR_CUDA, err[0] ? "a wait inside a block returned without a timeout"
-                                    : "the wait returned without the word or a timeout");
+  if (err[0] && err[1] && err[2]) return fail(ODBA_ERR_TIMEOUT, "the waits ran out and raised the error words");
+  return fail(ODBA_ERR_CUDA, !err[0]   ? "the wait returned without the word or a timeout"
+                             : !err[1] ? "a wait inside a block returned without a timeout"
+                                       : "the one-warp wait returned without a timeout");
 }
 
 int tune_set(int elem_size, int len_bucket, int count_bucket, int plan) {

@@ -1,12 +1,15 @@
-// Bounded hand-off of swath-edge rows between blocks (the swath pipeline).
+// Bounded hand-off of swath-edge rows between blocks or warps (the swath
+// pipelines).
 //
-// The producing block's feeding warp publishes "rows stored so far" with a
-// gpu-scope release; the consuming block's feeder acquires the word before it
-// reads rows it has not seen published (PipeGate::ready, polled between its
-// other duties: dtw_block.cuh).  Every wait is bounded: a feeder none of whose
-// duties could go on for the gate's limit (%globaltimer) raises the launch's
-// error word and goes on, a compute warp does so after four times the limit,
-// and every other waiter that sees the word stops waiting too.
+// The producer (a block's feeding warp, dtw_block.cuh, or a warp with a swath of
+// its own, dtw_warp.cuh) publishes "rows stored so far" with a gpu-scope
+// release; the consumer acquires the word before it reads rows it has not seen
+// published: a feeder polls it between its other duties (ready), a warp with a
+// swath of its own waits (wait).  Every wait is bounded: such a warp, or a
+// feeder none of whose duties could go on, raises the launch's error word after
+// the gate's limit (%globaltimer) and goes on, a block's compute warp does so
+// after four times the limit, and every other waiter that sees the word stops
+// waiting too.
 #pragma once
 
 #include <cstdint>
@@ -52,6 +55,21 @@ struct PipeGate {
       return true;
     }
     return false;
+  }
+  // bounded wait until rows [0, k) may be read (one thread)
+  __device__ __forceinline__ void wait(int k) {
+    unsigned long long t0 = 0;
+    for (unsigned it = 0; !ready(k); ++it) {
+      const unsigned long long now = global_timer_ns();
+      if (it == 0) {
+        t0 = now;
+      } else if (now - t0 > limit_ns) {
+        fail();
+        avail = 0x7fffffff;
+        return;
+      }
+      __nanosleep(128);
+    }
   }
   __device__ __forceinline__ void fail() { atomicExch(err, 1u); }
   __device__ __forceinline__ unsigned *error() { return err; }

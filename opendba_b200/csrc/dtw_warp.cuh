@@ -1,5 +1,5 @@
-// One warp sweeps one swath of a cost matrix (distances only): the form that
-// fills the GPU with many matrices at the least cost per cell.
+// One warp sweeps one swath of a cost matrix: the form that fills the GPU with
+// many matrices at the least cost per cell.
 //
 // Rows come in chunks of 32 pairs.  The warp stages a chunk's samples and
 // left-edge values in shared memory while it sweeps the chunk before, collects
@@ -16,6 +16,12 @@
 // float series of 2000-8000 samples (all pairs): 4.5 cycles per cell, padding
 // and fill included, 141 ms (a form that shuffled and packed the samples and
 // stored the edge from one lane by branch: 147).
+//
+// PATH records moves (dtw_path.cuh), for rounds large enough to fill the GPU
+// with one warp per swath: per step and lane 2 * WarpMoves<T>::kWords words, row
+// a's then row b's (float: D and U plane of 32 bits; double: one word, D in its
+// low half): word of (step t, lane l, row) of a swath at
+// ((t * 32 + l) * 2 + row) * kWords.
 #pragma once
 
 #include <type_traits>
@@ -35,6 +41,31 @@ struct WarpSmem {
   alignas(16) T sink[2 * kWarpChunk];  // where the lanes without a right edge store
 };
 
+// Words of a row's moves per step and lane.
+template <typename T>
+struct WarpMoves;
+template <>
+struct WarpMoves<float> {
+  static constexpr int kBits = 32, kWords = 2;
+  using V = uint4;
+  static __device__ __forceinline__ V pack(const unsigned (&w)[4]) {
+    return make_uint4(w[0], w[1], w[2], w[3]);
+  }
+};
+template <>
+struct WarpMoves<double> {
+  static constexpr int kBits = 16, kWords = 1;
+  using V = uint2;
+  static __device__ __forceinline__ V pack(const unsigned (&w)[4]) { return make_uint2(w[0], w[1]); }
+};
+
+// The gate of a warp that sweeps a matrix's swaths in turn: nothing to wait for.
+struct SoloGate {
+  static constexpr bool kActive = false;
+  __device__ __forceinline__ void wait(int) {}
+  __device__ __forceinline__ void publish(int) {}
+};
+
 // One swath for one warp.
 template <typename T>
 struct SwathJob {
@@ -49,21 +80,23 @@ struct SwathJob {
   bool free_diag0;    // column c0 is a reference swath-left column (c0 % 1024 == 0, c0 > 0)
   bool track = false; // keep the right edge's EdgeStat (needs edge_out)
   T corner_init;      // diagonal input of lane 0 at its first row
+  unsigned *words = nullptr;  // move words of this swath (PATH)
 };
 
 // Sweeps one swath.  last: the swath holds column n - 1; corner then receives
-// cell (m - 1, n - 1) in every lane.  Returns the right edge's EdgeStat in
-// every lane (the big value unless job.track).
-template <typename T, int R>
+// cell (m - 1, n - 1) in every lane (not with PATH).  Returns the right edge's
+// EdgeStat in every lane (the big value unless job.track).  Gate: the left edge
+// is another warp's, which publishes its rows, and the right edge is published.
+template <typename T, int R, bool PATH = false, typename Gate = SoloGate>
 __device__ __forceinline__ EdgeStat<T> sweep_warp(const SwathJob<T> &job, WarpSmem<T> &sm, bool last,
-                                                  T &corner) {
+                                                  T &corner, Gate gate = Gate()) {
   using V2 = typename Pair2<T>::V;
   const int lane = threadIdx.x & 31;
   const int r0 = job.r0, rows = job.m - r0;
   const T init = r0 ? T(0) : Num<T>::big();
   EdgeStat<T> st{Num<T>::big(), Num<T>::big()};
   if (rows <= 0) {  // open start over a single row: all zeros
-    if (last) corner = init;
+    if (last && !PATH) corner = init;
     return st;
   }
   const int pairs = (rows + 1) / 2, steps = pairs + 31;
@@ -81,11 +114,22 @@ __device__ __forceinline__ EdgeStat<T> sweep_warp(const SwathJob<T> &job, WarpSm
   const bool last_is_b = ((rows - 1) & 1) != 0;
   const bool oe_top = job.open_end && job.m >= 2;  // a single-row matrix has no open-end rule
   // the lane and register of column n - 1
-  const int cap_lane = last ? (job.n - 1 - job.c0) / R : 0;
-  const int capj = last && lane == cap_lane ? job.n - 1 - job.c0 - cap_lane * R : -1;
+  const bool cap_last = last && !PATH;
+  const int cap_lane = cap_last ? (job.n - 1 - job.c0) / R : 0;
+  const int capj = cap_last && lane == cap_lane ? job.n - 1 - job.c0 - cap_lane * R : -1;
   // steps [slow0, slow1) run the slow form
-  const int slow0 = oe_top ? last_pair : last ? last_pair + cap_lane : steps;
-  const int slow1 = oe_top ? last_pair + 32 : last ? slow0 + 1 : steps;
+  const int slow0 = oe_top ? last_pair : cap_last ? last_pair + cap_lane : steps;
+  const int slow1 = oe_top ? last_pair + 32 : cap_last ? slow0 + 1 : steps;
+  using Moves = typename WarpMoves<T>::V;
+  Moves *wp = PATH ? reinterpret_cast<Moves *>(job.words) + lane : nullptr;
+
+  // the left edge's rows of pairs [0, k)
+  auto await = [&](int k) {
+    if (Gate::kActive && has_in) {
+      if (lane == 0) gate.wait(2 * k < rows ? 2 * k : rows);
+      __syncwarp();
+    }
+  };
 
   // this lane's row pair of the next chunk
   T nx0 = T(0), nx1 = T(0), ne0 = T(0), ne1 = T(0);
@@ -112,6 +156,7 @@ __device__ __forceinline__ EdgeStat<T> sweep_warp(const SwathJob<T> &job, WarpSm
     }
   };
   if (!has_in) sm.ein[2 * lane] = sm.ein[2 * lane + 1] = Num<T>::big();
+  await(kWarpChunk);
   load(lane);
   put(lane);
   __syncwarp();
@@ -120,6 +165,7 @@ __device__ __forceinline__ EdgeStat<T> sweep_warp(const SwathJob<T> &job, WarpSm
   const V2 *es = reinterpret_cast<const V2 *>(sm.ein);
   for (int t0 = 0; t0 < steps; t0 += kWarpChunk) {
     const int lim = steps - t0 < kWarpChunk ? steps - t0 : kWarpChunk;
+    await(t0 + 2 * kWarpChunk);
     load(t0 + kWarpChunk + lane);
     const XPair<T> *xs = sm.x + ((t0 - lane) & (2 * kWarpChunk - 1));
     auto step = [&](auto slow_c, int s) {
@@ -132,14 +178,15 @@ __device__ __forceinline__ EdgeStat<T> sweep_warp(const SwathJob<T> &job, WarpSm
       lb = lane0 ? ev.y : lb;
       const T diag = dg;
       dg = lb;
-      unsigned word = 0u;
+      unsigned word[4] = {0u, 0u, 0u, 0u};
       const int k = t0 + s - lane;
       const bool top = SLOW && oe_top && k == last_pair;
       T c2 = cap;
-      a_last = step_row_pair<T, R, false, SLOW, SLOW>(col, yv, xv, la, lb, diag, top && !last_is_b,
-                                                      top && last_is_b, fd0, word, capj, last_is_b,
-                                                      c2);
-      if (SLOW) cap = k == last_pair ? c2 : cap;
+      a_last = step_row_pair<T, R, PATH, SLOW, SLOW && !PATH, PATH ? WarpMoves<T>::kBits : 8>(
+          col, yv, xv, la, lb, diag, top && !last_is_b, top && last_is_b, fd0, word, capj, last_is_b,
+          c2);
+      if (SLOW && !PATH) cap = k == last_pair ? c2 : cap;
+      if (PATH) wp[(size_t)(t0 + s) * 32] = WarpMoves<T>::pack(word);
       V2 v;
       v.x = a_last;
       v.y = col[R - 1];
@@ -180,6 +227,10 @@ __device__ __forceinline__ EdgeStat<T> sweep_warp(const SwathJob<T> &job, WarpSm
     }
     put(t0 + kWarpChunk + lane);
     __syncwarp();
+    if (Gate::kActive && has_out && lane == 0) {
+      const int stored = 2 * (t0 - 31 + lim);
+      if (stored > 0) gate.publish(stored < rows ? stored : rows);
+    }
   }
   if (job.track) {
 #pragma unroll
@@ -191,7 +242,7 @@ __device__ __forceinline__ EdgeStat<T> sweep_warp(const SwathJob<T> &job, WarpSm
     st.emin = __shfl_sync(kFull, st.emin, 0);
     st.etop = __shfl_sync(kFull, st.etop, (last_pair + 31) & 31);
   }
-  if (last) corner = __shfl_sync(kFull, cap, cap_lane);
+  if (cap_last) corner = __shfl_sync(kFull, cap, cap_lane);
   return st;
 }
 

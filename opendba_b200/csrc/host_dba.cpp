@@ -1728,31 +1728,46 @@ int run_jobs(const T *h_series, const uint64_t *h_lens, const int *job_begin, co
       }
       flags_now();
       cudaGraphExec_t exec[2] = {nullptr, nullptr};
-      for (int g = 0; g < 2; ++g) {
-        cudaGraph_t graph;
-        check_cuda(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "graph capture");
-        const T *cin = ptr<T>(cbuf[g]);
-        T *cout = ptr<T>(cbuf[1 - g]);
-        const int rc = sizeof(T) == 4
-            ? odba_dba_batch_round_f32((const float *)cin, ptr<uint64_t>(d_coff), ptr<int>(d_clen), ptr<int>(d_flags),
-                                       ptr<int>(d_mbeg), ptr<int>(d_mend), njobs, max_clen,
-                                       (const float *)js.ds.data.p, ptr<uint64_t>(js.ds.offs), ptr<uint64_t>(js.ds.lens),
-                                       ptr<int>(d_mseries), ptr<int>(d_mjob), ptr<int>(d_order), n, h_mlens.data(),
-                                       mjob.data(), h_clen.data(), size_flags.data(), (float *)cout,
-                                       ptr<uint32_t>(d_counts), ptr<double>(d_deltas), nullptr, nullptr, rws.p,
-                                       rws.bytes, st)
-            : odba_dba_batch_round_f64((const double *)cin, ptr<uint64_t>(d_coff), ptr<int>(d_clen), ptr<int>(d_flags),
-                                       ptr<int>(d_mbeg), ptr<int>(d_mend), njobs, max_clen,
-                                       (const double *)js.ds.data.p, ptr<uint64_t>(js.ds.offs), ptr<uint64_t>(js.ds.lens),
-                                       ptr<int>(d_mseries), ptr<int>(d_mjob), ptr<int>(d_order), n, h_mlens.data(),
-                                       mjob.data(), h_clen.data(), size_flags.data(), (double *)cout,
-                                       ptr<uint32_t>(d_counts), ptr<double>(d_deltas), nullptr, nullptr, rws.p,
-                                       rws.bytes, st);
-        check_cuda(cudaStreamEndCapture(st, &graph), "graph capture");
-        check(rc, "batched DBA round (capture)");
-        check_cuda(cudaGraphInstantiate(&exec[g], graph, 0), "graph instantiate");
-        cudaGraphDestroy(graph);
-      }
+      auto drop = [&] {
+        for (int g = 0; g < 2; ++g)
+          if (exec[g]) cudaGraphExecDestroy(exec[g]);
+      };
+      auto by_warp = [&](const std::vector<int> &fl) {
+        return odba::dba_batch_by_warp<T>(h_mlens.data(), mjob.data(), n, h_clen.data(), fl.data(), njobs);
+      };
+      int captured = 0;  // active jobs when the graphs' path kernel was chosen
+      bool warps = false;
+      auto capture = [&] {
+        drop();
+        captured = live;
+        warps = by_warp(size_flags);
+        for (int g = 0; g < 2; ++g) {
+          cudaGraph_t graph;
+          check_cuda(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "graph capture");
+          const T *cin = ptr<T>(cbuf[g]);
+          T *cout = ptr<T>(cbuf[1 - g]);
+          const int rc = sizeof(T) == 4
+              ? odba_dba_batch_round_f32((const float *)cin, ptr<uint64_t>(d_coff), ptr<int>(d_clen), ptr<int>(d_flags),
+                                         ptr<int>(d_mbeg), ptr<int>(d_mend), njobs, max_clen,
+                                         (const float *)js.ds.data.p, ptr<uint64_t>(js.ds.offs), ptr<uint64_t>(js.ds.lens),
+                                         ptr<int>(d_mseries), ptr<int>(d_mjob), ptr<int>(d_order), n, h_mlens.data(),
+                                         mjob.data(), h_clen.data(), size_flags.data(), (float *)cout,
+                                         ptr<uint32_t>(d_counts), ptr<double>(d_deltas), nullptr, nullptr, rws.p,
+                                         rws.bytes, st)
+              : odba_dba_batch_round_f64((const double *)cin, ptr<uint64_t>(d_coff), ptr<int>(d_clen), ptr<int>(d_flags),
+                                         ptr<int>(d_mbeg), ptr<int>(d_mend), njobs, max_clen,
+                                         (const double *)js.ds.data.p, ptr<uint64_t>(js.ds.offs), ptr<uint64_t>(js.ds.lens),
+                                         ptr<int>(d_mseries), ptr<int>(d_mjob), ptr<int>(d_order), n, h_mlens.data(),
+                                         mjob.data(), h_clen.data(), size_flags.data(), (double *)cout,
+                                         ptr<uint32_t>(d_counts), ptr<double>(d_deltas), nullptr, nullptr, rws.p,
+                                         rws.bytes, st);
+          check_cuda(cudaStreamEndCapture(st, &graph), "graph capture");
+          check(rc, "batched DBA round (capture)");
+          check_cuda(cudaGraphInstantiate(&exec[g], graph, 0), "graph instantiate");
+          cudaGraphDestroy(graph);
+        }
+      };
+      capture();
       int cur = 0;
       for (int round = 0; round < max_rounds && live; ++round) {
         check_cuda(cudaMemcpyAsync(d_flags.p, h_flags.data(), njobs * sizeof(int), cudaMemcpyHostToDevice, st), "flags");
@@ -1764,7 +1779,7 @@ int run_jobs(const T *h_series, const uint64_t *h_lens, const int *job_begin, co
                                    cudaMemcpyDeviceToHost, st), "wait error word");
         check_cuda(cudaStreamSynchronize(st), "batched round");
         if (wait_err) {
-          for (int g = 0; g < 2; ++g) cudaGraphExecDestroy(exec[g]);
+          drop();
           return ODBA_ERR_TIMEOUT;
         }
         for (int j = 0; j < njobs; ++j) {
@@ -1782,8 +1797,16 @@ int run_jobs(const T *h_series, const uint64_t *h_lens, const int *job_begin, co
         flags_now();
         // the next round reads the means just written (the other buffer)
         cur = 1 - cur;
+        // with half of its jobs done a round may suit a block per swath
+        if (warps && live && 2 * live <= captured) {
+          captured = live;
+          if (!by_warp(h_flags) && ws_for(h_flags) <= rws.bytes) {
+            for (int j = 0; j < njobs; ++j) size_flags[j] = h_flags[j];
+            capture();
+          }
+        }
       }
-      for (int g = 0; g < 2; ++g) cudaGraphExecDestroy(exec[g]);
+      drop();
     }
   } else if (live) {
     // plain: job by job, one round per call, synchronizing every round (performDBA's loop)

@@ -121,6 +121,10 @@ int prefix_chop_launch(const T *prefix, uint64_t P, const T *series, const uint6
 template <typename T>
 size_t dba_batch_workspace_bytes(const uint64_t *h_mlens, const int *h_mjob, int nmem,
                                  const uint64_t *h_clen, const int *h_flags, int njobs);
+// Whether such a round's path DTW goes by one warp per swath (large rounds).
+template <typename T>
+bool dba_batch_by_warp(const uint64_t *h_mlens, const int *h_mjob, int nmem, const uint64_t *h_clen,
+                       const int *h_flags, int njobs);
 template <typename T>
 int dba_batch_launch(const T *centroids, const unsigned long long *coff, const int *clen,
                      const int *jflags, const int *mbeg, const int *mend, int njobs, int max_clen,
