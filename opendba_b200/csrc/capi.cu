@@ -21,7 +21,6 @@ int fail(int status, const char *msg) {
 }
 
 namespace {
-constexpr uint64_t kScratchKeepBytes = uint64_t(256) << 20;
 constexpr int kScratchDevices = 64;
 
 // The current device's scratch pool, or null (no stream-ordered pools).
@@ -52,19 +51,26 @@ cudaMemPool_t scratch_pool() {
 
 cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t stream) {
   const cudaMemPool_t pool = scratch_pool();
-  if (!pool) return cudaMallocAsync(p, bytes, stream);
-  cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, stream);
-  if (e == cudaErrorMemoryAllocation) {
+  auto once = [&] {
+    if (bytes > kScratchKeepBytes) return cudaMalloc(p, bytes);
+    return pool ? cudaMallocFromPoolAsync(p, bytes, pool, stream) : cudaMallocAsync(p, bytes, stream);
+  };
+  cudaError_t e = once();
+  if (e == cudaErrorMemoryAllocation && pool) {
     cudaGetLastError();
     cudaStreamSynchronize(stream);
     cudaMemPoolTrimTo(pool, 0);
-    e = cudaMallocFromPoolAsync(p, bytes, pool, stream);
+    e = once();
   }
   return e;
 }
 
 void scratch_free(void *p, size_t bytes, cudaStream_t stream) {
   if (!p) return;
+  if (bytes > kScratchKeepBytes) {
+    cudaFree(p);
+    return;
+  }
   cudaFreeAsync(p, stream);
   if (bytes >= kScratchSyncBytes) cudaStreamSynchronize(stream);
 }

@@ -18,13 +18,17 @@ int fail(int status, const char *msg);
 int check_launch(const char *what);
 // Returns ODBA_OK if the current device is a compute capability 10.x part.
 int require_sm100();
-// Stream-ordered scratch of the host-buffer entry points, from a pool of the
-// library's own per device that keeps up to 256 MB mapped between calls (the
-// default pool unmaps what is freed at every synchronisation: mapping the
-// scratch again cost 0.4-0.7 ms a call).  Memory beyond that goes back when a
-// block of kScratchSyncBytes or more is freed (which waits for the stream: the
-// pool looks at its size when it is synchronised with), all of it when an
-// allocation fails or when the program asks (scratch_trim).
+// Scratch of the host-buffer entry points, in the order of one stream.  Blocks of
+// up to kScratchKeepBytes come from a pool of the library's own per device that
+// keeps up to as much mapped between calls (the default pool unmaps what is
+// freed at every synchronisation: mapping the scratch again cost 0.4-0.7 ms a
+// call).  What it holds beyond that goes back when a block of kScratchSyncBytes
+// or more is freed (which waits for the stream: the pool looks at its size when
+// it is synchronised with), all of it when an allocation fails or when the
+// program asks (scratch_trim).  Larger blocks are plain allocations: mapping and
+// unmapping them through the pool takes 10 ms per GB (100 GB: 0.7-1.1 s and
+// 0.7-1.5 s, cudaMalloc 0.01 and cudaFree 0.05 s).
+constexpr size_t kScratchKeepBytes = size_t(256) << 20;
 constexpr size_t kScratchSyncBytes = size_t(16) << 20;
 cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t stream);
 void scratch_free(void *p, size_t bytes, cudaStream_t stream);

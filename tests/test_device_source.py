@@ -44,3 +44,12 @@ def test_every_sweep_has_an_error_word():
     for name in ("dba_round.cu", "dtw_pairwise.cu"):
         assert "NoGate()" not in _source(name), name
     assert "return nullptr" not in _source("dtw_device.cuh")
+
+
+def test_large_scratch_is_not_mapped_through_the_pool():
+    # mapping and unmapping 100 GB through a pool takes two seconds, a plain
+    # allocation a sixtieth of one
+    text = _source("capi.cu")
+    alloc = text[text.index("cudaError_t scratch_alloc("):text.index("int scratch_trim()")]
+    assert "bytes > kScratchKeepBytes) return cudaMalloc(" in alloc
+    assert "cudaFree(p)" in alloc
