@@ -297,6 +297,8 @@ __device__ __forceinline__ bool sweep_block(const BlockJob<T> &job, BlockSmem<T>
   const bool oe_top = job.open_end && job.m >= 2 && job.top_band;
   const int cap_c = job.n - 1 - c_lane;         // 0 .. 7 in the lane that owns column n - 1
   const int capj = (CAP && cap_last) ? cap_c : -1;
+  // the step at which the lane that owns column n - 1 is on the last row
+  const int cap_step = (CAP && cap_last) ? last_pair + (((job.n - 1 - job.c0) / kBlkR) & 31) : -1;
   unsigned *wp = PATH ? job.words + (size_t)w * job.word_steps * 32 + lane : nullptr;
   const bool has_next = w + 1 < wact || job.edge_out != nullptr;  // somebody reads the edge ring
   const int *from = w ? &sm.done[w - 1] : &sm.staged;
@@ -332,11 +334,13 @@ __device__ __forceinline__ bool sweep_block(const BlockJob<T> &job, BlockSmem<T>
       }
       unsigned word[4] = {0u, 0u, 0u, 0u};
       const bool top = SLOW && oe_top && k == last_pair;
-      T c2 = cap;
       a_last = step_row_pair<T, kBlkR, PATH, SLOW, SLOW && CAP>(
-          col, yv, xv, la, lb, diag, top && !last_is_b, top && last_is_b, fd0, word, capj, last_is_b,
-          c2);
-      if (SLOW && CAP) cap = k == last_pair ? c2 : cap;
+          col, yv, xv, la, lb, diag, top && !last_is_b, top && last_is_b, fd0, word,
+          SLOW && CAP && k == last_pair && !last_is_b);
+      if (SLOW && CAP && t0 + s == cap_step) {  // (the last row in every lane's col)
+#pragma unroll
+        for (int j = 0; j < kBlkR; ++j) cap = capj == j ? col[j] : cap;
+      }
       V2 v;
       v.x = a_last;
       v.y = col[kBlkR - 1];

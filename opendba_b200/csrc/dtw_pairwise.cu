@@ -59,7 +59,7 @@ int whole_pairwise_launch(const T *series, const uint64_t *offsets, const uint64
   a.edge_stride = (max_len + 32 + 31) / 32 * 32;
   a.open_start = os;
   a.open_end = oe;
-  a.classes = size_classes(a.npairs, grid_size<T>() * kWarpsPerBlock);
+  a.classes = size_classes(a.npairs, grid_size<T>() * kWarpsPerBlock, max_len);
   cudaMemsetAsync(a.counter, 0, 16, stream);  // work counter and error word
   pairwise_kernel<T, RF, Tune<T>::RQ><<<grid_size<T>(), kWarpsPerBlock * 32, 0, stream>>>(a);
   return check_launch("pairwise DTW kernel");
@@ -542,42 +542,46 @@ bool plan_fits(int plan, unsigned long long npairs, uint64_t max_len, size_t ws_
 }
 
 // The pipeline pays while its blocks are few enough to run a pair's swaths side
-// by side: it takes a pair's steps a quarter to a half of the one-warp sweep's
+// by side: it takes a pair's steps a third to two thirds of the one-warp sweep's
 // time, but fills the GPU with a third as many pairs, and a second swath that is
-// nearly empty costs it a block all the same.  Measured on one B200 (one-warp
+// nearly empty costs it a block all the same.  Series of up to 160 samples are
+// swept by one warp in narrow lanes as fast.  Measured on one B200 (one-warp
 // time / pipeline time, all pairs of n series), float:
-//   2000-4000 samples  1431 / 1770 / 2016 / 2278 pairs  1.37 / 1.18 / 1.02 / 0.95
-//   1000-2000          1128 / 1431 / 1770               1.46 / 1.18 / 0.95
-//   1200-1500          780 / 1128 / 1770                1.42 / 1.01 / 0.68
-//   900-1100           861 / 1128                       1.17 / 0.92
-//   512-1024           861 / 1128 / 1431                1.23 / 1.08 / 0.90
-//   150-400            630 / 861                        1.22 / 0.92
-//   64-128             378 / 780                        1.14 / 0.71
-//   20-40              435 / 630                        1.02 / 0.72
+//   2000-4000 samples  1128 / 1431 / 1770 pairs         1.54 / 1.28 / 1.18
+//   1000-2000          1128 / 1431 / 1653 / 1770        1.40 / 1.14 / 1.03 / 0.97
+//   1200-1500          780 / 946 / 1128 / 1431          1.33 / 1.16 / 1.00 / 0.77
+//   900-1100           861 / 1035 / 1128                1.14 / 1.02 / 0.96
+//   512-1024           861 / 1128 / 1431                1.21 / 1.09 / 0.85
+//   150-400            435 / 630 / 780                  1.14 / 1.07 / 0.96
+//   180-250            190 / 378 / 561                  1.09 / 1.07 / 0.96
+//   129-160            66 / 378                         0.96 / 0.99
+//   64-128             190 / 378                        0.86 / 0.86
+//   20-40              190 / 435                        0.88 / 0.83
 // double:
-//   2000-4000          1770 / 2278                      1.34 / 1.13
-//   1000-2000          1770 / 2016                      1.15 / 1.04
-//   900-1100           861 / 1128 / 1431                1.39 / 1.13 / 0.89
-//   512-1024           1128 / 1431                      1.17 / 0.98
-//   150-400            630 / 861 / 1128                 1.15 / 1.08 / 0.81
-//   64-128             378 / 780                        1.14 / 0.70
-//   20-40              276 / 630                        0.93 / 0.57
+//   2000-4000          1431 / 1653 / 1770               1.53 / 1.39 / 1.13
+//   1000-2000          1431 / 1653 / 1770               1.22 / 1.09 / 1.04
+//   1200-1500          946 / 1128 / 1431                1.24 / 1.09 / 0.84
+//   900-1100           861 / 1035 / 1128                1.23 / 1.05 / 0.94
+//   512-1024           1035 / 1128 / 1431               1.23 / 1.05 / 0.94
+//   150-400            435 / 630 / 780                  1.33 / 1.06 / 0.98
+//   180-250            190 / 378 / 561                  1.13 / 1.14 / 0.72
+//   129-160            66 / 378                         0.83 / 0.99
+//   64-128             190 / 378                        0.78 / 0.78
 // Above one pair per resident warp (1776) the workspace that does not know the
 // number of pairs would not hold the pipeline's edges, so the rule ends there.
 template <typename T>
 int rule_of_thumb(unsigned long long npairs, uint64_t max_len) {
   const unsigned long long slots = (unsigned long long)grid_size<T>() * kWarpsPerBlock;
   const uint64_t swaths = (max_len + kBlkCols - 1) / kBlkCols;
-  const bool f32 = sizeof(T) == 4;
   unsigned long long most;
   if (swaths >= 3)
     most = slots;
   else if (swaths == 2)
-    most = max_len >= 1536 ? (f32 ? slots * 15 / 16 : slots) : (f32 ? slots * 5 / 8 : slots * 2 / 3);
+    most = max_len < 1536 ? slots * 5 / 8 : sizeof(T) == 4 ? slots * 15 / 16 : slots;
   else if (max_len >= 256)
-    most = max_len >= 512 ? (f32 ? slots * 2 / 3 : slots * 3 / 4) : (f32 ? slots * 3 / 7 : slots / 2);
+    most = max_len >= 512 ? slots * 2 / 3 : slots * 2 / 5;
   else
-    most = f32 || max_len >= 64 ? slots / 4 : 0;
+    most = max_len > 160 ? slots / 4 : 0;
   return npairs < most ? ODBA_PLAN_SWATH_PIPELINE : ODBA_PLAN_WHOLE_PAIR;
 }
 

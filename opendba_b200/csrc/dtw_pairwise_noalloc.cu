@@ -136,7 +136,7 @@ int pairwise_noalloc(const T *series, const uint64_t *offsets, const uint64_t *l
   a.edge_stride = stride;
   a.open_start = os ? 1 : 0;
   a.open_end = oe ? 1 : 0;
-  a.classes = size_classes(a.npairs, grid * kWarpsPerBlock);
+  a.classes = size_classes(a.npairs, grid * kWarpsPerBlock, max_len);
   // the counter is the only state that must start at zero
   cudaError_t e = cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), stream);
   if (e != cudaSuccess) return fail(ODBA_ERR_CUDA, "clearing the work counter failed");

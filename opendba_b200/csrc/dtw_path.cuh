@@ -73,51 +73,49 @@ __device__ __forceinline__ T row_pair_cell(T d, T up, T diag, T left, bool top, 
 // Two rows of a lane's R columns, row b one column behind row a: the two
 // chains interleave, and since row a at column j reads the old col[j - 1] as its
 // diagonal before row b writes the new one, no column changes registers (in
-// column order all of them would rotate).  CAP: cap receives the value of column
-// capj in row a (capb: in row b).
+// column order all of them would rotate).  PASS: with `pass` set row b is row a
+// again (row a is the matrix's last; its costs are then in col).
 template <typename T>
 struct RowPairState {
   T a_left, a_diag, b_left, b_diag, va_prev;
   unsigned w[4];
 };
-template <typename T, int R, bool PATH, bool TOP, bool CAP, int BITS, int J>
+template <typename T, int R, bool PATH, bool TOP, bool PASS, int BITS, int J>
 struct RowPairCols {
   static __device__ __forceinline__ void run(T (&col)[R], const YCols<T, R> &yv,
                                              RowDiffs<T, R> &df, RowPairState<T> &z, bool top_a,
-                                             bool top_b, bool fd0, int capj, bool capb, T &cap) {
+                                             bool top_b, bool fd0, bool pass) {
     if constexpr (J < R) {
       const T up = col[J];
       const T va = row_pair_cell<T, PATH, TOP, BITS, 0, J>(df.a(yv, J), up, z.a_diag, z.a_left,
                                                            top_a, J == 0 && fd0, z.w);
       z.a_diag = up;
       z.a_left = va;
-      if (CAP) cap = (capj == J && !capb) ? va : cap;
       if constexpr (J > 0) {
-        const T vb = row_pair_cell<T, PATH, TOP, BITS, 1, J - 1>(
+        T vb = row_pair_cell<T, PATH, TOP, BITS, 1, J - 1>(
             df.b(yv, J - 1), z.va_prev, z.b_diag, z.b_left, top_b, J == 1 && fd0, z.w);
+        if (PASS) vb = pass ? z.va_prev : vb;
         z.b_diag = z.va_prev;
         z.b_left = vb;
         col[J - 1] = vb;
-        if (CAP) cap = (capj == J - 1 && capb) ? vb : cap;
       }
       z.va_prev = va;
-      RowPairCols<T, R, PATH, TOP, CAP, BITS, J + 1>::run(col, yv, df, z, top_a, top_b, fd0, capj,
-                                                          capb, cap);
+      RowPairCols<T, R, PATH, TOP, PASS, BITS, J + 1>::run(col, yv, df, z, top_a, top_b, fd0, pass);
     }
   }
 };
 // words: the step's moves (BITS / 8 of them; PATH).
-template <typename T, int R, bool PATH, bool TOP, bool CAP, int BITS = 8>
+template <typename T, int R, bool PATH, bool TOP, bool PASS, int BITS = 8>
 __device__ __forceinline__ T step_row_pair(T (&col)[R], const YCols<T, R> &yv, const XPair<T> &x,
                                            T la, T lb, T dg, bool top_a, bool top_b, bool fd0,
-                                           unsigned (&words)[4], int capj, bool capb, T &cap) {
+                                           unsigned (&words)[4], bool pass) {
   static_assert(!PATH || R <= BITS, "a bit per column");
   RowPairState<T> z{la, dg, lb, la, T(0), {0u, 0u, 0u, 0u}};
   RowDiffs<T, R> df(x);
-  RowPairCols<T, R, PATH, TOP, CAP, BITS, 0>::run(col, yv, df, z, top_a, top_b, fd0, capj, capb, cap);
+  RowPairCols<T, R, PATH, TOP, PASS, BITS, 0>::run(col, yv, df, z, top_a, top_b, fd0, pass);
   col[R - 1] = row_pair_cell<T, PATH, TOP, BITS, 1, R - 1>(
       df.b(yv, R - 1), z.va_prev, z.b_diag, z.b_left, top_b, R == 1 && fd0, z.w);
-  if (CAP) cap = (capj == R - 1 && capb) ? col[R - 1] : cap;
+  if (PASS) col[R - 1] = pass ? z.va_prev : col[R - 1];
   if (PATH) {
     if (BITS == 8) {
       words[0] = z.w[0] | z.w[1];

@@ -8,7 +8,7 @@
 // branches.  Lanes outside the matrix compute values nobody reads: above the
 // first row a lane is re-set when it reaches it (the first 31 steps), below the
 // last row nothing is stored; only the steps that need the open-end top row or
-// the last cell run a slower form.
+// the last cell run a slower form, and a last swath ends with the last cell.
 //
 // What bounds it: the issue port.  A float cell is half a packed subtraction, a
 // three-input minimum and a multiply-add, 3.9 cycles per warp cell and scheduler
@@ -99,13 +99,13 @@ __device__ __forceinline__ EdgeStat<T> sweep_warp(const SwathJob<T> &job, WarpSm
     if (last && !PATH) corner = init;
     return st;
   }
-  const int pairs = (rows + 1) / 2, steps = pairs + 31;
+  const int pairs = (rows + 1) / 2;
   YCols<T, R> yv;
   yv.load(job.y, job.c0 + lane * R, job.n);
   T col[R];
 #pragma unroll
   for (int j = 0; j < R; ++j) col[j] = init;
-  T a_last = init, dg = init, cap = T(0);
+  T a_last = init, dg = init;
   const bool lane0 = lane == 0, lane31 = lane == 31;
   const T dinit = lane0 ? job.corner_init : init;
   const bool fd0 = job.free_diag0 && lane0;
@@ -113,13 +113,14 @@ __device__ __forceinline__ EdgeStat<T> sweep_warp(const SwathJob<T> &job, WarpSm
   const int last_pair = (rows - 1) >> 1;
   const bool last_is_b = ((rows - 1) & 1) != 0;
   const bool oe_top = job.open_end && job.m >= 2;  // a single-row matrix has no open-end rule
-  // the lane and register of column n - 1
+  // the lane and register of column n - 1, and the step that computes the last
+  // cell: the last one of a last swath, which has no right edge
   const bool cap_last = last && !PATH;
   const int cap_lane = cap_last ? (job.n - 1 - job.c0) / R : 0;
-  const int capj = cap_last && lane == cap_lane ? job.n - 1 - job.c0 - cap_lane * R : -1;
-  // steps [slow0, slow1) run the slow form
-  const int slow0 = oe_top ? last_pair : cap_last ? last_pair + cap_lane : steps;
-  const int slow1 = oe_top ? last_pair + 32 : cap_last ? slow0 + 1 : steps;
+  const int capj = cap_last ? job.n - 1 - job.c0 - cap_lane * R : -1;
+  const int steps = cap_last ? last_pair + cap_lane + 1 : pairs + 31;
+  // the steps from slow0 on run the slow form
+  const int slow0 = oe_top ? last_pair : cap_last ? steps - 1 : steps;
   using Moves = typename WarpMoves<T>::V;
   Moves *wp = PATH ? reinterpret_cast<Moves *>(job.words) + lane : nullptr;
 
@@ -163,8 +164,15 @@ __device__ __forceinline__ EdgeStat<T> sweep_warp(const SwathJob<T> &job, WarpSm
 
   V2 *os = reinterpret_cast<V2 *>(lane31 ? sm.eout : sm.sink);
   const V2 *es = reinterpret_cast<const V2 *>(sm.ein);
-  for (int t0 = 0; t0 < steps; t0 += kWarpChunk) {
-    const int lim = steps - t0 < kWarpChunk ? steps - t0 : kWarpChunk;
+  // One copy of each form of the step: what runs next to other swath widths has
+  // to share the instruction cache with them.  Double has a loop of its own for
+  // the chunks without a slow step all the same (kApart): beside the slow form its
+  // two rows' chains were scheduled one after the other (one pair of 1000 x 1000
+  // 0.62 ms so, 0.37 apart; 100 series of 1000-4000 13.6 and 12.6); float 147 us
+  // and 142 ms either way.
+  constexpr bool kApart = sizeof(T) == 8;
+  auto chunk = [&](auto mixed_c, int t0, int lim) {
+    constexpr bool MIXED = decltype(mixed_c)::value;
     await(t0 + 2 * kWarpChunk);
     load(t0 + kWarpChunk + lane);
     const XPair<T> *xs = sm.x + ((t0 - lane) & (2 * kWarpChunk - 1));
@@ -181,19 +189,15 @@ __device__ __forceinline__ EdgeStat<T> sweep_warp(const SwathJob<T> &job, WarpSm
       unsigned word[4] = {0u, 0u, 0u, 0u};
       const int k = t0 + s - lane;
       const bool top = SLOW && oe_top && k == last_pair;
-      T c2 = cap;
       a_last = step_row_pair<T, R, PATH, SLOW, SLOW && !PATH, PATH ? WarpMoves<T>::kBits : 8>(
-          col, yv, xv, la, lb, diag, top && !last_is_b, top && last_is_b, fd0, word, capj, last_is_b,
-          c2);
-      if (SLOW && !PATH) cap = k == last_pair ? c2 : cap;
+          col, yv, xv, la, lb, diag, top && !last_is_b, top && last_is_b, fd0, word,
+          SLOW && k == last_pair && !last_is_b);
       if (PATH) wp[(size_t)(t0 + s) * 32] = WarpMoves<T>::pack(word);
       V2 v;
       v.x = a_last;
       v.y = col[R - 1];
       os[s] = v;
     };
-    // one copy of each form of the step: what runs next to other swath widths
-    // has to share the instruction cache with them
     for (int s = 0; s < lim;) {
       if (t0 == 0 && s == lane) {  // the lane's first row pair
         dg = dinit;
@@ -201,12 +205,13 @@ __device__ __forceinline__ EdgeStat<T> sweep_warp(const SwathJob<T> &job, WarpSm
         for (int j = 0; j < R; ++j) col[j] = init;
       }
       int s1 = t0 == 0 ? s + 1 : lim;
-      if (t0 + s < slow0 || t0 + s >= slow1) {
-        if (t0 + s < slow0 && s1 > slow0 - t0) s1 = slow0 - t0;
+      if (!MIXED || t0 + s < slow0) {
+        if (MIXED && s1 > slow0 - t0) s1 = slow0 - t0;
 #pragma unroll 1
         for (; s < s1; ++s) step(std::false_type{}, s);
       } else {
-        step(std::true_type{}, s++);
+        step(std::true_type{}, s);
+        ++s;
       }
     }
     __syncwarp();
@@ -231,7 +236,16 @@ __device__ __forceinline__ EdgeStat<T> sweep_warp(const SwathJob<T> &job, WarpSm
       const int stored = 2 * (t0 - 31 + lim);
       if (stored > 0) gate.publish(stored < rows ? stored : rows);
     }
-  }
+  };
+  int t0 = 0;
+  if (kApart)
+    for (; t0 < steps; t0 += kWarpChunk) {
+      const int lim = steps - t0 < kWarpChunk ? steps - t0 : kWarpChunk;
+      if (t0 + lim > slow0) break;
+      chunk(std::false_type{}, t0, lim);
+    }
+  for (; t0 < steps; t0 += kWarpChunk)
+    chunk(std::true_type{}, t0, steps - t0 < kWarpChunk ? steps - t0 : kWarpChunk);
   if (job.track) {
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1)
@@ -242,7 +256,12 @@ __device__ __forceinline__ EdgeStat<T> sweep_warp(const SwathJob<T> &job, WarpSm
     st.emin = __shfl_sync(kFull, st.emin, 0);
     st.etop = __shfl_sync(kFull, st.etop, (last_pair + 31) & 31);
   }
-  if (cap_last) corner = __shfl_sync(kFull, cap, cap_lane);
+  if (cap_last) {
+    T cap = T(0);
+#pragma unroll
+    for (int j = 0; j < R; ++j) cap = capj == j ? col[j] : cap;
+    corner = __shfl_sync(kFull, cap, cap_lane);
+  }
   return st;
 }
 

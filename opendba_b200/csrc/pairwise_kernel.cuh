@@ -47,17 +47,21 @@ struct PairwiseArgs {
 // kSizeClasses times and take, each time, the pairs of one class of matrix
 // size (sixteenths of max_len^2, the largest class first), so that the pairs
 // left for the end are the small ones.  A skipped pair costs an atomic and two
-// loads.  100 double series of 1000-4000 samples (2.8 pairs per warp): 14.30 ms
-// in index order, 14.48 / 13.99 / 13.45 with 4 / 8 / 16 classes; 300 float
-// series of 2000-8000 (25 per warp): 142.0 and 141.3.  Below two pairs per warp
-// nearly all start at once and the skips cost more than the order gives (64
-// series, 1.1 per warp: 288 and 296 us); above kClassWaves the tail is less
-// than the skips.
+// loads, so it has to be a small part of the longest pair's time, which is what
+// the order can save: max_len^2 of at least kClassLen2 per pair of the launch.
+// One class / sixteen: float, 100 series (4950 pairs) of 100-300 samples 0.096 /
+// 0.130 ms, 500-1000 0.464 / 0.492, 1000-2000 1.710 / 1.714; 300 of 2000-8000
+// 142.0 / 141.3; double, 100 of 500-1000 1.496 / 1.492, 1000-2000 5.21 / 5.02,
+// 1000-4000 13.4 / 12.6.  Below two pairs per warp nearly all start at once;
+// above kClassWaves the tail is less than the skips.
 constexpr int kSizeClasses = 16;
-constexpr unsigned long long kClassWaves = 64;
+constexpr unsigned long long kClassWaves = 64, kClassLen2 = 400;
 
-inline int size_classes(unsigned long long npairs, int warps) {
-  return npairs >= 2ull * warps && npairs <= kClassWaves * warps ? kSizeClasses : 1;
+inline int size_classes(unsigned long long npairs, int warps, unsigned long long max_len) {
+  return npairs >= 2ull * warps && npairs <= kClassWaves * warps &&
+                 max_len * max_len >= kClassLen2 * npairs
+             ? kSizeClasses
+             : 1;
 }
 
 __device__ __forceinline__ long long row_start(long long s, long long n) {
@@ -108,12 +112,13 @@ __device__ __forceinline__ bool shortcut_fires(const EdgeStat<T> &st, int m, T &
 }
 
 // Full swaths use RF registers per lane (swath width 32*RF); the last, partial
-// swath uses the smallest multiple of RQ registers that covers it.  RQ = 8:
-// every width is code of its own, and the warps of an SM run different widths
-// next to each other.  With RQ = 4 (8 float widths) and five copies of the step
-// per width they spend half of their time waiting for instructions: pairs of
-// 8-48 series of 200-2000 samples took 4.46 ms, with two copies and RQ = 8
-// 1.57, RQ = 16 1.54; full-width work pays 0.4% for RQ = 8 and 2% for 16.
+// swath uses the smallest multiple of RQ registers that covers it, and a matrix of
+// up to 128 columns 4 (200 series of 20-60 samples: 0.16 ms with 8, 0.087 so).
+// RQ = 8: every width is code of its own, and the warps of an SM run different
+// widths next to each other.  With RQ = 4 (8 float widths) and five copies of the
+// step per width they spend half of their time waiting for instructions: pairs of
+// 8-48 series of 200-2000 samples took 4.46 ms, with two copies and RQ = 8 1.57,
+// RQ = 16 1.54; full-width work pays 0.4% for RQ = 8 and 2% for 16.
 template <typename T, int RF, int RQ>
 __device__ void sweep_pair(SwathJob<T> job, WarpSmem<T> &sm, T *e0, T *e1, T &corner) {
   constexpr int W = 32 * RF;
@@ -131,7 +136,9 @@ __device__ void sweep_pair(SwathJob<T> job, WarpSmem<T> &sm, T *e0, T *e1, T &co
     const int rneed = (width + 31) / 32;
     const int rq = (rneed + RQ - 1) / RQ * RQ;
     EdgeStat<T> st{Num<T>::big(), Num<T>::big()};
-    if (rq >= RF) {
+    if (job.n <= 128) {
+      st = sweep_warp<T, 4>(job, sm, last, corner);
+    } else if (rq >= RF) {
       st = sweep_warp<T, RF>(job, sm, last, corner);
     } else {
       switch (rq / RQ) {
