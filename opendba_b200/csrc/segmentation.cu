@@ -81,6 +81,7 @@ __device__ __forceinline__ unsigned char seg_byte(double v) {
 struct SegParams {
   int spb, k_max, minseg, dw, smem_optin;
   int fast;  // the shared memory holds the fast form's rows
+  int smem;  // bytes of dynamic shared memory
 };
 
 // DP extent from the reference's dynamic shared-memory layout.
@@ -205,6 +206,44 @@ __device__ __forceinline__ bool seg_plain_value(float v) {
 }
 __device__ __forceinline__ bool seg_plain_value(double v) {
   return v == v && (unsigned long long)__double_as_longlong(v) != 0x8000000000000000ull;
+}
+
+// The segment bounds of a block whose medians the exchange sort has to give
+// (segment_sort_kernel), left in the place of its medians: NaNs whose payload no
+// arithmetic gives, with the bound in the low 16 bits.
+template <typename T>
+struct SegPending;
+template <>
+struct SegPending<float> {
+  static constexpr unsigned kTag = 0x7fdb0000u;
+  static __device__ __forceinline__ float put(unsigned short b) { return __uint_as_float(kTag | b); }
+  static __device__ __forceinline__ bool is(float v) {
+    return (__float_as_uint(v) & 0xffff0000u) == kTag;
+  }
+  static __device__ __forceinline__ unsigned short get(float v) {
+    return (unsigned short)__float_as_uint(v);
+  }
+};
+template <>
+struct SegPending<double> {
+  static constexpr unsigned long long kTag = 0x7ffdba0000000000ull;
+  static __device__ __forceinline__ double put(unsigned short b) {
+    return __longlong_as_double((long long)(kTag | b));
+  }
+  static __device__ __forceinline__ bool is(double v) {
+    return ((unsigned long long)__double_as_longlong(v) & ~0xffffull) == kTag;
+  }
+  static __device__ __forceinline__ unsigned short get(double v) {
+    return (unsigned short)__double_as_longlong(v);
+  }
+};
+
+// The median of samples lb .. rb-1 of a block sorted within its segments
+// (segmentation.hpp:327-332).
+template <typename T>
+__device__ __forceinline__ T seg_median(const T *sorted, int lb, int rb) {
+  const int mid = (lb + rb) / 2;
+  return ((lb - rb) % 2) ? sorted[mid] : (sorted[mid] + sorted[mid + 1]) / 2;
 }
 
 template <typename T>
@@ -421,56 +460,99 @@ __global__ void __launch_bounds__(kSegThreads) segment_kernel(const T *series,
     if (seg > test_k) out[seg - 1] = SegLim<T>::hi();
   // the move table is dead: its space takes the sorted samples where they fit
   T *sorted = reinterpret_cast<T *>((reinterpret_cast<uintptr_t>(kpath) + 15) & ~uintptr_t(15));
-  const bool room = size_t(k_max + 1) * W * 2 >= size_t(spb + 2) * sizeof(T) + 16;
-  const T *res = od;
-  if (__syncthreads_and(plain) && room) {
-    // every sample to its rank within its segment (equal samples by index).
-    // One thread per segment with an exchange sort is serial in the longest
-    // segment, and the reference's down-averaging makes the upper third of
-    // each block one such segment (170 of 512 samples with minseg 4).
-    for (int i = t; i < spb + 2; i += blockDim.x) {
-      int lo = 0, hi = test_k;  // bp[lo] * dw <= i < bp[hi] * dw
-      const int last = bp[test_k] * dw < N ? bp[test_k] * dw : N;
-      const T v = od[i];
-      if (i >= last) {
-        sorted[i] = v;
-        continue;
-      }
-      while (hi - lo > 1) {
-        const int mid = (lo + hi) / 2;
-        if (bp[mid] * dw <= i) lo = mid; else hi = mid;
-      }
-      const int lb = bp[lo] * dw;
-      const int rb = bp[hi] * dw < N ? bp[hi] * dw : N;
-      int rank = 0;
-      for (int j = lb; j < rb; ++j) {
-        const T w = od[j];
-        rank += int(w < v) | int(w == v && j < i);
-      }
-      sorted[lb + rank] = v;
+  const bool room = smem_raw + sp.smem >= reinterpret_cast<unsigned char *>(sorted + spb + 2);
+  if (!__syncthreads_and(plain) || !room) {
+    for (int seg = t + 1; seg <= test_k; seg += blockDim.x) out[seg - 1] = SegPending<T>::put(bp[seg]);
+    return;
+  }
+  // every sample to its rank within its segment (equal samples by index).
+  // One thread per segment with an exchange sort is serial in the longest
+  // segment, and the reference's down-averaging makes the upper third of
+  // each block one such segment (170 of 512 samples with minseg 4).
+  for (int i = t; i < spb + 2; i += blockDim.x) {
+    int lo = 0, hi = test_k;  // bp[lo] * dw <= i < bp[hi] * dw
+    const int last = bp[test_k] * dw < N ? bp[test_k] * dw : N;
+    const T v = od[i];
+    if (i >= last) {
+      sorted[i] = v;
+      continue;
     }
-    res = sorted;
-  } else {
-    for (int seg = t + 1; seg <= test_k; seg += blockDim.x) {
-      int rb = bp[seg] * dw;
-      if (rb > N) rb = N;
-      const int lb = bp[seg - 1] * dw;
-      for (int i = lb; i < rb - 1; ++i)
-        for (int j = i + 1; j < rb; ++j)
-          if (od[i] > od[j]) {
-            const T tmp = od[i];
-            od[i] = od[j];
-            od[j] = tmp;
-          }
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) / 2;
+      if (bp[mid] * dw <= i) lo = mid; else hi = mid;
     }
+    const int lb = bp[lo] * dw;
+    const int rb = bp[hi] * dw < N ? bp[hi] * dw : N;
+    int rank = 0;  // (no NaN: equal samples before this one come first)
+    for (int j = lb; j < i; ++j) rank += int(od[j] <= v);
+    for (int j = i + 1; j < rb; ++j) rank += int(od[j] < v);
+    sorted[lb + rank] = v;
   }
   __syncthreads();
   for (int seg = t + 1; seg <= test_k; seg += blockDim.x) {
     int rb = bp[seg] * dw;
     if (rb > N) rb = N;
+    out[seg - 1] = seg_median(sorted, bp[seg - 1] * dw, rb);
+  }
+}
+
+// The medians of the blocks segment_kernel left bounds for: those with a NaN or
+// a negative zero, whose order is the exchange sort's own, and those too long
+// for the rank sort's copy.  One thread per segment, as the reference has it; a
+// kernel of its own, since the serial sort of a long segment beside the DP's
+// 1024 threads keeps a whole SM waiting (1 M samples with negative zeros, minimum
+// segment 9: 37 ms in one kernel, 22 in blocks of 256 threads).
+constexpr int kSegSortThreads = 256;
+template <typename T>
+__global__ void __launch_bounds__(kSegSortThreads) segment_sort_kernel(const T *series,
+                                                                       const uint64_t *offsets,
+                                                                       const uint64_t *lens,
+                                                                       const unsigned long long *seg_base,
+                                                                       SegParams sp, T *medians) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int t = threadIdx.x, s = blockIdx.x, by = blockIdx.y;
+  const long orig_N = long(lens[s]);
+  const int spb = sp.spb, dw = sp.dw, k_max = sp.k_max;
+  if ((long)by * spb >= orig_N) return;
+  T *out = medians + seg_base[s] + (unsigned long long)by * k_max;
+  if (!SegPending<T>::is(out[0])) return;
+  const T *x = series + offsets[s] + (long)by * spb;
+  const int N = (long)(by + 1) * spb > orig_N ? int(orig_N % spb) : spb;
+  T *od = reinterpret_cast<T *>(smem_raw);                                // spb samples + 2
+  unsigned short *bp = reinterpret_cast<unsigned short *>(od + spb + 2);  // k_max + 1
+  __shared__ int segs;
+  if (t == 0) {
+    segs = 0;
+    bp[0] = 0;
+  }
+  __syncthreads();
+  for (int i = t; i < spb + 2; i += blockDim.x)
+    od[i] = (i < spb && (long)by * spb + i < orig_N) ? x[i] : T(0);
+  for (int seg = t + 1; seg <= k_max; seg += blockDim.x)
+    if (SegPending<T>::is(out[seg - 1])) {
+      bp[seg] = SegPending<T>::get(out[seg - 1]);
+      atomicMax(&segs, seg);
+    }
+  __syncthreads();
+  const int test_k = segs;
+  for (int seg = t + 1; seg <= test_k; seg += blockDim.x) {
+    int rb = bp[seg] * dw;
+    if (rb > N) rb = N;
     const int lb = bp[seg - 1] * dw;
-    const int mid = (lb + rb) / 2;
-    out[seg - 1] = ((lb - rb) % 2) ? res[mid] : (res[mid] + res[mid + 1]) / 2;
+    for (int i = lb; i < rb - 1; ++i)
+      for (int j = i + 1; j < rb; ++j)
+        if (od[i] > od[j]) {
+          const T tmp = od[i];
+          od[i] = od[j];
+          od[j] = tmp;
+        }
+  }
+  __syncthreads();
+  for (int seg = t + 1; seg <= test_k; seg += blockDim.x) {
+    int rb = bp[seg] * dw;
+    if (rb > N) rb = N;
+    const int lb = bp[seg - 1] * dw < N ? bp[seg - 1] * dw : N;
+    out[seg - 1] = seg_median(od, lb, rb);
   }
 }
 
@@ -507,12 +589,17 @@ int segment_launch(const T *series, const uint64_t *offsets, const uint64_t *len
   // segment lengths the general form alone fits
   sp.fast = segment_smem_bytes<T>(sp.spb, sp.k_max, true) <= size_t(sp.smem_optin);
   const size_t smem = segment_smem_bytes<T>(sp.spb, sp.k_max, sp.fast != 0);
+  sp.smem = int(smem);
   if (smem > size_t(sp.smem_optin))
     return fail(ODBA_ERR_INVALID_ARGUMENT, "minimum segment length needs more shared memory than the device has");
   cudaFuncSetAttribute(segment_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
   if (n < 1 || max_blocks < 1) return ODBA_OK;
   dim3 grid(n, max_blocks);
   segment_kernel<T><<<grid, kSegThreads, smem, stream>>>(series, offsets, lens, seg_base, sp, medians);
+  const size_t sort_smem = size_t(sp.spb + 2) * sizeof(T) + size_t(sp.k_max + 2) * 2;
+  cudaFuncSetAttribute(segment_sort_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sort_smem));
+  segment_sort_kernel<T><<<grid, kSegSortThreads, sort_smem, stream>>>(series, offsets, lens, seg_base,
+                                                                       sp, medians);
   return check_launch("segmentation kernel");
 }
 
