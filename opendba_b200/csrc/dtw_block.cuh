@@ -74,6 +74,8 @@ struct BlockSmem {
   alignas(16) T sink[2 * kBlkRing];
   int done[kBlkWarps];                // steps done by each compute warp
   int staged, drained;                // row pairs staged / stored by the feeder
+  unsigned *err;                      // the launch's error word, and the limit of the
+  unsigned long long limit_ns;        // compute warps' waits (read only when one is long)
   unsigned long long task;
 };
 
@@ -93,21 +95,22 @@ __device__ __forceinline__ unsigned long long warp_timer_ns() {
 
 // Waits until the counter is at least v (every lane of the calling warp);
 // one that has to wait waits for `more` instead, so that a neighbour of nearly
-// the same pace is not waited for again at every chunk.  Bounded: past limit_ns
-// the launch's error word is raised; a word already up ends the wait.
-__device__ __forceinline__ void wait_count(const int *p, int v, int more, unsigned *err,
-                                           unsigned long long limit_ns) {
+// the same pace is not waited for again at every chunk.  Bounded: past the
+// block's limit the launch's error word is raised; a word already up ends the
+// wait.
+template <typename T>
+__device__ __forceinline__ void wait_count(const int *p, int v, int more, const BlockSmem<T> &sm) {
   if (smem_count(p) < v) {
     unsigned long long t0 = 0;
     for (unsigned it = 0; smem_count(p) < more; ++it) {
       __nanosleep(it < 4 ? 64u << it : 1000u);
       if ((it & 63u) == 63u) {
-        if (*reinterpret_cast<volatile unsigned *>(err)) break;
+        if (*reinterpret_cast<volatile unsigned *>(sm.err)) break;
         const unsigned long long now = global_timer_ns();
         if (t0 == 0) {
           t0 = now;
-        } else if (now - t0 > limit_ns) {
-          atomicExch(err, 1u);
+        } else if (now - t0 > sm.limit_ns) {
+          atomicExch(sm.err, 1u);
           break;
         }
       }
@@ -173,6 +176,10 @@ __device__ __forceinline__ bool sweep_block(const BlockJob<T> &job, BlockSmem<T>
   if (threadIdx.x < kBlkWarps) sm.done[threadIdx.x] = 0;
   if (threadIdx.x == kBlkWarps) sm.staged = 0;
   if (threadIdx.x == kBlkWarps + 1) sm.drained = 0;
+  if (threadIdx.x == kBlkWarps + 2) {
+    sm.err = gate.error();
+    sm.limit_ns = 4 * gate.limit();  // past every wait of a feeder
+  }
   __syncthreads();
 
   if (w == kBlkWarps) {
@@ -365,36 +372,40 @@ __device__ __forceinline__ bool sweep_block(const BlockJob<T> &job, BlockSmem<T>
   // the steps at which some lane is on row m - 1 are slow where that row has
   // rules of its own (open end) or its value is wanted
   const bool slow_end = oe_top || (CAP && cap_last);
-  const unsigned long long wait_limit = 4 * gate.limit();  // past every wait of a feeder
-#pragma unroll 1
-  for (int t0 = 0; t0 < steps; t0 += kBlkChunk) {
+  // a chunk with its waits before and its count after
+  auto turn = [&](auto fill_c, auto slow_c, int t0) {
     // this chunk's left-edge pairs, and room in the right-edge ring
     int need = t0 + kBlkChunk;
     need = need < pairs ? need : pairs;
     if (w) need = need + 31 < steps ? need + 31 : steps;
     const int most = w ? steps : pairs;
-    wait_count(from, need, need + kBlkSlack < most ? need + kBlkSlack : most, gate.error(),
-               wait_limit);
+    wait_count(from, need, need + kBlkSlack < most ? need + kBlkSlack : most, sm);
     if (has_next) {
       const int room = t0 + kBlkChunk - 31 - kBlkRing;
       if (room > 0) {
         // (the right neighbour can go on to step t0 - 39 whatever this warp does)
         const int v = room < pairs ? room : pairs, more = room + 4 * kBlkChunk;
-        wait_count(to, v, more < pairs ? more : pairs, gate.error(), wait_limit);
+        wait_count(to, v, more < pairs ? more : pairs, sm);
       }
     }
-    if (slow_end && t0 + kBlkChunk > last_pair)
-      chunk(std::true_type{}, std::true_type{}, t0);
-    else if (t0 < 32)
-      chunk(std::true_type{}, std::false_type{}, t0);
-    else
-      chunk(std::false_type{}, std::false_type{}, t0);
+    chunk(fill_c, slow_c, t0);
     __syncwarp();
     if (lane31) {
       __threadfence_block();
       *reinterpret_cast<volatile int *>(&sm.done[w]) = t0 + kBlkChunk;
     }
-  }
+  };
+  // Each form of the chunk in a loop of its own: beside one another in one loop
+  // they spoil each other's schedule (double, a round of 100 members of 1000-4000,
+  // open end: 1.41 ms in one loop, 1.32 so).
+  const int slow_from = !slow_end ? steps : last_pair >= kBlkChunk ? last_pair + 1 - kBlkChunk : 0;
+  int t0 = 0;
+#pragma unroll 1
+  for (; t0 < 32 && t0 < slow_from; t0 += kBlkChunk) turn(std::true_type{}, std::false_type{}, t0);
+#pragma unroll 1
+  for (; t0 < slow_from; t0 += kBlkChunk) turn(std::false_type{}, std::false_type{}, t0);
+#pragma unroll 1
+  for (; t0 < steps; t0 += kBlkChunk) turn(std::true_type{}, std::true_type{}, t0);
   corner = cap;
   return CAP && cap_last && capj >= 0 && capj < kBlkR;
 }
