@@ -564,8 +564,10 @@ __launch_bounds__(kBlkThreads, sizeof(T) == 4 ? kRoundBlocksF32 : kRoundBlocksF6
 // all members too large) a task is a member, swath after swath, with two edge
 // columns per warp.
 //
-// What bounds it is the issue port: 12 warps per SM (8 in double), 2000 float
-// members of 3000-8000 samples 11.1 cycles per cell and scheduler.
+// What bounds it is the issue port, with 12 warps per SM (8 in double): 2000 float
+// members of 3000-8000 samples take 12.0 cycles per warp cell and scheduler, fill
+// and padding included, against 11.1 in a loop of nothing but path cells (a block
+// per swath 15.5).
 constexpr int kRoundWarpBlocksF32 = 3, kRoundWarpBlocksF64 = 2;
 template <typename T, int R, typename Gate>
 __device__ __forceinline__ EdgeStat<T> path_warp_swath(const SwathJob<T> &job, WarpSmem<T> &sm,
@@ -1296,49 +1298,53 @@ int pipe_bands() {
   return forced > 0 ? (forced < kMaxBands ? forced : kMaxBands) : 1;
 }
 
-// Whether a round of `tasks` (member, 1024-column swath) pairs, the most swaths
-// of a member being max_swaths, fills the GPU with one warp per swath.  At full
-// load the one-warp sweep takes three quarters of the block sweep's issue slots
-// per cell; the block sweep ends a chain of swaths in a quarter of the steps, and
-// the longer the chains the more of them it takes to hide their ends.  One
-// B200, block time / one-warp time of a round (centroid of a middling member):
-//   float, 1 swath   100-400 samples    1000 / 1500 / 2000 / 2500 tasks  0.99 / 1.03 / 1.10 / 1.10
-//                    400-800            1000 / 2000 / 2500               0.93 / 0.94 / 1.07
-//          2         1000-2000          1200 / 1600 / 2000 / 2400        0.97 / 1.01 / 1.11 / 1.28
-//          3         2000-4000          1200 / 1800 / 2100 / 2700        0.81 / 0.99 / 1.03 / 1.04
-//          5-6       3000-8000          1800 / 2700 / 3000 / 3600        0.92 / 1.02 / 0.98 / 1.07
-//          12-13     8000-16000         2400 / 3000 / 3900               0.92 / 0.96 / 1.04
-//   double, 1        100-400            500 / 700 / 900                  0.99 / 1.11 / 1.24
-//                    400-800            300 / 500 / 700                  0.79 / 1.01 / 1.23
-//          2         1000-2000          400 / 600 / 800                  0.82 / 1.03 / 1.15
-//          3-4       2000-4000          600 / 1200                       0.86 / 1.13
-//          5-6       3000-8000          1200 / 1500 / 1800               0.96 / 1.02 / 1.03
-//          11-12     8000-16000         1200 / 1650                      0.96 / 0.99
-// Larger ones: 2000 float members of 3000-8000 25.2 ms (block) and 20.0, 1000
-// double ones 28.2 and 22.3.
+// Whether a round fills the GPU with one warp per swath.  units: its work, the
+// rows of all (member, 1024-column swath) pairs over the most rows of a member;
+// max_swaths: the most swaths of a member.  At full load the one-warp sweep
+// takes three quarters of the block sweep's issue slots per cell; the block sweep
+// ends a chain of swaths in a quarter of the steps, and the longer the chains the
+// more of them it takes to hide their ends.  One B200, block time / one-warp time
+// of a round (lengths even over the range, centroid of a middling member):
+//   float, 1 swath   100-400 samples    630 / 940 / 1250 / 1560 units    0.99 / 1.03 / 1.10 / 1.10
+//                    400-800            750 / 1500 / 1880                0.93 / 0.94 / 1.07
+//          2         1000-2000          900 / 1200 / 1500 / 1800         0.97 / 1.01 / 1.11 / 1.28
+//          3         2000-4000          900 / 1350 / 1580 / 2030         0.81 / 0.99 / 1.03 / 1.04
+//          5-6       3000-8000          1240 / 1860 / 2060 / 2480        0.92 / 1.02 / 0.98 / 1.07
+//          12-13     8000-16000         1800 / 2250 / 2930               0.92 / 0.96 / 1.04
+//   double, 1        100-400            310 / 440 / 560                  0.99 / 1.11 / 1.24
+//                    400-800            230 / 380 / 530                  0.79 / 1.01 / 1.23
+//          2         1000-2000          300 / 450 / 600                  0.82 / 1.03 / 1.15
+//          3-4       2000-4000          450 / 900                        0.86 / 1.13
+//          5-6       3000-8000          830 / 1040 / 1240                0.96 / 1.02 / 1.03
+//          11-12     8000-16000         900 / 1240                       0.96 / 0.99
+// Few long members among short ones leave the long chains alone at the end (float,
+// 300 members of 200-20000, log-even, 3600 pairs in 611 units: 7.6 ms by blocks,
+// 11.0 by warps), so the rule counts work, not pairs.  Larger rounds: 2000 float
+// members of 3000-8000 25.2 ms (block) and 20.0, 1000 double ones 28.2 and 21.7.
 template <typename T>
-bool fills_with_warps(unsigned long long tasks, int max_swaths) {
+bool fills_with_warps(unsigned long long units, int max_swaths) {
   const unsigned long long slots = (unsigned long long)round_warp_grid<T>() * kRoundWarps;
-  if (sizeof(T) == 4)
-    return max_swaths <= 4 ? tasks * 5 >= slots * 6 : max_swaths <= 8 ? tasks * 5 >= slots * 8 : tasks >= slots * 2;
-  return max_swaths <= 2   ? tasks * 2 >= slots
-         : max_swaths <= 4 ? tasks * 6 >= slots * 5
-         : max_swaths <= 8 ? tasks * 2 >= slots * 3
-                           : tasks * 4 >= slots * 7;
+  // percent of the resident warps
+  const unsigned pc = sizeof(T) == 4 ? (max_swaths <= 4 ? 85 : max_swaths <= 8 ? 150 : 160)
+                                     : (max_swaths <= 2   ? 38
+                                        : max_swaths <= 4 ? 63
+                                        : max_swaths <= 8 ? 90
+                                                          : 110);
+  return units * 100 >= slots * pc;
 }
 
-// Workspace layout for nmem members / njobs jobs with the given totals; tasks:
-// (member, 1024-column swath) pairs of active members.
+// Workspace layout for nmem members / njobs jobs with the given totals; units:
+// the active members' work (fills_with_warps).
 template <typename T>
 RoundLayout round_layout(int nmem, int njobs, unsigned long long words,
                          unsigned long long ranges, unsigned long long maxm, int max_swaths = 0,
-                         unsigned long long rows = 0, unsigned long long tasks = 0) {
+                         unsigned long long rows = 0, unsigned long long units = 0) {
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
   RoundLayout L;
   L.edge_stride = (maxm + 32 + 31) / 32 * 32;
   L.pipe = max_swaths > 0 && size_t(nmem) * 2 * L.edge_stride * sizeof(T) <= kPipeEdgeBytes;
   L.nbands = L.pipe ? pipe_bands() : 1;
-  L.one_warp = max_swaths > 0 && (!L.pipe || (L.nbands == 1 && fills_with_warps<T>(tasks, max_swaths)));
+  L.one_warp = max_swaths > 0 && (!L.pipe || (L.nbands == 1 && fills_with_warps<T>(units, max_swaths)));
   L.max_swaths = L.one_warp ? max_swaths * (kBlkCols / warp_cols<T>()) : max_swaths;
   const size_t edge_cols = L.pipe ? size_t(nmem)
                            : L.one_warp ? size_t(round_warp_grid<T>()) * kRoundWarps : 0;
@@ -1373,12 +1379,12 @@ template <typename T>
 void host_totals(const uint64_t *h_lens, const int *h_mjob, int nmem, const uint64_t *h_clen,
                  const int *h_flags, unsigned long long &words, unsigned long long &ranges,
                  unsigned long long &maxm, int *max_swaths = nullptr,
-                 unsigned long long *rows = nullptr, unsigned long long *tasks = nullptr) {
+                 unsigned long long *rows = nullptr, unsigned long long *units = nullptr) {
   words = ranges = 0;
   maxm = 1;
   if (max_swaths) *max_swaths = 1;
   if (rows) *rows = 0;
-  if (tasks) *tasks = 0;
+  unsigned long long work = 0;
   for (int k = 0; k < nmem; ++k) {
     const int j = h_mjob ? h_mjob[k] : 0;
     const int f = h_flags[j];
@@ -1389,8 +1395,9 @@ void host_totals(const uint64_t *h_lens, const int *h_mjob, int nmem, const uint
     if ((unsigned long long)g.m > maxm) maxm = g.m;
     if (max_swaths && g.swaths > *max_swaths) *max_swaths = g.swaths;
     if (rows) *rows += (unsigned long long)g.m;
-    if (tasks) *tasks += (unsigned long long)g.swaths;
+    work += (unsigned long long)g.m * g.swaths;
   }
+  if (units) *units = work / maxm;
 }
 
 // Planning, range clearing and the path DTW of a round (everything before
@@ -1478,10 +1485,10 @@ size_t dba_round_workspace_bytes(const uint64_t *h_lens, int n, uint64_t Lc, int
   const uint64_t clen = Lc;
   const int flags = (os ? 1 : 0) | (oe ? 2 : 0) | 4;
   int ms = 1;
-  unsigned long long rows = 0, tasks = 0;
-  host_totals<T>(h_lens, nullptr, n, &clen, &flags, words, ranges, maxm, &ms, &rows, &tasks);
+  unsigned long long rows = 0, units = 0;
+  host_totals<T>(h_lens, nullptr, n, &clen, &flags, words, ranges, maxm, &ms, &rows, &units);
   if (Lc > maxm) maxm = Lc;
-  return round_layout<T>(n, 1, words, ranges, maxm, ms, rows, tasks).total;
+  return round_layout<T>(n, 1, words, ranges, maxm, ms, rows, units).total;
 }
 
 namespace {
@@ -1527,10 +1534,10 @@ RoundLayout single_job_layout(const uint64_t *h_lens, int n, uint64_t Lc, int fl
   unsigned long long words, ranges, maxm;
   const uint64_t clen = Lc;
   int ms = 1;
-  unsigned long long rows = 0, tasks = 0;
-  host_totals<T>(h_lens, nullptr, n, &clen, &flags, words, ranges, maxm, &ms, &rows, &tasks);
+  unsigned long long rows = 0, units = 0;
+  host_totals<T>(h_lens, nullptr, n, &clen, &flags, words, ranges, maxm, &ms, &rows, &units);
   if (Lc > maxm) maxm = Lc;
-  return round_layout<T>(n, 1, words, ranges, maxm, ms, rows, tasks);
+  return round_layout<T>(n, 1, words, ranges, maxm, ms, rows, units);
 }
 
 }  // namespace
@@ -1612,11 +1619,11 @@ size_t dba_batch_workspace_bytes(const uint64_t *h_mlens, const int *h_mjob, int
                                  const uint64_t *h_clen, const int *h_flags, int njobs) {
   unsigned long long words, ranges, maxm;
   int ms = 1;
-  unsigned long long rows = 0, tasks = 0;
-  host_totals<T>(h_mlens, h_mjob, nmem, h_clen, h_flags, words, ranges, maxm, &ms, &rows, &tasks);
+  unsigned long long rows = 0, units = 0;
+  host_totals<T>(h_mlens, h_mjob, nmem, h_clen, h_flags, words, ranges, maxm, &ms, &rows, &units);
   for (int j = 0; j < njobs; ++j)
     if (h_clen[j] > maxm) maxm = h_clen[j];
-  return round_layout<T>(nmem, njobs, words, ranges, maxm, ms, rows, tasks).total;
+  return round_layout<T>(nmem, njobs, words, ranges, maxm, ms, rows, units).total;
 }
 
 template <typename T>
@@ -1624,11 +1631,11 @@ bool dba_batch_by_warp(const uint64_t *h_mlens, const int *h_mjob, int nmem, con
                        const int *h_flags, int njobs) {
   unsigned long long words, ranges, maxm;
   int ms = 1;
-  unsigned long long rows = 0, tasks = 0;
-  host_totals<T>(h_mlens, h_mjob, nmem, h_clen, h_flags, words, ranges, maxm, &ms, &rows, &tasks);
+  unsigned long long rows = 0, units = 0;
+  host_totals<T>(h_mlens, h_mjob, nmem, h_clen, h_flags, words, ranges, maxm, &ms, &rows, &units);
   for (int j = 0; j < njobs; ++j)
     if (h_clen[j] > maxm) maxm = h_clen[j];
-  return round_layout<T>(nmem, njobs, words, ranges, maxm, ms, rows, tasks).one_warp;
+  return round_layout<T>(nmem, njobs, words, ranges, maxm, ms, rows, units).one_warp;
 }
 template bool dba_batch_by_warp<float>(const uint64_t *, const int *, int, const uint64_t *,
                                        const int *, int);
@@ -1646,11 +1653,11 @@ int dba_batch_launch(const T *centroids, const unsigned long long *coff, const i
                      cudaStream_t stream) {
   unsigned long long words, ranges, maxm;
   int ms = 1;
-  unsigned long long rows = 0, tasks = 0;
-  host_totals<T>(h_mlens, h_mjob, nmem, h_clen, h_flags, words, ranges, maxm, &ms, &rows, &tasks);
+  unsigned long long rows = 0, units = 0;
+  host_totals<T>(h_mlens, h_mjob, nmem, h_clen, h_flags, words, ranges, maxm, &ms, &rows, &units);
   for (int j = 0; j < njobs; ++j)
     if (h_clen[j] > maxm) maxm = h_clen[j];
-  const RoundLayout L = round_layout<T>(nmem, njobs, words, ranges, maxm, ms, rows, tasks);
+  const RoundLayout L = round_layout<T>(nmem, njobs, words, ranges, maxm, ms, rows, units);
   if (ws_bytes < L.total) return fail(ODBA_ERR_WORKSPACE_TOO_SMALL, "DBA batch workspace too small");
   RoundArgs<T> a;
   a.centroids = centroids;
@@ -2470,10 +2477,10 @@ size_t prefix_chop_workspace_bytes(const uint64_t *h_lens, int n, uint64_t P) {
   const uint64_t clen = P;
   const int flags = kChopFlags;
   int ms = 1;
-  unsigned long long tasks = 0;
-  host_totals<T>(h_lens, nullptr, n, &clen, &flags, words, ranges, maxm, &ms, nullptr, &tasks);
+  unsigned long long units = 0;
+  host_totals<T>(h_lens, nullptr, n, &clen, &flags, words, ranges, maxm, &ms, nullptr, &units);
   if (P > maxm) maxm = P;
-  return round_layout<T>(n, 1, words, ranges, maxm, ms, 0, tasks).total;
+  return round_layout<T>(n, 1, words, ranges, maxm, ms, 0, units).total;
 }
 
 template <typename T>
@@ -2484,10 +2491,10 @@ int prefix_chop_launch(const T *prefix, uint64_t P, const T *series, const uint6
   const uint64_t clen = P;
   const int flags = kChopFlags;
   int ms = 1;
-  unsigned long long tasks = 0;
-  host_totals<T>(h_lens, nullptr, n, &clen, &flags, words, ranges, maxm, &ms, nullptr, &tasks);
+  unsigned long long units = 0;
+  host_totals<T>(h_lens, nullptr, n, &clen, &flags, words, ranges, maxm, &ms, nullptr, &units);
   if (P > maxm) maxm = P;
-  const RoundLayout L = round_layout<T>(n, 1, words, ranges, maxm, ms, 0, tasks);
+  const RoundLayout L = round_layout<T>(n, 1, words, ranges, maxm, ms, 0, units);
   if (ws_bytes < L.total) return fail(ODBA_ERR_WORKSPACE_TOO_SMALL, "prefix chop workspace too small");
   char *base = static_cast<char *>(ws);
   int *single = reinterpret_cast<int *>(base + L.off_single);

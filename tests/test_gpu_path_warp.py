@@ -29,10 +29,15 @@ def _signal(rng, L, dtype):
     return (np.repeat(rng.normal(0, 1, L // 9 + 1), 9)[:L] + rng.normal(0, 0.1, L)).astype(dtype)
 
 
-def _many(kinds, cols, dtype):
-    """Copies of the kinds in turn: a good deal more swaths than the rule asks."""
-    swaths = -(-cols // 1024)
-    n = (3000 if dtype == np.float32 else 1400) // swaths + 1
+def _many(kinds, lc, dtype, open_end=0, leader=False):
+    """Copies of the kinds in turn: more work, in swaths of the most rows, than the
+    resident warps (1776 float, 1184 double) times what the rule asks."""
+    flip = [leader or (open_end and lc < len(k)) for k in kinds]
+    rows = np.array([lc if f else len(k) for f, k in zip(flip, kinds)])
+    swaths = np.array([-(-(len(k) if f else lc) // 1024) for f, k in zip(flip, kinds)])
+    wide = swaths.max() > 4
+    need = (1776 * (1.5 if wide else 0.95)) if dtype == np.float32 else 1184 * (1.0 if wide else 0.7)
+    n = int(need * rows.max() / (rows * swaths).mean()) + len(kinds)
     return [kinds[k % len(kinds)] for k in range(n)]
 
 
@@ -44,7 +49,7 @@ def test_lane_and_chunk_edges(env, mode, cols, dtype):
     rng = np.random.default_rng([cols, mode[0], mode[1]])
     centroid = _signal(rng, cols, dtype)
     kinds = [_signal(rng, L, dtype) for L in ROWS]
-    members = _many(kinds, cols, dtype)
+    members = _many(kinds, cols, dtype, mode[1])
     ds = api.DeviceSeries.from_host(members)
     got = api.dba_round_ranges(torch.from_numpy(centroid).cuda(), ds, *mode).cpu().numpy()
     want = O.member_ranges(centroid, kinds, *mode, fma_mode=1)
@@ -60,9 +65,11 @@ def test_whole_round_and_paths(env, mode, dtype):
     torch, api, _ = env
     rng = np.random.default_rng([9, mode[0], mode[1]])
     centroid = _signal(rng, 300, dtype)
-    kinds = [_signal(rng, L, dtype) for L in (40, 299, 301, 600, 1100, 1700, 2300, 3300)]
-    kinds.append(np.concatenate([centroid, np.full(2500, centroid[-1], dtype=dtype)]))
-    members = _many(kinds, 300, dtype)
+    lens = (40, 299, 301, 600, 1100, 1700, 2300, 3300) if mode[1] else (40, 250, 299, 300, 301, 410)
+    kinds = [_signal(rng, L, dtype) for L in lens]
+    if mode[1]:
+        kinds.append(np.concatenate([centroid, np.full(2500, centroid[-1], dtype=dtype)]))
+    members = _many(kinds, 300, dtype, mode[1])
     ds = api.DeviceSeries.from_host(members)
     c = torch.from_numpy(centroid).cuda()
     mean, counts, delta, _ = api.dba_round(c, ds, *mode)
@@ -104,7 +111,7 @@ def test_prefix_chop_of_many_series(env, dtype):
         return pos.cpu().numpy(), hist.cpu().numpy()
 
     few = chop(kinds)
-    many = chop(_many(kinds, 1024, dtype))
+    many = chop(_many(kinds, 260, dtype, leader=True))
     for k in range(len(many[0])):
         assert many[0][k] == few[0][k % len(kinds)]
         assert np.array_equal(many[1][k], few[1][k % len(kinds)])
