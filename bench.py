@@ -518,7 +518,7 @@ def main():
                          "peak_basis": f"{SMS} SMs x {FP32_LANES} FP32 lanes x {f_mhz:.0f} MHz "
                                        f"(median sampled) / {OPS_PER_CELL} ops per cell",
                          "frac_at_max_clock": achieved / peak_max,
-                         "kernel": "pairwise_kernel<float,32,4>", "kernel_ms": kms,
+                         "kernel": "pairwise_kernel<float,32,8>", "kernel_ms": kms,
                          "hbm_peak_gbs_measured": hbm_gbs},
             "e2e": {"value": e2e_value, "unit": "GCUPS", "h2d_bytes_per_step": h2d,
                     "d2h_bytes_per_step": d2h, "seconds_per_step": e2e_sec,

@@ -5,8 +5,9 @@
 // Every warp of the grid pulls pairs from a device work counter, largest pair
 // index first (with length-sorted input that is roughly largest cost first),
 // and sweeps the pair swath by swath with the register wavefront of
-// dtw_device.cuh.  The swath right-edge column goes through a per-warp
-// ping-pong buffer in global memory (L2-resident in practice).
+// dtw_warp.cuh; few pairs go through the swath pipeline below, a block per
+// swath (dtw_block.cuh).  The swath right-edge column goes through a per-warp
+// (per-pair) ping-pong buffer in global memory (L2-resident in practice).
 //
 // Output: the reference's upper-triangle layout, pair (s, j), s < j, at
 // index s*n - s*(s+1)/2 + (j - s - 1) (clustering.cuh:4-6), with
