@@ -232,6 +232,7 @@ __device__ __forceinline__ bool sweep_block(const BlockJob<T> &job, BlockSmem<T>
         }
         if (ok) {
           __threadfence_block();
+          __syncwarp();  // lane 0 has acquired the rows for all
           // (past pair k1 the slots still hold older pairs)
           const int k = staged + (lane >> 1);
           if (k < k1) {

@@ -28,6 +28,14 @@ def test_feeder_decides_by_one_read():
     assert "smem_count(" not in feeder and "global_timer_ns(" not in feeder
 
 
+def test_lanes_read_what_lane_0_acquired_after_a_warp_barrier():
+    text = _source("dtw_block.cuh")
+    staged = text[text.index("gate.ready("):text.index("__ldcg(job.edge_in")]
+    assert "__syncwarp()" in staged
+    text = _source("dtw_warp.cuh")
+    assert "__syncwarp()" in text[text.index("gate.wait("):text.index("__ldcg(")]
+
+
 def test_waits_of_the_sweep_take_the_launch_limit():
     # the limit a launch (or the self-test) gives is the one its sweep's waits
     # run out by, and there is no second wait beside them to test instead
