@@ -568,15 +568,27 @@ bool plan_fits(int plan, unsigned long long npairs, uint64_t max_len, size_t ws_
 //   180-250            190 / 378 / 561                  1.13 / 1.14 / 0.72
 //   129-160            66 / 378                         0.83 / 0.99
 //   64-128             190 / 378                        0.78 / 0.78
+// A pair list (reads against one or a few series) gains less: the one-warp kernel
+// starts no more blocks than it has tasks for, the pipeline adds the launch that
+// applies the open-end shortcut.  Reads against one series of their median
+// length, float / double:
+//   500-5000 samples   300 / 1200 tasks         2.66 / 1.22    2.66 / 1.43
+//   1000-2000          300 / 700 / 1200         1.66 / 1.27 / 0.82    1.67 / 1.36 / 0.86
+//   700-1000           100 / 300 / 700          1.42 / 1.20 / 0.81    1.57 / 1.31 / 0.98
+//   512-700            100 / 300                1.10 / 0.96    1.25 / 1.04
+//   300-500            30 / 300                 0.99 / 0.90    0.85 / 0.76
+//   150-250            30 / 300                 0.80 / 0.78    0.67 / 0.66
 // Above one pair per resident warp (1776) the workspace that does not know the
 // number of pairs would not hold the pipeline's edges, so the rule ends there.
 template <typename T>
-int rule_of_thumb(unsigned long long npairs, uint64_t max_len) {
+int rule_of_thumb(unsigned long long npairs, uint64_t max_len, bool list = false) {
   const unsigned long long slots = (unsigned long long)grid_size<T>() * kWarpsPerBlock;
   const uint64_t swaths = (max_len + kBlkCols - 1) / kBlkCols;
   unsigned long long most;
   if (swaths >= 3)
     most = slots;
+  else if (list)
+    most = swaths == 2 ? slots / 2 : max_len >= 512 ? slots / 6 : 0;
   else if (swaths == 2)
     most = max_len < 1536 ? slots * 5 / 8 : sizeof(T) == 4 ? slots * 15 / 16 : slots;
   else if (max_len >= 256)
@@ -588,7 +600,8 @@ int rule_of_thumb(unsigned long long npairs, uint64_t max_len) {
 
 // Chooses the plan; *measure tells the caller to time the launch for the table.
 template <typename T>
-int choose_plan(unsigned long long npairs, uint64_t max_len, size_t ws_bytes, bool *measure) {
+int choose_plan(unsigned long long npairs, uint64_t max_len, size_t ws_bytes, bool *measure,
+                bool list = false) {
   const int e = sizeof(T) == 8 ? 1 : 0, lb = bucket_of(max_len), cb = bucket_of(npairs);
   std::lock_guard<std::mutex> g(g_tune_mu);
   harvest_locked(false);
@@ -611,7 +624,7 @@ int choose_plan(unsigned long long npairs, uint64_t max_len, size_t ws_bytes, bo
     if (c.rate[p] > 0 && plan_fits<T>(p, npairs, max_len, ws_bytes) && (!best || c.rate[p] > c.rate[best]))
       best = p;
   if (best) return best;
-  const int r = rule_of_thumb<T>(npairs, max_len);
+  const int r = rule_of_thumb<T>(npairs, max_len, list);
   if (plan_fits<T>(r, npairs, max_len, ws_bytes)) return r;
   for (int p = 1; p < ODBA_PLAN_COUNT; ++p)
     if (plan_fits<T>(p, npairs, max_len, ws_bytes)) return p;
@@ -628,9 +641,9 @@ void record_pending(unsigned long long npairs, uint64_t max_len, int plan, cudaE
 
 template <typename T, typename F>
 int run_planned(unsigned long long npairs, uint64_t max_len, size_t ws_bytes, cudaStream_t stream,
-                F &&launch) {
+                bool list, F &&launch) {
   bool measure = false;
-  const int plan = choose_plan<T>(npairs, max_len, ws_bytes, &measure);
+  const int plan = choose_plan<T>(npairs, max_len, ws_bytes, &measure, list);
   if (!plan) return fail(ODBA_ERR_WORKSPACE_TOO_SMALL, "workspace too small");
   cudaEvent_t a = nullptr, b = nullptr;
   if (measure && (cudaEventCreate(&a) != cudaSuccess || cudaEventCreate(&b) != cudaSuccess)) {
@@ -674,7 +687,7 @@ int pairwise_range_launch(const T *series, const uint64_t *offsets, const uint64
                           cudaStream_t stream) {
   if (n < 2 || pend <= pbeg) return ODBA_OK;
   const unsigned long long npairs = pend - pbeg;
-  return run_planned<T>(npairs, max_len, ws_bytes, stream, [&](int plan) {
+  return run_planned<T>(npairs, max_len, ws_bytes, stream, false, [&](int plan) {
     switch (plan) {
       case ODBA_PLAN_WHOLE_PAIR_HALF_SWATH:
         return whole_pairwise_launch<T, Tune<T>::RF / 2>(series, offsets, lens, n, max_len, os, oe,
@@ -706,7 +719,7 @@ int pairlist_launch(const T *series, const uint64_t *offsets, const uint64_t *le
                     const odba_pair_task *tasks, unsigned long long ntasks, uint64_t max_len,
                     T *dists, void *workspace, size_t ws_bytes, cudaStream_t stream) {
   if (ntasks == 0) return ODBA_OK;
-  return run_planned<T>(ntasks, max_len, ws_bytes, stream, [&](int plan) {
+  return run_planned<T>(ntasks, max_len, ws_bytes, stream, true, [&](int plan) {
     switch (plan) {
       case ODBA_PLAN_WHOLE_PAIR_HALF_SWATH:
         return whole_pairlist_launch<T, Tune<T>::RF / 2>(series, offsets, lens, tasks, ntasks,
