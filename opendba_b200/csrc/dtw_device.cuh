@@ -64,9 +64,11 @@ struct Num<float> {
     return r;
   }
 };
-// Costs are never NaN and never -0 (they start at +0 or d*d and only grow), so
-// a compare-and-select minimum gives the same bits as fmin without fmin's NaN
-// handling, which costs several extra instructions per call in double.
+// Costs of finite samples are never NaN and never -0 (they start at +0 or d*d and
+// only grow), so a compare-and-select minimum gives the same bits as fmin
+// without fmin's NaN handling, which costs several extra instructions per call
+// in double.  With a NaN cost the order of the arguments decides (b wins only if
+// it compares less).
 template <>
 struct Num<double> {
   static __device__ __forceinline__ double big() { return DBL_MAX; }

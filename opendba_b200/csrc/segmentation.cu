@@ -1,6 +1,6 @@
 // Adaptive k-segmentation (adaptive_device_segmentation, segmentation.hpp:48-337).
 //
-// One 256-thread CTA per block of 256*dw raw samples (dw = ceil(minseg/3)):
+// One CTA per block of 256*dw raw samples (dw = ceil(minseg/3)):
 // down-average by dw, 8-bit quantise against the block's range, then the
 // Bellman k-segment DP on integer squared errors, with a binary search on k
 // for the largest k whose segments are all at least minseg/dw long, and the
